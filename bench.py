@@ -700,7 +700,7 @@ def run_bse_batched(args):
     line = {"metric": "BSE TFLOP/s", "value": tf, "unit": "TFLOP/s", "n_gpus": ws, "steps": K, "warmup": W,
             "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
             "data": "synthetic", "config": cfg,
-            "roofline": {"kernel": "k_lu_batched", "bound": "tensor", "achieved": tf, "peak": peak64,
+            "roofline": {"kernel": "k_lu_update", "bound": "tensor", "achieved": tf, "peak": peak64,
                          "unit": "TFLOP/s", "frac": tf / peak64, "traffic": None,
                          "peak_source": "FP64 cuBLAS ZGEMM 4096^3 measured in this run"},
             "max_rel_err_vs_lapack": err,

@@ -106,3 +106,39 @@ def test_split_lu_phi_scale_and_unrefined_error(gpu_lib):
         errs[steps] = max(np.abs(out[i] - refs[i]).max() / np.abs(refs[i]).max() for i in range(len(refs)))
     assert 1e-9 < errs[0] < 1e-2, errs
     assert errs[8] < 1e-12, errs
+
+
+@pytest.mark.gpu
+def test_batched_lu_at_block_edges(gpu_lib):
+    """Sizes around the 32-column panels, the 64-column blocks, the 512 rows of
+    one register row per thread and the 1024 rows past which a panel stays in
+    global memory, each with rows that need interchanges, in one batch."""
+    from tups_b200.bse_batched import Instances, solve
+    sizes = [1, 7, 16, 31, 32, 33, 63, 64, 65, 96, 97, 128, 129, 513, 577, 1089]
+    rng = np.random.default_rng(29)
+    gam, chi, nls = [], [], []
+    for n in sizes:
+        nl = next(k for k in (9, 5, 3, 1) if n % k == 0)
+        c = rng.standard_normal((nl, nl, n // nl)) + 1j * rng.standard_normal((nl, nl, n // nl))
+        g = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        # |Gamma chi|_2 <= 0.9 (|g|_2 below 3 sqrt(n), blocks by their own norm) ...
+        g *= 0.9 / (3.0 * np.sqrt(n) * max(np.linalg.norm(c[:, :, i], 2) for i in range(n // nl)))
+        gam.append(np.asfortranarray(g))
+        chi.append(np.asfortranarray(c))
+        nls.append(nl)
+    inst = Instances(n=np.array(sizes, dtype=np.int32), nl=np.array(nls, dtype=np.int32), scale=np.ones(len(sizes)),
+                     gamma=gam, chi=chi, q=np.zeros((len(sizes), 3), dtype=np.int32))
+    for i, (got, g, c) in enumerate(zip(solve(inst), gam, chi)):
+        ref = LU.bse_lu(g, c, 1.0)
+        # ... so cond(A) <= 1.9 / 0.1, and the forward error is at most about 4 n eps cond
+        assert np.abs(got - ref).max() <= 4 * sizes[i] * 2.3e-16 * 19 * np.abs(ref).max(), sizes[i]
+    # rows far from the diagonal as pivots: A = I - chi with chi cyclic shifts per frequency block
+    n = 130
+    g = np.zeros((n, n), dtype=np.complex128, order="F")
+    g[np.arange(n), (np.arange(n) + 67) % n] = 5.0 + rng.uniform(0.0, 1.0, n)
+    g += 0.01 * rng.standard_normal((n, n))
+    inst = Instances(n=np.array([n], dtype=np.int32), nl=np.array([1], dtype=np.int32), scale=np.ones(1), gamma=[g],
+                     chi=[np.ones((1, 1, n), dtype=np.complex128, order="F")], q=np.zeros((1, 3), dtype=np.int32))
+    ref = LU.bse_lu(g, inst.chi[0], 1.0)
+    cond = np.linalg.cond(np.eye(n) - g)
+    assert np.abs(solve(inst)[0] - ref).max() <= 4 * n * 2.3e-16 * cond * np.abs(ref).max()

@@ -10,7 +10,7 @@ Gaussian, Hermitian-symmetrised and scaled so that the spectral radius of
 Gamma chi is `rho` (estimated by power iteration).
 
 ``solve`` runs ``tups_bse_lu_batched``: F = (1 - c Gamma chi)^{-1} Gamma
-(or Phi = F - Gamma) for all instances in one persistent launch.
+(or Phi = F - Gamma) for all instances together.
 """
 from __future__ import annotations
 

@@ -4,12 +4,24 @@
 //   F = (1 - c Gamma chi)^{-1} Gamma,   Phi = F - Gamma,
 // per (q, channel) instance with n = Nl*Nnu and chi block-diagonal in nu.
 //
-// One persistent launch: each CTA takes the next instance from an atomic
-// counter (instances queued largest first), forms A = I - c Gamma chi (cost
-// n^2 Nl), factors P A = L U with partial pivoting (blocked, panel width 32,
-// trailing rank-32 updates on the FP64 tensor cores), and solves L U F = P
-// Gamma in place for all n right-hand sides.  Caller-owned buffers only; the
-// instance table lives in a static device array.
+// Right-looking LU with partial pivoting of [A | Gamma], A = I - c Gamma chi,
+// in blocks of 64 columns, every step one launch over all instances that
+// still have a block:
+//   k_lu_panel   one CTA per instance factors the block's columns and inverts
+//                its unit lower 64 x 64 diagonal factor in place,
+//   k_lu_rows    column tiles: the block's row interchanges, then
+//                U12 = L11^{-1} P A12 (and the same of the right-hand sides),
+//   k_lu_update  32 x 32 tiles of [A22 | F2] -= L21 U12,
+// then, with the upper diagonal factors inverted (k_lu_invert), back
+// substitution from each instance's last block:
+//   k_lu_rows    X_b = U_bb^{-1} F_b,      k_lu_update   F_above -= U_above,b X_b.
+// The forward substitution of the right-hand sides is part of the update, so
+// rows of L left of the block are never interchanged.  The products run on the
+// FP64 tensor cores.  One CTA per instance for the whole solve, which this
+// replaces, left most SMs idle and its largest instance alone at the end.
+//
+// Caller-owned buffers only; the instance table and the interchange maps live
+// in static device arrays.
 #include <algorithm>
 #include <cstdio>
 #include <numeric>
@@ -22,12 +34,14 @@ namespace {
 
 using tups::cplx;
 using tups::cmk;
-using tups::lud::cabs1;
-using tups::lud::rank_update;
+using tups::lud::dmma8;
+using tups::lud::kPanelCols;
+using tups::lud::kPanelRows;
+using tups::lud::kPanelThreads;
+using tups::lud::PanelShared;
 
 constexpr int kLuMaxInst = 16384;
-constexpr int NB = 32;
-constexpr int LU_THREADS = 256;
+constexpr int NB = 2 * kPanelCols;  // 64
 
 struct LuDesc {
   long long g_off;  // complex offset of Gamma_i / F_i / A_i (n^2 each)
@@ -37,192 +51,465 @@ struct LuDesc {
   double scale;     // c
 };
 
+// the interchanges of one block as a gather: block row k takes row src[k];
+// rows below the block that changed, (row << 6 | block row it takes)
+struct LuMap {
+  int src[NB];
+  int moved[NB];
+  int count;
+};
+
 __device__ LuDesc g_lu_desc[kLuMaxInst];
-__device__ int g_lu_next;
+__device__ LuMap g_lu_map[kLuMaxInst];
 __device__ int g_lu_status[kLuMaxInst];
 
-// one instance: A = I - s Gamma chi; P A = L U; F = Gamma -> A^{-1} Gamma
-__device__ void lu_instance(const LuDesc& d, const cplx* __restrict__ Gam, const cplx* __restrict__ chi_all,
-                            cplx* __restrict__ Fout, cplx* __restrict__ Aw, int* __restrict__ piv_all, int inst) {
-  __shared__ double s_val[LU_THREADS / 32];
-  __shared__ int s_idx[LU_THREADS / 32];
-  __shared__ int s_piv;
-  __shared__ cplx s_inv;
+// ---- A = I - c Gamma chi, F = Gamma ---------------------------------------------
+// One thread per (row, nu) line: the line's nl entries of Gamma are loaded once
+// (LMAX registers) and give its nl entries of A; the lanes run over rows at
+// one nu, so a chi entry is one address per warp.  Sums over l1 ascending.
+// LMAX = 0: any nl, the line re-read for every l2.
+template <int LMAX>
+__device__ void form_lines(const LuDesc& d, const cplx* __restrict__ G, const cplx* __restrict__ chi,
+                           cplx* __restrict__ A, cplx* __restrict__ F) {
   const int n = d.n, nl = d.nl, nf = n / nl;
-  const size_t n2 = (size_t)n * n;
+  const size_t lines = (size_t)n * nf;
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < lines; t += (size_t)gridDim.x * blockDim.x) {
+    const int row = (int)(t % n), nu = (int)(t / n);
+    cplx g[LMAX > 0 ? LMAX : 1];
+    if constexpr (LMAX > 0) {
+#pragma unroll
+      for (int l = 0; l < LMAX; l++)
+        if (l < nl) g[l] = G[row + (size_t)n * (l * nf + nu)];
+    }
+    for (int l2 = 0; l2 < nl; l2++) {
+      const int col = l2 * nf + nu;
+      const size_t e = row + (size_t)n * col;
+      cplx acc = cmk(0.0, 0.0);
+      if constexpr (LMAX > 0) {
+#pragma unroll
+        for (int l1 = 0; l1 < LMAX; l1++)
+          if (l1 < nl) acc = tups::cfma(g[l1], chi[l1 + nl * (l2 + (size_t)nl * nu)], acc);
+      } else {
+        for (int l1 = 0; l1 < nl; l1++)
+          acc = tups::cfma(G[row + (size_t)n * (l1 * nf + nu)], chi[l1 + nl * (l2 + (size_t)nl * nu)], acc);
+      }
+      A[e] = cmk((row == col ? 1.0 : 0.0) - d.scale * acc.x, -d.scale * acc.y);
+      F[e] = G[e];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_lu_form(const cplx* __restrict__ Gam, const cplx* __restrict__ chi_all,
+                                                 cplx* __restrict__ Fout, cplx* __restrict__ Aw) {
+  const LuDesc d = g_lu_desc[blockIdx.y];
+  if (blockIdx.x == 0 && threadIdx.x == 0) g_lu_status[blockIdx.y] = 0;
   const cplx* G = Gam + d.g_off;
   const cplx* chi = chi_all + d.c_off;
   cplx* A = Aw + d.g_off;
   cplx* F = Fout + d.g_off;
-  int* ipiv = piv_all + d.p_off;
+  if (d.nl <= 1) form_lines<1>(d, G, chi, A, F);
+  else if (d.nl <= 5) form_lines<5>(d, G, chi, A, F);
+  else if (d.nl <= 9) form_lines<9>(d, G, chi, A, F);
+  else if (d.nl <= 13) form_lines<13>(d, G, chi, A, F);
+  else form_lines<0>(d, G, chi, A, F);
+}
+
+// ---- one block of 64 columns ------------------------------------------------------
+constexpr int kInvLd = NB + 1;
+
+struct LuPanelShared {
+  PanelShared p;
+  int orig[kPanelRows];  // where a row's content stood before the block
+  int moved;
+  int row[2 * NB], cur[2 * NB];  // replay of the interchanges (tall blocks)
+  union {
+    tups::lud::HalfShared half;
+    struct {
+      cplx M[NB * kInvLd], T[kPanelCols * kPanelCols];  // [col][row]
+    };
+  };
+};
+
+// M <- M^{-1}, a 64 x 64 triangle (unit lower, or UP: upper) in shared memory
+// with the pitch kInvLd: 16 x 16 diagonal blocks by substitution, one thread
+// per column, then merged pairwise, inv([X 0; Y Z]) = [X' 0; -Z' Y X' Z'] and
+// its mirror.  A zero pivot divides by one (its instance is reported
+// singular).  T: 1024 complex of scratch.  At least 64 threads.
+template <bool UP>
+__device__ void invert_triangle(cplx* __restrict__ M, cplx* __restrict__ T) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  // A = I - s Gamma chi, F = Gamma
-  for (size_t e = tid; e < n2; e += nt) {
-    const int row = (int)(e % n), col = (int)(e / n);
-    const int l2 = col / nf, nu = col % nf;
-    cplx acc = cmk(0.0, 0.0);
-    for (int l1 = 0; l1 < nl; l1++)
-      acc = tups::cfma(G[row + (size_t)n * (l1 * nf + nu)], chi[l1 + nl * (l2 + (size_t)nl * nu)], acc);
-    A[e] = cmk((row == col ? 1.0 : 0.0) - d.scale * acc.x, -d.scale * acc.y);
-    F[e] = G[e];
+  if (tid < 64) {
+    const int b = tid & 48, c = tid & 15;
+    const cplx* D = M + b * kInvLd + b;
+    cplx x[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) x[r] = cmk(r == c ? 1.0 : 0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int k = UP ? 15 - i : i;
+      if (UP) {
+        const cplx u = D[k * kInvLd + k];
+        if (u.x != 0.0 || u.y != 0.0) x[k] = tups::cmul(x[k], tups::lud::crecip1(u));
+      }
+#pragma unroll
+      for (int r = 0; r < 16; r++)
+        if (UP ? r < k : r > k) x[r] = tups::lud::cfnma(D[k * kInvLd + r], x[k], x[r]);
+    }
+    __syncwarp();  // a 16-column block belongs to half a warp
+#pragma unroll
+    for (int r = 0; r < 16; r++) M[(b + c) * kInvLd + b + r] = x[r];
   }
   __syncthreads();
-  int singular = 0;
-  for (int j0 = 0; j0 < n; j0 += NB) {
-    const int jb = min(NB, n - j0);
-    // ---- panel factorization, columns j0 .. j0+jb-1 ----
-    for (int c = j0; c < j0 + jb; c++) {
-      double best = -1.0;
-      int bi = c;
-      for (int r = c + tid; r < n; r += nt) {
-        const double v = cabs1(A[r + (size_t)n * c]);
-        if (v > best) {
-          best = v;
-          bi = r;
-        }
+  for (int s = 16; s < NB; s *= 2) {
+    const int s2 = s * s, per = NB / (2 * s) * s2;
+    for (int e = tid; e < per; e += nt) {  // T = Y X' (lower) or Y Z' (upper)
+      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
+      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
+      cplx a0 = cmk(0.0, 0.0), a1 = a0;
+      for (int k = 0; k < s; k += 2) {
+        a0 = tups::cfma(M[(x0 + k) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k], a0);
+        a1 = tups::cfma(M[(x0 + k + 1) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k + 1], a1);
       }
-      // warp then block argmax (lowest row index on ties, as izamax)
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) {
-          best = ov;
-          bi = oi;
-        }
-      }
-      if ((tid & 31) == 0) {
-        s_val[tid >> 5] = best;
-        s_idx[tid >> 5] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double bv = s_val[0];
-        int bx = s_idx[0];
-        for (int w = 1; w < nt / 32; w++)
-          if (s_val[w] > bv || (s_val[w] == bv && s_idx[w] < bx)) {
-            bv = s_val[w];
-            bx = s_idx[w];
-          }
-        s_piv = bx;
-        ipiv[c] = bx;
-        const cplx pv = A[bx + (size_t)n * c];
-        if (bv == 0.0) {
-          s_inv = cmk(0.0, 0.0);
-          if (!singular) g_lu_status[inst] = c + 1;
-          singular = 1;
-        } else {
-          s_inv = tups::crecip(pv);
-        }
-      }
-      __syncthreads();
-      const int p = s_piv;
-      if (p != c)
-        for (int col = j0 + tid; col < j0 + jb; col += nt) {
-          const cplx t = A[c + (size_t)n * col];
-          A[c + (size_t)n * col] = A[p + (size_t)n * col];
-          A[p + (size_t)n * col] = t;
-        }
-      __syncthreads();
-      const cplx inv = s_inv;
-      for (int r = c + 1 + tid; r < n; r += nt) A[r + (size_t)n * c] = tups::cmul(A[r + (size_t)n * c], inv);
-      __syncthreads();
-      const int ncols = j0 + jb - (c + 1), nrows = n - (c + 1);
-      for (int e = tid; e < ncols * nrows; e += nt) {
-        const int r = c + 1 + e % nrows, col = c + 1 + e / nrows;
-        A[r + (size_t)n * col] =
-            tups::csub(A[r + (size_t)n * col], tups::cmul(A[r + (size_t)n * c], A[c + (size_t)n * col]));
-      }
-      __syncthreads();
+      T[e] = tups::cadd(a0, a1);  // [pair][c][r]
     }
-    // ---- the panel's interchanges on the columns outside it ----
-    for (int c = j0; c < j0 + jb; c++) {
-      const int p = ipiv[c];
-      if (p != c)
-        for (int col = tid; col < n; col += nt) {
-          if (col >= j0 && col < j0 + jb) continue;
-          const cplx t = A[c + (size_t)n * col];
-          A[c + (size_t)n * col] = A[p + (size_t)n * col];
-          A[p + (size_t)n * col] = t;
-        }
-      __syncthreads();
+    __syncthreads();
+    for (int e = tid; e < per; e += nt) {  // Y = -Z' T or -X' T
+      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
+      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;
+      const cplx* t = T + (e - r);
+      cplx a0 = cmk(0.0, 0.0), a1 = a0;
+      for (int k = 0; k < s; k += 2) {
+        a0 = tups::lud::cfnma(M[(y0 + k) * kInvLd + y0 + r], t[k], a0);
+        a1 = tups::lud::cfnma(M[(y0 + k + 1) * kInvLd + y0 + r], t[k + 1], a1);
+      }
+      M[(x0 + c) * kInvLd + y0 + r] = tups::cadd(a0, a1);
     }
-    const int rest = n - j0 - jb;
-    if (rest <= 0) continue;
-    // ---- U12 = L11^{-1} A12 ----
-    for (int col = j0 + jb + tid; col < n; col += nt)
-      for (int rr = 1; rr < jb; rr++) {
-        cplx acc = A[j0 + rr + (size_t)n * col];
-        for (int kk = 0; kk < rr; kk++)
-          acc = tups::csub(acc, tups::cmul(A[j0 + rr + (size_t)n * (j0 + kk)], A[j0 + kk + (size_t)n * col]));
-        A[j0 + rr + (size_t)n * col] = acc;
-      }
-    __syncthreads();
-    // ---- A22 -= L21 U12 ----
-    rank_update(A + (j0 + jb) + (size_t)n * (j0 + jb), A + (j0 + jb) + (size_t)n * j0, A + j0 + (size_t)n * (j0 + jb),
-                 rest, rest, jb, n, n, n);
-    __syncthreads();
-  }
-  // ---- solve: F <- P F, L Y = F, U X = Y ----
-  for (int c = 0; c < n; c++) {
-    const int p = ipiv[c];
-    if (p != c)
-      for (int col = tid; col < n; col += nt) {
-        const cplx t = F[c + (size_t)n * col];
-        F[c + (size_t)n * col] = F[p + (size_t)n * col];
-        F[p + (size_t)n * col] = t;
-      }
-    __syncthreads();
-  }
-  for (int j0 = 0; j0 < n; j0 += NB) {
-    const int jb = min(NB, n - j0);
-    for (int col = tid; col < n; col += nt)
-      for (int rr = 1; rr < jb; rr++) {
-        cplx acc = F[j0 + rr + (size_t)n * col];
-        for (int kk = 0; kk < rr; kk++)
-          acc = tups::csub(acc, tups::cmul(A[j0 + rr + (size_t)n * (j0 + kk)], F[j0 + kk + (size_t)n * col]));
-        F[j0 + rr + (size_t)n * col] = acc;
-      }
-    __syncthreads();
-    const int rest = n - j0 - jb;
-    if (rest > 0) rank_update(F + (j0 + jb), A + (j0 + jb) + (size_t)n * j0, F + j0, rest, n, jb, n, n, n);
-    __syncthreads();
-  }
-  const int nblk = (n + NB - 1) / NB;
-  for (int bk = nblk - 1; bk >= 0; bk--) {
-    const int j0 = bk * NB, jb = min(NB, n - j0);
-    for (int col = tid; col < n; col += nt)
-      for (int rr = jb - 1; rr >= 0; rr--) {
-        cplx acc = F[j0 + rr + (size_t)n * col];
-        for (int kk = rr + 1; kk < jb; kk++)
-          acc = tups::csub(acc, tups::cmul(A[j0 + rr + (size_t)n * (j0 + kk)], F[j0 + kk + (size_t)n * col]));
-        const cplx u = A[j0 + rr + (size_t)n * (j0 + rr)];
-        F[j0 + rr + (size_t)n * col] = (u.x == 0.0 && u.y == 0.0) ? acc : tups::cmul(acc, tups::crecip(u));
-      }
-    __syncthreads();
-    if (j0 > 0) rank_update(F, A + (size_t)n * j0, F + j0, j0, n, jb, n, n, n);
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(LU_THREADS, 2) k_lu_batched(const cplx* __restrict__ Gam, const cplx* __restrict__ chi,
-                                                           cplx* __restrict__ F, cplx* __restrict__ Aw,
-                                                           int* __restrict__ ipiv, int n_inst, int want_phi) {
-  __shared__ int s_inst;
-  while (true) {
-    if (threadIdx.x == 0) s_inst = atomicAdd(&g_lu_next, 1);
-    __syncthreads();
-    const int i = s_inst;
-    __syncthreads();
-    if (i >= n_inst) break;
-    const LuDesc d = g_lu_desc[i];
-    lu_instance(d, Gam, chi, F, Aw, ipiv, i);
-    if (want_phi) {
-      const size_t n2 = (size_t)d.n * d.n;
-      for (size_t e = threadIdx.x; e < n2; e += blockDim.x)
-        F[d.g_off + e] = tups::csub(F[d.g_off + e], Gam[d.g_off + e]);
+// the triangle of the diagonal block at (j0, j0), identity past jb, into M
+template <bool UP>
+__device__ void load_triangle(const cplx* __restrict__ A, int n, int j0, int jb, cplx* __restrict__ M) {
+  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+    const int r = e % NB, c = e / NB;
+    const bool in = r < jb && c < jb && (UP ? r <= c : r > c);
+    M[c * kInvLd + r] = in ? A[j0 + r + (size_t)n * (j0 + c)] : cmk(r == c ? 1.0 : 0.0, 0.0);
+  }
+  __syncthreads();
+}
+
+template <bool UP>
+__device__ void store_triangle(cplx* __restrict__ A, int n, int j0, int jb, const cplx* __restrict__ M) {
+  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+    const int r = e % NB, c = e / NB;
+    if (r < jb && c < jb && (UP ? r <= c : r > c)) A[j0 + r + (size_t)n * (j0 + c)] = M[c * kInvLd + r];
+  }
+}
+
+// Columns [j0, j0 + 64) of every instance (one CTA each): two 32-column panels
+// with a 32-wide update between them, the interchange map, and the unit lower
+// diagonal factor replaced by its inverse (nothing later needs the factor).
+// RPT: rows per thread in registers, 0 = columns in global memory.
+// A serial chain of column steps: bound by barrier and FP64 latency, not by
+// bandwidth; its SMs' FP64 pipes idle between the steps.
+template <int RPT>
+__global__ void __launch_bounds__(kPanelThreads, 1) k_lu_panel(cplx* __restrict__ Aw, int* __restrict__ piv_all,
+                                                               int step) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  LuPanelShared& S = *reinterpret_cast<LuPanelShared*>(smraw);
+  const int inst = blockIdx.x, tid = threadIdx.x;
+  const LuDesc d = g_lu_desc[inst];
+  const int n = d.n, j0 = step * NB, jb = min(NB, n - j0), je = j0 + jb;
+  cplx* A = Aw + d.g_off;
+  int* ipiv = piv_all + d.p_off;
+  LuMap& map = g_lu_map[inst];
+  for (int i = tid; i < kPanelRows; i += kPanelThreads) S.p.loc[i] = S.orig[i] = i;
+  if (tid == 0) S.moved = 0;
+  __syncthreads();
+  auto track = [&](int c, int p) {
+    if (RPT > 0) {
+      const int x = S.orig[c - j0];
+      S.orig[c - j0] = S.orig[p - j0];
+      S.orig[p - j0] = x;
+    }
+  };
+  for (int h0 = j0; h0 < je; h0 += kPanelCols) {
+    const int kb = min(kPanelCols, je - h0);
+    if (h0 > j0) tups::lud::panel_half(A, n, j0, kb, S.half);
+    if constexpr (RPT > 0)
+      tups::lud::panel_factor<RPT>(A, n, h0, kb, j0, je, ipiv, &g_lu_status[inst], S.p, track);
+    else
+      tups::lud::panel_factor_global(A, n, h0, kb, j0, je, ipiv, &g_lu_status[inst], S.p, track);
+  }
+  // the interchange map: block rows take src, the rows below that changed take
+  // a block row (an interchange always involves the block)
+  if (RPT > 0) {
+    if (tid < NB) map.src[tid] = tid < jb ? j0 + S.orig[tid] : 0;
+    for (int i = jb + tid; i < n - j0; i += kPanelThreads)
+      if (S.orig[i] != i) map.moved[atomicAdd(&S.moved, 1)] = (j0 + i) << 6 | S.orig[i];
+  } else if (tid == 0) {
+    int cnt = jb;
+    for (int k = 0; k < jb; k++) {
+      S.row[k] = j0 + k;
+      S.cur[k] = k;
+    }
+    for (int k = 0; k < jb; k++) {
+      const int p = ipiv[j0 + k];
+      int x = p < je ? p - j0 : jb;
+      if (p >= je) {
+        while (x < cnt && S.row[x] != p) x++;
+        if (x == cnt) {
+          S.row[cnt] = p;
+          S.cur[cnt++] = x;
+        }
+      }
+      const int t = S.cur[k];
+      S.cur[k] = S.cur[x];
+      S.cur[x] = t;
+    }
+    for (int k = 0; k < NB; k++) map.src[k] = k < jb ? S.row[S.cur[k]] : 0;
+    for (int x = jb; x < cnt; x++) map.moved[x - jb] = S.row[x] << 6 | S.cur[x];
+    S.moved = cnt - jb;
+  }
+  __syncthreads();
+  if (tid == 0) map.count = S.moved;
+  load_triangle<false>(A, n, j0, jb, S.M);
+  invert_triangle<false>(S.M, S.T);
+  store_triangle<false>(A, n, j0, jb, S.M);
+}
+
+// U_bb^{-1} over U_bb for every diagonal block of every instance, off the
+// chain of panels: the back substitution reads nothing else of them
+__global__ void __launch_bounds__(256) k_lu_invert(cplx* __restrict__ Aw) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* M = reinterpret_cast<cplx*>(smraw);
+  const LuDesc d = g_lu_desc[blockIdx.y];
+  const int n = d.n, j0 = blockIdx.x * NB, jb = min(NB, n - j0);
+  if (j0 >= n) return;
+  cplx* A = Aw + d.g_off;
+  load_triangle<true>(A, n, j0, jb, M);
+  invert_triangle<true>(M, M + NB * kInvLd);
+  store_triangle<true>(A, n, j0, jb, M);
+}
+constexpr size_t kInvertSmem = ((size_t)NB * kInvLd + kPanelCols * kPanelCols) * sizeof(cplx);
+
+// column c of [A right of the block | F] (forward) or of F (backward)
+__device__ __forceinline__ cplx* rhs_column(cplx* A, cplx* F, int n, int right, int c) {
+  return c < right ? A + (size_t)n * (n - right + c) : F + (size_t)n * (c - right);
+}
+
+// first row of the block of launch `step`: the step-th from the top, or from
+// the bottom (BACK)
+template <bool BACK>
+__device__ __forceinline__ int block_start(int n, int step) {
+  return BACK ? ((n + NB - 1) / NB - 1 - step) * NB : step * NB;
+}
+
+// ---- block row: X[block, tile] = T (P X)[block, tile], T = L11^{-1} or U_bb^{-1} ----
+// 32 columns per CTA, a warp per 8 of them and all 64 rows, so the triangle's
+// skipped 16 x 16 blocks shorten every warp alike.  The interchanges are a
+// gather: all reads of the tile end before its first write.
+constexpr int RW_BN = 32, RW_THREADS = 4 * RW_BN, RW_LDL = NB + 2, RW_LDB = NB + 4;
+constexpr size_t kRowsSmem = ((size_t)NB * RW_LDL + RW_BN * RW_LDB) * sizeof(cplx);
+
+__device__ __forceinline__ void lu_cp_async16(void* sdst, const void* gsrc, bool valid) {
+  unsigned sz = valid ? 16u : 0u;
+  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz));
+}
+
+template <bool BACK>
+__global__ void __launch_bounds__(RW_THREADS, 2) k_lu_rows(cplx* __restrict__ Aw, cplx* __restrict__ Fout, int step) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* sL = reinterpret_cast<cplx*>(smraw);  // [k][m]
+  cplx* sB = sL + NB * RW_LDL;                // [col][k]
+  const int inst = blockIdx.y;
+  const LuDesc d = g_lu_desc[inst];
+  const int n = d.n, j0 = block_start<BACK>(n, step), jb = min(NB, n - j0), je = j0 + jb;
+  const int right = BACK ? 0 : n - je, width = right + n, c0 = blockIdx.x * RW_BN;
+  if (c0 >= width) return;
+  cplx* A = Aw + d.g_off;
+  cplx* F = Fout + d.g_off;
+  const LuMap& map = g_lu_map[inst];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
+  constexpr int kStep = RW_THREADS / NB;
+  const int tm = tid % NB, tc = tid / NB;  // this thread's row and first column of both operands
+  const int srow = BACK ? j0 + tm : map.src[tm];
+#pragma unroll
+  for (int i = 0; i < RW_BN / kStep; i++) {
+    const int c = c0 + tc + kStep * i;
+    const bool in = tm < jb && c < width;
+    lu_cp_async16(&sB[(tc + kStep * i) * RW_LDB + tm], in ? rhs_column(A, F, n, right, c) + srow : A, in);
+  }
+#pragma unroll
+  for (int i = 0; i < NB / kStep; i++) {
+    const int k = tc + kStep * i;
+    const bool in = tm < jb && k < jb && (BACK ? tm <= k : tm > k);
+    lu_cp_async16(&sL[k * RW_LDL + tm], in ? A + j0 + tm + (size_t)n * (j0 + k) : A, in);
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  // the rows below the block that take a block row
+  cplx v[RW_BN / kStep];
+  const int cnt = BACK ? 0 : map.count, mv = tm < cnt ? map.moved[tm] : 0;
+  if (!BACK && tm < cnt) {
+#pragma unroll
+    for (int i = 0; i < RW_BN / kStep; i++) {
+      const int c = c0 + tc + kStep * i;
+      if (c < width) v[i] = rhs_column(A, F, n, right, c)[j0 + (mv & 63)];
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  if (!BACK) {
+    if (tid < NB) sL[tid * RW_LDL + tid] = cmk(1.0, 0.0);
+    if (tm < cnt) {
+#pragma unroll
+      for (int i = 0; i < RW_BN / kStep; i++) {
+        const int c = c0 + tc + kStep * i;
+        if (c < width) rhs_column(A, F, n, right, c)[mv >> 6] = v[i];
+      }
     }
     __syncthreads();
   }
+  double re[4][4] = {}, im[4][4] = {};
+  const cplx* b = sB + (warp * 8 + gid) * RW_LDB;
+#pragma unroll
+  for (int k8 = 0; k8 < NB; k8 += 8) {
+    const cplx b0 = b[k8 + tig], b1 = b[k8 + tig + 4];
+    const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      if (BACK ? k8 < 16 * t : k8 >= 16 * (t + 1)) continue;
+      const cplx* l = sL + (k8 + tig) * RW_LDL + 16 * t + gid;
+      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * RW_LDL], a3 = l[4 * RW_LDL + 8];
+      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+      dmma8(re[t], ar, br);
+      dmma8(re[t], an, bi);
+      dmma8(im[t], ar, bi);
+      dmma8(im[t], ai, br);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 4; t++)
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int m = 16 * t + gid + (x >= 2 ? 8 : 0), c = c0 + warp * 8 + 2 * tig + (x & 1);
+      if (m < jb && c < width) rhs_column(A, F, n, right, c)[j0 + m] = cmk(re[t][x], im[t][x]);
+    }
+}
+
+// ---- update: C -= L21 U12 (forward), F_above -= U_above,b X_b (backward) -----------
+// 32 x 32 complex tiles, 4 warps of 16 x 16, K = 64 in two cp.async stages of
+// 16, three real tensor-core products per complex one (as the BSE GEMM).
+constexpr int UP_BM = 32, UP_BN = 32, UP_BK = 16, UP_LDL = UP_BM + 2, UP_LDR = UP_BK + 4;
+
+template <bool BACK>
+__global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cplx* __restrict__ Fout, int step) {
+  __shared__ __align__(16) cplx sL[2][UP_BK][UP_LDL];
+  __shared__ __align__(16) cplx sR[2][UP_BN][UP_LDR];
+  const LuDesc& d = g_lu_desc[blockIdx.y];
+  const int n = d.n, j0 = block_start<BACK>(n, step), je = min(j0 + NB, n);
+  const int first = BACK ? 0 : je, rows = BACK ? j0 : n - je;  // rows of C
+  const int right = BACK ? 0 : n - je, width = right + n;
+  const int tiles_m = (rows + UP_BM - 1) / UP_BM;
+  if (tiles_m == 0) return;
+  const int m0 = (int)(blockIdx.x % tiles_m) * UP_BM, n0 = (int)(blockIdx.x / tiles_m) * UP_BN;
+  if (n0 >= width) return;
+  cplx* A = Aw + d.g_off;
+  cplx* F = Fout + d.g_off;
+  const int K = je - j0, ktiles = (K + UP_BK - 1) / UP_BK;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm0 = (warp % 2) * 16, wn0 = (warp / 2) * 16;
+  const int gid = lane >> 2, tig = lane & 3;
+  // this thread's fixed row of A, column of B and their k offsets
+  const int am = tid % UP_BM, ak = tid / UP_BM, bk = tid % UP_BK, bc = tid / UP_BK;
+  const cplx* pa = A + first + min(m0 + am, rows - 1) + (size_t)n * j0;
+  const bool okm = m0 + am < rows;
+  const cplx* pb[4];
+  bool okc[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = n0 + bc + 8 * i;
+    okc[i] = c < width;
+    pb[i] = rhs_column(A, F, n, right, min(c, width - 1)) + j0;
+  }
+  auto load = [&](int st, int kt) {
+    const int k0 = kt * UP_BK;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int k = k0 + ak + 4 * i;
+      lu_cp_async16(&sL[st][ak + 4 * i][am], k < K ? pa + (size_t)n * k : pa, okm && k < K);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      lu_cp_async16(&sR[st][bc + 8 * i][bk], k0 + bk < K ? pb[i] + k0 + bk : pb[i], okc[i] && k0 + bk < K);
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  double p1[2][4] = {}, p2[2][4] = {}, p3[2][4] = {};
+  load(0, 0);
+  for (int kt = 0; kt < ktiles; kt++) {
+    const int cur = kt & 1;
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    if (kt + 1 < ktiles) load(cur ^ 1, kt + 1);
+#pragma unroll
+    for (int k8 = 0; k8 < UP_BK; k8 += 8) {
+      const int mb = wm0 + gid;
+      const cplx v0 = sL[cur][k8 + tig][mb], v1 = sL[cur][k8 + tig][mb + 8];
+      const cplx v2 = sL[cur][k8 + tig + 4][mb], v3 = sL[cur][k8 + tig + 4][mb + 8];
+      const double are[4] = {v0.x, v1.x, v2.x, v3.x}, aim[4] = {v0.y, v1.y, v2.y, v3.y};
+      const double asum[4] = {v0.x + v0.y, v1.x + v1.y, v2.x + v2.y, v3.x + v3.y};
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int nb = wn0 + j * 8 + gid;
+        const cplx w0 = sR[cur][nb][k8 + tig], w1 = sR[cur][nb][k8 + tig + 4];
+        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y}, bsum[2] = {w0.x + w0.y, w1.x + w1.y};
+        dmma8(p1[j], are, bre);
+        dmma8(p2[j], aim, bim);
+        dmma8(p3[j], asum, bsum);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int row = m0 + wm0 + gid + (x >= 2 ? 8 : 0), col = n0 + wn0 + j * 8 + 2 * tig + (x & 1);
+      if (row < rows && col < width) {
+        cplx* c = rhs_column(A, F, n, right, col) + first + row;
+        const cplx v = *c;
+        *c = cmk(v.x - (p1[j][x] - p2[j][x]), v.y - (p3[j][x] - p1[j][x] - p2[j][x]));
+      }
+    }
+}
+
+// F -= Gamma
+__global__ void __launch_bounds__(256) k_lu_phi(const cplx* __restrict__ Gam, cplx* __restrict__ Fout) {
+  const LuDesc& d = g_lu_desc[blockIdx.y];
+  const size_t n2 = (size_t)d.n * d.n;
+  const cplx* G = Gam + d.g_off;
+  cplx* F = Fout + d.g_off;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n2; e += (size_t)gridDim.x * blockDim.x)
+    F[e] = tups::csub(F[e], G[e]);
+}
+
+// opt-in shared-memory sizes, once per device
+bool lu_prepare(int dev) {
+  static bool done[64] = {};
+  if (dev >= 0 && dev < 64 && done[dev]) return true;
+  const int ps = (int)sizeof(LuPanelShared), rs = (int)kRowsSmem;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (cudaFuncSetAttribute(k_lu_panel<0>, attr, ps) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_panel<1>, attr, ps) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_panel<2>, attr, ps) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_invert, attr, (int)kInvertSmem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_rows<false>, attr, rs) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_rows<true>, attr, rs) != cudaSuccess)
+    return false;
+  if (dev >= 0 && dev < 64) done[dev] = true;
+  return true;
 }
 
 }  // namespace
@@ -241,30 +528,52 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
     co += (long long)nl[i] * nl[i] * (n[i] / nl[i]);
     po += n[i];
   }
-  // largest first: the queue order is a permutation of the packed layout
+  // largest first: the instances that still have a block are the first ones
   std::vector<int> order(n_inst);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
   std::vector<LuDesc> queued(n_inst);
   for (int i = 0; i < n_inst; i++) queued[i] = desc[order[i]];
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int zero = 0;
-  std::vector<int> zeros(n_inst, 0);
-  if (cudaMemcpyToSymbolAsync(g_lu_desc, queued.data(), n_inst * sizeof(LuDesc), 0, cudaMemcpyHostToDevice, st) !=
-          cudaSuccess ||
-      cudaMemcpyToSymbolAsync(g_lu_next, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyToSymbolAsync(g_lu_status, zeros.data(), n_inst * sizeof(int), 0, cudaMemcpyHostToDevice, st) !=
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || !lu_prepare(dev) ||
+      cudaMemcpyToSymbolAsync(g_lu_desc, queued.data(), n_inst * sizeof(LuDesc), 0, cudaMemcpyHostToDevice, st) !=
           cudaSuccess) {
     cudaGetLastError();
     return TUPS_ERR_CUDA;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::min(n_inst, 2 * sms);
-  k_lu_batched<<<grid, LU_THREADS, 0, st>>>(reinterpret_cast<const cplx*>(gamma), reinterpret_cast<const cplx*>(chi),
-                                            reinterpret_cast<cplx*>(out), reinterpret_cast<cplx*>(work), ipiv, n_inst,
-                                            want_phi);
+  const cplx* G = reinterpret_cast<const cplx*>(gamma);
+  cplx* A = reinterpret_cast<cplx*>(work);
+  cplx* F = reinterpret_cast<cplx*>(out);
+  const int nmax = queued[0].n;
+  const unsigned eg = (unsigned)std::min<long long>(((long long)nmax * nmax + 255) / 256, 512);
+  const auto tiles = [](long long rows, long long cols) {
+    return (unsigned)((rows + UP_BM - 1) / UP_BM * ((cols + UP_BN - 1) / UP_BN));
+  };
+  // grid rows of at most 65535 instances (n_inst <= 16384)
+  k_lu_form<<<dim3(eg, n_inst), 256, 0, st>>>(G, reinterpret_cast<const cplx*>(chi), F, A);
+  int live = n_inst;
+  for (int step = 0; step * NB < nmax; step++) {
+    const int j0 = step * NB;
+    while (queued[live - 1].n <= j0) live--;
+    const int rows = nmax - j0, below = std::max(0, rows - NB);
+    const size_t ps = sizeof(LuPanelShared);
+    if (rows <= kPanelThreads) k_lu_panel<1><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
+    else if (rows <= kPanelRows) k_lu_panel<2><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
+    else k_lu_panel<0><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
+    const long long width = (long long)below + nmax;
+    k_lu_rows<false><<<dim3((unsigned)((width + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);
+    if (below > 0) k_lu_update<false><<<dim3(tiles(below, width), live), 128, 0, st>>>(A, F, step);
+  }
+  k_lu_invert<<<dim3((unsigned)((nmax + NB - 1) / NB), n_inst), 256, kInvertSmem, st>>>(A);
+  live = n_inst;
+  for (int step = 0; step * NB < nmax; step++) {
+    while (queued[live - 1].n <= step * NB) live--;
+    const int above = ((nmax + NB - 1) / NB - 1 - step) * NB;
+    k_lu_rows<true><<<dim3((unsigned)((nmax + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);
+    if (above > 0) k_lu_update<true><<<dim3(tiles(above, nmax), live), 128, 0, st>>>(A, F, step);
+  }
+  if (want_phi) k_lu_phi<<<dim3(eg, n_inst), 256, 0, st>>>(G, F);
   if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
   if (status) {
     std::vector<int> st_q(n_inst);

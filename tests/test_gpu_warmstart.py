@@ -163,3 +163,36 @@ def test_sweep_trains_on_solver_runs_and_reports_the_gain(gpu_lib):
     # within that band: their fixed points agree to ~1e-6, not to 1e-10
     assert s["max_final_sigma_rel_diff"] <= 1e-4
     assert s["warm_iterations_mean"] <= s["cold_iterations_mean"] + 1.0
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (35, 33, 2, 17, 31), (260, 64, 1, 16, 33), (1030, 129, 2, 66, 65)],
+                         ids=["one", "odd", "edge", "long"])
+def test_mlp_layers_at_tile_edges(gpu_lib, shape):
+    """Widths and batches around the 32 x 16 output tiles, the four k ranges of
+    a cluster and its 256-wide k chunks, aligned and unaligned rows; one Adam
+    step over a gathered minibatch against the float64 oracle."""
+    from tups_b200.warmstart import MLP
+    n_in, hidden, layers, n_out, batch = shape
+    net = MLP(n_in, n_out, hidden, layers, max_batch=batch, seed=3)
+    rng = np.random.default_rng(19)
+    p = net.get_params()
+    x = rng.normal(size=(batch, n_in)).astype(np.float32)
+    t = rng.normal(size=(batch, n_out)).astype(np.float32)
+    y_ref, _ = OW.mlp_forward(p, net.widths, x)
+    # a sum of n FP32 products is off by at most about n eps of the sum of magnitudes
+    tol = 4 * max(n_in, hidden) * 6e-8
+    assert parity.rel(net.forward(x), y_ref) <= max(tol, 1e-6)
+    loss, g = net.gradients(x, t)
+    loss_ref, g_ref = OW.mlp_loss_grad(p, net.widths, x, t)
+    assert abs(loss - loss_ref) <= MLP_TOL * loss_ref
+    assert parity.rel(g, g_ref) <= MLP_TOL
+    # the first Adam step moves a parameter by lr g / (|g| + eps): compared where |g| is far above rounding
+    net.train(x, t, batch=batch, epochs=1, lr=1e-2, weight_decay=0.1, seed=5)
+    layout, _ = OW.mlp_layout(net.widths)
+    want = p.astype(np.float64)
+    for wo, bo, fin, fout in layout:
+        want[wo:bo] *= 1.0 - 1e-2 * 0.1
+    want -= 1e-2 * g_ref / (np.abs(g_ref) + 1e-8)
+    big = np.abs(g_ref) > 1e-3 * np.abs(g_ref).max()
+    assert np.abs(net.get_params() - want)[big].max() <= 1e-2 * 2 * MLP_TOL / 1e-3
+    net.close()

@@ -10,8 +10,10 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "../../include/tups_b200.h"
@@ -35,7 +37,7 @@ struct tups_mlp {
   float* t = nullptr;          // target batch (max_batch, n_out)
   std::vector<float*> z, a;    // per hidden layer: pre-activation, activation
   float* y = nullptr;          // output (max_batch, n_out)
-  float* dz[2] = {};           // backward ping-pong (max_batch, max width)
+  std::vector<float*> dz;      // per linear layer: gradient of its output (max_batch, width)
   double* loss = nullptr;      // device loss slots
   int loss_slots = 0;
   float* data_x = nullptr;     // resident training set
@@ -64,11 +66,6 @@ int mlp_cuda(tups_mlp* m, cudaError_t e, const char* what) {
     if (_rc != TUPS_OK) return _rc; \
   } while (0)
 
-int launched(tups_mlp* m, const char* name) {
-  m->launches++;
-  return mlp_cuda(m, cudaGetLastError(), name);
-}
-
 template <typename T>
 int mlp_alloc(tups_mlp* m, T** p, size_t count) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T) + 16);
@@ -82,209 +79,441 @@ int mlp_alloc(tups_mlp* m, T** p, size_t count) {
 
 __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-// Epilogues of the tiled GEMM
-enum { EPI_STORE = 0, EPI_BIAS_SILU = 1, EPI_BIAS = 2, EPI_DSILU = 3 };
-
-// C(m, n) = sum_k A(m, k) B(k, n) with A(m, k) = A[m*sam + k*sak] and
-// B(k, n) = B[k*sbk + n*sbn]; 64 x 64 tile per CTA, 4 x 4 per thread.
-//   EPI_STORE:     C = acc
-//   EPI_BIAS_SILU: C = acc + bias[n] (pre-activation), C2 = silu(C)
-//   EPI_BIAS:      C = acc + bias[n]
-//   EPI_DSILU:     C = acc * silu'(aux[m, n])
-template <int EPI>
-__global__ void __launch_bounds__(256) k_mlp_gemm(int M, int N, int K, const float* __restrict__ A, int sam, int sak,
-                                                  const float* __restrict__ B, int sbk, int sbn,
-                                                  const float* __restrict__ bias, const float* __restrict__ aux,
-                                                  float* __restrict__ C, float* __restrict__ C2) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[4][4];
+// 4 floats of a row from k on, those past len (and, with !in, all) as zeros
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, int k, int len, bool vec, bool in) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  if (vec) {
+    const unsigned sz = in && k < len ? 16u : 0u;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(sz ? src + k : src), "r"(sz));
+  } else {
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-  const bool a_kfast = sak == 1, b_kfast = sbk == 1;
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int e = threadIdx.x; e < BK * BM; e += 256) {
-      const int kk = a_kfast ? e % BK : e / BM;
-      const int mm = a_kfast ? e / BK : e % BM;
-      const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? A[(size_t)gm * sam + (size_t)gk * sak] : 0.0f;
-      const int kb = b_kfast ? e % BK : e / BN;
-      const int nn = b_kfast ? e / BK : e % BN;
-      const int gn = n0 + nn, gkb = k0 + kb;
-      Bs[kb][nn] = (gn < N && gkb < K) ? B[(size_t)gkb * sbk + (size_t)gn * sbn] : 0.0f;
+    for (int i = 0; i < 4; i++) {
+      const unsigned sz = in && k + i < len ? 4u : 0u;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d + 4 * i), "l"(sz ? src + k + i : src),
+                   "r"(sz));
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) av[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    __syncthreads();
   }
+}
+
+// ---- layer products: C(m, n) = sum_k X(m, k) W(k, n) ------------------------------
+//
+// A minibatch has few rows (32 in training), so a layer is a thin product bound
+// by latency: 32 x 16 output tiles, and the sum over k split over the four CTAs
+// of a cluster (partial tiles added through distributed shared memory, in rank
+// order) and over the eight warps of a CTA, each thread 4 x 4 outputs over
+// float4 steps of k.  A CTA loads its whole k range (up to kKC) at once.
+//   forward (WT = false): W(k, n) = W[n * ldw + k], rows of W along k
+//   backward (WT = true): W(k, n) = W[k * ldw + n]
+// rows: optional gather of X's rows by index.
+// 964 -> 512 at 32 rows: 120 -> about 6 us (eight CTAs of 64 x 64 before); a
+// training step of 964 -> 3 x 512 -> 968 at 32 rows: 650 -> 60 us.
+enum { EPI_BIAS_SILU = 1, EPI_BIAS = 2, EPI_DSILU = 3, EPI_MSE = 4 };
+
+struct LinArgs {
+  int M, N, K;
+  const float* X;
+  const int* rows;
+  const int* trows;   // the same of the targets
+  const float* W;
+  const float* bias;  // EPI_BIAS*, EPI_MSE
+  const float* aux;   // EPI_DSILU: z (M, N); EPI_MSE: targets
+  float* C;           // pre-activation, output or gradient (M, N)
+  float* C2;          // EPI_BIAS_SILU: silu(C)
+  double* loss;       // EPI_MSE: += sum (y - t)^2 / (M N); C = 2 (y - t) / (M N)
+  double inv;
+  bool w_fresh;       // W may have been written by the launch just before
+};
+
+// Programmatic dependent launch: a kernel starts while its predecessor drains,
+// loads what that one does not write and then waits for it.  Dependents are
+// released after the wait, so at any kernel's start everything up to its
+// predecessor's predecessor is complete.
+__device__ __forceinline__ void wait_predecessor() {
+  asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+constexpr int kTM = 32, kTN = 16, kKC = 256, kSplit = 4, kLinThreads = 256;
+constexpr int kXP = kKC + 4, kWP = kTN + 4;  // pitches: float4 rows on distinct banks
+constexpr size_t kLinSmem = ((size_t)(kTM + kTN) * kXP > (size_t)kTM * kXP + (size_t)kKC * kWP
+                                 ? (size_t)(kTM + kTN) * kXP : (size_t)kTM * kXP + (size_t)kKC * kWP) * sizeof(float);
+
+template <int EPI, bool WT>
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kLinThreads) k_mlp_linear(LinArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* Xs = sm;             // [m][k]
+  float* Ws = sm + kTM * kXP; // [n][k], WT: [k][n]
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int n0 = (int)(blockIdx.x / kSplit) * kTN, m0 = (int)blockIdx.y * kTM;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kper = ((a.K + kSplit - 1) / kSplit + 31) / 32 * 32;
+  const int kbeg = rank * kper, kend = min(a.K, kbeg + kper);
+  const bool xv = a.K % 4 == 0 && (reinterpret_cast<size_t>(a.X) & 15) == 0;
+  const bool wv = (WT ? a.N : a.K) % 4 == 0 && (reinterpret_cast<size_t>(a.W) & 15) == 0;
+  const int g = lane >> 2, q = lane & 3;
+  float acc[4][4] = {};
+  // a row is up to 64 float4 steps of k: 64 threads per row, all copies in flight at once
+  const int k = tid % (kKC / 4) * 4, r0 = tid / (kKC / 4);
+  constexpr int kRows = kLinThreads / (kKC / 4);
+  auto load_w = [&](int kc) {
+    const int len = min(kKC, kend - kc), len4 = (len + 3) / 4;
+    if (!WT && k < 4 * len4) {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int m = m0 + ty + 16 * i;
-    if (m >= M) continue;
+      for (int i = 0; i < kTN / kRows; i++) {
+        const int n = r0 + i * kRows;
+        const bool in = n0 + n < a.N;
+        cp_async4(Ws + n * kXP + k, in ? a.W + (size_t)(n0 + n) * a.K + kc : a.W, k, len, wv, in);
+      }
+    }
+    if (WT) {
+      const int n = tid % (kTN / 4) * 4, left = min(kTN, a.N - n0);
+      for (int kk = tid / (kTN / 4); kk < 4 * len4; kk += kLinThreads / (kTN / 4))
+        cp_async4(Ws + kk * kWP + n, kk < len ? a.W + (size_t)(kc + kk) * a.N + n0 : a.W, n, left, wv, kk < len);
+    }
+  };
+  if (!a.w_fresh && kbeg < kend) load_w(kbeg);
+  wait_predecessor();
+  // what this thread's output needs besides the product, ahead of it
+  constexpr int kTile = kTM * kTN, kOwn = kTile / kSplit;  // each CTA finishes a quarter of the rows
+  const int eo = rank * kOwn + tid, mo = m0 + eo / kTN, no = n0 + eo % kTN;
+  const bool own = tid < kOwn && mo < a.M && no < a.N;
+  const size_t oo = (size_t)mo * a.N + no;
+  float bias = 0.0f, aux = 0.0f;
+  if (own) {
+    if (EPI != EPI_DSILU) bias = a.bias[no];
+    if (EPI == EPI_DSILU) aux = a.aux[oo];
+    if (EPI == EPI_MSE) aux = a.aux[a.trows ? (size_t)a.trows[mo] * a.N + no : oo];
+  }
+  for (int kc = kbeg; kc < kend; kc += kKC) {
+    const int len = min(kKC, kend - kc), len4 = (len + 3) / 4;
+    if (kc > kbeg) __syncthreads();
+    if (kc > kbeg || a.w_fresh) load_w(kc);
+    if (k < 4 * len4) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = n0 + tx + 16 * j;
-      if (n >= N) continue;
-      const size_t o = (size_t)m * N + n;
-      float v = acc[i][j];
-      if (EPI == EPI_BIAS_SILU) {
-        v += bias[n];
-        C[o] = v;
-        C2[o] = v * sigmoid(v);
-      } else if (EPI == EPI_BIAS) {
-        C[o] = v + bias[n];
-      } else if (EPI == EPI_DSILU) {
-        const float z = aux[o];
-        const float s = sigmoid(z);
-        C[o] = v * (s * (1.0f + z * (1.0f - s)));
-      } else {
-        C[o] = v;
+      for (int i = 0; i < kTM / kRows; i++) {
+        const int m = r0 + i * kRows;
+        const bool in = m0 + m < a.M;
+        const float* src = a.X;
+        if (in) src += (size_t)(a.rows ? a.rows[m0 + m] : m0 + m) * a.K + kc;
+        cp_async4(Xs + m * kXP + k, src, k, len, xv, in);
+      }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    for (int k4 = warp; k4 < len4; k4 += kLinThreads / 32) {
+      float4 x[4], w[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) x[i] = *reinterpret_cast<const float4*>(Xs + (g + 8 * i) * kXP + 4 * k4);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        w[j] = *reinterpret_cast<const float4*>(WT ? Ws + (4 * k4 + j) * kWP + 4 * q : Ws + (q + 4 * j) * kXP + 4 * k4);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (WT) {
+          const float xk[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            acc[i][0] = fmaf(xk[k], w[k].x, acc[i][0]);
+            acc[i][1] = fmaf(xk[k], w[k].y, acc[i][1]);
+            acc[i][2] = fmaf(xk[k], w[k].z, acc[i][2]);
+            acc[i][3] = fmaf(xk[k], w[k].w, acc[i][3]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            acc[i][j] = fmaf(x[i].x, w[j].x, acc[i][j]);
+            acc[i][j] = fmaf(x[i].y, w[j].y, acc[i][j]);
+            acc[i][j] = fmaf(x[i].z, w[j].z, acc[i][j]);
+            acc[i][j] = fmaf(x[i].w, w[j].w, acc[i][j]);
+          }
+        }
       }
     }
   }
-}
-
-// db[n] = sum_m dz[m, n]
-__global__ void k_mlp_colsum(const float* __restrict__ dz, float* __restrict__ db, int M, int N) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.0f;
-  for (int m = 0; m < M; m++) s += dz[(size_t)m * N + n];
-  db[n] = s;
-}
-
-// dy = 2 (y - t) / (M N); loss[slot] += sum (y - t)^2 / (M N)
-__global__ void k_mlp_mse(const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ dy,
-                          size_t n, double inv, double* loss) {
-  double s = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float d = y[i] - t[i];
-    dy[i] = (float)(2.0 * inv) * d;
-    s += (double)d * d;
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double sh[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = s;
+  // the warps' partial tiles, then the cluster's
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += sh[w];
-    atomicAdd(loss, tot * inv);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) sm[warp * kTile + (g + 8 * i) * kTN + (WT ? 4 * q + j : q + 4 * j)] = acc[i][j];
+  __syncthreads();
+  float* part = sm + (kLinThreads / 32) * kTile;
+  for (int e = tid; e < kTile; e += kLinThreads) {
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kLinThreads / 32; w++) v += sm[w * kTile + e];
+    part[e] = v;
+  }
+  cluster.sync();
+  double sq = 0.0;
+  if (own) {
+    float v = 0.0f;
+#pragma unroll
+    for (int r = 0; r < kSplit; r++) v += cluster.map_shared_rank(part, r)[eo];
+    if (EPI == EPI_BIAS_SILU) {
+      v += bias;
+      a.C[oo] = v;
+      a.C2[oo] = v * sigmoid(v);
+    } else if (EPI == EPI_BIAS) {
+      a.C[oo] = v + bias;
+    } else if (EPI == EPI_DSILU) {
+      const float s = sigmoid(aux);
+      a.C[oo] = v * (s * (1.0f + aux * (1.0f - s)));
+    } else {
+      const float d = v + bias - aux;
+      a.C[oo] = (float)(2.0 * a.inv) * d;
+      sq = (double)d * d;
+    }
+  }
+  if (EPI == EPI_MSE && tid < kOwn) {
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (lane == 0) atomicAdd(a.loss, sq * a.inv);
+  }
+  cluster.sync();  // the partial tile stays until every rank has read it
+}
+
+// ---- gradients of all layers, and the Adam step on them ------------------------------
+//
+// dW_l(o, i) = sum_b dZ_l[b, o] X_l[b, i] and db_l(o) = sum_b dZ_l[b, o], one
+// launch over the 32 x 64 tiles of every layer; with ADAM the tile steps its
+// parameters at once (Kingma & Ba 2015, bias-corrected step lr_t, decoupled
+// weight decay on W only, Loshchilov & Hutter 2019) instead of storing the
+// gradient: parameters and moments are read and written once.
+constexpr int kMaxLinear = 17, kGradTO = 32;
+
+struct GradLayer {
+  const float* dz;    // (M, fout)
+  const float* in;    // (., fin)
+  const int* rows;    // optional gather of in's rows
+  int fout, fin, tile0, tiles_i;
+  size_t w_off, b_off;
+};
+
+struct GradArgs {
+  GradLayer l[kMaxLinear];
+  int layers, M;
+  float* grads;              // ADAM = false
+  float *p, *m, *v;          // ADAM = true
+  float lr_t, b1, b2, eps_t, decay;
+};
+
+// one step of parameter p with moments m and v
+__device__ __forceinline__ void adam(const GradArgs& a, float g, float decay, float& p, float& m, float& v) {
+  m = a.b1 * m + (1.0f - a.b1) * g;
+  v = a.b2 * v + (1.0f - a.b2) * g * g;
+  p = p * decay - a.lr_t * m / (sqrtf(v) + a.eps_t);
+}
+
+template <bool ADAM>
+__global__ void __launch_bounds__(kLinThreads, 4) k_mlp_grad(const __grid_constant__ GradArgs a) {
+  constexpr int TO = kGradTO, TI = 64, KB = 32, PER = TO / 8;
+  __shared__ __align__(16) float Ds[KB][TO];
+  __shared__ __align__(16) float Is[KB][TI];
+  int l = 0;
+  while (l + 1 < a.layers && (int)blockIdx.x >= a.l[l + 1].tile0) l++;
+  const GradLayer& L = a.l[l];
+  const int t = (int)blockIdx.x - L.tile0;
+  const int o0 = t / L.tiles_i * TO, i0 = t % L.tiles_i * TI;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool bias = i0 == 0 && tid < TO;
+  float acc[PER][2] = {}, bsum = 0.0f;
+  // the tile's parameters and moments do not depend on the gradient: their
+  // loads go out first
+  float p[PER][2], m[PER][2], v[PER][2];
+  if (ADAM) {
+#pragma unroll
+    for (int k = 0; k < PER; k++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int o = o0 + warp * PER + k, i = i0 + lane + 32 * j;
+        if (o < L.fout && i < L.fin) {
+          const size_t w = L.w_off + (size_t)o * L.fin + i;
+          p[k][j] = a.p[w];
+          m[k][j] = a.m[w];
+          v[k][j] = a.v[w];
+        }
+      }
+  }
+  wait_predecessor();
+  for (int b0 = 0; b0 < a.M; b0 += KB) {
+    if (b0 > 0) __syncthreads();
+    const int nb = min(KB, a.M - b0);
+#pragma unroll
+    for (int e = tid; e < KB * TO; e += 256) {
+      const int b = e / TO, c = e % TO;
+      Ds[b][c] = b < nb && o0 + c < L.fout ? L.dz[(size_t)(b0 + b) * L.fout + o0 + c] : 0.0f;
+    }
+#pragma unroll
+    for (int e = tid; e < KB * TI; e += 256) {
+      const int b = e / TI, c = e % TI;
+      Is[b][c] = b < nb && i0 + c < L.fin
+                     ? L.in[(size_t)(L.rows ? L.rows[b0 + b] : b0 + b) * L.fin + i0 + c] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int b = 0; b < nb; b++) {
+      const float4 d0 = *reinterpret_cast<const float4*>(&Ds[b][warp * PER]);
+      const float d[PER] = {d0.x, d0.y, d0.z, d0.w};
+      const float x0 = Is[b][lane], x1 = Is[b][lane + 32];
+#pragma unroll
+      for (int k = 0; k < PER; k++) {
+        acc[k][0] = fmaf(d[k], x0, acc[k][0]);
+        acc[k][1] = fmaf(d[k], x1, acc[k][1]);
+      }
+    }
+    if (bias)
+      for (int b = 0; b < nb; b++) bsum += Ds[b][tid];
+  }
+#pragma unroll
+  for (int k = 0; k < PER; k++)
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int o = o0 + warp * PER + k, i = i0 + lane + 32 * j;
+      if (o < L.fout && i < L.fin) {
+        const size_t w = L.w_off + (size_t)o * L.fin + i;
+        if (ADAM) {
+          adam(a, acc[k][j], a.decay, p[k][j], m[k][j], v[k][j]);
+          a.p[w] = p[k][j];
+          a.m[w] = m[k][j];
+          a.v[w] = v[k][j];
+        } else {
+          a.grads[w] = acc[k][j];
+        }
+      }
+    }
+  if (bias && o0 + tid < L.fout) {
+    const size_t w = L.b_off + o0 + tid;
+    if (ADAM) {
+      float bp = a.p[w], bm = a.m[w], bv = a.v[w];
+      adam(a, bsum, 1.0f, bp, bm, bv);
+      a.p[w] = bp;
+      a.m[w] = bm;
+      a.v[w] = bv;
+    } else {
+      a.grads[w] = bsum;
+    }
   }
 }
 
-// Adam (Kingma & Ba 2015) with bias-corrected step size lr_t
-__global__ void k_mlp_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                           float* __restrict__ v, size_t n, float lr_t, float b1, float b2, float eps_t) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr_t * mi / (sqrtf(vi) + eps_t);
-  }
+template <class Args>
+int launch_dependent(tups_mlp* m, const char* name, void (*kernel)(Args), dim3 grid, size_t smem, const Args& a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kLinThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = m->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  m->launches++;
+  return mlp_cuda(m, cudaLaunchKernelEx(&cfg, kernel, a), name);
 }
 
-__global__ void k_mlp_scale(float* __restrict__ p, size_t n, float f) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] *= f;
+template <int EPI, bool WT>
+int linear(tups_mlp* m, const LinArgs& a) {
+  const dim3 grid((unsigned)((a.N + kTN - 1) / kTN * kSplit), (unsigned)((a.M + kTM - 1) / kTM));
+  return launch_dependent(m, "k_mlp_linear", k_mlp_linear<EPI, WT>, grid, kLinSmem, a);
 }
 
-// rows of a resident set: out[i, :] = src[idx[i], :]
-__global__ void k_mlp_gather(const float* __restrict__ src, const int* __restrict__ idx, float* __restrict__ out,
-                             int rows, int cols) {
-  const size_t n = (size_t)rows * cols;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(e / cols), c = (int)(e % cols);
-    out[e] = src[(size_t)idx[r] * cols + c];
-  }
-}
-
-unsigned grid1d(size_t n, int threads) {
-  const size_t b = (n + threads - 1) / threads;
-  return (unsigned)std::min<size_t>(std::max<size_t>(b, 1), 148 * 8);
-}
-
-template <int EPI>
-int gemm(tups_mlp* m, int M, int N, int K, const float* A, int sam, int sak, const float* B, int sbk, int sbn,
-         const float* bias, const float* aux, float* C, float* C2) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  k_mlp_gemm<EPI><<<grid, 256, 0, m->stream>>>(M, N, K, A, sam, sak, B, sbk, sbn, bias, aux, C, C2);
-  return launched(m, "k_mlp_gemm");
+// opt-in shared memory of every instantiation that linear() launches
+int linear_prepare(tups_mlp* m) {
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  MTRY(mlp_cuda(m, cudaFuncSetAttribute(k_mlp_linear<EPI_BIAS_SILU, false>, attr, (int)kLinSmem), "k_mlp_linear"));
+  MTRY(mlp_cuda(m, cudaFuncSetAttribute(k_mlp_linear<EPI_BIAS, false>, attr, (int)kLinSmem), "k_mlp_linear"));
+  MTRY(mlp_cuda(m, cudaFuncSetAttribute(k_mlp_linear<EPI_MSE, false>, attr, (int)kLinSmem), "k_mlp_linear"));
+  return mlp_cuda(m, cudaFuncSetAttribute(k_mlp_linear<EPI_DSILU, true>, attr, (int)kLinSmem), "k_mlp_linear");
 }
 
 int n_linear(const tups_mlp* m) { return m->n_layers + 1; }
 
-// forward of the batch in m->x (batch rows) into m->y
-int forward(tups_mlp* m, int batch) {
-  const float* in = m->x;
+// forward of `batch` rows of x (gathered by rows, or consecutive); the last
+// layer gives m->y, or with targets t the loss into loss and its gradient
+// with respect to the output
+int forward(tups_mlp* m, int batch, const float* x, const int* rows, const float* t, double* loss) {
+  const float* in = x;
   for (int l = 0; l < n_linear(m); l++) {
-    const int fin = m->width[l], fout = m->width[l + 1];
-    const float* W = m->params + m->w_off[l];
-    const float* b = m->params + m->b_off[l];
-    // Z = in W^T + b: A(m, k) = in[m*fin + k], B(k, n) = W[n*fin + k]
+    LinArgs a{};
+    a.M = batch;
+    a.N = m->width[l + 1];
+    a.K = m->width[l];
+    a.X = in;
+    a.rows = l == 0 ? rows : nullptr;
+    a.w_fresh = l == 0;  // the previous step's update
+    a.W = m->params + m->w_off[l];
+    a.bias = m->params + m->b_off[l];
     if (l < m->n_layers) {
-      MTRY(gemm<EPI_BIAS_SILU>(m, batch, fout, fin, in, fin, 1, W, 1, fin, b, nullptr, m->z[l], m->a[l]));
+      a.C = m->z[l];
+      a.C2 = m->a[l];
+      MTRY((linear<EPI_BIAS_SILU, false>(m, a)));
       in = m->a[l];
+    } else if (!t) {
+      a.C = m->y;
+      MTRY((linear<EPI_BIAS, false>(m, a)));
     } else {
-      MTRY(gemm<EPI_BIAS>(m, batch, fout, fin, in, fin, 1, W, 1, fin, b, nullptr, m->y, nullptr));
+      a.C = m->dz[l];
+      a.aux = t;
+      a.trows = rows;
+      a.loss = loss;
+      a.inv = 1.0 / ((double)batch * m->n_out);
+      MTRY((linear<EPI_MSE, false>(m, a)));
     }
   }
   return TUPS_OK;
 }
 
-// loss into m->loss[slot] and gradients of the batch in m->x / m->t into m->grads
-int backward(tups_mlp* m, int batch, int slot) {
-  const size_t ny = (size_t)batch * m->n_out;
-  float* dcur = m->dz[0];
-  k_mlp_mse<<<grid1d(ny, 256), 256, 0, m->stream>>>(m->y, m->t, dcur, ny, 1.0 / (double)ny, m->loss + slot);
-  MTRY(launched(m, "k_mlp_mse"));
-  for (int l = n_linear(m) - 1; l >= 0; l--) {
-    const int fin = m->width[l], fout = m->width[l + 1];
-    const float* in = l == 0 ? m->x : m->a[l - 1];
-    // dW(o, i) = sum_b dZ[b, o] in[b, i]: A(m=o, k=b) = dZ[b*fout + o], B(k=b, n=i) = in[b*fin + i]
-    MTRY(gemm<EPI_STORE>(m, fout, fin, batch, dcur, 1, fout, in, fin, 1, nullptr, nullptr, m->grads + m->w_off[l],
-                         nullptr));
-    k_mlp_colsum<<<(fout + 127) / 128, 128, 0, m->stream>>>(dcur, m->grads + m->b_off[l], batch, fout);
-    MTRY(launched(m, "k_mlp_colsum"));
-    if (l > 0) {
-      // dZ_{l-1}(b, i) = sum_o dZ[b, o] W[o, i] * silu'(Z_{l-1}(b, i))
-      float* dnext = dcur == m->dz[0] ? m->dz[1] : m->dz[0];
-      const float* W = m->params + m->w_off[l];
-      MTRY(gemm<EPI_DSILU>(m, batch, fin, fout, dcur, fout, 1, W, fin, 1, nullptr, m->z[l - 1], dnext, nullptr));
-      dcur = dnext;
-    }
+// gradients of the batch whose forward (with targets) just ran: into m->grads,
+// or with lr > 0 as one Adam step
+int backward(tups_mlp* m, int batch, const float* x, const int* rows, float lr, float weight_decay) {
+  for (int l = n_linear(m) - 1; l > 0; l--) {
+    // dZ_{l-1}(b, i) = sum_o dZ_l[b, o] W_l[o, i] silu'(Z_{l-1}(b, i))
+    LinArgs a{};
+    a.M = batch;
+    a.N = m->width[l];
+    a.K = m->width[l + 1];
+    a.X = m->dz[l];
+    a.W = m->params + m->w_off[l];
+    a.aux = m->z[l - 1];
+    a.C = m->dz[l - 1];
+    MTRY((linear<EPI_DSILU, true>(m, a)));
   }
-  return TUPS_OK;
-}
-
-int adam_step(tups_mlp* m, float lr, float b1, float b2, float eps) {
-  m->adam_t++;
-  const double bc1 = 1.0 - std::pow((double)b1, (double)m->adam_t);
-  const double bc2 = 1.0 - std::pow((double)b2, (double)m->adam_t);
-  // step with bias correction folded into the step size and epsilon
-  const float lr_t = (float)(lr * std::sqrt(bc2) / bc1);
-  const float eps_t = (float)(eps * std::sqrt(bc2));
-  k_mlp_adam<<<grid1d(m->n_params, 256), 256, 0, m->stream>>>(m->params, m->grads, m->adam_m, m->adam_v,
-                                                               m->n_params, lr_t, b1, b2, eps_t);
-  return launched(m, "k_mlp_adam");
+  GradArgs g{};
+  g.layers = n_linear(m);
+  g.M = batch;
+  int tiles = 0;
+  for (int l = 0; l < g.layers; l++) {
+    GradLayer& L = g.l[l];
+    L.dz = m->dz[l];
+    L.in = l == 0 ? x : m->a[l - 1];
+    L.rows = l == 0 ? rows : nullptr;
+    L.fout = m->width[l + 1];
+    L.fin = m->width[l];
+    L.tile0 = tiles;
+    L.tiles_i = (L.fin + 63) / 64;
+    L.w_off = m->w_off[l];
+    L.b_off = m->b_off[l];
+    tiles += (L.fout + kGradTO - 1) / kGradTO * L.tiles_i;
+  }
+  g.grads = m->grads;
+  if (lr > 0.0f) {
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    m->adam_t++;
+    const double bc1 = 1.0 - std::pow((double)b1, (double)m->adam_t);
+    const double bc2 = 1.0 - std::pow((double)b2, (double)m->adam_t);
+    // step with bias correction folded into the step size and epsilon
+    g.p = m->params;
+    g.m = m->adam_m;
+    g.v = m->adam_v;
+    g.b1 = b1;
+    g.b2 = b2;
+    g.lr_t = (float)(lr * std::sqrt(bc2) / bc1);
+    g.eps_t = (float)(eps * std::sqrt(bc2));
+    g.decay = weight_decay > 0.0f ? 1.0f - lr * weight_decay : 1.0f;
+    return launch_dependent(m, "k_mlp_grad", k_mlp_grad<true>, dim3(tiles), 0, g);
+  }
+  return launch_dependent(m, "k_mlp_grad", k_mlp_grad<false>, dim3(tiles), 0, g);
 }
 
 int h2d(tups_mlp* m, void* dst, const void* src, size_t bytes) {
@@ -348,22 +577,28 @@ extern "C" int tups_mlp_create(int n_in, int n_hidden, int n_layers, int n_out, 
   m->n_params = off;
   int rc = set_dev(m);
   if (!rc) rc = mlp_cuda(m, cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking), "stream");
-  const int wmax = std::max(std::max(n_in, n_hidden), n_out);
-  if (!rc) rc = mlp_alloc(m, &m->params, m->n_params);
-  if (!rc) rc = mlp_alloc(m, &m->grads, m->n_params);
-  if (!rc) rc = mlp_alloc(m, &m->adam_m, m->n_params);
-  if (!rc) rc = mlp_alloc(m, &m->adam_v, m->n_params);
-  if (!rc) rc = mlp_alloc(m, &m->x, (size_t)max_batch * n_in);
-  if (!rc) rc = mlp_alloc(m, &m->t, (size_t)max_batch * n_out);
-  if (!rc) rc = mlp_alloc(m, &m->y, (size_t)max_batch * n_out);
+  if (!rc) rc = linear_prepare(m);
+  // every buffer of the network in one allocation (one cudaMalloc and one
+  // cudaFree instead of one per buffer)
   m->z.assign(n_layers, nullptr);
   m->a.assign(n_layers, nullptr);
-  for (int l = 0; l < n_layers && !rc; l++) {
-    rc = mlp_alloc(m, &m->z[l], (size_t)max_batch * n_hidden);
-    if (!rc) rc = mlp_alloc(m, &m->a[l], (size_t)max_batch * n_hidden);
+  m->dz.assign(n_layers + 1, nullptr);
+  std::vector<std::pair<float**, size_t>> want = {
+      {&m->params, m->n_params}, {&m->grads, m->n_params}, {&m->adam_m, m->n_params}, {&m->adam_v, m->n_params},
+      {&m->x, (size_t)max_batch * n_in}, {&m->t, (size_t)max_batch * n_out}, {&m->y, (size_t)max_batch * n_out}};
+  for (int l = 0; l < n_layers; l++) {
+    want.push_back({&m->z[l], (size_t)max_batch * n_hidden});
+    want.push_back({&m->a[l], (size_t)max_batch * n_hidden});
   }
-  if (!rc) rc = mlp_alloc(m, &m->dz[0], (size_t)max_batch * wmax);
-  if (!rc) rc = mlp_alloc(m, &m->dz[1], (size_t)max_batch * wmax);
+  for (int l = 0; l <= n_layers; l++) want.push_back({&m->dz[l], (size_t)max_batch * m->width[l + 1]});
+  size_t total = 0;
+  for (const auto& w : want) total += (w.second + 63) / 64 * 64;
+  float* arena = nullptr;
+  if (!rc) rc = mlp_alloc(m, &arena, total);
+  for (const auto& w : want) {
+    *w.first = arena;
+    if (arena) arena += (w.second + 63) / 64 * 64;
+  }
   if (!rc) rc = mlp_cuda(m, cudaMemsetAsync(m->params, 0, m->n_params * sizeof(float), m->stream), "memset");
   if (!rc) rc = mlp_cuda(m, cudaMemsetAsync(m->adam_m, 0, m->n_params * sizeof(float), m->stream), "memset");
   if (!rc) rc = mlp_cuda(m, cudaMemsetAsync(m->adam_v, 0, m->n_params * sizeof(float), m->stream), "memset");
@@ -413,7 +648,7 @@ extern "C" int tups_mlp_forward(tups_mlp* m, const float* x, int batch, float* y
   MTRY(set_dev(m));
   MTRY(check_batch(m, batch));
   MTRY(h2d(m, m->x, x, (size_t)batch * m->n_in * sizeof(float)));
-  MTRY(forward(m, batch));
+  MTRY(forward(m, batch, m->x, nullptr, nullptr, nullptr));
   return d2h(m, y, m->y, (size_t)batch * m->n_out * sizeof(float));
 }
 
@@ -429,8 +664,8 @@ extern "C" int tups_mlp_gradients(tups_mlp* m, const float* x, const float* t, i
   MTRY(h2d(m, m->x, x, (size_t)batch * m->n_in * sizeof(float)));
   MTRY(h2d(m, m->t, t, (size_t)batch * m->n_out * sizeof(float)));
   MTRY(mlp_cuda(m, cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream), "memset"));
-  MTRY(forward(m, batch));
-  MTRY(backward(m, batch, 0));
+  MTRY(forward(m, batch, m->x, nullptr, m->t, m->loss));
+  MTRY(backward(m, batch, m->x, nullptr, 0.0f, 0.0f));
   if (loss) MTRY(d2h(m, loss, m->loss, sizeof(double)));
   if (grad) MTRY(d2h(m, grad, m->grads, m->n_params * sizeof(float)));
   return mlp_cuda(m, cudaStreamSynchronize(m->stream), "synchronize");
@@ -471,23 +706,8 @@ extern "C" int tups_mlp_train(tups_mlp* m, const float* x, const float* t, int n
     MTRY(h2d(m, m->idx, all_idx.data() + (size_t)e * n_samples, n_samples * sizeof(int)));
     for (int b = 0; b < per_epoch; b++) {
       const int r0 = b * batch, rows = std::min(batch, n_samples - r0);
-      k_mlp_gather<<<grid1d((size_t)rows * m->n_in, 256), 256, 0, m->stream>>>(m->data_x, m->idx + r0, m->x, rows,
-                                                                              m->n_in);
-      MTRY(launched(m, "k_mlp_gather"));
-      k_mlp_gather<<<grid1d((size_t)rows * m->n_out, 256), 256, 0, m->stream>>>(m->data_t, m->idx + r0, m->t, rows,
-                                                                               m->n_out);
-      MTRY(launched(m, "k_mlp_gather"));
-      MTRY(forward(m, rows));
-      MTRY(backward(m, rows, e));
-      if (weight_decay > 0.0f) {
-        // decoupled weight decay (Loshchilov & Hutter 2019) on the weights only
-        for (int l = 0; l < n_linear(m); l++) {
-          const size_t nw = (size_t)m->width[l] * m->width[l + 1];
-          k_mlp_scale<<<grid1d(nw, 256), 256, 0, m->stream>>>(m->params + m->w_off[l], nw, 1.0f - lr * weight_decay);
-          MTRY(launched(m, "k_mlp_scale"));
-        }
-      }
-      MTRY(adam_step(m, lr, 0.9f, 0.999f, 1e-8f));
+      MTRY(forward(m, rows, m->data_x, m->idx + r0, m->data_t, m->loss + e));
+      MTRY(backward(m, rows, m->data_x, m->idx + r0, lr, weight_decay));
     }
   }
   if (loss_per_epoch && epochs > 0) {

@@ -13,6 +13,7 @@
 #include <string>
 
 #include "tups_device.cuh"
+#include "zgemm_tile.cuh"
 
 namespace tups {
 
@@ -132,237 +133,63 @@ __global__ void __launch_bounds__(256) k_bse_prep_ab(BsePtrs P, const cplx* __re
   else prep_chi_gamma<LMAX>(P, chi_ph, chi_pp, B, q_begin, Nz, Nf, Nl, blockIdx.x - nA, chs);
 }
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc, bool valid) {
-  unsigned sz = valid ? 16u : 0u;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(sdst)), "l"(gsrc), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// D += A*B on 16x8x8 f64 tiles (row.col): a[4], b[2], c[4] per thread
-__device__ __forceinline__ void dmma16x8x8(double* c, const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
-// Batched complex GEMM on the FP64 tensor cores with the BSE epilogue.
-// CTA tile BM x BN (complex), K step BK; WM x WN warps, warp tile
-// (16 TM) x (8 TN).  Left operand L = [A | F] (Nz x 2Nz), right R = [F ; B].
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, bool M3>
-__global__ void __launch_bounds__(WM* WN * 32) k_bse_gemm(BsePtrs P, const cplx* __restrict__ A,
-                                                          const cplx* __restrict__ B, int q_begin, int Nz,
-                                                          double one_minus_f) {
-  constexpr int TM = BM / WM / 16, TN = BN / WN / 8;
-  constexpr int LDL = BM + 2;  // conflict-free 16-byte fragment loads
-  constexpr int LDR = BK + 4;
-  constexpr int NT = WM * WN * 32;
+// Batched complex GEMM on the FP64 tensor cores with the BSE epilogue:
+// [A | F] (Nz x 2Nz) times [F ; B], tiles of ZgemmTile (zgemm_tile.cuh).
+template <class Tile, int BK, int MINB>
+__global__ void __launch_bounds__(Tile::NT, MINB) k_bse_gemm(BsePtrs P, const cplx* __restrict__ A,
+                                                             const cplx* __restrict__ B, int q_begin, int Nz,
+                                                             double one_minus_f) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  cplx* sL = reinterpret_cast<cplx*>(smraw);           // [STAGES][BK][LDL]
-  cplx* sR = sL + (size_t)STAGES * BK * LDL;           // [STAGES][BN][LDR]
-
   const int inst = blockIdx.y;
   const int q = q_begin + inst / 4, r = inst % 4;
   const size_t n2 = (size_t)Nz * Nz;
-  const cplx* Ai = A + n2 * inst;
-  const cplx* Bi = B + n2 * inst;
-  const cplx* Fq = P.F[r] + n2 * q;
-  cplx* Gq = P.G[r] + n2 * q;
-  const int tiles_m = (Nz + BM - 1) / BM;
-  const int m0 = (blockIdx.x % tiles_m) * BM, n0 = (blockIdx.x / tiles_m) * BN;
-  const int K = 2 * Nz;
-  const int ktiles = (K + BK - 1) / BK;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm0 = (warp % WM) * (16 * TM), wn0 = (warp / WM) * (8 * TN);
-  const int gid = lane >> 2, tig = lane & 3;
-
-  auto load_stage = [&](int stage, int kt) {
-    const int k0 = kt * BK;
-    cplx* dL = sL + (size_t)stage * BK * LDL;
-    cplx* dR = sR + (size_t)stage * BN * LDR;
-    for (int e = tid; e < BK * BM; e += NT) {
-      int m = e % BM, kk = e / BM;
-      int gm = m0 + m, gk = k0 + kk;
-      bool ok = gm < Nz && gk < K;
-      const cplx* src = Ai;
-      if (ok) src = gk < Nz ? Ai + gm + (size_t)Nz * gk : Fq + gm + (size_t)Nz * (gk - Nz);
-      cp_async16(dL + kk * LDL + m, src, ok);
-    }
-    for (int e = tid; e < BK * BN; e += NT) {
-      int kk = e % BK, n = e / BK;
-      int gn = n0 + n, gk = k0 + kk;
-      bool ok = gn < Nz && gk < K;
-      const cplx* src = Fq;
-      if (ok) src = gk < Nz ? Fq + gk + (size_t)Nz * gn : Bi + (gk - Nz) + (size_t)Nz * gn;
-      cp_async16(dR + n * LDR + kk, src, ok);
-    }
-  };
-
-  // M3: three real products per complex one (Gauss): P1 = Ar Br, P2 = Ai Bi,
-  // P3 = (Ar + Ai)(Br + Bi); Re = P1 - P2, Im = P3 - P1 - P2.  Otherwise four:
-  // Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br (accumulated in p1 = Re, p2 = Im).
-  double p1[TM][TN][4], p2[TM][TN][4], p3[M3 ? TM : 1][M3 ? TN : 1][4];
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        p1[i][j][e] = p2[i][j][e] = 0.0;
-        if (M3) p3[M3 ? i : 0][M3 ? j : 0][e] = 0.0;
-      }
-
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; s++) {
-    if (s < ktiles) load_stage(s, s);
-    cp_async_commit();
-  }
-  for (int kt = 0; kt < ktiles; kt++) {
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();
-    {
-      int nk = kt + STAGES - 1;
-      if (nk < ktiles) load_stage(nk % STAGES, nk);
-      cp_async_commit();
-    }
-    const cplx* cL = sL + (size_t)(kt % STAGES) * BK * LDL;
-    const cplx* cR = sR + (size_t)(kt % STAGES) * BN * LDR;
-#pragma unroll
-    for (int k8 = 0; k8 < BK; k8 += 8) {
-      double are[TM][4], aim[TM][4], anim[TM][4], bre[TN][2], bim[TN][2];
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const int mb = wm0 + i * 16 + gid;
-        cplx v0 = cL[(k8 + tig) * LDL + mb];
-        cplx v1 = cL[(k8 + tig) * LDL + mb + 8];
-        cplx v2 = cL[(k8 + tig + 4) * LDL + mb];
-        cplx v3 = cL[(k8 + tig + 4) * LDL + mb + 8];
-        are[i][0] = v0.x; aim[i][0] = v0.y;
-        are[i][1] = v1.x; aim[i][1] = v1.y;
-        are[i][2] = v2.x; aim[i][2] = v2.y;
-        are[i][3] = v3.x; aim[i][3] = v3.y;
-#pragma unroll
-        for (int e = 0; e < 4; e++) anim[i][e] = -aim[i][e];
-      }
-#pragma unroll
-      for (int j = 0; j < TN; j++) {
-        const int nb = wn0 + j * 8 + gid;
-        cplx w0 = cR[nb * LDR + k8 + tig];
-        cplx w1 = cR[nb * LDR + k8 + tig + 4];
-        bre[j][0] = w0.x; bim[j][0] = w0.y;
-        bre[j][1] = w1.x; bim[j][1] = w1.y;
-      }
-      if (M3) {
-        double asum[TM][4], bsum[TN][2];
-#pragma unroll
-        for (int i = 0; i < TM; i++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) asum[i][e] = are[i][e] + aim[i][e];
-#pragma unroll
-        for (int j = 0; j < TN; j++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) bsum[j][e] = bre[j][e] + bim[j][e];
-#pragma unroll
-        for (int i = 0; i < TM; i++)
-#pragma unroll
-          for (int j = 0; j < TN; j++) {
-            dmma16x8x8(p1[i][j], are[i], bre[j]);
-            dmma16x8x8(p2[i][j], aim[i], bim[j]);
-            dmma16x8x8(p3[M3 ? i : 0][M3 ? j : 0], asum[i], bsum[j]);
-          }
-      } else {
-#pragma unroll
-        for (int i = 0; i < TM; i++)
-#pragma unroll
-          for (int j = 0; j < TN; j++) {
-            dmma16x8x8(p1[i][j], are[i], bre[j]);
-            dmma16x8x8(p1[i][j], anim[i], bim[j]);
-            dmma16x8x8(p2[i][j], are[i], bim[j]);
-            dmma16x8x8(p2[i][j], aim[i], bre[j]);
-          }
-      }
-    }
-  }
-  cp_async_wait<0>();
-  double cre[TM][TN][4], cim[TM][TN][4];
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        if (M3) {
-          cre[i][j][e] = p1[i][j][e] - p2[i][j][e];
-          cim[i][j][e] = p3[M3 ? i : 0][M3 ? j : 0][e] - p1[i][j][e] - p2[i][j][e];
-        } else {
-          cre[i][j][e] = p1[i][j][e];
-          cim[i][j][e] = p2[i][j][e];
-        }
-      }
-
+  // constant indices keep the parameter struct out of local memory
+  const cplx* Fq = (r == 0 ? P.F[0] : r == 1 ? P.F[1] : r == 2 ? P.F[2] : P.F[3]) + n2 * q;
+  cplx* Gq = (r == 0 ? P.G[0] : r == 1 ? P.G[1] : r == 2 ? P.G[2] : P.G[3]) + n2 * q;
+  const double s = r == 0 ? P.scale[0] : r == 1 ? P.scale[1] : r == 2 ? P.scale[2] : P.scale[3];
+  const int tiles_m = (Nz + Tile::BM - 1) / Tile::BM;
+  const int m0 = (int)(blockIdx.x % tiles_m) * Tile::BM, n0 = (int)(blockIdx.x / tiles_m) * Tile::BN;
+  Tile t;
+  t.run(BseSource<BK>{A + n2 * inst, Fq, B + n2 * inst, Nz, m0, n0}, reinterpret_cast<cplx*>(smraw), Nz - m0, Nz - n0);
   // epilogue: Phi = s * C + (1-f) (F - Gamma), written over Gamma
-  const double s = P.scale[r];
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        int row = m0 + wm0 + i * 16 + gid + (e >= 2 ? 8 : 0);
-        int col = n0 + wn0 + j * 8 + 2 * tig + (e & 1);
-        if (row < Nz && col < Nz) {
-          size_t idx = row + (size_t)Nz * col;
-          cplx f = Fq[idx], g = Gq[idx];
-          Gq[idx] = cmk(s * cre[i][j][e] + one_minus_f * (f.x - g.x), s * cim[i][j][e] + one_minus_f * (f.y - g.y));
-        }
-      }
+  t.each(Nz - m0, Nz - n0, [&](int row, int col, cplx c) {
+    const size_t idx = (m0 + row) + (size_t)Nz * (n0 + col);
+    const cplx f = Fq[idx], g = Gq[idx];
+    Gq[idx] = cmk(s * c.x + one_minus_f * (f.x - g.x), s * c.y + one_minus_f * (f.y - g.y));
+  });
 }
 
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, bool M3>
+template <int TM, int TN, int WM, int WN, int BK, int ST, int MINB>
 static int run_gemm(tups_ctx* ctx, const BsePtrs& P, int q_begin, int q_count) {
+  using Tile = ZgemmTile<TM, TN, WM, WN, BK, ST, true>;
   const int Nz = ctx->d.Nz;
-  constexpr int LDL = BM + 2, LDR = BK + 4;
-  size_t sm = (size_t)STAGES * (BK * LDL + BN * LDR) * sizeof(cplx);
-  auto kern = k_bse_gemm<BM, BN, BK, WM, WN, STAGES, M3>;
-  if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  auto kern = k_bse_gemm<Tile, BK, MINB>;
+  if (Tile::kSmem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem);
     if (e != cudaSuccess) return cuda_check(ctx, e, "k_bse_gemm smem attribute");
   }
-  int tiles = ((Nz + BM - 1) / BM) * ((Nz + BN - 1) / BN);
-  dim3 grid(tiles, 4 * q_count);
-  kern<<<grid, WM * WN * 32, sm, ctx->stream>>>(P, ctx->s.bse_A, ctx->s.bse_B, q_begin, Nz,
-                                                1.0 - ctx->p.f_damping);
+  const int tiles = ((Nz + Tile::BM - 1) / Tile::BM) * ((Nz + Tile::BN - 1) / Tile::BN);
+  kern<<<dim3(tiles, 4 * q_count), Tile::NT, Tile::kSmem, ctx->stream>>>(P, ctx->s.bse_A, ctx->s.bse_B, q_begin, Nz,
+                                                                          1.0 - ctx->p.f_damping);
   return after_launch(ctx, "k_bse_gemm");
 }
 
 // Tile candidates of the FP64 BSE GEMM for Nz >= 32, all with three real
 // products per complex one: they differ in CTA tile, warps and pipeline
 // depth, never in the order of any element's K sum, so every candidate
-// writes the same bits.  Index 0 is the choice measured best on a B200 before
-// the tuner existed: 32 x 32 tiles of 4 warps (16 x 16 each), two cp.async
-// stages (38 KB of shared memory, 5 CTAs per SM): 8x8 / Nl = 5 (Nz = 160)
-// 1.79 ms, against 1.93 ms with three stages, 2.01 ms with BK = 32 and
-// 2.13 ms with four products; 16x16 / Nl = 9 (Nz = 576) 480 ms, against
-// 541 ms for 64 x 64 tiles of 8 warps with four products, 656 ms with three.
+// writes the same bits.  Index 0 is the choice measured best on a B200: 32 x 32
+// tiles of 4 warps (16 x 16 each), three stages of 16 columns, 3 CTAs per SM
+// (the second fragment set needs 170 registers).  8x8 / Nl = 5 (Nz = 160):
+// 1.62 ms, four stages 1.64, 16 x 64 tiles 2.0; Nz = 110, where a 16-row tile
+// wastes least: 0.165, 0.162, 0.164 ms of the tuner's sample.
 struct BseCand {
   const char* name;
   int (*run)(tups_ctx*, const BsePtrs&, int, int);
 };
 static const BseCand kBseCands[] = {
-    {"32x32x16_w2x2_s2", run_gemm<32, 32, 16, 2, 2, 2, true>},
-    {"32x32x16_w2x2_s3", run_gemm<32, 32, 16, 2, 2, 3, true>},
-    {"64x32x16_w4x2_s2", run_gemm<64, 32, 16, 4, 2, 2, true>},
-    {"32x64x16_w2x4_s2", run_gemm<32, 64, 16, 2, 4, 2, true>},
-    {"32x32x32_w2x2_s2", run_gemm<32, 32, 32, 2, 2, 2, true>},
+    {"32x32x16_w2x2_s3", run_gemm<1, 2, 2, 2, 16, 3, 3>},
+    {"32x32x16_w2x2_s4", run_gemm<1, 2, 2, 2, 16, 4, 3>},
+    {"16x64x16_w1x4_s3", run_gemm<1, 2, 1, 4, 16, 3, 3>},
 };
 constexpr int kNumBseCands = sizeof(kBseCands) / sizeof(kBseCands[0]);
 
@@ -590,7 +417,7 @@ int launch_bse_chunk(tups_ctx* ctx, int q_begin, int q_count) {
     rc = bse_choice(ctx, P, q_begin, q_count, &choice);
     if (!rc) rc = kBseCands[choice].run(ctx, P, q_begin, q_count);
   } else {
-    rc = run_gemm<16, 16, 16, 1, 2, 3, true>(ctx, P, q_begin, q_count);
+    rc = run_gemm<1, 1, 1, 2, 16, 3, 6>(ctx, P, q_begin, q_count);
   }
   phase_end(ctx, TUPS_PHASE_BSE_GEMM);
   return rc;

@@ -1,0 +1,52 @@
+"""The crossing on a B200 at sizes around its tiles: element lists and columns
+that no tile divides, sums of one and several stages, the short-sum and the
+long-sum tiles, both product forms, one form factor."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import tups_oracle as O
+import parity
+
+pytestmark = pytest.mark.gpu
+
+# FP64 sums of a few hundred terms against the oracle's: 1e-12 of the largest
+TOL = 1e-12
+
+
+@pytest.mark.parametrize("products", [3, 4])
+@pytest.mark.parametrize("case", [
+    dict(Nx=4, Nf=6, neighbours=1),
+    dict(Nx=4, Nf=18, neighbours=1),
+    dict(Nx=4, Nf=6, neighbours=2),
+    dict(Nx=6, Nf=14, neighbours=2),
+    dict(Nx=4, Nf=10, neighbours=3),
+], ids=["nl1_nf6", "nl1_nf18", "nl5_nf6", "nl5_nf14_nx6", "nl9_nf10"])
+def test_crossing_at_tile_edges(gpu_lib, case, products):
+    from tups_b200 import Solver
+    p = O.Params(beta=3.0, U=2.0, nParticle=0.95, f_damping=0.5, ite_max=10, **case)
+    st = O.initialize(p)
+    sol = Solver(parity.to_solver_params(p))
+    sol.set_crossing_products(products)
+    rng = np.random.default_rng(case["Nf"] + products)
+    shape = (sol.Nz, sol.Nz, sol.Nb)
+    G = {r: rng.standard_normal(shape) + 1j * rng.standard_normal(shape) for r in "dmst"}
+    sol.calculate_expSqR()
+    sol.calculate_expqSR()
+    for w in ("phbar_to_ph", "pp_to_ph", "ph_to_pp", "phbar_to_pp"):
+        getattr(sol, "calc_M_" + w)()
+    for r in "dmst":
+        sol.set_vertex(r, 1, G[r])
+    sol.calc_PhiR(0)
+    sol.calculate_PAE()
+    O.calculate_expSqR(st)
+    O.calculate_expqSR(st)
+    for r in "dmst":
+        st.G[r] = G[r].copy()
+    O.calc_PhiR(st)
+    O.calc_M(st)
+    O.calculate_PAE(st)
+    for r in "dmst":
+        assert parity.rel(sol.F(r), st.F[r]) <= TOL, r
+    sol.close()

@@ -602,14 +602,16 @@ extern "C" int tups_get_PhiR(tups_ctx* ctx, int channel, double* h) {
 extern "C" int tups_get_M(tups_ctx* ctx, int which, double* h) {
   if (!ctx || which < 0 || which > 3 || !h) return TUPS_ERR_BADARG;
   const auto& d = ctx->d;
-  const size_t nl4 = (size_t)d.Nl * d.Nl * d.Nl * d.Nl;
+  const size_t nl2 = (size_t)d.Nl * d.Nl, nl4 = nl2 * nl2;
   std::vector<cplx> m(nl4 * d.NIBZ * d.NR);
   TRY(copy_d2h(ctx, m.data(), ctx->s.M[which], m.size() * sizeof(cplx)));
   cplx* out = reinterpret_cast<cplx*>(h);
   for (int R = 0; R < d.NR; R++)
     for (int q = 0; q < d.Nb; q++) {
       const int Qi = q / (d.Nf / 2);
-      std::memcpy(out + nl4 * (q + (size_t)d.Nb * R), m.data() + nl4 * (Qi + (size_t)d.NIBZ * R), nl4 * sizeof(cplx));
+      // the device keeps (l3, l4, R) fastest, then (l1, l2), then Q
+      for (size_t t = 0; t < nl4; t++)
+        out[nl4 * (q + (size_t)d.Nb * R) + t] = m[(Qi * nl2 + t % nl2) * (nl2 * d.NR) + R * nl2 + t / nl2];
     }
   return TUPS_OK;
 }

@@ -243,9 +243,10 @@ __global__ void k_M(cplx* __restrict__ M, int which, const double* __restrict__ 
   const int nl4 = Nl * Nl * Nl * Nl;
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (size_t)nl4 * NIBZ * NR) return;
-  int t = (int)(e % nl4);
-  const int Q = (int)((e / nl4) % NIBZ), R = (int)(e / ((size_t)nl4 * NIBZ));
-  const int l1 = t % Nl, l2 = (t / Nl) % Nl, l3 = (t / (Nl * Nl)) % Nl, l4 = t / (Nl * Nl * Nl);
+  // stored as the crossing GEMM's right operand: (l3, l4, R) fastest, then (l1, l2), then Q
+  const int nl2 = Nl * Nl, K = nl2 * NR, k = (int)(e % K), R = k / nl2;
+  const int l12 = (int)((e / K) % nl2), Q = (int)(e / ((size_t)K * nl2));
+  const int l1 = l12 % Nl, l2 = l12 / Nl, l3 = k % nl2 % Nl, l4 = k % nl2 / Nl;
   const int qx = qibz_xy[2 * Q] - 1, qy = qibz_xy[2 * Q + 1] - 1;  // 0-based
   const int Nc = Nx * Ny;
   auto ff = [&](int kx, int ky, int l) { return FF[kx + Nx * (ky + Ny * l)]; };

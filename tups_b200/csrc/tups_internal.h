@@ -37,6 +37,8 @@ struct DeviceTables {
   cplx* tw_y = nullptr;       // (Ny*Ng)
   int4* pae_elems = nullptr;  // crossing: elements per (pair, family, W), see pae.cu
   int* pae_counts = nullptr;
+  long long* pae_xoff = nullptr;  // crossing: a list's place in the gathered operand
+  cplx* pae_x = nullptr;          // crossing: the gathered operand of one chunk of frequencies
 };
 
 struct DeviceState {
@@ -54,7 +56,7 @@ struct DeviceState {
   cplx* bse_B = nullptr;      // chi*Gamma
   size_t bse_chunk = 0;       // instances per chunk
   cplx* PhiR[4] = {};         // (Nz*Nz, Nf/2, NR)
-  cplx* M[4] = {};            // (Nl^4, NIBZ, NR): 0 phbar_to_ph 1 pp_to_ph 2 ph_to_pp 3 phbar_to_pp
+  cplx* M[4] = {};            // (Nl^2 NR, Nl^2, NIBZ): 0 phbar_to_ph 1 pp_to_ph 2 ph_to_pp 3 phbar_to_pp
   cplx* chi_aux_ph = nullptr; // (Nl*nbox, Nb)
   cplx* chi_aux_pp = nullptr;
   cplx* LChi = nullptr;       // (Nb, Nz): slot fastest
@@ -120,7 +122,8 @@ struct tups_ctx {
   // host copies of small state
   double F_max_prev[4] = {0, 0, 0, 0};
   bool have_exp = false, have_M = false, have_phir = false, have_green = false;
-  int pae_max_tiles[2] = {0, 0};  // longest element list of each family
+  std::vector<int> pae_cnt;         // crossing: length of each element list
+  std::vector<int> pae_chunks[2];   // crossing: first frequency of each chunk of a family, then Nf/2
   tups::DeviceTables t;
   tups::DeviceState s;
   tups::ReadoutBufs rd;

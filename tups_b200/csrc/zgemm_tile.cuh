@@ -41,8 +41,12 @@ __device__ __forceinline__ void zg_dmma(double* c, const double* a, const double
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
+// Without AHEAD the fragments of a step are read when it starts: fewer
+// registers, so more CTAs per SM, which is the better side for short sums (a
+// 64-column LU update: 5 CTAs per SM 6.4 ms, 3 with AHEAD 9.6).
+//
 // WM x WN warps of 16 TM x 8 TN
-template <int TM, int TN, int WM, int WN, int BK, int ST, bool M3>
+template <int TM, int TN, int WM, int WN, int BK, int ST, bool M3, bool AHEAD = true>
 struct ZgemmTile {
   static constexpr int BM = 16 * TM * WM, BN = 8 * TN * WN, NW = WM * WN, NT = 32 * NW;
   static constexpr int LDL = BM + 2, LDR = BK + 4;  // conflict-free 16-byte fragment reads
@@ -100,7 +104,7 @@ struct ZgemmTile {
         }
       }
     };
-    cplx fa[2][TM][4], fb[2][TN][2];
+    cplx fa[AHEAD ? 2 : 1][TM][4], fb[AHEAD ? 2 : 1][TN][2];
     auto fetch = [&](int buf, int st, int k8) {
       const cplx* cL = sL + (size_t)st * BK * LDL + (k8 + tig) * LDL + wm0 + gid;
       const cplx* cR = sR + (size_t)st * BN * LDR + (wn0 + gid) * LDR + k8 + tig;
@@ -131,27 +135,36 @@ struct ZgemmTile {
       asm volatile("cp.async.commit_group;\n" ::);
       ldst = ldst + 1 == ST ? 0 : ldst + 1;
     };
-    land();
+    if (AHEAD) land();
     if (wm0 >= rows || wn0 >= cols) {
       for (int kt = 0; kt < ktiles; kt++) {
+        if (!AHEAD) land();
         refill(kt);
-        land();
+        if (AHEAD) land();
       }
       return;
     }
-    fetch(0, 0, 0);
+    if (AHEAD) fetch(0, 0, 0);
     for (int kt = 0; kt < ktiles; kt++) {
+      if (!AHEAD) {
+        land();
+        refill(kt);
+      }
 #pragma unroll
       for (int kk = 0; kk < KB; kk++) {
-        const int cur = kk & 1;
-        if (kk == KB - 1) {
+        const int cur = AHEAD ? kk & 1 : 0;
+        if (!AHEAD) {
+          fetch(0, st, 8 * kk);
+          if (kk == KB - 1) st = st + 1 == ST ? 0 : st + 1;
+        } else if (kk == KB - 1) {
           land();
           st = st + 1 == ST ? 0 : st + 1;
           fetch(cur ^ 1, st, 0);  // past the last stage: stale content, unused
         } else {
           fetch(cur ^ 1, st, 8 * (kk + 1));
         }
-        if (kk == 0) refill(kt);
+        if (AHEAD && kk == 0) refill(kt);
+        if (!AHEAD && kk > 0 && 8 * kk >= src.depth(kt)) continue;  // a short last stage
         double ar[TM][4], ai[TM][4], as[TM][4];
 #pragma unroll
         for (int i = 0; i < TM; i++)

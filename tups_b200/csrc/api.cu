@@ -57,10 +57,8 @@ int copy_h2d(tups_ctx* ctx, void* dev, const void* host, size_t bytes) {
 
 int green_async(tups_ctx* ctx, int cal_chi) {
   tups::phase_begin(ctx, TUPS_PHASE_GREEN);
-  TRY(tups::launch_sigma_hartree(ctx));
   TRY(tups::launch_bisection(ctx, cal_chi, kMuMaxSteps));
-  TRY(tups::launch_grt(ctx));
-  TRY(tups::launch_gkw(ctx));
+  TRY(tups::launch_green(ctx));
   tups::phase_end(ctx, TUPS_PHASE_GREEN);
   ctx->have_green = true;
   return TUPS_OK;

@@ -5,6 +5,7 @@
 #include <cmath>
 #include <vector>
 
+#include "spline.cuh"
 #include "tups_device.cuh"
 
 namespace tups {
@@ -48,68 +49,26 @@ __global__ void k_chi0_products(const cplx* __restrict__ Grt, const cplx* __rest
 // FDfit + nfourier('Bosonic') at every IBZ point of `narr` fine-grid arrays
 // (SRC/parquet_chi.f90:242-257, SRC/MATH_mod.f90:95-212); one CTA per
 // (IBZ point, array); out[arr][ip * Nf/2 + k]
-__global__ void k_spline_bosonic(const cplx* __restrict__ data, const int* __restrict__ ibz, cplx* __restrict__ out,
-                                 int Nx, int Ny, int Ng, int Nf, int NIBZ, double beta) {
-  extern __shared__ double sp[];
-  double* r = sp;
-  double* qv = sp + Nf;
-  double* u = sp + 2 * Nf;
-  double* xm = sp + 3 * Nf;
+__global__ void __launch_bounds__(128) k_spline_bosonic(const cplx* __restrict__ data, const double* __restrict__ tab,
+                                                        const cplx* __restrict__ ph, const int* __restrict__ ibz, cplx* __restrict__ out, int Nx,
+                                                        int Ny, int Ng, int Nf, int NIBZ, double beta) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const SplineShared S = spline_bind(smraw, Nf);
   const int ip = blockIdx.x, arr = blockIdx.y;
   const int nh = Nf / 2;
   const int n1 = Nx * Ng, n2 = Ny * Ng;
   const int i = ibz[3 * ip * nh], j = ibz[3 * ip * nh + 1];
   const int x = (i - 1) * Ng, y = (j - 1) * Ng;
   const cplx* d = data + (size_t)arr * n1 * n2 * Nf;
-  for (int t = threadIdx.x; t < Nf; t += blockDim.x) r[t] = d[x + (size_t)n1 * (y + (size_t)n2 * t)].x;
-  __syncthreads();
-  const int L = Nf - 1;
-  const double delta = beta / L;
-  if (threadIdx.x == 0) {
-    const double dt = beta / (double)(Nf - 1);
-    const double fd1 = (-25.0 * r[0] + 48.0 * r[1] - 36.0 * r[2] + 16.0 * r[3] - 3.0 * r[4]) / 12.0 / dt;
-    const double fd2 =
-        (25.0 * r[L] - 48.0 * r[L - 1] + 36.0 * r[L - 2] - 16.0 * r[L - 3] + 3.0 * r[L - 4]) / 12.0 / dt;
-    qv[0] = -0.5;
-    u[0] = (3.0 / delta) * ((r[1] - r[0]) / delta - fd1);
-    for (int kk = 2; kk <= L; kk++) {
-      const double p = qv[kk - 2] / 2.0 + 2.0;
-      qv[kk - 1] = -1.0 / 2.0 / p;
-      u[kk - 1] = 3.0 / (delta * delta) * (r[kk] + r[kk - 2] - 2.0 * r[kk - 1]);
-      u[kk - 1] = (u[kk - 1] - u[kk - 2] / 2.0) / p;
-    }
-    qv[L] = 0.5;
-    u[L] = (3.0 / delta) * (fd2 - (r[L] - r[L - 1]) / delta);
-    xm[L] = (u[L] - qv[L] * u[L - 1]) / (qv[L] * qv[L - 1] + 1.0);
-    for (int kk = L; kk >= 1; kk--) xm[kk - 1] = qv[kk - 1] * xm[kk] + u[kk - 1];
-  }
-  __syncthreads();
+  for (int t = threadIdx.x; t < Nf; t += blockDim.x) S.r[t] = d[x + (size_t)n1 * (y + (size_t)n2 * t)].x;
+  spline_fit(S, tab, Nf, beta);
   cplx* o = out + (size_t)arr * NIBZ * nh + (size_t)ip * nh;
-  for (int w = threadIdx.x + 1; w <= nh; w += blockDim.x) {
-    const double om = 2.0 * (w - 1) * M_PI / beta;
-    double cr = 0.0, ci = 0.0;
-    for (int jj = 1; jj <= L; jj++) {
-      const double a = r[jj - 1], c = xm[jj - 1] / 2.0;
-      const double b = (r[jj] - r[jj - 1]) / delta - (2.0 * xm[jj - 1] + xm[jj]) * delta / 6.0;
-      const double dd = (xm[jj] - xm[jj - 1]) / (6.0 * delta);
-      if (fabs(om) < 1e-6) {
-        cr += a * delta + 0.5 * b * delta * delta + c * delta * delta * delta / 3.0 +
-              dd * delta * delta * delta * delta / 4.0;
-        continue;
-      }
-      const double om2 = om * om, om3 = om2 * om, om4 = om3 * om;
-      double sp1, cp1, sm1, cm1;
-      sincos(om * delta * jj, &sp1, &cp1);
-      sincos(om * delta * (jj - 1), &sm1, &cm1);
-      const double p1r = (-6.0 * dd) / om4 + (b + 2.0 * delta * c + 3.0 * delta * delta * dd) / om2;
-      const double p1i =
-          (2.0 * c + 6.0 * delta * dd) / om3 + (-a - delta * b - delta * delta * c - delta * delta * delta * dd) / om;
-      const double p2r = 6.0 * dd / om4 - b / om2;
-      const double p2i = -2.0 * c / om3 + a / om;
-      cr += cp1 * p1r - sp1 * p1i + cm1 * p2r - sm1 * p2i;
-      ci += cp1 * p1i + sp1 * p1r + cm1 * p2i + sm1 * p2r;
-    }
-    o[w - 1] = cmk(cr, ci);
+  const int groups = blockDim.x / kSplineLanes;
+  for (int w0 = 0; w0 < nh; w0 += groups) {
+    const int w = w0 + threadIdx.x / kSplineLanes;
+    const int wc = min(w, nh - 1);
+    const cplx c = spline_transform(S, 2.0 * wc * M_PI / beta, ph + (size_t)Nf * wc, Nf, beta);
+    if (threadIdx.x % kSplineLanes == 0 && w < nh) o[w] = c;
   }
 }
 
@@ -190,14 +149,26 @@ __global__ void __launch_bounds__(256) k_sus(const cplx* __restrict__ F0, const 
   const size_t n2 = (size_t)Nz * Nz;
   // in-box: i = l*Nf + nu  <->  extended index l*nbox + nu + f_range*Nf
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < Nz; i += blockDim.x) {
+  // lanes over rows, a warp per eighth of the columns, eight loads in flight:
+  // one read of F (a thread per row left three warps of eight idle
+  // and one load in flight: 8x8 / Nl = 5 159 -> 140 us)
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, parts = blockDim.x >> 5;
+  for (int i = lane; i < Nz; i += 32) {
     const int ei = (i / Nf) * nbox + i % Nf + f_range * Nf;
     cplx rs[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-    for (int jc = 0; jc < Nz; jc++) {
-      const int ej = (jc / Nf) * nbox + jc % Nf + f_range * Nf;
-      const cplx f = F[i + (size_t)Nz * jc + n2 * q];
+    for (int j0 = part; j0 < Nz; j0 += 8 * parts) {
+      cplx f[8];
 #pragma unroll
-      for (int ff = 0; ff < 4; ff++) rs[ff] = cfma(f, v[ff * ne + ej], rs[ff]);
+      for (int u = 0; u < 8; u++)
+        if (j0 + u * parts < Nz) f[u] = F[i + (size_t)Nz * (j0 + u * parts) + n2 * q];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int jc = j0 + u * parts;
+        if (jc >= Nz) break;
+        const int ej = (jc / Nf) * nbox + jc % Nf + f_range * Nf;
+#pragma unroll
+        for (int ff = 0; ff < 4; ff++) rs[ff] = cfma(f[u], v[ff * ne + ej], rs[ff]);
+      }
     }
 #pragma unroll
     for (int ff = 0; ff < 4; ff++) {
@@ -240,27 +211,30 @@ __global__ void __launch_bounds__(256) k_sus(const cplx* __restrict__ F0, const 
 }
 
 // symmetrize_array (SRC/parquet_util.f90:1215-1272) for `narr` IBZ arrays of
-// nfreq frequencies: one thread per (array, frequency), reference loop order
-__global__ void k_symmetrize_batch(const cplx* __restrict__ in, cplx* __restrict__ out, const int* __restrict__ symlist,
-                                   const int* __restrict__ symq, int narr, int nfreq, int Nx, int Ny, int nxibz,
-                                   int NIBZ) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= narr * nfreq) return;
-  const int a = t / nfreq, nu = t % nfreq;
+// nfreq frequencies: a warp per (array, momentum) as k_symmetrize of the SDE
+__global__ void __launch_bounds__(128) k_symmetrize_batch(const cplx* __restrict__ in, cplx* __restrict__ out,
+                                                          const int* __restrict__ symlist,
+                                                          const int* __restrict__ symq, int narr, int nfreq, int Nx,
+                                                          int Ny, int NIBZ) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int nk = Nx * Ny;
+  if (t >= narr * nk) return;
+  const int a = t / nk, k = t % nk, kx = k / Ny + 1, ky = k % Ny + 1;
   const cplx* src = in + (size_t)a * NIBZ * nfreq;
-  cplx* dst = out + (size_t)a * Nx * Ny * nfreq;
-  for (int k = 0; k < Nx * Ny; k++) dst[(size_t)k * nfreq + nu] = cmk(0.0, 0.0);
-  int ip = 0;
-  for (int qx = 1; qx <= nxibz; qx++)
-    for (int qy = 1; qy <= qx; qy++, ip++) {
-      const cplx v = src[(size_t)ip * nfreq + nu];
-      for (int s = 0; s < NS; s++) {
-        if (!symlist[NS * ip + s]) continue;
-        const int sx = symq[2 * (NS * ip + s)], sy = symq[2 * (NS * ip + s) + 1];
-        const size_t o = ((size_t)(sx - 1) * Ny + sy - 1) * nfreq + nu;
-        dst[o] = cadd(dst[o], v);
+  cplx* dst = out + ((size_t)a * nk + k) * nfreq;
+  for (int nu0 = 0; nu0 < nfreq; nu0 += 32) {
+    const int nu = nu0 + lane;
+    cplx acc = cmk(0.0, 0.0);
+    for (int p0 = 0; p0 < NS * NIBZ; p0 += 32) {
+      const int p = p0 + lane;
+      const bool hit = p < NS * NIBZ && symlist[p] && symq[2 * p] == kx && symq[2 * p + 1] == ky;
+      for (unsigned m = __ballot_sync(0xffffffffu, hit); m; m &= m - 1) {
+        const int ip = (p0 + __ffs(m) - 1) / NS;
+        if (nu < nfreq) acc = cadd(acc, src[(size_t)ip * nfreq + nu]);
       }
     }
+    if (nu < nfreq) dst[nu] = acc;
+  }
 }
 
 int launch_readout(tups_ctx* ctx) {
@@ -277,8 +251,8 @@ int launch_readout(tups_ctx* ctx) {
   k_chi0_products<<<cdiv(ng, 256), 256, 0, ctx->stream>>>(ctx->s.Grt, rd.ffg, rd.prod, n1, n2, d.Nf);
   if ((rc = after_launch(ctx, "k_chi0_products"))) return rc;
   if ((rc = launch_fft2d_batch(ctx, rd.prod, rd.prod_ft, 10 * d.Nf, 0))) return rc;
-  k_spline_bosonic<<<dim3(d.NIBZ, 10), 64, 4 * (size_t)d.Nf * sizeof(double), ctx->stream>>>(
-      rd.prod_ft, ctx->t.ibz, rd.chi0, d.Nx, d.Ny, d.Ngrain, d.Nf, d.NIBZ, ctx->p.beta);
+  k_spline_bosonic<<<dim3(d.NIBZ, 10), 128, spline_smem(d.Nf), ctx->stream>>>(
+      rd.prod_ft, ctx->t.spline, ctx->t.ph_bose, ctx->t.ibz, rd.chi0, d.Nx, d.Ny, d.Ngrain, d.Nf, d.NIBZ, ctx->p.beta);
   if ((rc = after_launch(ctx, "k_spline_bosonic"))) return rc;
   // susceptibilities
   k_GG<<<dim3(d.Nb, d.nbox), 128, 2 * (size_t)d.Nc * sizeof(cplx), ctx->stream>>>(
@@ -295,11 +269,11 @@ int launch_readout(tups_ctx* ctx) {
   if ((rc = after_launch(ctx, "k_sus"))) return rc;
   // whole-BZ arrays: 16 sus (channel, ff) + 10 chi0 arrays
   const int nh = d.Nf / 2;
-  k_symmetrize_batch<<<cdiv(16 * nh, 64), 64, 0, ctx->stream>>>(rd.sus, rd.sus_bz, ctx->t.symlist, ctx->t.symq, 16,
-                                                                  nh, d.Nx, d.Ny, d.Nx_IBZ, d.NIBZ);
+  k_symmetrize_batch<<<cdiv(16 * d.Nc, 4), 128, 0, ctx->stream>>>(rd.sus, rd.sus_bz, ctx->t.symlist, ctx->t.symq, 16,
+                                                                   nh, d.Nx, d.Ny, d.NIBZ);
   if ((rc = after_launch(ctx, "k_symmetrize_batch"))) return rc;
-  k_symmetrize_batch<<<cdiv(10 * nh, 64), 64, 0, ctx->stream>>>(rd.chi0, rd.chi0_bz, ctx->t.symlist, ctx->t.symq, 10,
-                                                                  nh, d.Nx, d.Ny, d.Nx_IBZ, d.NIBZ);
+  k_symmetrize_batch<<<cdiv(10 * d.Nc, 4), 128, 0, ctx->stream>>>(rd.chi0, rd.chi0_bz, ctx->t.symlist, ctx->t.symq, 10,
+                                                                   nh, d.Nx, d.Ny, d.NIBZ);
   return after_launch(ctx, "k_symmetrize_batch");
 }
 

@@ -2,6 +2,7 @@
 // calc_LChi/PhChi/PPChi (:439-574), the Sigma_V accumulation (:116-221),
 // symmetrize_array (SRC/parquet_util.f90:1215-1272) and the U^2 term
 // calc_order_2nd (:264-338) with FDfit/nfourier (SRC/MATH_mod.f90:95-212).
+#include "spline.cuh"
 #include "tups_device.cuh"
 
 namespace tups {
@@ -40,8 +41,8 @@ __global__ void k_sde_chis(SdePtrs P, const cplx* __restrict__ cph, const cplx* 
   const int W = ibz[3 * q + 2];
   // Lambda contribution, only the l3 = l4 = 1 block
   cplx lc = cmk(0.0, 0.0);
-  if (i < Nf && threadIdx.y == 0) {
-    for (int j = 0; j < nbox; j++) {
+  if (i < Nf) {
+    for (int j = threadIdx.y; j < nbox; j += blockDim.y) {
       const int l40 = j - fr * Nf + 1;
       const cplx c = cph_q[j];
       if (l40 > 0 && l40 < Nf + 1) {
@@ -54,7 +55,7 @@ __global__ void k_sde_chis(SdePtrs P, const cplx* __restrict__ cph, const cplx* 
       }
     }
   }
-  // the (l4, j) columns are split over the 8 thread rows of the CTA
+  // the (l4, j) columns, and the box above, are split over the 8 thread rows of the CTA
   // (blockDim = 32 x 8): 8x the parallelism of one thread per row
   cplx ph = cmk(0.0, 0.0), pp = cmk(0.0, 0.0);
   const cplx* Pd = P.Phi[0] + n2 * q;
@@ -72,14 +73,17 @@ __global__ void k_sde_chis(SdePtrs P, const cplx* __restrict__ cph, const cplx* 
     pp = cfma(Ps[idx], b, pp);
     pp = cfma(Pt[idx], b, pp);
   }
-  __shared__ cplx red_ph[8][32], red_pp[8][32];
+  __shared__ cplx red_ph[8][32], red_pp[8][32], red_l[8][32];
   red_ph[threadIdx.y][threadIdx.x] = ph;
   red_pp[threadIdx.y][threadIdx.x] = pp;
+  red_l[threadIdx.y][threadIdx.x] = lc;
   __syncthreads();
   if (threadIdx.y != 0 || !active) return;
-  for (int y = 1; y < (int)blockDim.y; y++) {
+#pragma unroll
+  for (int y = 1; y < 8; y++) {
     ph = cadd(ph, red_ph[y][threadIdx.x]);
     pp = cadd(pp, red_pp[y][threadIdx.x]);
+    lc = cadd(lc, red_l[y][threadIdx.x]);
   }
   const size_t o = (size_t)q + (size_t)gridDim.y * i;  // gridDim.y = Nb
   LChi[o] = lc;
@@ -112,38 +116,41 @@ __global__ void __launch_bounds__(256) k_sde_sigma(const cplx* __restrict__ Gkw,
   const double mu = scal[S_MU];
   const int mkx = (Nx - kx) % Nx, mky = (Ny - ky) % Ny;
   double sre = 0.0, sim = 0.0;
-  for (int q = threadIdx.x; q < Nb; q += blockDim.x) {
+  // threads over (star image s, slot q), q fastest.  The form factors are real,
+  // so each image's sum over l3 is taken first and meets its Green's functions
+  // once
+  for (int t = threadIdx.x; t < NS * Nb; t += blockDim.x) {
+    const int s = t / Nb, q = t - s * Nb;
     // local slot q of this context is global slot slot0 + q
     const int w = ibz[3 * (slot0 + q) + 2];
     const int Qi = (slot0 + q) / nh;
+    if (!symlist[NS * Qi + s]) continue;
     // row i of slot q at q + Nb i
     const cplx* Lq = LChi + q;
     const cplx* Pq = PhChi + q;
     const cplx* Qq = PPChi + q;
-    cplx acc = cmk(0.0, 0.0);
-    for (int s = 0; s < NS; s++) {
-      if (!symlist[NS * Qi + s]) continue;
-      const int sx = symq[2 * (NS * Qi + s)] - 1, sy = symq[2 * (NS * Qi + s) + 1] - 1;
-      const int kqx = (kx + sx) % Nx, kqy = (ky + sy) % Ny;
-      const cplx gkq = get_green(Gkw, SigmaH, Ek, kqx, kqy, k0 + w - 1, Nx, Ny, Nf, beta, mu);
-      const int qmkx = (mkx + sx) % Nx, qmky = (mky + sy) % Ny, qmkw = (Nf + 1 - k0) + w - 1;
-      const cplx gqmk = get_green(Gkw, SigmaH, Ek, qmkx, qmky, qmkw, Nx, Ny, Nf, beta, mu);
-      const cplx gkmq =
-          get_green(Gkw, SigmaH, Ek, (Nx - qmkx) % Nx, (Ny - qmky) % Ny, -qmkw + Nf + 1, Nx, Ny, Nf, beta, mu);
-      for (int l3 = 0; l3 < Nl; l3++) {
-        const double ffi = FFinv[s + NS * (kx + Nx * (ky + Ny * l3))];
-        const size_t i3 = (size_t)Nb * (l3 * Nf + k0 - 1);
-        acc = cadd(acc, cscale(cmul(gkq, Lq[i3]), ffi));
-        acc = cadd(acc, cscale(cmul(gkq, Pq[i3]), ffi));
-        acc = cadd(acc, cscale(cmul(gqmk, Qq[i3]), ffi));
-        if (w == 1) continue;
-        const size_t i3m = (size_t)Nb * (l3 * Nf + Nf - k0);
-        const double fs = ffi * (double)signs[l3];
-        acc = cadd(acc, cscale(cmul(gkmq, cconj(Lq[i3m])), fs));
-        acc = cadd(acc, cscale(cmul(gkmq, cconj(Pq[i3m])), fs));
-        acc = cadd(acc, cscale(cmul(cconj(gkq), cconj(Qq[i3m])), fs));
-      }
+    const int sx = symq[2 * (NS * Qi + s)] - 1, sy = symq[2 * (NS * Qi + s) + 1] - 1;
+    const int kqx = (kx + sx) % Nx, kqy = (ky + sy) % Ny;
+    const cplx gkq = get_green(Gkw, SigmaH, Ek, kqx, kqy, k0 + w - 1, Nx, Ny, Nf, beta, mu);
+    const int qmkx = (mkx + sx) % Nx, qmky = (mky + sy) % Ny, qmkw = (Nf + 1 - k0) + w - 1;
+    const cplx gqmk = get_green(Gkw, SigmaH, Ek, qmkx, qmky, qmkw, Nx, Ny, Nf, beta, mu);
+    const cplx gkmq =
+        get_green(Gkw, SigmaH, Ek, (Nx - qmkx) % Nx, (Ny - qmky) % Ny, -qmkw + Nf + 1, Nx, Ny, Nf, beta, mu);
+    cplx a = cmk(0.0, 0.0), b = a, c = a, e = a;
+    for (int l3 = 0; l3 < Nl; l3++) {
+      const double ffi = FFinv[s + NS * (kx + Nx * (ky + Ny * l3))];
+      const size_t i3 = (size_t)Nb * (l3 * Nf + k0 - 1);
+      a = cadd(a, cscale(cadd(Lq[i3], Pq[i3]), ffi));
+      b = cadd(b, cscale(Qq[i3], ffi));
+      if (w == 1) continue;
+      const size_t i3m = (size_t)Nb * (l3 * Nf + Nf - k0);
+      const double fs = ffi * (double)signs[l3];
+      c = cadd(c, cscale(cadd(Lq[i3m], Pq[i3m]), fs));
+      e = cadd(e, cscale(Qq[i3m], fs));
     }
+    cplx acc = cfma(gqmk, b, cmul(gkq, a));
+    acc = cfma(gkmq, cconj(c), acc);
+    acc = cfma(cconj(gkq), cconj(e), acc);
     sre += acc.x;
     sim += acc.y;
   }
@@ -152,30 +159,33 @@ __global__ void __launch_bounds__(256) k_sde_sigma(const cplx* __restrict__ Gkw,
   if (threadIdx.x == 0) SigmaV[(size_t)ik * Nf + k0 - 1] = cmk(-pref * sre, -pref * sim);
 }
 
-// Sigma(BZ) from Sigma_V(IBZ) (symmetrize_array) plus the U^2 term; one
-// thread per frequency does the whole scatter for it, in the reference's order
-__global__ void k_symmetrize(const cplx* __restrict__ SigmaV, const cplx* __restrict__ order2,
-                             const int* __restrict__ ibz, const int* __restrict__ symlist, const int* __restrict__ symq,
-                             cplx* __restrict__ Sigma, int Nx, int Ny, int Nf, int nxibz, int use_U2) {
-  // one thread per output (k, nu): the sum, in the reference's (ip, s) loop
-  // order, of the IBZ values whose star images land on k (one per k on an
-  // even lattice), plus the U^2 term
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)Nx * Ny * Nf) return;
-  const int nu = (int)(e % Nf), k = (int)(e / Nf);
+// Sigma(BZ) from Sigma_V(IBZ) (symmetrize_array) plus the U^2 term.  A warp per
+// momentum k: its lanes test the (ip, s) pairs 32 at a time for the star images
+// that land on k (one per k on an even lattice), then run over the frequencies,
+// adding the IBZ values in the reference's (ip, s) order.
+__global__ void __launch_bounds__(128) k_symmetrize(const cplx* __restrict__ SigmaV, const cplx* __restrict__ order2,
+                                                    const int* __restrict__ symlist, const int* __restrict__ symq,
+                                                    cplx* __restrict__ Sigma, int Nx, int Ny, int Nf, int nibz,
+                                                    int use_U2) {
+  const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (k >= Nx * Ny) return;
   const int kx = k / Ny + 1, ky = k % Ny + 1;
-  cplx acc = cmk(0.0, 0.0);
-  int ip = 0;
-  for (int qx = 1; qx <= nxibz; qx++)
-    for (int qy = 1; qy <= qx; qy++, ip++)
-      for (int s = 0; s < NS; s++) {
-        if (!symlist[NS * ip + s]) continue;
-        if (symq[2 * (NS * ip + s)] == kx && symq[2 * (NS * ip + s) + 1] == ky)
-          acc = cadd(acc, SigmaV[(size_t)ip * Nf + nu]);
+  for (int nu0 = 0; nu0 < Nf; nu0 += 32) {
+    const int nu = nu0 + lane;
+    cplx acc = cmk(0.0, 0.0);
+    for (int p0 = 0; p0 < NS * nibz; p0 += 32) {
+      const int p = p0 + lane;
+      const bool hit = p < NS * nibz && symlist[p] && symq[2 * p] == kx && symq[2 * p + 1] == ky;
+      for (unsigned m = __ballot_sync(0xffffffffu, hit); m; m &= m - 1) {
+        const int ip = (p0 + __ffs(m) - 1) / NS;
+        if (nu < Nf) acc = cadd(acc, SigmaV[(size_t)ip * Nf + nu]);
       }
-  if (use_U2) acc = cadd(acc, order2[e]);
-  Sigma[e] = acc;
-  (void)ibz;
+    }
+    if (nu < Nf) {
+      const size_t e = (size_t)k * Nf + nu;
+      Sigma[e] = use_U2 ? cadd(acc, order2[e]) : acc;
+    }
+  }
 }
 
 // GGG(r, tau) = G(r,tau)^2 G(-r, beta-tau) U^2 (SRC/parquet_SDE.f90:297-305)
@@ -190,69 +200,29 @@ __global__ void k_ggg(const cplx* __restrict__ Grt, cplx* __restrict__ out, int 
 }
 
 // FDfit + nfourier (cubic spline with clamped end slopes, integrated exactly
-// against e^{i om tau}) for one k per CTA; writes order_2nd(k, nu).  Thread 0
-// solves the tridiagonal spline system, the others then sum over intervals.
-__global__ void k_nfourier(const cplx* __restrict__ GGG, cplx* __restrict__ order2, int Nx, int Ny, int Ng, int Nf,
-                           double beta) {
-  extern __shared__ double sp[];
-  double* r = sp;
-  double* qv = sp + Nf;
-  double* u = sp + 2 * Nf;
-  double* xm = sp + 3 * Nf;
+// against e^{i om tau}) for one k per CTA; writes order_2nd(k, nu).
+__global__ void __launch_bounds__(128) k_nfourier(const cplx* __restrict__ GGG, const double* __restrict__ tab,
+                                                  const cplx* __restrict__ ph, cplx* __restrict__ order2, int Nx, int Ny, int Ng, int Nf,
+                                                  double beta) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const SplineShared S = spline_bind(smraw, Nf);
   const int k = blockIdx.x;
   const int kx = k / Ny, ky = k % Ny;
   const int n1 = Nx * Ng, n2 = Ny * Ng;
   const int kxc = kx * Ng, kyc = ky * Ng;
-  const int L = Nf - 1;
-  const double delta = beta / L;
-  for (int t = threadIdx.x; t < Nf; t += blockDim.x) r[t] = GGG[kxc + (size_t)n1 * (kyc + (size_t)n2 * t)].x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double dt = beta / (Nf - 1);
-    // FDfit (SRC/MATH_mod.f90:95-107)
-    const double fd1 = (-25.0 * r[0] + 48.0 * r[1] - 36.0 * r[2] + 16.0 * r[3] - 3.0 * r[4]) / 12.0 / dt;
-    const double fd2 =
-        (25.0 * r[L] - 48.0 * r[L - 1] + 36.0 * r[L - 2] - 16.0 * r[L - 3] + 3.0 * r[L - 4]) / 12.0 / dt;
-    // spline second derivatives (SRC/MATH_mod.f90:140-168)
-    qv[0] = -0.5;
-    u[0] = (3.0 / delta) * ((r[1] - r[0]) / delta - fd1);
-    for (int kk = 2; kk <= L; kk++) {
-      const double p = qv[kk - 2] / 2.0 + 2.0;
-      qv[kk - 1] = -1.0 / 2.0 / p;
-      u[kk - 1] = 3.0 / (delta * delta) * (r[kk] + r[kk - 2] - 2.0 * r[kk - 1]);
-      u[kk - 1] = (u[kk - 1] - u[kk - 2] / 2.0) / p;
-    }
-    qv[L] = 0.5;
-    u[L] = (3.0 / delta) * (fd2 - (r[L] - r[L - 1]) / delta);
-    xm[L] = (u[L] - qv[L] * u[L - 1]) / (qv[L] * qv[L - 1] + 1.0);
-    for (int kk = L; kk >= 1; kk--) xm[kk - 1] = qv[kk - 1] * xm[kk] + u[kk - 1];
-  }
-  __syncthreads();
+  for (int t = threadIdx.x; t < Nf; t += blockDim.x) S.r[t] = GGG[kxc + (size_t)n1 * (kyc + (size_t)n2 * t)].x;
+  spline_fit(S, tab, Nf, beta);
   const size_t base = (size_t)k * Nf;
-  for (int i = threadIdx.x + 1; i <= Nf / 2; i += blockDim.x) {
-    const double om = (2.0 * i - 1.0) * M_PI / beta;
-    const double om2 = om * om, om3 = om2 * om, om4 = om3 * om;
-    double cr = 0.0, ci = 0.0;
-    for (int j = 1; j <= L; j++) {
-      const double a = r[j - 1], c = xm[j - 1] / 2.0;
-      const double b = (r[j] - r[j - 1]) / delta - (2.0 * xm[j - 1] + xm[j]) * delta / 6.0;
-      const double d = (xm[j] - xm[j - 1]) / (6.0 * delta);
-      double sp1, cp1, sm1, cm1;
-      sincos(om * delta * j, &sp1, &cp1);
-      sincos(om * delta * (j - 1), &sm1, &cm1);
-      // explus*(p1r + i p1i) + ex*(p2r + i p2i), SRC/MATH_mod.f90:200-207
-      const double p1r = (-6.0 * d) / om4 + (b + 2.0 * delta * c + 3.0 * delta * delta * d) / om2;
-      const double p1i =
-          (2.0 * c + 6.0 * delta * d) / om3 + (-a - delta * b - delta * delta * c - delta * delta * delta * d) / om;
-      const double p2r = 6.0 * d / om4 - b / om2;
-      const double p2i = -2.0 * c / om3 + a / om;
-      cr += cp1 * p1r - sp1 * p1i + cm1 * p2r - sm1 * p2i;
-      ci += cp1 * p1i + sp1 * p1r + cm1 * p2i + sm1 * p2r;
-    }
+  const int groups = blockDim.x / kSplineLanes;
+  for (int i0 = 1; i0 <= Nf / 2; i0 += groups) {
+    const int i = i0 + threadIdx.x / kSplineLanes;
+    const int ic = min(i, Nf / 2);
+    const cplx c = spline_transform(S, (2.0 * ic - 1.0) * M_PI / beta, ph + (size_t)Nf * (ic - 1), Nf, beta);
+    if (threadIdx.x % kSplineLanes || i > Nf / 2) continue;
     // SRC/parquet_SDE.f90:325-330
     const int nu = Nf / 2 + 1 - i;
-    order2[base + nu - 1] = cmk(cr, -ci);
-    order2[base + Nf - nu] = cmk(cr, ci);
+    order2[base + nu - 1] = cmk(c.x, -c.y);
+    order2[base + Nf - nu] = c;
   }
 }
 
@@ -288,13 +258,12 @@ int launch_sde(tups_ctx* ctx) {
     k_ggg<<<cdiv(n, 256), 256, 0, ctx->stream>>>(ctx->s.Grt, ctx->s.Grt_work, n1, n2, d.Nf, ctx->p.U);
     if ((rc = after_launch(ctx, "k_ggg"))) return rc;
     if ((rc = launch_fft2d(ctx, ctx->s.Grt_work, ctx->s.GGG, 0))) return rc;
-    k_nfourier<<<d.Nc, 64, 4 * (size_t)d.Nf * sizeof(double), ctx->stream>>>(ctx->s.GGG, ctx->s.order2, d.Nx, d.Ny,
-                                                                            d.Ngrain, d.Nf, ctx->p.beta);
+    k_nfourier<<<d.Nc, 128, spline_smem(d.Nf), ctx->stream>>>(ctx->s.GGG, ctx->t.spline, ctx->t.ph_fermi, ctx->s.order2,
+                                                              d.Nx, d.Ny, d.Ngrain, d.Nf, ctx->p.beta);
     if ((rc = after_launch(ctx, "k_nfourier"))) return rc;
   }
-  k_symmetrize<<<cdiv((long long)d.Nc * d.Nf, 128), 128, 0, ctx->stream>>>(ctx->s.SigmaV, ctx->s.order2, ctx->t.ibz, ctx->t.symlist,
-                                                       ctx->t.symq, ctx->s.Sigma, d.Nx, d.Ny, d.Nf, d.Nx_IBZ,
-                                                       ctx->p.use_U2);
+  k_symmetrize<<<cdiv(d.Nc, 4), 128, 0, ctx->stream>>>(ctx->s.SigmaV, ctx->s.order2, ctx->t.symlist, ctx->t.symq,
+                                                       ctx->s.Sigma, d.Nx, d.Ny, d.Nf, d.NIBZ, ctx->p.use_U2);
   return after_launch(ctx, "k_symmetrize");
 }
 

@@ -655,6 +655,30 @@ static int upload_tables(tups_ctx* ctx) {
     }
     TRY(upload(ctx, &t.tw_tau, tw));
   }
+  // multipliers of the spline's tridiagonal elimination (SRC/MATH_mod.f90:140-155)
+  {
+    std::vector<double> tab((size_t)2 * Nf, 0.0);
+    tab[0] = -0.5;
+    for (int k = 1; k < Nf; k++) {
+      const double p = tab[k - 1] / 2.0 + 2.0;
+      tab[k] = -1.0 / 2.0 / p;
+      tab[Nf + k] = 1.0 / p;
+    }
+    TRY(upload(ctx, &t.spline, tab));
+    // its phases at the interval ends, rounded as om * delta * j
+    const double delta = ctx->p.beta / (Nf - 1);
+    for (int bose = 0; bose < 2; bose++) {
+      std::vector<cplx> ph((size_t)Nf * (Nf / 2));
+      for (int i = 0; i < Nf / 2; i++) {
+        const double om = bose ? 2.0 * i * M_PI / ctx->p.beta : (2.0 * (i + 1) - 1.0) * M_PI / ctx->p.beta;
+        for (int j = 0; j < Nf; j++) {
+          const double a = om * delta * j;
+          ph[j + (size_t)Nf * i] = make_double2(std::cos(a), std::sin(a));
+        }
+      }
+      TRY(upload(ctx, bose ? &t.ph_bose : &t.ph_fermi, ph));
+    }
+  }
   for (int dim = 0; dim < 2; dim++) {
     int n = (dim == 0 ? Nx : Ny) * Ng;
     std::vector<cplx> tw(n);

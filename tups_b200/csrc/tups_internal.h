@@ -33,6 +33,9 @@ struct DeviceTables {
   cplx* expSqR = nullptr;     // (NIBZ, NR, 8)
   cplx* expqSR = nullptr;     // (Nc, NR, 8), k index (ky-1)*Nx+kx
   cplx* tw_tau = nullptr;     // (Nf tau, Nf nu) e^{-i nu_n tau_i}
+  double* spline = nullptr;   // elimination of the clamped spline: [q | 1/p], Nf each
+  cplx* ph_fermi = nullptr;   // (Nf tau, Nf/2): e^{i om tau}, om = (2i - 1) pi / beta
+  cplx* ph_bose = nullptr;    // the same for om = 2 w pi / beta
   cplx* tw_x = nullptr;       // (Nx*Ng) e^{-2 pi i m / n1}
   cplx* tw_y = nullptr;       // (Ny*Ng)
   int4* pae_elems = nullptr;  // crossing: elements per (pair, family, W), see pae.cu
@@ -252,10 +255,9 @@ int cuda_check(tups_ctx* ctx, cudaError_t e, const char* what);
 int after_launch(tups_ctx* ctx, const char* name);
 
 // kernel drivers (each returns TUPS_OK or an error code)
-int launch_sigma_hartree(tups_ctx* ctx);
 int launch_bisection(tups_ctx* ctx, int cal_chi, int max_steps);
-int launch_grt(tups_ctx* ctx);
-int launch_gkw(tups_ctx* ctx);
+// G(r, tau), G(k, nu) and Sigma_H for the mu of launch_bisection
+int launch_green(tups_ctx* ctx);
 int launch_chi(tups_ctx* ctx, int q_begin, int q_count);
 int launch_bse_chunk(tups_ctx* ctx, int q_begin, int q_count);
 // slices the next BSE call will use (0 = FP64), see bse.cu

@@ -35,10 +35,10 @@ namespace {
 using tups::cplx;
 using tups::cmk;
 using tups::lud::dmma8;
+using tups::lud::kInvLd;
 using tups::lud::kPanelCols;
 using tups::lud::kPanelRows;
 using tups::lud::kPanelThreads;
-using tups::lud::PanelShared;
 
 constexpr int kLuMaxInst = 16384;
 constexpr int NB = 2 * kPanelCols;  // 64
@@ -115,97 +115,11 @@ __global__ void __launch_bounds__(256) k_lu_form(const cplx* __restrict__ Gam, c
 }
 
 // ---- one block of 64 columns ------------------------------------------------------
-constexpr int kInvLd = NB + 1;
-
 struct LuPanelShared {
-  PanelShared p;
-  int orig[kPanelRows];  // where a row's content stood before the block
+  tups::lud::BlockShared b;
   int moved;
   int row[2 * NB], cur[2 * NB];  // replay of the interchanges (tall blocks)
-  union {
-    tups::lud::HalfShared half;
-    struct {
-      cplx M[NB * kInvLd], T[kPanelCols * kPanelCols];  // [col][row]
-    };
-  };
 };
-
-// M <- M^{-1}, a 64 x 64 triangle (unit lower, or UP: upper) in shared memory
-// with the pitch kInvLd: 16 x 16 diagonal blocks by substitution, one thread
-// per column, then merged pairwise, inv([X 0; Y Z]) = [X' 0; -Z' Y X' Z'] and
-// its mirror.  A zero pivot divides by one (its instance is reported
-// singular).  T: 1024 complex of scratch.  At least 64 threads.
-template <bool UP>
-__device__ void invert_triangle(cplx* __restrict__ M, cplx* __restrict__ T) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid < 64) {
-    const int b = tid & 48, c = tid & 15;
-    const cplx* D = M + b * kInvLd + b;
-    cplx x[16];
-#pragma unroll
-    for (int r = 0; r < 16; r++) x[r] = cmk(r == c ? 1.0 : 0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const int k = UP ? 15 - i : i;
-      if (UP) {
-        const cplx u = D[k * kInvLd + k];
-        if (u.x != 0.0 || u.y != 0.0) x[k] = tups::cmul(x[k], tups::lud::crecip1(u));
-      }
-#pragma unroll
-      for (int r = 0; r < 16; r++)
-        if (UP ? r < k : r > k) x[r] = tups::lud::cfnma(D[k * kInvLd + r], x[k], x[r]);
-    }
-    __syncwarp();  // a 16-column block belongs to half a warp
-#pragma unroll
-    for (int r = 0; r < 16; r++) M[(b + c) * kInvLd + b + r] = x[r];
-  }
-  __syncthreads();
-  for (int s = 16; s < NB; s *= 2) {
-    const int s2 = s * s, per = NB / (2 * s) * s2;
-    for (int e = tid; e < per; e += nt) {  // T = Y X' (lower) or Y Z' (upper)
-      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
-      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
-      cplx a0 = cmk(0.0, 0.0), a1 = a0;
-      for (int k = 0; k < s; k += 2) {
-        a0 = tups::cfma(M[(x0 + k) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k], a0);
-        a1 = tups::cfma(M[(x0 + k + 1) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k + 1], a1);
-      }
-      T[e] = tups::cadd(a0, a1);  // [pair][c][r]
-    }
-    __syncthreads();
-    for (int e = tid; e < per; e += nt) {  // Y = -Z' T or -X' T
-      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
-      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;
-      const cplx* t = T + (e - r);
-      cplx a0 = cmk(0.0, 0.0), a1 = a0;
-      for (int k = 0; k < s; k += 2) {
-        a0 = tups::lud::cfnma(M[(y0 + k) * kInvLd + y0 + r], t[k], a0);
-        a1 = tups::lud::cfnma(M[(y0 + k + 1) * kInvLd + y0 + r], t[k + 1], a1);
-      }
-      M[(x0 + c) * kInvLd + y0 + r] = tups::cadd(a0, a1);
-    }
-    __syncthreads();
-  }
-}
-
-// the triangle of the diagonal block at (j0, j0), identity past jb, into M
-template <bool UP>
-__device__ void load_triangle(const cplx* __restrict__ A, int n, int j0, int jb, cplx* __restrict__ M) {
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int r = e % NB, c = e / NB;
-    const bool in = r < jb && c < jb && (UP ? r <= c : r > c);
-    M[c * kInvLd + r] = in ? A[j0 + r + (size_t)n * (j0 + c)] : cmk(r == c ? 1.0 : 0.0, 0.0);
-  }
-  __syncthreads();
-}
-
-template <bool UP>
-__device__ void store_triangle(cplx* __restrict__ A, int n, int j0, int jb, const cplx* __restrict__ M) {
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int r = e % NB, c = e / NB;
-    if (r < jb && c < jb && (UP ? r <= c : r > c)) A[j0 + r + (size_t)n * (j0 + c)] = M[c * kInvLd + r];
-  }
-}
 
 // Columns [j0, j0 + 64) of every instance (one CTA each): two 32-column panels
 // with a 32-wide update between them, the interchange map, and the unit lower
@@ -224,30 +138,23 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_lu_panel(cplx* __restrict_
   cplx* A = Aw + d.g_off;
   int* ipiv = piv_all + d.p_off;
   LuMap& map = g_lu_map[inst];
-  for (int i = tid; i < kPanelRows; i += kPanelThreads) S.p.loc[i] = S.orig[i] = i;
+  for (int i = tid; i < kPanelRows; i += kPanelThreads) S.b.orig[i] = i;
   if (tid == 0) S.moved = 0;
   __syncthreads();
   auto track = [&](int c, int p) {
     if (RPT > 0) {
-      const int x = S.orig[c - j0];
-      S.orig[c - j0] = S.orig[p - j0];
-      S.orig[p - j0] = x;
+      const int x = S.b.orig[c - j0];
+      S.b.orig[c - j0] = S.b.orig[p - j0];
+      S.b.orig[p - j0] = x;
     }
   };
-  for (int h0 = j0; h0 < je; h0 += kPanelCols) {
-    const int kb = min(kPanelCols, je - h0);
-    if (h0 > j0) tups::lud::panel_half(A, n, j0, kb, S.half);
-    if constexpr (RPT > 0)
-      tups::lud::panel_factor<RPT>(A, n, h0, kb, j0, je, ipiv, &g_lu_status[inst], S.p, track);
-    else
-      tups::lud::panel_factor_global(A, n, h0, kb, j0, je, ipiv, &g_lu_status[inst], S.p, track);
-  }
+  tups::lud::block_factor<RPT, NB>(A, n, j0, jb, j0, je, ipiv, &g_lu_status[inst], S.b, track);
   // the interchange map: block rows take src, the rows below that changed take
   // a block row (an interchange always involves the block)
   if (RPT > 0) {
-    if (tid < NB) map.src[tid] = tid < jb ? j0 + S.orig[tid] : 0;
+    if (tid < NB) map.src[tid] = tid < jb ? j0 + S.b.orig[tid] : 0;
     for (int i = jb + tid; i < n - j0; i += kPanelThreads)
-      if (S.orig[i] != i) map.moved[atomicAdd(&S.moved, 1)] = (j0 + i) << 6 | S.orig[i];
+      if (S.b.orig[i] != i) map.moved[atomicAdd(&S.moved, 1)] = (j0 + i) << 6 | S.b.orig[i];
   } else if (tid == 0) {
     int cnt = jb;
     for (int k = 0; k < jb; k++) {
@@ -274,9 +181,6 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_lu_panel(cplx* __restrict_
   }
   __syncthreads();
   if (tid == 0) map.count = S.moved;
-  load_triangle<false>(A, n, j0, jb, S.M);
-  invert_triangle<false>(S.M, S.T);
-  store_triangle<false>(A, n, j0, jb, S.M);
 }
 
 // U_bb^{-1} over U_bb for every diagonal block of every instance, off the
@@ -288,9 +192,9 @@ __global__ void __launch_bounds__(256) k_lu_invert(cplx* __restrict__ Aw) {
   const int n = d.n, j0 = blockIdx.x * NB, jb = min(NB, n - j0);
   if (j0 >= n) return;
   cplx* A = Aw + d.g_off;
-  load_triangle<true>(A, n, j0, jb, M);
-  invert_triangle<true>(M, M + NB * kInvLd);
-  store_triangle<true>(A, n, j0, jb, M);
+  tups::lud::load_triangle<true>(A, n, j0, jb, M);
+  tups::lud::invert_triangle<true>(M, M + NB * kInvLd);
+  tups::lud::store_triangle<true>(A, n, j0, jb, M);
 }
 constexpr size_t kInvertSmem = ((size_t)NB * kInvLd + kPanelCols * kPanelCols) * sizeof(cplx);
 

@@ -1,14 +1,12 @@
 // Device pieces shared by the batched LU kernels (lu.cu, lu_split.cu):
-// complex 1-norm for pivoting, the rank-K (K <= 32) update on the FP64
-// tensor cores and the factorisation of one 32-column panel by one CTA.
+// the factorisation of a block of 64 columns by one CTA as two 32-column
+// panels, and the inversion of its 64 x 64 triangles.
 #pragma once
 
 #include "tups_device.cuh"
 
 namespace tups {
 namespace lud {
-
-constexpr int kRankMaxK = 32;
 
 static __device__ __forceinline__ double cabs1(cplx a) { return fabs(a.x) + fabs(a.y); }
 
@@ -18,62 +16,6 @@ static __device__ __forceinline__ void dmma8(double* c, const double* a, const d
       "{%0,%1,%2,%3};\n"
       : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
-// C[m x p] -= A[m x K] B[K x p], K <= 32, column-major with leading dim ld
-// (all three inside the same n x n matrix or RHS block).  Warp tiles of
-// 16 x 32 on the FP64 tensor cores, fragments straight from global memory.
-static __device__ void rank_update(cplx* C, const cplx* A, const cplx* B, int m, int p, int K, int ldc, int lda,
-                                   int ldb) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int gid = lane >> 2, tig = lane & 3;
-  const int tm = (m + 15) / 16, tp = (p + 31) / 32;
-  for (int t = warp; t < tm * tp; t += nwarps) {
-    const int r0 = (t % tm) * 16, c0 = (t / tm) * 32;
-    double cre[4][4], cim[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        const int r = r0 + gid + (x >= 2 ? 8 : 0), c = c0 + j * 8 + 2 * tig + (x & 1);
-        cplx v = (r < m && c < p) ? C[r + (size_t)ldc * c] : cmk(0.0, 0.0);
-        cre[j][x] = v.x;
-        cim[j][x] = v.y;
-      }
-#pragma unroll
-    for (int k8 = 0; k8 < kRankMaxK; k8 += 8) {
-      if (k8 >= K) break;
-      double are[4], aim[4], apos[4];
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        const int r = r0 + gid + (x & 1 ? 8 : 0), k = k8 + tig + (x >= 2 ? 4 : 0);
-        cplx v = (r < m && k < K) ? A[r + (size_t)lda * k] : cmk(0.0, 0.0);
-        // C -= A B  ==  C += (-A) B
-        are[x] = -v.x;
-        aim[x] = -v.y;
-        apos[x] = v.y;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int c = c0 + j * 8 + gid;
-        const int k0 = k8 + tig, k1 = k8 + tig + 4;
-        cplx w0 = (c < p && k0 < K) ? B[k0 + (size_t)ldb * c] : cmk(0.0, 0.0);
-        cplx w1 = (c < p && k1 < K) ? B[k1 + (size_t)ldb * c] : cmk(0.0, 0.0);
-        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y};
-        dmma8(cre[j], are, bre);   // -Are Bre
-        dmma8(cre[j], apos, bim);  // +Aim Bim
-        dmma8(cim[j], are, bim);   // -Are Bim
-        dmma8(cim[j], aim, bre);   // -Aim Bre
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        const int r = r0 + gid + (x >= 2 ? 8 : 0), c = c0 + j * 8 + 2 * tig + (x & 1);
-        if (r < m && c < p) C[r + (size_t)ldc * c] = cmk(cre[j][x], cim[j][x]);
-      }
-  }
 }
 
 // ---- factorisation of one panel of up to 32 columns by one CTA -----------------
@@ -136,7 +78,7 @@ static __device__ __forceinline__ void warp_argmax(unsigned& hi, unsigned& lo, i
 // c.  Interchanges are applied to the columns [ca, cb) of the enclosing block
 // and, through track(c, p), recorded by the caller.  n - h0 <= RPT * 512.
 // `loc` holds the identity on entry and on return.
-template <int RPT, class Track>
+template <int RPT, int COLS, class Track>
 static __device__ void panel_factor(cplx* __restrict__ A, int n, int h0, int kb, int ca, int cb, int* __restrict__ ipiv,
                                     int* __restrict__ status, PanelShared& S, Track track) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -276,7 +218,7 @@ static __device__ void panel_factor(cplx* __restrict__ A, int n, int h0, int kb,
     // and their pivots, each from where its content stood (a row named twice
     // gets the same value twice)
     const int ncol = cb - ca - w;
-    constexpr int kMove = 2 * kPanelSub, kMaxMove = kMove * (2 * kPanelCols) / kPanelThreads;
+    constexpr int kMove = 2 * kPanelSub, kMaxMove = (kMove * COLS + kPanelThreads - 1) / kPanelThreads;
     cplx v[kMaxMove];
     const int ms = tid % kMove, mk = ms % kPanelSub;  // this thread's row of the exchange
     const int mdst = mk >= w ? h0 : ms < kPanelSub ? jj + mk : S.piv[mk];
@@ -447,6 +389,121 @@ static __device__ void panel_factor_global(cplx* __restrict__ A, int n, int h0, 
     }
     __syncthreads();
   }
+}
+
+// ---- one block of 64 columns by one CTA ------------------------------------------
+constexpr int kBlock = 2 * kPanelCols, kInvLd = kBlock + 1;
+
+struct BlockShared {
+  PanelShared p;
+  int orig[kPanelRows];  // where a row's content stood before the block
+  union {
+    HalfShared half;
+    struct {
+      cplx M[kBlock * kInvLd], T[kPanelCols * kPanelCols];  // [col][row]
+    };
+  };
+};
+
+// M <- M^{-1}, a 64 x 64 triangle (unit lower, or UP: upper) in shared memory
+// with the pitch kInvLd: 16 x 16 diagonal blocks by substitution, one thread
+// per column, then merged pairwise, inv([X 0; Y Z]) = [X' 0; -Z' Y X' Z'] and
+// its mirror.  A zero pivot divides by one (its instance is reported
+// singular).  T: 1024 complex of scratch.  At least 64 threads.
+template <bool UP>
+static __device__ void invert_triangle(cplx* __restrict__ M, cplx* __restrict__ T) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  if (tid < 64) {
+    const int b = tid & 48, c = tid & 15;
+    const cplx* D = M + b * kInvLd + b;
+    cplx x[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) x[r] = cmk(r == c ? 1.0 : 0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int k = UP ? 15 - i : i;
+      if (UP) {
+        const cplx u = D[k * kInvLd + k];
+        if (u.x != 0.0 || u.y != 0.0) x[k] = cmul(x[k], crecip1(u));
+      }
+#pragma unroll
+      for (int r = 0; r < 16; r++)
+        if (UP ? r < k : r > k) x[r] = cfnma(D[k * kInvLd + r], x[k], x[r]);
+    }
+    __syncwarp();  // a 16-column block belongs to half a warp
+#pragma unroll
+    for (int r = 0; r < 16; r++) M[(b + c) * kInvLd + b + r] = x[r];
+  }
+  __syncthreads();
+  for (int s = 16; s < kBlock; s *= 2) {
+    const int s2 = s * s, per = kBlock / (2 * s) * s2;
+    for (int e = tid; e < per; e += nt) {  // T = Y X' (lower) or Y Z' (upper)
+      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
+      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
+      cplx a0 = cmk(0.0, 0.0), a1 = a0;
+      for (int k = 0; k < s; k += 2) {
+        a0 = cfma(M[(x0 + k) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k], a0);
+        a1 = cfma(M[(x0 + k + 1) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k + 1], a1);
+      }
+      T[e] = cadd(a0, a1);  // [pair][c][r]
+    }
+    __syncthreads();
+    for (int e = tid; e < per; e += nt) {  // Y = -Z' T or -X' T
+      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
+      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;
+      const cplx* t = T + (e - r);
+      cplx a0 = cmk(0.0, 0.0), a1 = a0;
+      for (int k = 0; k < s; k += 2) {
+        a0 = cfnma(M[(y0 + k) * kInvLd + y0 + r], t[k], a0);
+        a1 = cfnma(M[(y0 + k + 1) * kInvLd + y0 + r], t[k + 1], a1);
+      }
+      M[(x0 + c) * kInvLd + y0 + r] = cadd(a0, a1);
+    }
+    __syncthreads();
+  }
+}
+
+// the triangle of the diagonal block at (j0, j0), identity past jb, into M
+template <bool UP>
+static __device__ void load_triangle(const cplx* __restrict__ A, int n, int j0, int jb, cplx* __restrict__ M) {
+  for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
+    const int r = e % kBlock, c = e / kBlock;
+    const bool in = r < jb && c < jb && (UP ? r <= c : r > c);
+    M[c * kInvLd + r] = in ? A[j0 + r + (size_t)n * (j0 + c)] : cmk(r == c ? 1.0 : 0.0, 0.0);
+  }
+  __syncthreads();
+}
+
+template <bool UP>
+static __device__ void store_triangle(cplx* __restrict__ A, int n, int j0, int jb, const cplx* __restrict__ M) {
+  for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
+    const int r = e % kBlock, c = e / kBlock;
+    if (r < jb && c < jb && (UP ? r <= c : r > c)) A[j0 + r + (size_t)n * (j0 + c)] = M[c * kInvLd + r];
+  }
+}
+
+
+// Columns [j0, j0 + jb), jb <= 64, rows j0 .. n-1: two 32-column panels with a
+// 32-wide update between them, then the unit lower diagonal factor replaced by
+// its inverse (nothing later needs the factor).  RPT: rows per thread in
+// registers, 0 = columns in global memory.  Interchanges as panel_factor's.
+// Ends with a barrier.
+template <int RPT, int COLS, class Track>
+static __device__ void block_factor(cplx* __restrict__ A, int n, int j0, int jb, int ca, int cb, int* __restrict__ ipiv,
+                                    int* __restrict__ status, BlockShared& S, Track track) {
+  const int je = j0 + jb;
+  for (int i = threadIdx.x; i < kPanelRows; i += kPanelThreads) S.p.loc[i] = i;
+  __syncthreads();
+  for (int h0 = j0; h0 < je; h0 += kPanelCols) {
+    const int kb = min(kPanelCols, je - h0);
+    if (h0 > j0) panel_half(A, n, j0, kb, S.half);
+    if constexpr (RPT > 0) panel_factor<RPT, COLS>(A, n, h0, kb, ca, cb, ipiv, status, S.p, track);
+    else panel_factor_global(A, n, h0, kb, ca, cb, ipiv, status, S.p, track);
+  }
+  load_triangle<false>(A, n, j0, jb, S.M);
+  invert_triangle<false>(S.M, S.T);
+  store_triangle<false>(A, n, j0, jb, S.M);
+  __syncthreads();
 }
 
 }  // namespace lud

@@ -8,14 +8,14 @@
 // contiguous buffers:
 //  * A = I - c Gamma chi (chi block-diagonal in nu, n^2 Nl per instance).
 //  * Blocked right-looking LU with partial pivoting, blocks of 128 columns.
-//    The panel (all rows, 128 columns) is factored in FP64 by one CTA per
-//    instance, in sub-panels of 32 with the sub-panel updates on the FP64
-//    tensor cores; the trailing update A22 -= L21 U12 (K = 128) runs on the
-//    int8 tensor cores as an Ozaki split GEMM with s slices (ozaki.cu), so
-//    the factors are those of a matrix within about 10^(1.1-2s) of A.
-//  * X = U^{-1} L^{-1} P Gamma: 128-row diagonal blocks in FP64 (sub-blocks
-//    of 32 plus FP64 tensor-core updates), the off-diagonal updates on the
-//    int8 path.
+//    The block is factored in FP64 as two panels of 64 columns, one CTA per
+//    instance each (lu_device.cuh), with the second panel's update over 32 x 32
+//    tiles between them; the trailing update A22 -= L21 U12 (K = 128) runs on
+//    the int8 tensor cores as an Ozaki split GEMM with s slices (ozaki.cu),
+//    so the factors are those of a matrix within about 10^(1.1-2s) of A.
+//  * X = U^{-1} L^{-1} P Gamma: 128-row diagonal blocks in FP64 through the
+//    inverses of their 64 x 64 triangles (FP64 tensor cores), the off-diagonal
+//    updates on the int8 path.
 //  * Refinement: R = Gamma - A X = Gamma - X + c Gamma (chi X) in FP64 (the
 //    GEMM on the FP64 tensor cores, three real products per complex one);
 //    stop when max|R| <= tol max|Gamma| for every instance of the group (or
@@ -32,15 +32,12 @@
 
 #include "lu_device.cuh"
 #include "tups_device.cuh"
+#include "zgemm_tile.cuh"
 
 namespace tups {
 namespace {
 
-using lud::cabs1;
-using lud::rank_update;
-
 constexpr int LS_NB = 128;      // block of the split-precision updates
-constexpr int LS_SUB = 32;      // inner block of the FP64 work
 constexpr int LS_THREADS = 256;
 constexpr int LS_EPI_SUB = 2;   // OzRun::epi: C -= A B
 
@@ -68,12 +65,11 @@ __device__ double block_max(double v) {
   return m;
 }
 
-// Gg = Xg = Gamma_i, Ag = I - c Gamma_i chi_i (sums over l1 ascending, as the
+// Gg = Gamma_i, Ag = I - c Gamma_i chi_i (sums over l1 ascending, as the
 // FP64 LU form in lu.cu)
 __global__ void __launch_bounds__(LS_THREADS) k_ls_form(const LsDesc* __restrict__ desc, const cplx* __restrict__ gamma,
                                                         const cplx* __restrict__ chi_all, cplx* __restrict__ Gg,
-                                                        cplx* __restrict__ Xg, cplx* __restrict__ Ag,
-                                                        unsigned long long* gmax, int n) {
+                                                        cplx* __restrict__ Ag, unsigned long long* gmax, int n) {
   const int i = blockIdx.y;
   const LsDesc d = desc[i];
   const int nl = d.nl, nf = n / nl;
@@ -88,7 +84,6 @@ __global__ void __launch_bounds__(LS_THREADS) k_ls_form(const LsDesc* __restrict
     for (int l1 = 0; l1 < nl; l1++) acc = cfma(G[row + (size_t)n * (l1 * nf + nu)], chi[l1 + nl * (l2 + (size_t)nl * nu)], acc);
     const cplx g = G[e];
     Gg[n2 * i + e] = g;
-    Xg[n2 * i + e] = g;
     Ag[n2 * i + e] = cmk((row == col ? 1.0 : 0.0) - d.scale * acc.x, -d.scale * acc.y);
     mx = fmax(mx, fmax(fabs(g.x), fabs(g.y)));
   }
@@ -96,242 +91,287 @@ __global__ void __launch_bounds__(LS_THREADS) k_ls_form(const LsDesc* __restrict
   if (threadIdx.x == 0) atomic_max_nonneg(&gmax[i], mx);
 }
 
-// one column b[0:kb] = L^{-1} b (L unit lower, kb <= 32) with the column in
-// registers: b[r] -= L[r, k] b[k] for k < r in ascending order
-__device__ __forceinline__ void col_lower(const cplx* __restrict__ L, int ldl, cplx* b, int kb) {
-  cplx v[LS_SUB];
-#pragma unroll
-  for (int r = 0; r < LS_SUB; r++) v[r] = r < kb ? b[r] : cmk(0.0, 0.0);
-#pragma unroll
-  for (int r = 1; r < LS_SUB; r++) {
-    if (r < kb) {
-      cplx acc = v[r];
-#pragma unroll
-      for (int k = 0; k < r; k++) acc = csub(acc, cmul(L[r + (size_t)ldl * k], v[k]));
-      v[r] = acc;
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < LS_SUB; r++)
-    if (r < kb) b[r] = v[r];
-}
+// ---- 128-column block ------------------------------------------------------------
+using lud::BlockShared;
+using lud::kBlock;
+using lud::kInvLd;
+using lud::kPanelRows;
+using lud::kPanelThreads;
 
-// one column b[0:kb] = U^{-1} b (U upper with its diagonal, kb <= 32)
-__device__ __forceinline__ void col_upper(const cplx* __restrict__ U, int ldu, cplx* b, int kb) {
-  cplx v[LS_SUB];
-#pragma unroll
-  for (int r = 0; r < LS_SUB; r++) v[r] = r < kb ? b[r] : cmk(0.0, 0.0);
-#pragma unroll
-  for (int r = LS_SUB - 1; r >= 0; r--) {
-    if (r < kb) {
-      cplx acc = v[r];
-#pragma unroll
-      for (int k = r + 1; k < LS_SUB; k++)
-        if (k < kb) acc = csub(acc, cmul(U[r + (size_t)ldu * k], v[k]));
-      const cplx u = U[r + (size_t)ldu * r];
-      v[r] = (u.x == 0.0 && u.y == 0.0) ? acc : cmul(acc, crecip(u));
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < LS_SUB; r++)
-    if (r < kb) b[r] = v[r];
-}
+struct LsPanelShared {
+  BlockShared b;
+  cplx x[32 * (kBlock + 4)];  // [column][row]: columns of the block right of the panel
+};
 
-// Panel [j0, j0 + jb) of every instance of the group (one CTA each): partial
-// pivoting LU of rows j0..n-1 in sub-panels of 32, within the panel's columns
-// (k_ls_rows applies its interchanges to the other columns and forms U12).
-__global__ void __launch_bounds__(LS_THREADS) k_ls_panel(cplx* __restrict__ Ag, int* __restrict__ ipiv_all,
-                                                         int* __restrict__ status, int n, int j0, int jb) {
-  __shared__ double s_val[LS_THREADS / 32];
-  __shared__ int s_idx[LS_THREADS / 32];
-  __shared__ int s_piv;
-  __shared__ cplx s_inv;
-  const int i = blockIdx.x;
+// Columns [j0, j0 + 64) of the block [J0, JE), one CTA per instance: the panel
+// with its interchanges on all the block's columns, L11^{-1} over L11, and for
+// the first panel U12 = L11^{-1} A12 of the block's other columns (32 at a time,
+// 16 x 8 warp tiles).  worig[r]: the row whose content, as it stood before the
+// block, row r now holds.  With the block's last panel the instance's whole
+// permutation follows: perm'[r] = perm[worig[r]].  RPT as in block_factor.
+template <int RPT>
+__global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict__ Ag, int* __restrict__ ipiv_all,
+                                                               int* __restrict__ worig_all, int* __restrict__ wtmp_all,
+                                                               int* __restrict__ perm_all, int* __restrict__ status,
+                                                               int n, int j0, int J0, int JE) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  LsPanelShared& S = *reinterpret_cast<LsPanelShared*>(smraw);
+  const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int jb = min(kBlock, JE - j0), je = j0 + jb;
   cplx* A = Ag + (size_t)n * n * i;
-  int* ipiv = ipiv_all + (size_t)n * i;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int je = j0 + jb;
-  for (int jj = j0; jj < je; jj += LS_SUB) {
-    const int kb = min(LS_SUB, je - jj);
-    for (int c = jj; c < jj + kb; c++) {
-      double best = -1.0;
-      int bi = c;
-      for (int r = c + tid; r < n; r += nt) {
-        const double v = cabs1(A[r + (size_t)n * c]);
-        if (v > best) {
-          best = v;
-          bi = r;
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) {
-          best = ov;
-          bi = oi;
-        }
-      }
-      if ((tid & 31) == 0) {
-        s_val[tid >> 5] = best;
-        s_idx[tid >> 5] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double bv = s_val[0];
-        int bx = s_idx[0];
-        for (int w = 1; w < nt / 32; w++)
-          if (s_val[w] > bv || (s_val[w] == bv && s_idx[w] < bx)) {
-            bv = s_val[w];
-            bx = s_idx[w];
-          }
-        s_piv = bx;
-        ipiv[c] = bx;
-        if (bv == 0.0) {
-          s_inv = cmk(0.0, 0.0);
-          if (status[i] == 0) status[i] = c + 1;
-        } else {
-          s_inv = crecip(A[bx + (size_t)n * c]);
-        }
-      }
-      __syncthreads();
-      const int p = s_piv;
-      if (p != c)
-        for (int col = jj + tid; col < jj + kb; col += nt) {
-          const cplx t = A[c + (size_t)n * col];
-          A[c + (size_t)n * col] = A[p + (size_t)n * col];
-          A[p + (size_t)n * col] = t;
-        }
-      __syncthreads();
-      const cplx inv = s_inv;
-      for (int r = c + 1 + tid; r < n; r += nt) A[r + (size_t)n * c] = cmul(A[r + (size_t)n * c], inv);
-      __syncthreads();
-      const int ncols = jj + kb - (c + 1), nrows = n - (c + 1);
-      for (int e = tid; e < ncols * nrows; e += nt) {
-        const int r = c + 1 + e % nrows, col = c + 1 + e / nrows;
-        A[r + (size_t)n * col] = csub(A[r + (size_t)n * col], cmul(A[r + (size_t)n * c], A[c + (size_t)n * col]));
-      }
-      __syncthreads();
-    }
-    // this sub-panel's interchanges on the other columns of the panel
-    for (int c = jj; c < jj + kb; c++) {
-      const int p = ipiv[c];
-      if (p != c)
-        for (int col = j0 + tid; col < je; col += nt) {
-          if (col >= jj && col < jj + kb) continue;
-          const cplx t = A[c + (size_t)n * col];
-          A[c + (size_t)n * col] = A[p + (size_t)n * col];
-          A[p + (size_t)n * col] = t;
-        }
-      __syncthreads();
-    }
-    const int rc = je - jj - kb;
-    if (rc > 0) {
-      for (int col = tid; col < rc; col += nt)
-        col_lower(A + jj + (size_t)n * jj, n, A + jj + (size_t)n * (jj + kb + col), kb);
-      __syncthreads();
-      rank_update(A + (jj + kb) + (size_t)n * (jj + kb), A + (jj + kb) + (size_t)n * jj, A + jj + (size_t)n * (jj + kb),
-                  n - jj - kb, rc, kb, n, n, n);
-      __syncthreads();
-    }
+  int* worig = worig_all + (size_t)n * i;
+  for (int r = j0 + tid; r < n; r += kPanelThreads) {
+    const int o = j0 == J0 ? r : worig[r];
+    if (RPT > 0) S.b.orig[r - j0] = o;
+    else worig[r] = o;
   }
-}
-
-// Columns outside the panel [j0, j0 + jb), LS_COLS per CTA (grid (column
-// chunks, instances)): the panel's row interchanges, thread per column, then
-// for the columns right of the panel U12 = L11^{-1} A12 in sub-blocks of 32
-// (column in registers) with the FP64 tensor-core update between them.
-constexpr int LS_COLS = 128;
-
-__global__ void __launch_bounds__(LS_COLS) k_ls_rows(cplx* __restrict__ Ag, const int* __restrict__ ipiv_all, int n,
-                                                     int j0, int jb) {
-  const int i = blockIdx.y;
-  cplx* A = Ag + (size_t)n * n * i;
-  const int* ipiv = ipiv_all + (size_t)n * i;
-  const int je = j0 + jb;
-  const int c0 = blockIdx.x * LS_COLS;
-  const int col = c0 + threadIdx.x;
-  if (col < n && (col < j0 || col >= je)) {
-    cplx* x = A + (size_t)n * col;
-    for (int c = j0; c < je; c++) {
-      const int p = ipiv[c];
-      if (p != c) {
-        const cplx t = x[c];
-        x[c] = x[p];
-        x[p] = t;
-      }
-    }
-  }
-  const int ca = max(c0, je), cb = min(c0 + LS_COLS, n);  // this CTA's columns of A12
-  if (ca >= cb) return;
   __syncthreads();
-  for (int jj = j0; jj < je; jj += LS_SUB) {
-    const int kb = min(LS_SUB, je - jj);
-    if (col >= ca && col < cb) col_lower(A + jj + (size_t)n * jj, n, A + jj + (size_t)n * col, kb);
+  auto track = [&](int c, int p) {
+    int* o = RPT > 0 ? S.b.orig - j0 : worig;
+    const int x = o[c];
+    o[c] = o[p];
+    o[p] = x;
+  };
+  lud::block_factor<RPT, LS_NB>(A, n, j0, jb, J0, JE, ipiv_all + (size_t)n * i, &status[i], S.b, track);
+  if (RPT > 0)
+    for (int r = j0 + tid; r < n; r += kPanelThreads) worig[r] = S.b.orig[r - j0];
+  if (je == JE) {
+    int *perm = perm_all + (size_t)n * i, *tmp = wtmp_all + (size_t)n * i;
     __syncthreads();
-    if (jj + kb < je)
-      rank_update(A + (jj + kb) + (size_t)n * ca, A + (jj + kb) + (size_t)n * jj, A + jj + (size_t)n * ca,
-                  je - jj - kb, cb - ca, kb, n, n, n);
+    for (int r = J0 + tid; r < n; r += kPanelThreads) tmp[r] = J0 == 0 ? worig[r] : perm[worig[r]];
+    __syncthreads();
+    for (int r = J0 + tid; r < n; r += kPanelThreads) perm[r] = tmp[r];
+    return;
+  }
+  // L11^{-1} is still in S.b.M (unit diagonal included)
+  const int gid = lane >> 2, tig = lane & 3, m0 = (warp >> 2) * 16, cn = (warp & 3) * 8;
+  for (int c0 = je; c0 < JE; c0 += 32) {
+    for (int e = tid; e < 32 * kBlock; e += kPanelThreads) {
+      const int r = e % kBlock, c = e / kBlock;
+      S.x[c * (kBlock + 4) + r] = c0 + c < JE ? A[j0 + r + (size_t)n * (c0 + c)] : cmk(0.0, 0.0);
+    }
+    __syncthreads();
+    double re[4] = {}, im[4] = {};
+    for (int k8 = 0; k8 < m0 + 16; k8 += 8) {
+      const cplx* l = S.b.M + (k8 + tig) * kInvLd + m0 + gid;
+      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * kInvLd], a3 = l[4 * kInvLd + 8];
+      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+      const cplx* x = S.x + (cn + gid) * (kBlock + 4) + k8 + tig;
+      const double br[2] = {x[0].x, x[4].x}, bi[2] = {x[0].y, x[4].y};
+      lud::dmma8(re, ar, br);
+      lud::dmma8(re, an, bi);
+      lud::dmma8(im, ar, bi);
+      lud::dmma8(im, ai, br);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + cn + 2 * tig + (e & 1);
+      if (c < JE) A[j0 + r + (size_t)n * c] = cmk(re[e], im[e]);
+    }
     __syncthreads();
   }
 }
 
-// X <- P X: every thread applies the whole interchange sequence to its columns
-__global__ void __launch_bounds__(LS_THREADS) k_ls_perm(cplx* __restrict__ Xg, const int* __restrict__ ipiv_all, int n) {
-  const int i = blockIdx.y;
-  cplx* X = Xg + (size_t)n * n * i;
-  const int* ipiv = ipiv_all + (size_t)n * i;
-  for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x) {
-    cplx* x = X + (size_t)n * col;
-    for (int c = 0; c < n; c++) {
-      const int p = ipiv[c];
-      if (p != c) {
-        const cplx t = x[c];
-        x[c] = x[p];
-        x[p] = t;
-      }
+// A[j1.., j1..JE) -= A[j1.., J0..j1) A[J0..j1, j1..JE): the block's second panel
+using LsTile = ZgemmTile<1, 2, 2, 2, 16, 2, true, false>;
+
+struct LsSource {
+  const cplx *l, *r;
+  int n, K, n0;
+  __device__ int ktiles() const { return (K + 15) / 16; }
+  __device__ int depth(int kt) const { return min(16, K - 16 * kt); }
+  __device__ size_t ldl() const { return (size_t)n; }
+  __device__ const cplx* left(int kt) const { return l + (size_t)n * 16 * kt; }
+  __device__ const cplx* right(int kt) const { return r + 16 * kt; }
+  __device__ size_t roff(int c) const { return (size_t)n * (n0 + c); }
+};
+
+__global__ void __launch_bounds__(LsTile::NT, 5) k_ls_mid(cplx* __restrict__ Ag, int n, int J0, int j1, int JE) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* A = Ag + (size_t)n * n * blockIdx.z;
+  const int m0 = blockIdx.x * LsTile::BM, n0 = blockIdx.y * LsTile::BN, rows = n - j1 - m0, cols = JE - j1 - n0;
+  LsTile t;
+  t.run(LsSource{A + j1 + m0 + (size_t)n * J0, A + J0 + (size_t)n * j1, n, j1 - J0, n0}, reinterpret_cast<cplx*>(smraw),
+        rows, cols);
+  t.each(rows, cols, [&](int row, int col, cplx v) {
+    cplx* c = A + (j1 + m0 + row) + (size_t)n * (j1 + n0 + col);
+    *c = csub(*c, v);
+  });
+}
+
+// U_bb^{-1} over the upper 64 x 64 diagonal triangles, off the chain of panels
+__global__ void __launch_bounds__(256) k_ls_invert(cplx* __restrict__ Ag, int n) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* M = reinterpret_cast<cplx*>(smraw);
+  const int j0 = blockIdx.x * kBlock, jb = min(kBlock, n - j0);
+  cplx* A = Ag + (size_t)n * n * blockIdx.y;
+  lud::load_triangle<true>(A, n, j0, jb, M);
+  lud::invert_triangle<true>(M, M + kBlock * kInvLd);
+  lud::store_triangle<true>(A, n, j0, jb, M);
+}
+constexpr size_t kLsInvertSmem = ((size_t)kBlock * kInvLd + lud::kPanelCols * lud::kPanelCols) * sizeof(cplx);
+
+// ---- solves with a 128-row diagonal block [j0, j0 + jb) on LT_COLS columns per CTA ----
+// T is the block's unit lower (or, BACK, upper) triangle; its 64 x 64 diagonal
+// triangles hold their inverses, so X = T^{-1} X is three products per tile,
+// lower: X1 = I1 X1, X2 -= L21 X1, X2 = I2 X2.  A warp takes 8 columns and two
+// of the four 16-row strips, the first with the last, so that the triangles'
+// skipped strips cost every warp the same.
+// ROWS: the columns of A outside the block first take the block's interchanges
+// (worig), all reads of a tile before its first write; those left of the
+// block take nothing else.
+constexpr int LT_COLS = 16, LT_LDL = kBlock + 2, LT_LDX = LS_NB + 4;
+constexpr size_t kTriSmem = ((size_t)kBlock * LT_LDL + LT_COLS * LT_LDX) * sizeof(cplx);
+enum { TRI_ROWS = 0, TRI_FWD = 1, TRI_BACK = 2 };
+
+__device__ __forceinline__ void ls_cp_async16(void* sdst, const void* gsrc, bool valid) {
+  unsigned sz = valid ? 16u : 0u;
+  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz));
+}
+
+// out = sgn (x + ...): KIND 0 lower triangle (unit diagonal implied), 1 upper
+// triangle, 2 full block; rows r0.. (64) of the tile from rows k0.. (64) of it;
+// KIND 2 subtracts from the tile, the triangles replace it
+template <int KIND>
+__device__ __forceinline__ void tri_stage(const cplx* __restrict__ A, int n, int row, int col, int nr, int nk, cplx* sL,
+                                          cplx* sX, int r0, int k0) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
+#pragma unroll 8
+  for (int i = 0; i < kBlock * kBlock / 128; i++) {
+    const int m = tid % kBlock, k = tid / kBlock + 2 * i;
+    const bool in = m < nr && k < nk && (KIND == 0 ? m > k : KIND == 1 ? m <= k : true);
+    ls_cp_async16(sL + k * LT_LDL + m, in ? A + row + m + (size_t)n * (col + k) : A, in);
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (KIND == 0) {
+    if (tid < kBlock) sL[tid * LT_LDL + tid] = cmk(1.0, 0.0);
+    __syncthreads();
+  }
+  const int cn = (warp & 1) * 8;
+  double re[2][4] = {}, im[2][4] = {};
+  const cplx* x = sX + (cn + gid) * LT_LDX + k0 + tig;
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int t = u == 0 ? warp >> 1 : 3 - (warp >> 1);
+    const int ka = KIND == 1 ? 16 * t : 0, kz = KIND == 0 ? 16 * (t + 1) : kBlock;
+    for (int k8 = ka; k8 < kz; k8 += 8) {
+      const cplx* l = sL + (k8 + tig) * LT_LDL + 16 * t + gid;
+      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * LT_LDL], a3 = l[4 * LT_LDL + 8];
+      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+      const double br[2] = {x[k8].x, x[k8 + 4].x}, bi[2] = {x[k8].y, x[k8 + 4].y};
+      lud::dmma8(re[u], ar, br);
+      lud::dmma8(re[u], an, bi);
+      lud::dmma8(im[u], ar, bi);
+      lud::dmma8(im[u], ai, br);
     }
   }
+  __syncthreads();  // every warp has read the tile and the operand
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int t = u == 0 ? warp >> 1 : 3 - (warp >> 1);
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      cplx* d = sX + (cn + 2 * tig + (e & 1)) * LT_LDX + r0 + 16 * t + gid + (e >= 2 ? 8 : 0);
+      *d = KIND == 2 ? cmk(d->x - re[u][e], d->y - im[u][e]) : cmk(re[u][e], im[u][e]);
+    }
+  }
+  __syncthreads();
 }
 
-// forward substitution on the diagonal block [j0, j0 + jb) (unit lower),
-// LS_COLS columns of the right-hand sides per CTA
-__global__ void __launch_bounds__(LS_COLS) k_ls_fwd_diag(const cplx* __restrict__ Ag, cplx* __restrict__ Xg, int n,
-                                                         int j0, int jb) {
-  const int i = blockIdx.y;
+template <int MODE>
+__global__ void __launch_bounds__(128, 2) k_ls_tri(const cplx* __restrict__ Ag, cplx* Xg, const int* __restrict__ worig_all,
+                                                   int n, int j0, int jb) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int s_moved[LS_NB];
+  __shared__ int s_cnt;
+  cplx* sL = reinterpret_cast<cplx*>(smraw);  // [k][m]
+  cplx* sX = sL + kBlock * LT_LDL;            // [column][row]
+  const int i = blockIdx.y, tid = threadIdx.x, je = j0 + jb;
   const cplx* A = Ag + (size_t)n * n * i;
   cplx* X = Xg + (size_t)n * n * i;
-  const int je = j0 + jb;
-  const int ca = blockIdx.x * LS_COLS, cb = min(ca + LS_COLS, n);
-  const int col = ca + threadIdx.x;
-  for (int jj = j0; jj < je; jj += LS_SUB) {
-    const int kb = min(LS_SUB, je - jj);
-    if (col < cb) col_lower(A + jj + (size_t)n * jj, n, X + jj + (size_t)n * col, kb);
+  // ROWS: the columns are those of A outside the block, left ones first
+  const int ncol = MODE == TRI_ROWS ? n - jb : n, c0 = blockIdx.x * LT_COLS;
+  auto column = [&](int c) {
+    return X + (size_t)n * (MODE == TRI_ROWS && c0 + c >= j0 ? c0 + c + jb : c0 + c);
+  };
+  const int nc = min(LT_COLS, ncol - c0);
+  int src = j0 + tid;
+  if (MODE == TRI_ROWS) {
+    const int* worig = worig_all + (size_t)n * i;
+    if (tid == 0) s_cnt = 0;
     __syncthreads();
-    if (jj + kb < je)
-      rank_update(X + (jj + kb) + (size_t)n * ca, A + (jj + kb) + (size_t)n * jj, X + jj + (size_t)n * ca,
-                  je - jj - kb, cb - ca, kb, n, n, n);
+    if (tid < jb) src = worig[j0 + tid];
+    for (int r = je + tid; r < n; r += 128)
+      if (worig[r] != r) s_moved[atomicAdd(&s_cnt, 1)] = r;
+  }
+#pragma unroll
+  for (int c = 0; c < LT_COLS; c++) {
+    const bool in = tid < jb && c < nc;
+    ls_cp_async16(sX + c * LT_LDX + tid, in ? column(c) + src : X, in);
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (MODE == TRI_ROWS) {
+    // rows below the block that take a block row: each interchange moves one
+    const int cnt = s_cnt;
+    cplx v[LT_COLS];
+    const int dst = tid < cnt ? s_moved[tid] : 0;
+    const int from = tid < cnt ? worig_all[(size_t)n * i + dst] : 0;
+#pragma unroll
+    for (int c = 0; c < LT_COLS; c++)
+      if (tid < cnt && c < nc) v[c] = column(c)[from];
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < LT_COLS; c++)
+      if (tid < cnt && c < nc) column(c)[dst] = v[c];
+  }
+  // a tile of left columns only is done with the interchanges; a mixed one
+  // solves all its columns and stores the right ones
+  const bool solve = MODE != TRI_ROWS || c0 + nc > j0;
+  const int b1 = min(jb, kBlock), b2 = jb - b1;
+  if (!solve) {
+#pragma unroll
+    for (int c = 0; c < LT_COLS; c++)
+      if (tid < jb && c < nc) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
+    return;
+  }
+  if (MODE == TRI_ROWS && c0 < j0) {
+#pragma unroll
+    for (int c = 0; c < LT_COLS; c++)
+      if (tid < jb && c0 + c < j0) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
     __syncthreads();
   }
+  if (MODE == TRI_BACK) {
+    if (b2 > 0) {
+      tri_stage<1>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sX, kBlock, kBlock);
+      tri_stage<2>(A, n, j0, j0 + kBlock, b1, b2, sL, sX, 0, kBlock);
+    }
+    tri_stage<1>(A, n, j0, j0, b1, b1, sL, sX, 0, 0);
+  } else {
+    tri_stage<0>(A, n, j0, j0, b1, b1, sL, sX, 0, 0);
+    if (b2 > 0) {
+      tri_stage<2>(A, n, j0 + kBlock, j0, b2, b1, sL, sX, kBlock, 0);
+      tri_stage<0>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sX, kBlock, kBlock);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < LT_COLS; c++)
+    if (tid < jb && c < nc && (MODE != TRI_ROWS || c0 + c >= j0)) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
 }
 
-// back substitution on the diagonal block [j0, j0 + jb) (upper), LS_COLS
-// columns per CTA
-__global__ void __launch_bounds__(LS_COLS) k_ls_bwd_diag(const cplx* __restrict__ Ag, cplx* __restrict__ Xg, int n,
-                                                         int j0, int jb) {
+// X = P Y: row r from row perm[r]
+__global__ void __launch_bounds__(LS_THREADS) k_ls_gather(const cplx* __restrict__ Yg, const int* __restrict__ perm_all,
+                                                          cplx* __restrict__ Xg, int n) {
   const int i = blockIdx.y;
-  const cplx* A = Ag + (size_t)n * n * i;
-  cplx* X = Xg + (size_t)n * n * i;
-  const int ca = blockIdx.x * LS_COLS, cb = min(ca + LS_COLS, n);
-  const int col = ca + threadIdx.x;
-  const int nsub = (jb + LS_SUB - 1) / LS_SUB;
-  for (int t = nsub - 1; t >= 0; t--) {
-    const int jj = j0 + t * LS_SUB, kb = min(LS_SUB, j0 + jb - jj);
-    if (col < cb) col_upper(A + jj + (size_t)n * jj, n, X + jj + (size_t)n * col, kb);
-    __syncthreads();
-    if (jj > j0)
-      rank_update(X + j0 + (size_t)n * ca, A + j0 + (size_t)n * jj, X + jj + (size_t)n * ca, jj - j0, cb - ca, kb, n,
-                  n, n);
-    __syncthreads();
+  const size_t n2 = (size_t)n * n;
+  const int* perm = perm_all + (size_t)n * i;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n2; e += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(e % n);
+    Xg[n2 * i + e] = Yg[n2 * i + (e - r) + perm[r]];
   }
 }
 
@@ -353,91 +393,31 @@ __global__ void __launch_bounds__(LS_THREADS) k_ls_chimul(const LsDesc* __restri
   }
 }
 
-__device__ __forceinline__ void ls_cp_async16(void* sdst, const void* gsrc, bool valid) {
-  unsigned sz = valid ? 16u : 0u;
-  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz));
-}
+// R = Gamma - X + c Gamma Y on the FP64 tensor cores (the BSE GEMM's tile)
+using RsTile = ZgemmTile<1, 2, 2, 2, 16, 3, true>;
 
-// R = Gamma - X + c Gamma Y on the FP64 tensor cores: 32 x 32 complex tiles,
-// 4 warps of 16 x 16, two cp.async stages, three real products per complex
-// one (P1 = Ar Br, P2 = Ai Bi, P3 = (Ar + Ai)(Br + Bi))
-constexpr int RS_BM = 32, RS_BN = 32, RS_BK = 16, RS_LDL = RS_BM + 2, RS_LDR = RS_BK + 4;
-
-__global__ void __launch_bounds__(128) k_ls_resid(const LsDesc* __restrict__ desc, const cplx* __restrict__ Gg,
-                                                  const cplx* __restrict__ Yg, const cplx* __restrict__ Xg,
-                                                  cplx* __restrict__ Rg, unsigned long long* rmax, int n) {
-  __shared__ __align__(16) cplx sL[2][RS_BK][RS_LDL];
-  __shared__ __align__(16) cplx sR[2][RS_BN][RS_LDR];
+__global__ void __launch_bounds__(RsTile::NT, 3) k_ls_resid(const LsDesc* __restrict__ desc, const cplx* __restrict__ Gg,
+                                                            const cplx* __restrict__ Yg, const cplx* __restrict__ Xg,
+                                                            cplx* __restrict__ Rg, unsigned long long* rmax, int n) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int i = blockIdx.y;
   const size_t n2 = (size_t)n * n;
-  const cplx* Gi = Gg + n2 * i;
-  const cplx* Yi = Yg + n2 * i;
-  const int tiles_m = (n + RS_BM - 1) / RS_BM;
-  const int m0 = (blockIdx.x % tiles_m) * RS_BM, n0 = (blockIdx.x / tiles_m) * RS_BN;
-  const int ktiles = (n + RS_BK - 1) / RS_BK;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm0 = (warp % 2) * 16, wn0 = (warp / 2) * 16;
-  const int gid = lane >> 2, tig = lane & 3;
-  auto load = [&](int st, int kt) {
-    const int k0 = kt * RS_BK;
-    for (int e = tid; e < RS_BK * RS_BM; e += 128) {
-      const int m = e % RS_BM, kk = e / RS_BM, gm = m0 + m, gk = k0 + kk;
-      const bool ok = gm < n && gk < n;
-      ls_cp_async16(&sL[st][kk][m], ok ? Gi + gm + (size_t)n * gk : Gi, ok);
-    }
-    for (int e = tid; e < RS_BK * RS_BN; e += 128) {
-      const int kk = e % RS_BK, c = e / RS_BK, gc = n0 + c, gk = k0 + kk;
-      const bool ok = gc < n && gk < n;
-      ls_cp_async16(&sR[st][c][kk], ok ? Yi + gk + (size_t)n * gc : Yi, ok);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  double p1[2][4] = {}, p2[2][4] = {}, p3[2][4] = {};
-  load(0, 0);
-  for (int kt = 0; kt < ktiles; kt++) {
-    const int cur = kt & 1;
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-    if (kt + 1 < ktiles) load(cur ^ 1, kt + 1);
-#pragma unroll
-    for (int k8 = 0; k8 < RS_BK; k8 += 8) {
-      const int mb = wm0 + gid;
-      const cplx v0 = sL[cur][k8 + tig][mb], v1 = sL[cur][k8 + tig][mb + 8];
-      const cplx v2 = sL[cur][k8 + tig + 4][mb], v3 = sL[cur][k8 + tig + 4][mb + 8];
-      const double are[4] = {v0.x, v1.x, v2.x, v3.x}, aim[4] = {v0.y, v1.y, v2.y, v3.y};
-      const double asum[4] = {v0.x + v0.y, v1.x + v1.y, v2.x + v2.y, v3.x + v3.y};
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int nb = wn0 + j * 8 + gid;
-        const cplx w0 = sR[cur][nb][k8 + tig], w1 = sR[cur][nb][k8 + tig + 4];
-        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y}, bsum[2] = {w0.x + w0.y, w1.x + w1.y};
-        lud::dmma8(p1[j], are, bre);
-        lud::dmma8(p2[j], aim, bim);
-        lud::dmma8(p3[j], asum, bsum);
-      }
-    }
-  }
+  const cplx *G = Gg + n2 * i, *X = Xg + n2 * i;
+  cplx* R = Rg + n2 * i;
+  const int tiles_m = (n + RsTile::BM - 1) / RsTile::BM;
+  const int m0 = (int)(blockIdx.x % tiles_m) * RsTile::BM, n0 = (int)(blockIdx.x / tiles_m) * RsTile::BN;
+  RsTile t;
+  t.run(LsSource{G + m0, Yg + n2 * i, n, n, n0}, reinterpret_cast<cplx*>(smraw), n - m0, n - n0);
   const double s = desc[i].scale;
-  const cplx* Xi = Xg + n2 * i;
-  cplx* Ri = Rg + n2 * i;
   double mx = 0.0;
-#pragma unroll
-  for (int j = 0; j < 2; j++)
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      const int row = m0 + wm0 + gid + (x >= 2 ? 8 : 0), col = n0 + wn0 + j * 8 + 2 * tig + (x & 1);
-      if (row < n && col < n) {
-        const size_t idx = row + (size_t)n * col;
-        const double cre = p1[j][x] - p2[j][x], cim = p3[j][x] - p1[j][x] - p2[j][x];
-        const cplx g = Gi[idx], xv = Xi[idx];
-        const cplx rv = cmk((g.x - xv.x) + s * cre, (g.y - xv.y) + s * cim);
-        Ri[idx] = rv;
-        mx = fmax(mx, fmax(fabs(rv.x), fabs(rv.y)));
-      }
-    }
+  t.each(n - m0, n - n0, [&](int row, int col, cplx c) {
+    const size_t e = (m0 + row) + (size_t)n * (n0 + col);
+    const cplx g = G[e], x = X[e], v = cmk((g.x - x.x) + s * c.x, (g.y - x.y) + s * c.y);
+    R[e] = v;
+    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+  });
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0) atomic_max_nonneg(&rmax[i], mx);
+  if ((threadIdx.x & 31) == 0) atomic_max_nonneg(&rmax[i], mx);
 }
 
 // X += D
@@ -472,7 +452,7 @@ struct LsLayout {
 LsLayout ls_layout(int b, int n, int slices) {
   LsLayout L;
   L.mat = up256((size_t)b * n * n * sizeof(cplx));
-  L.ipiv = up256((size_t)b * n * sizeof(int));
+  L.ipiv = up256((size_t)4 * b * n * sizeof(int));  // pivots, block map, scratch, permutation
   L.desc = up256((size_t)b * sizeof(LsDesc));
   L.norms = up256((size_t)2 * b * sizeof(unsigned long long));  // max|R_i|, max|Gamma_i|
   L.status = up256((size_t)b * sizeof(int) + sizeof(double));
@@ -513,15 +493,17 @@ int ls_gemm_sub(cudaStream_t st, void* ozw, int b, int M, int N, int K, const cp
   return oz_run(R, st, launches);
 }
 
-// X <- U^{-1} L^{-1} P X for every instance of the group
-int ls_solve(cudaStream_t st, cplx* Ag, cplx* Xg, const int* ipiv, void* ozw, int b, int n, int s, double* ozstat,
-             long long* launches) {
+// X = U^{-1} L^{-1} P Y for every instance of the group
+int ls_solve(cudaStream_t st, const cplx* Ag, const cplx* Yg, cplx* Xg, const int* perm, void* ozw, int b, int n, int s,
+             double* ozstat, long long* launches) {
   const long long n2 = (long long)n * n;
-  k_ls_perm<<<dim3((n + LS_THREADS - 1) / LS_THREADS, b), LS_THREADS, 0, st>>>(Xg, ipiv, n);
+  const dim3 eg((unsigned)std::min<size_t>(((size_t)n * n + LS_THREADS - 1) / LS_THREADS, 512), b);
+  const dim3 tg((n + LT_COLS - 1) / LT_COLS, b);
+  k_ls_gather<<<eg, LS_THREADS, 0, st>>>(Yg, perm, Xg, n);
   (*launches)++;
   for (int j0 = 0; j0 < n; j0 += LS_NB) {
     const int jb = std::min(LS_NB, n - j0), je = j0 + jb;
-    k_ls_fwd_diag<<<dim3((n + LS_COLS - 1) / LS_COLS, b), LS_COLS, 0, st>>>(Ag, Xg, n, j0, jb);
+    k_ls_tri<TRI_FWD><<<tg, 128, kTriSmem, st>>>(Ag, Xg, nullptr, n, j0, jb);
     (*launches)++;
     if (je < n) {
       int rc = ls_gemm_sub(st, ozw, b, n - je, n, jb, Ag + je + (size_t)n * j0, n, Xg + j0, n, Xg + je, n, n2, s,
@@ -532,7 +514,7 @@ int ls_solve(cudaStream_t st, cplx* Ag, cplx* Xg, const int* ipiv, void* ozw, in
   const int nblk = (n + LS_NB - 1) / LS_NB;
   for (int bk = nblk - 1; bk >= 0; bk--) {
     const int j0 = bk * LS_NB, jb = std::min(LS_NB, n - j0);
-    k_ls_bwd_diag<<<dim3((n + LS_COLS - 1) / LS_COLS, b), LS_COLS, 0, st>>>(Ag, Xg, n, j0, jb);
+    k_ls_tri<TRI_BACK><<<tg, 128, kTriSmem, st>>>(Ag, Xg, nullptr, n, j0, jb);
     (*launches)++;
     if (j0 > 0) {
       int rc = ls_gemm_sub(st, ozw, b, j0, n, jb, Ag + (size_t)n * j0, n, Xg + j0, n, Xg, n, n2, s, ozstat, launches);
@@ -540,6 +522,21 @@ int ls_solve(cudaStream_t st, cplx* Ag, cplx* Xg, const int* ipiv, void* ozw, in
     }
   }
   return cudaGetLastError() == cudaSuccess ? TUPS_OK : TUPS_ERR_CUDA;
+}
+
+// opt-in shared-memory sizes
+bool ls_prepare() {
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int ps = (int)sizeof(LsPanelShared), ts = (int)kTriSmem;
+  return cudaFuncSetAttribute(k_ls_panel<0>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_panel<1>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_panel<2>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_tri<TRI_ROWS>, attr, ts) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_tri<TRI_FWD>, attr, ts) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_tri<TRI_BACK>, attr, ts) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_invert, attr, (int)kLsInvertSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_mid, attr, (int)LsTile::kSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(k_ls_resid, attr, (int)RsTile::kSmem) == cudaSuccess;
 }
 
 }  // namespace
@@ -575,6 +572,10 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   (void)cudaGetLastError();
+  if (!ls_prepare()) {
+    (void)cudaGetLastError();
+    return TUPS_ERR_CUDA;
+  }
   long long launches = 0;
   const cplx* G = reinterpret_cast<const cplx*>(gamma);
   const cplx* CH = reinterpret_cast<const cplx*>(chi);
@@ -592,6 +593,7 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
     cplx* Yg = (cplx*)(p + 4 * L.mat);
     p += 5 * L.mat;
     int* ipiv = (int*)p;
+    int *worig = ipiv + (size_t)b * nn, *wtmp = worig + (size_t)b * nn, *perm = wtmp + (size_t)b * nn;
     p += L.ipiv;
     LsDesc* desc = (LsDesc*)p;
     p += L.desc;
@@ -611,31 +613,40 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
     const size_t n2 = (size_t)nn * nn;
     const dim3 eg((unsigned)std::min<size_t>((n2 + LS_THREADS - 1) / LS_THREADS, 512), b);
     if (cudaMemsetAsync(norms, 0, 2 * b * sizeof(unsigned long long), st) != cudaSuccess) return TUPS_ERR_CUDA;
-    k_ls_form<<<eg, LS_THREADS, 0, st>>>(desc, G, CH, Gg, Xg, Ag, norms + b, nn);
+    k_ls_form<<<eg, LS_THREADS, 0, st>>>(desc, G, CH, Gg, Ag, norms + b, nn);
     // P A = L U
     for (int j0 = 0; j0 < nn; j0 += LS_NB) {
       const int jb = std::min(LS_NB, nn - j0), je = j0 + jb;
-      k_ls_panel<<<b, LS_THREADS, 0, st>>>(Ag, ipiv, stat, nn, j0, jb);
-      if (jb < nn) k_ls_rows<<<dim3((nn + LS_COLS - 1) / LS_COLS, b), LS_COLS, 0, st>>>(Ag, ipiv, nn, j0, jb);
+      for (int h0 = j0; h0 < je; h0 += kBlock) {
+        const int rows = nn - h0;
+        if (h0 > j0)
+          k_ls_mid<<<dim3((rows + LsTile::BM - 1) / LsTile::BM, (je - h0 + LsTile::BN - 1) / LsTile::BN, b), LsTile::NT,
+                     LsTile::kSmem, st>>>(Ag, nn, j0, h0, je);
+        const auto panel = rows <= kPanelThreads ? k_ls_panel<1> : rows <= kPanelRows ? k_ls_panel<2> : k_ls_panel<0>;
+        panel<<<b, kPanelThreads, sizeof(LsPanelShared), st>>>(Ag, ipiv, worig, wtmp, perm, stat, nn, h0, j0, je);
+      }
+      if (jb < nn)
+        k_ls_tri<TRI_ROWS><<<dim3((nn - jb + LT_COLS - 1) / LT_COLS, b), 128, kTriSmem, st>>>(Ag, Ag, worig, nn, j0, jb);
       if (je < nn) {
         int rc = ls_gemm_sub(st, ozw, b, nn - je, nn - je, jb, Ag + je + (size_t)nn * j0, nn, Ag + j0 + (size_t)nn * je,
                              nn, Ag + je + (size_t)nn * je, nn, (long long)n2, slices, ozstat, &launches);
         if (rc) return rc;
       }
     }
+    k_ls_invert<<<dim3((nn + kBlock - 1) / kBlock, b), 256, kLsInvertSmem, st>>>(Ag, nn);
     if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
-    int rc = ls_solve(st, Ag, Xg, ipiv, ozw, b, nn, slices, ozstat, &launches);
+    int rc = ls_solve(st, Ag, Gg, Xg, perm, ozw, b, nn, slices, ozstat, &launches);
     if (rc) return rc;
     // refinement: residual in FP64; stop once max|R_i| <= tol max|Gamma_i| for
     // every instance of the group, else correct with the split-precision factors
     int steps = 0;
-    const int tiles = ((nn + RS_BM - 1) / RS_BM) * ((nn + RS_BN - 1) / RS_BN);
+    const int tiles = ((nn + RsTile::BM - 1) / RsTile::BM) * ((nn + RsTile::BN - 1) / RsTile::BN);
     std::vector<unsigned long long> hn(2 * b);
     std::vector<double> rel(b, 0.0);
     for (;;) {
       if (cudaMemsetAsync(norms, 0, b * sizeof(unsigned long long), st) != cudaSuccess) return TUPS_ERR_CUDA;
       k_ls_chimul<<<eg, LS_THREADS, 0, st>>>(desc, CH, Xg, Yg, nn);
-      k_ls_resid<<<dim3(tiles, b), 128, 0, st>>>(desc, Gg, Yg, Xg, Rg, norms, nn);
+      k_ls_resid<<<dim3(tiles, b), RsTile::NT, RsTile::kSmem, st>>>(desc, Gg, Yg, Xg, Rg, norms, nn);
       if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
       if (cudaMemcpyAsync(hn.data(), norms, 2 * b * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st) !=
               cudaSuccess ||
@@ -652,9 +663,9 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
         worst = std::max(worst, rel[k]);
       }
       if (worst <= tol || steps >= max_refine) break;
-      rc = ls_solve(st, Ag, Rg, ipiv, ozw, b, nn, slices, ozstat, &launches);
+      rc = ls_solve(st, Ag, Rg, Yg, perm, ozw, b, nn, slices, ozstat, &launches);
       if (rc) return rc;
-      k_ls_update<<<eg, LS_THREADS, 0, st>>>(Xg, Rg, nn);
+      k_ls_update<<<eg, LS_THREADS, 0, st>>>(Xg, Yg, nn);
       steps++;
     }
     k_ls_scatter<<<eg, LS_THREADS, 0, st>>>(desc, Xg, Gg, OUT, nn, want_phi);

@@ -26,6 +26,7 @@
 #include <mutex>
 
 #include "tups_device.cuh"
+#include "zgemm_tile.cuh"
 
 namespace {
 
@@ -56,120 +57,101 @@ int scratch_address(int dev, cplx** out) {
   return TUPS_OK;
 }
 
-// A = Gamma chi, B = chi Gamma for instances [i0, i0+n) into the scratch
-__global__ void k_noalloc_prep(const cplx* __restrict__ G, const cplx* __restrict__ chi, cplx* __restrict__ A,
-                               cplx* __restrict__ B, int i0, int Nz, int Nf, int Nl) {
+// A = Gamma chi, B = chi Gamma for instances [i0, i0+n) into the scratch, sums
+// over the form factor ascending.  The first nA CTAs of an instance form A: a
+// thread per (row, nu) line loads the line's Nl entries of Gamma once (NA_LMAX
+// registers at a time) for its Nl outputs, lanes over rows at one nu, so a chi
+// entry is one address per warp.  The rest form B: a warp per column, lanes
+// over nu, chi[:, :, 32 nu] staged in shared memory ([l1 + Nl l2][lane], pitch
+// 33) when it fits.
+constexpr int NA_LMAX = 16, NA_STAGE = 13;  // Nl up to which chi is staged
+
+template <int LMAX>
+__device__ __forceinline__ void na_gamma_chi(const cplx* __restrict__ Gm, const cplx* __restrict__ ch,
+                                             cplx* __restrict__ Ai, int Nz, int Nf, int Nl, int cta, int ncta) {
+  const size_t lines = (size_t)Nz * Nf;
+  for (size_t t = (size_t)cta * blockDim.x + threadIdx.x; t < lines; t += (size_t)ncta * blockDim.x) {
+    const int row = (int)(t % Nz), nu = (int)(t / Nz);
+    cplx g[LMAX];
+#pragma unroll
+    for (int l = 0; l < LMAX; l++)
+      if (l < Nl) g[l] = Gm[row + (size_t)Nz * (l * Nf + nu)];
+    for (int l2 = 0; l2 < Nl; l2++) {
+      const cplx* c = ch + Nl * (l2 + (size_t)Nl * nu);
+      cplx acc = tups::cmk(0.0, 0.0);
+#pragma unroll
+      for (int l = 0; l < LMAX; l++)
+        if (l < Nl) acc = tups::cfma(g[l], c[l], acc);
+      for (int l = LMAX; l < Nl; l++) acc = tups::cfma(Gm[row + (size_t)Nz * (l * Nf + nu)], c[l], acc);
+      Ai[row + (size_t)Nz * (l2 * Nf + nu)] = acc;
+    }
+  }
+}
+
+template <int LMAX>
+__global__ void __launch_bounds__(256) k_noalloc_prep(const cplx* __restrict__ G, const cplx* __restrict__ chi,
+                                                      cplx* __restrict__ A, cplx* __restrict__ B, int i0, int Nz,
+                                                      int Nf, int Nl, int nA) {
+  extern __shared__ cplx chs[];
   const int li = blockIdx.y;
   const size_t n2 = (size_t)Nz * Nz;
   const cplx* Gm = G + n2 * (i0 + li);
   const cplx* ch = chi + (size_t)Nl * Nl * Nf * (i0 + li);
-  cplx* Ai = A + n2 * li;
-  cplx* Bi = B + n2 * li;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n2; e += (size_t)gridDim.x * blockDim.x) {
-    const int row = (int)(e % Nz), col = (int)(e / Nz);
-    const int l2 = col / Nf, nu = col % Nf;
+  if ((int)blockIdx.x < nA) {
+    na_gamma_chi<LMAX>(Gm, ch, A + n2 * li, Nz, Nf, Nl, blockIdx.x, nA);
+    return;
+  }
+  const int cta = blockIdx.x - nA, nchunk = (Nf + 31) / 32, nu0 = (cta % nchunk) * 32;
+  const int lane = threadIdx.x & 31, nu = nu0 + lane, col = cta / nchunk * 8 + (threadIdx.x >> 5);
+  const bool staged = Nl <= NA_STAGE;
+  if (staged)
+    for (int e = threadIdx.x; e < Nl * Nl * min(32, Nf - nu0); e += 256) {
+      const int ll = e % (Nl * Nl), j = e / (Nl * Nl);
+      chs[ll * 33 + j] = ch[(size_t)ll + (size_t)Nl * Nl * (nu0 + j)];
+    }
+  __syncthreads();
+  if (nu >= Nf || col >= Nz) return;
+  const cplx* Gc = Gm + (size_t)Nz * col + nu;
+  cplx* Bc = B + n2 * li + (size_t)Nz * col + nu;
+  cplx g[LMAX];
+#pragma unroll
+  for (int l = 0; l < LMAX; l++)
+    if (l < Nl) g[l] = Gc[l * Nf];
+  for (int l1 = 0; l1 < Nl; l1++) {
+    auto c = [&](int l2) { return staged ? chs[(l1 + Nl * l2) * 33 + lane] : ch[l1 + Nl * (l2 + (size_t)Nl * nu)]; };
     cplx acc = tups::cmk(0.0, 0.0);
-    for (int l1 = 0; l1 < Nl; l1++)
-      acc = tups::cfma(Gm[row + (size_t)Nz * (l1 * Nf + nu)], ch[l1 + Nl * (l2 + (size_t)Nl * nu)], acc);
-    Ai[e] = acc;
-    const int r1 = row / Nf, rnu = row % Nf;
-    cplx acb = tups::cmk(0.0, 0.0);
-    for (int l = 0; l < Nl; l++)
-      acb = tups::cfma(ch[r1 + Nl * (l + (size_t)Nl * rnu)], Gm[(l * Nf + rnu) + (size_t)Nz * col], acb);
-    Bi[e] = acb;
+#pragma unroll
+    for (int l = 0; l < LMAX; l++)
+      if (l < Nl) acc = tups::cfma(c(l), g[l], acc);
+    for (int l = LMAX; l < Nl; l++) acc = tups::cfma(c(l), Gc[l * Nf], acc);
+    Bc[l1 * Nf] = acc;
   }
 }
 
-__device__ __forceinline__ void na_cp_async16(void* sdst, const void* gsrc, bool valid) {
-  unsigned sz = valid ? 16u : 0u;
-  unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz));
-}
+// Phi = s [A | F] [F ; B] + (1-f)(F - Gamma) over Gamma, the BSE GEMM's tile with
+// four real products per complex one (three measured 12 % less exact here)
+constexpr int NB_BK = 16, NB_PER_SM = 4;
+using NaTile = tups::ZgemmTile<1, 2, 2, 2, NB_BK, 3, false>;
 
-__device__ __forceinline__ void na_dmma(double* c, const double* a, const double* b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
-// Phi = s [A | F] [F ; B] + (1-f)(F - Gamma) over Gamma, 32x32 complex tiles,
-// 4 warps of 16x16, two-stage cp.async pipeline, K step 16
-constexpr int NB_BM = 32, NB_BN = 32, NB_BK = 16, NB_LDL = NB_BM + 2, NB_LDR = NB_BK + 4;
-
-__global__ void __launch_bounds__(128) k_noalloc_gemm(cplx* __restrict__ G, const cplx* __restrict__ F,
-                                                      const cplx* __restrict__ A, const cplx* __restrict__ B, int i0,
-                                                      int Nz, double s, double one_minus_f) {
-  __shared__ __align__(16) cplx sL[2][NB_BK][NB_LDL];
-  __shared__ __align__(16) cplx sR[2][NB_BN][NB_LDR];
+__global__ void __launch_bounds__(NaTile::NT, NB_PER_SM) k_noalloc_gemm(cplx* __restrict__ G, const cplx* __restrict__ F,
+                                                                        const cplx* __restrict__ A,
+                                                                        const cplx* __restrict__ B, int i0, int Nz,
+                                                                        double s, double one_minus_f) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int li = blockIdx.y;
   const size_t n2 = (size_t)Nz * Nz;
-  const cplx* Ai = A + n2 * li;
-  const cplx* Bi = B + n2 * li;
   const cplx* Fi = F + n2 * (i0 + li);
   cplx* Gi = G + n2 * (i0 + li);
-  const int tiles_m = (Nz + NB_BM - 1) / NB_BM;
-  const int m0 = (blockIdx.x % tiles_m) * NB_BM, n0 = (blockIdx.x / tiles_m) * NB_BN;
-  const int K = 2 * Nz, ktiles = (K + NB_BK - 1) / NB_BK;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm0 = (warp % 2) * 16, wn0 = (warp / 2) * 16;
-  const int gid = lane >> 2, tig = lane & 3;
-  auto load = [&](int st, int kt) {
-    const int k0 = kt * NB_BK;
-    for (int e = tid; e < NB_BK * NB_BM; e += 128) {
-      const int m = e % NB_BM, kk = e / NB_BM, gm = m0 + m, gk = k0 + kk;
-      const bool ok = gm < Nz && gk < K;
-      const cplx* src = Ai;
-      if (ok) src = gk < Nz ? Ai + gm + (size_t)Nz * gk : Fi + gm + (size_t)Nz * (gk - Nz);
-      na_cp_async16(&sL[st][kk][m], src, ok);
-    }
-    for (int e = tid; e < NB_BK * NB_BN; e += 128) {
-      const int kk = e % NB_BK, n = e / NB_BK, gn = n0 + n, gk = k0 + kk;
-      const bool ok = gn < Nz && gk < K;
-      const cplx* src = Fi;
-      if (ok) src = gk < Nz ? Fi + gk + (size_t)Nz * gn : Bi + (gk - Nz) + (size_t)Nz * gn;
-      na_cp_async16(&sR[st][n][kk], src, ok);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  double cre[2][4] = {}, cim[2][4] = {};
-  load(0, 0);
-  for (int kt = 0; kt < ktiles; kt++) {
-    const int cur = kt & 1;
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-    if (kt + 1 < ktiles) load(cur ^ 1, kt + 1);
-#pragma unroll
-    for (int k8 = 0; k8 < NB_BK; k8 += 8) {
-      const int mb = wm0 + gid;
-      const cplx v0 = sL[cur][k8 + tig][mb], v1 = sL[cur][k8 + tig][mb + 8];
-      const cplx v2 = sL[cur][k8 + tig + 4][mb], v3 = sL[cur][k8 + tig + 4][mb + 8];
-      const double are[4] = {v0.x, v1.x, v2.x, v3.x}, aim[4] = {v0.y, v1.y, v2.y, v3.y};
-      const double anim[4] = {-v0.y, -v1.y, -v2.y, -v3.y};
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int nb = wn0 + j * 8 + gid;
-        const cplx w0 = sR[cur][nb][k8 + tig], w1 = sR[cur][nb][k8 + tig + 4];
-        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y};
-        na_dmma(cre[j], are, bre);
-        na_dmma(cre[j], anim, bim);
-        na_dmma(cim[j], are, bim);
-        na_dmma(cim[j], aim, bre);
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 2; j++)
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      const int row = m0 + wm0 + gid + (x >= 2 ? 8 : 0), col = n0 + wn0 + j * 8 + 2 * tig + (x & 1);
-      if (row < Nz && col < Nz) {
-        const size_t idx = row + (size_t)Nz * col;
-        const cplx f = Fi[idx], g = Gi[idx];
-        Gi[idx] = tups::cmk(s * cre[j][x] + one_minus_f * (f.x - g.x), s * cim[j][x] + one_minus_f * (f.y - g.y));
-      }
-    }
+  const int tiles_m = (Nz + NaTile::BM - 1) / NaTile::BM;
+  const int m0 = (int)(blockIdx.x % tiles_m) * NaTile::BM, n0 = (int)(blockIdx.x / tiles_m) * NaTile::BN;
+  NaTile t;
+  t.run(tups::BseSource<NB_BK>{A + n2 * li, Fi, B + n2 * li, Nz, m0, n0}, reinterpret_cast<cplx*>(smraw), Nz - m0,
+        Nz - n0);
+  t.each(Nz - m0, Nz - n0, [&](int row, int col, cplx c) {
+    const size_t e = (m0 + row) + (size_t)Nz * (n0 + col);
+    const cplx f = Fi[e], g = Gi[e];
+    Gi[e] = tups::cmk(s * c.x + one_minus_f * (f.x - g.x), s * c.y + one_minus_f * (f.y - g.y));
+  });
 }
 
 }  // namespace
@@ -198,20 +180,42 @@ extern "C" int tups_bse_noalloc(int n_inst, int Nz, int Nf, int Nl, double* gamm
   if (rc != TUPS_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // instances per pass through the scratch; the instance index is gridDim.y
-  // of both kernels, at most 65535
-  const int chunk = (int)std::min<size_t>(kScratchComplex / per, 65535);
-  cplx* A = scratch;
-  cplx* B = scratch + (size_t)chunk * Nz * Nz;
+  // of both kernels, at most 65535.  Of the pass sizes that fit, the one whose
+  // GEMM grids fill their last waves best: 240 instances of Nz = 160 take 11
+  // passes of 23 (0.97 waves each) instead of 6 of 40 (1.69)
   const size_t n2 = (size_t)Nz * Nz;
-  const int tiles = ((Nz + NB_BM - 1) / NB_BM) * ((Nz + NB_BN - 1) / NB_BN);
+  const int cap = (int)std::min<size_t>(std::min<size_t>(kScratchComplex / per, 65535), (size_t)n_inst);
+  const int tiles = ((Nz + NaTile::BM - 1) / NaTile::BM) * ((Nz + NaTile::BN - 1) / NaTile::BN);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long slots = (long long)NB_PER_SM * sms;
+  auto waves = [&](int chunk) {
+    const long long full = (n_inst / chunk) * (((long long)chunk * tiles + slots - 1) / slots);
+    return full + ((long long)(n_inst % chunk) * tiles + slots - 1) / slots;
+  };
+  int chunk = cap;
+  for (int c = cap; c >= 1 && c > cap - 64 && 2 * c > cap; c--)
+    if (waves(c) < waves(chunk)) chunk = c;
+  cplx* A = scratch;
+  cplx* B = scratch + (size_t)cap * n2;
+  const int nA = (int)std::min<size_t>(((size_t)Nz * Nf + 255) / 256, 4096);
+  const int nB = ((Nf + 31) / 32) * ((Nz + 7) / 8);
+  const size_t smp = Nl <= NA_STAGE ? (size_t)Nl * Nl * 33 * sizeof(cplx) : 0;
+  const auto prep = Nl <= 1 ? k_noalloc_prep<1> : Nl <= 5 ? k_noalloc_prep<5> : Nl <= 9 ? k_noalloc_prep<9>
+                    : k_noalloc_prep<NA_LMAX>;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((smp > 48 * 1024 && cudaFuncSetAttribute(prep, attr, (int)smp) != cudaSuccess) ||
+      cudaFuncSetAttribute(k_noalloc_gemm, attr, (int)NaTile::kSmem) != cudaSuccess) {
+    cudaGetLastError();
+    return TUPS_ERR_CUDA;
+  }
   for (int i0 = 0; i0 < n_inst; i0 += chunk) {
     const int n = n_inst - i0 < chunk ? n_inst - i0 : chunk;
-    dim3 pg((unsigned)(n2 < 256 * 1024 ? (n2 + 255) / 256 : 1024), n);
-    k_noalloc_prep<<<pg, 256, 0, st>>>(reinterpret_cast<const cplx*>(gamma_phi), reinterpret_cast<const cplx*>(chi), A,
-                                       B, i0, Nz, Nf, Nl);
+    prep<<<dim3(nA + nB, n), 256, smp, st>>>(reinterpret_cast<const cplx*>(gamma_phi),
+                                             reinterpret_cast<const cplx*>(chi), A, B, i0, Nz, Nf, Nl, nA);
     if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
-    k_noalloc_gemm<<<dim3(tiles, n), 128, 0, st>>>(reinterpret_cast<cplx*>(gamma_phi), reinterpret_cast<const cplx*>(F),
-                                                   A, B, i0, Nz, scale, 1.0 - f_damping);
+    k_noalloc_gemm<<<dim3(tiles, n), NaTile::NT, NaTile::kSmem, st>>>(
+        reinterpret_cast<cplx*>(gamma_phi), reinterpret_cast<const cplx*>(F), A, B, i0, Nz, scale, 1.0 - f_damping);
     if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
   }
   return TUPS_OK;

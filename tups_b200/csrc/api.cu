@@ -28,10 +28,9 @@ int read_scalars(tups_ctx* ctx, double* out) {
   return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "synchronize");
 }
 
-// surface a status left by a device routine (bisection cap) and clear it
-int device_status(tups_ctx* ctx) {
-  double sc[tups::S_COUNT];
-  TRY(read_scalars(ctx, sc));
+// surface a status left by a device routine (bisection cap) in the scalars sc
+// and clear it
+int status_of(tups_ctx* ctx, const double* sc) {
   int st = (int)sc[tups::S_STATUS];
   if (st != 0) {
     double z = 0.0;
@@ -41,6 +40,12 @@ int device_status(tups_ctx* ctx) {
     return tups::set_error(ctx, st, "device routine reported an error");
   }
   return TUPS_OK;
+}
+
+int device_status(tups_ctx* ctx) {
+  double sc[tups::S_COUNT];
+  TRY(read_scalars(ctx, sc));
+  return status_of(ctx, sc);
 }
 
 int copy_d2h(tups_ctx* ctx, void* host, const void* dev, size_t bytes) {
@@ -232,19 +237,26 @@ static int copy_sigma_old(tups_ctx* ctx) {
       "SigmaOld = Sigma");
 }
 
-extern "C" int tups_conv(tups_ctx* ctx, tups_conv_info* info) {
-  if (!ctx) return TUPS_ERR_BADARG;
-  TRY(set_dev(ctx));
+// with_status: a device routine's pending error comes before the check, from
+// the same read of the scalars
+static int conv_impl(tups_ctx* ctx, tups_conv_info* info, bool with_status) {
   tups::phase_begin(ctx, TUPS_PHASE_CONV);
   TRY(tups::launch_conv(ctx));
   tups::phase_end(ctx, TUPS_PHASE_CONV);
   double sc[tups::S_COUNT];
   TRY(read_scalars(ctx, sc));
+  if (with_status) TRY(status_of(ctx, sc));
   tups_conv_info ci;
   const int rc = conv_finish(ctx, sc, &ci);
   TRY(copy_sigma_old(ctx));
   if (info) *info = ci;
   return rc;
+}
+
+extern "C" int tups_conv(tups_ctx* ctx, tups_conv_info* info) {
+  if (!ctx) return TUPS_ERR_BADARG;
+  TRY(set_dev(ctx));
+  return conv_impl(ctx, info, false);
 }
 
 extern "C" int tups_vertex_update(tups_ctx* ctx) {
@@ -485,9 +497,8 @@ static int iteration_impl(tups_ctx* ctx, int ite, tups_conv_info* info, bool wit
   TRY(tups::launch_pae(ctx));
   tups::phase_end(ctx, TUPS_PHASE_PAE);
   if (!ctx->p.oneshot || ite == ctx->p.ite_max - 1) TRY(sde_async(ctx));
-  TRY(device_status(ctx));
   tups_conv_info ci;
-  int rc = tups_conv(ctx, &ci);
+  int rc = conv_impl(ctx, &ci, true);
   if (info) *info = ci;
   if (rc) return rc;
   if (ite % 5 == 0 || ite == ctx->p.ite_max - 1 || ci.converged) {

@@ -384,33 +384,29 @@ int launch_phir(tups_ctx* ctx) {
 
 int launch_M(tups_ctx* ctx, int which) {
   const auto& d = ctx->d;
-  // IBZ momenta (1-based) and the star lists of the lattice vectors R
-  std::vector<int> qxy(2 * d.NIBZ), slR(NS * d.NR);
-  for (int Q = 0; Q < d.NIBZ; Q++) {
-    qxy[2 * Q] = ctx->ibz[3 * Q * (d.Nf / 2)];
-    qxy[2 * Q + 1] = ctx->ibz[3 * Q * (d.Nf / 2) + 1];
+  if (!ctx->t.ibz_xy) {
+    // IBZ momenta (1-based) and, behind them, the star lists of the lattice
+    // vectors R: kept with the context, so a run's four launches queue up
+    std::vector<int> tab(2 * (size_t)d.NIBZ + (size_t)NS * d.NR);
+    for (int Q = 0; Q < d.NIBZ; Q++) {
+      tab[2 * Q] = ctx->ibz[3 * Q * (d.Nf / 2)];
+      tab[2 * Q + 1] = ctx->ibz[3 * Q * (d.Nf / 2) + 1];
+    }
+    for (int R = 0; R < d.NR; R++)
+      for (int s = 0; s < NS; s++) tab[2 * (size_t)d.NIBZ + NS * R + s] = ctx->symlist[NS * R + s];
+    void* p = nullptr;
+    int rc = cuda_check(ctx, cudaMalloc(&p, tab.size() * sizeof(int)), "M tables");
+    if (rc) return rc;
+    ctx->allocations.push_back(p);
+    rc = cuda_check(ctx, cudaMemcpy(p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice), "M tables");
+    if (rc) return rc;
+    ctx->t.ibz_xy = (int*)p;
   }
-  for (int R = 0; R < d.NR; R++)
-    for (int s = 0; s < NS; s++) slR[NS * R + s] = ctx->symlist[NS * R + s];
-  int* dq = nullptr;
-  int* ds = nullptr;
-  int rc = cuda_check(ctx, cudaMalloc(&dq, qxy.size() * sizeof(int)), "M tables");
-  if (rc) return rc;
-  rc = cuda_check(ctx, cudaMalloc(&ds, slR.size() * sizeof(int)), "M tables");
-  if (rc) {
-    cudaFree(dq);
-    return rc;
-  }
-  cudaMemcpyAsync(dq, qxy.data(), qxy.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
-  cudaMemcpyAsync(ds, slR.data(), slR.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
   const size_t n = (size_t)d.Nl * d.Nl * d.Nl * d.Nl * d.NIBZ * d.NR;
-  k_M<<<cdiv(n, 128), 128, 0, ctx->stream>>>(ctx->s.M[which], which, ctx->t.FF, ctx->t.FF_inv, ctx->t.expqSR, dq, ds,
-                                             d.Nx, d.Ny, d.Nl, d.NIBZ, d.NR);
-  rc = after_launch(ctx, "k_M");
-  cudaStreamSynchronize(ctx->stream);
-  cudaFree(dq);
-  cudaFree(ds);
-  return rc;
+  k_M<<<cdiv(n, 128), 128, 0, ctx->stream>>>(ctx->s.M[which], which, ctx->t.FF, ctx->t.FF_inv, ctx->t.expqSR,
+                                             ctx->t.ibz_xy, ctx->t.ibz_xy + 2 * (size_t)d.NIBZ, d.Nx, d.Ny, d.Nl,
+                                             d.NIBZ, d.NR);
+  return after_launch(ctx, "k_M");
 }
 
 }  // namespace tups

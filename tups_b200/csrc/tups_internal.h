@@ -28,6 +28,7 @@ struct DeviceTables {
   double* lfac = nullptr;     // (8, Nl)
   int* ibz = nullptr;         // (Nred, 3): qx, qy, w (1-based)
   int* symlist = nullptr;     // (NIBZ, 8) 0/1
+  int* ibz_xy = nullptr;      // (NIBZ, 2) qx, qy and (NR, 8) star flags of R, see launch_M
   int* symq = nullptr;        // (NIBZ, 8, 2): S(q) 1-based (qx, qy)
   cplx* L[4] = {};            // Lambda_r (Nf, Nf, Nf/2)
   cplx* expSqR = nullptr;     // (NIBZ, NR, 8)

@@ -462,9 +462,8 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
     while (queued[live - 1].n <= j0) live--;
     const int rows = nmax - j0, below = std::max(0, rows - NB);
     const size_t ps = sizeof(LuPanelShared);
-    if (rows <= kPanelThreads) k_lu_panel<1><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
-    else if (rows <= kPanelRows) k_lu_panel<2><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
-    else k_lu_panel<0><<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
+    const auto panel = rows <= kPanelThreads ? k_lu_panel<1> : rows <= kPanelRows ? k_lu_panel<2> : k_lu_panel<0>;
+    panel<<<live, kPanelThreads, ps, st>>>(A, ipiv, step);
     const long long width = (long long)below + nmax;
     k_lu_rows<false><<<dim3((unsigned)((width + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);
     if (below > 0) k_lu_update<false><<<dim3(tiles(below, width), live), 128, 0, st>>>(A, F, step);

@@ -119,14 +119,19 @@ static __device__ void panel_factor(cplx* __restrict__ A, int n, int h0, int kb,
       for (int i = 0; i < RPT; i++) {
         const int r = h0 + tid + i * kPanelThreads;
         if (r >= jj && r < n) {
-          for (int t = 0; t < p0; t += kPanelSub) {
-            cplx l[kPanelSub];
+          cplx l[kPanelSub], m[kPanelSub];
 #pragma unroll
-            for (int x = 0; x < kPanelSub; x++) l[x] = A[r + (size_t)n * (h0 + t + x)];
+          for (int x = 0; x < kPanelSub; x++) l[x] = A[r + (size_t)n * (h0 + x)];
+          for (int t = 0; t < p0; t += kPanelSub) {
+            if (t + kPanelSub < p0)
+#pragma unroll
+              for (int x = 0; x < kPanelSub; x++) m[x] = A[r + (size_t)n * (h0 + t + kPanelSub + x)];
 #pragma unroll
             for (int x = 0; x < kPanelSub; x++)
 #pragma unroll
               for (int k = 0; k < kPanelSub; k++) a[i][k] = cfnma(l[x], S.u[t + x][k], a[i][k]);
+#pragma unroll
+            for (int x = 0; x < kPanelSub; x++) l[x] = m[x];
           }
         }
       }
@@ -335,8 +340,7 @@ static __device__ void panel_half(cplx* __restrict__ A, int n, int j0, int kb, H
 }
 
 // The same panel with its columns in global memory, for more rows than the
-// registers hold (n - h0 > kPanelRows): a pass over the column per step, as
-// many as 512 threads wide.
+// registers hold (n - h0 > kPanelRows): a pass over the columns per step.
 template <class Track>
 static __device__ void panel_factor_global(cplx* __restrict__ A, int n, int h0, int kb, int ca, int cb,
                                            int* __restrict__ ipiv, int* __restrict__ status, PanelShared& S,
@@ -435,31 +439,42 @@ static __device__ void invert_triangle(cplx* __restrict__ M, cplx* __restrict__ 
     for (int r = 0; r < 16; r++) M[(b + c) * kInvLd + b + r] = x[r];
   }
   __syncthreads();
+  // Y is s x s; a warp per 16 x 8 tile of a product
+  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5, gid = lane >> 2, tig = lane & 3;
+  auto product = [&](const cplx* L, int ldl, const cplx* R, int ldr, int s, int m0, int c0, double* re, double* im) {
+    for (int k8 = 0; k8 < s; k8 += 8) {
+      const cplx* l = L + (k8 + tig) * ldl + m0 + gid;
+      const cplx* r = R + (c0 + gid) * ldr + k8 + tig;
+      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * ldl], a3 = l[4 * ldl + 8], b0 = r[0], b1 = r[4];
+      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y}, br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
+      dmma8(re, ar, br);
+      dmma8(im, ar, bi);
+      dmma8(re, an, bi);
+      dmma8(im, ai, br);
+    }
+  };
   for (int s = 16; s < kBlock; s *= 2) {
-    const int s2 = s * s, per = kBlock / (2 * s) * s2;
-    for (int e = tid; e < per; e += nt) {  // T = Y X' (lower) or Y Z' (upper)
-      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
-      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
-      cplx a0 = cmk(0.0, 0.0), a1 = a0;
-      for (int k = 0; k < s; k += 2) {
-        a0 = cfma(M[(x0 + k) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k], a0);
-        a1 = cfma(M[(x0 + k + 1) * kInvLd + y0 + r], M[(x0 + c) * kInvLd + x0 + k + 1], a1);
+    const int per = s / 16 * (s / 8), tiles = kBlock / (2 * s) * per;
+    for (int pass = 0; pass < 2; pass++) {
+      // pass 0: T = Y X' (lower) or Y Z' (upper); pass 1: Y = -Z' T or -X' T
+      for (int t = warp; t < tiles; t += nw) {
+        const int b = t / per * 2 * s, m0 = t % per % (s / 16) * 16, c0 = t % per / (s / 16) * 8;
+        const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
+        cplx* Y = M + x0 * kInvLd + y0;
+        cplx* Tp = T + t / per * s * s;  // [c][r]
+        double re[4] = {}, im[4] = {};
+        if (pass == 0) product(Y, kInvLd, M + x0 * kInvLd + x0, kInvLd, s, m0, c0, re, im);
+        else product(M + y0 * kInvLd + y0, kInvLd, Tp, s, s, m0, c0, re, im);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + 2 * tig + (e & 1);
+          if (pass == 0) Tp[c * s + r] = cmk(re[e], im[e]);
+          else Y[c * kInvLd + r] = cmk(-re[e], -im[e]);
+        }
       }
-      T[e] = cadd(a0, a1);  // [pair][c][r]
+      __syncthreads();
     }
-    __syncthreads();
-    for (int e = tid; e < per; e += nt) {  // Y = -Z' T or -X' T
-      const int b = e / s2 * 2 * s, r = e % s, c = e % s2 / s;
-      const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;
-      const cplx* t = T + (e - r);
-      cplx a0 = cmk(0.0, 0.0), a1 = a0;
-      for (int k = 0; k < s; k += 2) {
-        a0 = cfnma(M[(y0 + k) * kInvLd + y0 + r], t[k], a0);
-        a1 = cfnma(M[(y0 + k + 1) * kInvLd + y0 + r], t[k + 1], a1);
-      }
-      M[(x0 + c) * kInvLd + y0 + r] = cadd(a0, a1);
-    }
-    __syncthreads();
   }
 }
 

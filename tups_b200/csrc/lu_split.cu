@@ -144,30 +144,32 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict_
     return;
   }
   // L11^{-1} is still in S.b.M (unit diagonal included)
-  const int gid = lane >> 2, tig = lane & 3, m0 = (warp >> 2) * 16, cn = (warp & 3) * 8;
+  const int gid = lane >> 2, tig = lane & 3, cn = (warp & 3) * 8;
   for (int c0 = je; c0 < JE; c0 += 32) {
     for (int e = tid; e < 32 * kBlock; e += kPanelThreads) {
       const int r = e % kBlock, c = e / kBlock;
       S.x[c * (kBlock + 4) + r] = c0 + c < JE ? A[j0 + r + (size_t)n * (c0 + c)] : cmk(0.0, 0.0);
     }
     __syncthreads();
-    double re[4] = {}, im[4] = {};
-    for (int k8 = 0; k8 < m0 + 16; k8 += 8) {
-      const cplx* l = S.b.M + (k8 + tig) * kInvLd + m0 + gid;
-      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * kInvLd], a3 = l[4 * kInvLd + 8];
-      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
-      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
-      const cplx* x = S.x + (cn + gid) * (kBlock + 4) + k8 + tig;
-      const double br[2] = {x[0].x, x[4].x}, bi[2] = {x[0].y, x[4].y};
-      lud::dmma8(re, ar, br);
-      lud::dmma8(re, an, bi);
-      lud::dmma8(im, ar, bi);
-      lud::dmma8(im, ai, br);
-    }
+    for (int m0 = (warp >> 2) * 16; m0 < kBlock; m0 += kPanelThreads / 128 * 16) {
+      double re[4] = {}, im[4] = {};
+      for (int k8 = 0; k8 < m0 + 16; k8 += 8) {
+        const cplx* l = S.b.M + (k8 + tig) * kInvLd + m0 + gid;
+        const cplx a0 = l[0], a1 = l[8], a2 = l[4 * kInvLd], a3 = l[4 * kInvLd + 8];
+        const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
+        const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+        const cplx* x = S.x + (cn + gid) * (kBlock + 4) + k8 + tig;
+        const double br[2] = {x[0].x, x[4].x}, bi[2] = {x[0].y, x[4].y};
+        lud::dmma8(re, ar, br);
+        lud::dmma8(re, an, bi);
+        lud::dmma8(im, ar, bi);
+        lud::dmma8(im, ai, br);
+      }
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + cn + 2 * tig + (e & 1);
-      if (c < JE) A[j0 + r + (size_t)n * c] = cmk(re[e], im[e]);
+      for (int e = 0; e < 4; e++) {
+        const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + cn + 2 * tig + (e & 1);
+        if (c < JE) A[j0 + r + (size_t)n * c] = cmk(re[e], im[e]);
+      }
     }
     __syncthreads();
   }

@@ -70,6 +70,28 @@ def test_zgemm_split_cta_pairs_match_the_emulation(gpu_lib, dims, s):
         assert parity.rel(got[b], emu) <= EMU_TOL, (b, parity.rel(got[b], emu))
 
 
+@pytest.mark.parametrize("K", [8, 65, 592, 593, 1184, 1185, 2369, 4737])
+def test_zgemm_split_at_the_slicers_edges(gpu_lib, K):
+    """Rows staged whole by eights and by fours or streamed, columns staged by
+    8, 4, 2 and 1 or read twice; lines of zeros, of one sign and near the ends
+    of the exponent range.  The slices are exact, so only the final conversions
+    differ: a few roundings of sums of at most 2 K products of line maxima."""
+    M, N, s = 37, 11, 4
+    rng = np.random.default_rng(K)
+    A = rng.normal(size=(1, M, K)) + 1j * rng.normal(size=(1, M, K))
+    B = rng.normal(size=(1, K, N)) + 1j * rng.normal(size=(1, K, N))
+    A[0, 1] *= 1e-305
+    A[0, 2] *= 1e200
+    A[0, 3] = 0.0
+    A[0, 4] = -abs(A[0, 4])
+    B[0, :, 1] = 0.0
+    B[0, :, 2] *= -1e-290
+    got = _zgemm_split(gpu_lib, A, B, s)[0]
+    emu = S.ozaki_zgemm(A[0], B[0], s)
+    unit = np.abs(A[0]).max(axis=1)[:, None] * np.abs(B[0]).max(axis=0)[None, :]
+    assert np.all(np.abs(got - emu) <= EMU_TOL * 2 * K * unit)
+
+
 def test_split_bse_against_fp64(gpu_lib):
     from oracle import tups_oracle as O
     from tups_b200 import Solver

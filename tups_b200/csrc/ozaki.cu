@@ -69,12 +69,12 @@ __device__ __forceinline__ OzLine oz_view(const OzOperand& o, int inst) {
 }
 
 // element (m, k) of a row operand (parts)
-__device__ __forceinline__ cplx oz_a(const OzLine& v, int m, int k) {
+__device__ __forceinline__ const cplx& oz_a(const OzLine& v, int m, int k) {
   return k < v.K1 ? v.p1[m + (size_t)v.ld1 * k] : v.p2[m + (size_t)v.ld2 * (k - v.K1)];
 }
 
 // element (k, j) of a column operand (parts)
-__device__ __forceinline__ cplx oz_b(const OzLine& v, int k, int j) {
+__device__ __forceinline__ const cplx& oz_b(const OzLine& v, int k, int j) {
   return k < v.K1 ? v.p1[k + (size_t)v.ld1 * j] : v.p2[(k - v.K1) + (size_t)v.ld2 * j];
 }
 
@@ -84,59 +84,148 @@ __device__ __forceinline__ int oz_exponent(double maxabs) {
   return e;
 }
 
-// The s int8 slices of v 2^-e (|v 2^-e| < 1) are the base-128 digits, most
-// significant first and carrying the sign of v, of t = trunc(v 2^(7s - e)):
-// the same bytes as the repeated a = trunc(128 r), r = 128 r - a of the
-// error-free splitting (all steps exact in FP64), with
-// one scaling and one conversion instead of 4 s FP64 operations.  |t| <
-// 2^(7s) <= 2^56, so t is an exact int64.
-__device__ __forceinline__ long long oz_fixed(double v, int e, int s) {
-  return __double2ll_rz(ldexp(v, OZ_SLICE_BITS * s - e));
-}
-// digit i (0 = most significant) of t as a byte
-__device__ __forceinline__ uint32_t oz_digit(long long t, int i, int s) {
-  const long long u = t < 0 ? -t : t;
-  const int d = (int)((u >> (OZ_SLICE_BITS * (s - 1 - i))) & 127);
-  return (uint32_t)(uint8_t)(int8_t)(t < 0 ? -d : d);
+// max(mx, |v.x|, |v.y|) that ignores NaN
+__device__ __forceinline__ double oz_absmax(double mx, cplx v) {
+  mx = fabs(v.x) > mx ? fabs(v.x) : mx;
+  return fabs(v.y) > mx ? fabs(v.y) : mx;
 }
 
-// Rows of A': one CTA per 32 rows of one instance.  out: [inst][s][M][Kpad].
-// Pass 1 finds each row's scale (a warp per 8 columns at a time, four loads
-// in flight per thread); pass 2 stages 32 x 64 complex tiles in shared
-// memory (eight loads in flight per thread) and writes each row's slices as
-// 8-byte runs.
-constexpr int OZ_RT = 64;  // columns per staged tile of the row slicer
-__global__ void __launch_bounds__(256, 3) k_oz_split_rows(OzOperand A, int M, int s, int Kpad, int8_t* __restrict__ out,
-                                                       double* __restrict__ rscale) {
-  const int inst = blockIdx.y;
-  const int m0 = blockIdx.x * 32;
-  const int Kc = A.K1 + A.K2;
-  const OzLine V = oz_view(A, inst);
-  __shared__ double smax[8][33];
-  __shared__ int sexp[32];
-  __shared__ cplx tile[OZ_RT][33];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  {
-    const int m = m0 + lane;
-    double mx0 = 0.0, mx1 = 0.0, mx2 = 0.0, mx3 = 0.0;
-    if (m < M) {
-      int k = w;
-      for (; k + 24 < Kc; k += 32) {
-        const cplx v0 = oz_a(V, m, k), v1 = oz_a(V, m, k + 8), v2 = oz_a(V, m, k + 16), v3 = oz_a(V, m, k + 24);
-        mx0 = fmax(mx0, fmax(fabs(v0.x), fabs(v0.y)));
-        mx1 = fmax(mx1, fmax(fabs(v1.x), fabs(v1.y)));
-        mx2 = fmax(mx2, fmax(fabs(v2.x), fabs(v2.y)));
-        mx3 = fmax(mx3, fmax(fabs(v3.x), fabs(v3.y)));
+// The s int8 slices of v 2^-e (|v 2^-e| < 1) are the base-128 digits, most
+// significant first and carrying the sign of v, of t = trunc(|v| 2^(7s - e)):
+// the same bytes as the repeated a = trunc(128 r), r = 128 r - a of the
+// error-free splitting (all steps exact in FP64), with
+// one scaling and one conversion instead of 4 s FP64 operations.  t <
+// 2^(7s) <= 2^56, so t is an exact int64.  2^(7s - e) is the product of two
+// normal doubles (e >= -1073: one of them is 1 except for lines below 2^-960).
+struct OzScale {
+  double f1, f2;
+};
+__device__ __forceinline__ OzScale oz_scale(int e, int s) {
+  const int k = OZ_SLICE_BITS * s - e, k1 = min(k, 1023);
+  return {__hiloint2double((k1 + 1023) << 20, 0), __hiloint2double((k - k1 + 1023) << 20, 0)};
+}
+// digit j (0 = least significant) of v in byte j & 3 of lo (j < 4) or hi: the
+// 7-bit groups of t spread to bytes, then, for v < 0, each negated as
+// (128 - d) ^ 128, which borrows from no neighbour.
+__device__ __forceinline__ void oz_digits(double v, const OzScale& sc, uint32_t& lo, uint32_t& hi) {
+  const unsigned long long u = (unsigned long long)__double2ll_rz(fabs(v) * sc.f1 * sc.f2);
+  auto spread = [](uint32_t x) {  // 28 bits -> 4 bytes of 7
+    x += 3u * (x & 0xfffc000u);
+    return x + (x & 0x3f803f80u);
+  };
+  const int neg = __double2hiint(v) >> 31;
+  const uint32_t bias = (uint32_t)neg & 0x80808080u, sg = (uint32_t)neg | 1u;
+  lo = (spread((uint32_t)u & 0xfffffffu) * sg + bias) ^ bias;
+  hi = (spread((uint32_t)(u >> 28) & 0xfffffffu) * sg + bias) ^ bias;
+}
+// bytes (column c, digit j) of four columns -> word j holds digit j of the four
+__device__ __forceinline__ void oz_transpose4(uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+  const uint32_t t0 = __byte_perm(w0, w1, 0x5140), t1 = __byte_perm(w2, w3, 0x5140);
+  const uint32_t t2 = __byte_perm(w0, w1, 0x7362), t3 = __byte_perm(w2, w3, 0x7362);
+  w0 = __byte_perm(t0, t1, 0x5410);
+  w1 = __byte_perm(t0, t1, 0x7632);
+  w2 = __byte_perm(t2, t3, 0x5410);
+  w3 = __byte_perm(t2, t3, 0x7632);
+}
+
+__device__ __forceinline__ void oz_cp_async16(void* sdst, const void* gsrc, bool valid) {
+  const unsigned sz = valid ? 16u : 0u;
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(sz));
+}
+
+constexpr size_t kOzLinesSmem = 74 * 1024;  // a CTA's whole rows or columns: three CTAs per SM
+
+// the slices of row entries k .. k + 7 (at(c): entry k + c; beyond Kc unused):
+// one 8-byte run per slice and part
+template <class At>
+__device__ __forceinline__ void oz_row_slices(At at, const OzScale& sc, int k, int Kc, int s, size_t slice_stride,
+                                              int8_t* row) {
+  double im[8];
+  uint32_t lo[8], hi[8];
+#pragma unroll
+  for (int part = 0; part < 2; part++) {
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      double v;
+      if (part == 0) {
+        const cplx x = at(c);
+        v = x.x;
+        im[c] = x.y;
+      } else {
+        v = im[c];
       }
-      for (; k < Kc; k += 8) {
-        const cplx v = oz_a(V, m, k);
-        mx0 = fmax(mx0, fmax(fabs(v.x), fabs(v.y)));
+      oz_digits(v, sc, lo[c], hi[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c += 4) {
+      oz_transpose4(lo[c], lo[c + 1], lo[c + 2], lo[c + 3]);
+      oz_transpose4(hi[c], hi[c + 1], hi[c + 2], hi[c + 3]);
+    }
+    int8_t* dst = row + k + (part ? Kc : 0);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (j >= s) continue;
+      const uint32_t a = j < 4 ? lo[j & 3] : hi[j & 3], b = j < 4 ? lo[4 + (j & 3)] : hi[4 + (j & 3)];
+      int8_t* o = dst + (size_t)(s - 1 - j) * slice_stride;
+      if ((Kc & 7) == 0) {
+        *reinterpret_cast<uint2*>(o) = make_uint2(a, b);
+      } else {
+        for (int c = 0; c < 8 && k + c < Kc; c++) o[c] = (int8_t)((c < 4 ? a : b) >> (8 * (c & 3)));
       }
     }
-    smax[w][lane] = fmax(fmax(mx0, mx1), fmax(mx2, mx3));
+  }
+}
+
+// zero the K padding [2 Kc, Kpad) of rows m0 .. m0 + R - 1
+template <int R>
+__device__ __forceinline__ void oz_row_padding(int8_t* base, int m0, int M, int Kc, int s, int Kpad, size_t slice_stride) {
+  const int pad = Kpad - 2 * Kc;
+  for (int x = threadIdx.x; x < R * pad * s; x += 256) {
+    const int b = x % pad, r = (x / pad) % R, i = x / (pad * R);
+    if (m0 + r < M) base[(size_t)i * slice_stride + (size_t)(m0 + r) * Kpad + 2 * Kc + b] = 0;
+  }
+}
+
+// Rows of A', whole rows staged: one CTA per R rows of one instance (out:
+// [inst][s][M][Kpad]), brought
+// into shared memory by cp.async, all of it in flight, and read there for the
+// scales and for the slices, so that A crosses HBM once.  Entry (row r,
+// column c) stands at oz_at<R>: the eight lanes of a quarter warp (one row,
+// columns 8 apart) meet on no bank, and neither do the copies (rows fastest).
+// Bound by HBM and by issue: 32 x 576 x 576 in six slices, 297 MB, takes 68 us
+// (4.4 TB/s); the streamed form below read A twice and took 168 us, 93 with
+// today's conversion.
+template <int R>
+__device__ __forceinline__ int oz_at(int r, int c) {
+  return (R == 8 ? c : c ^ ((c >> 5) & 1)) * R + ((r + (c >> 3)) & (R - 1));
+}
+template <int R>
+__global__ void __launch_bounds__(256) k_oz_split_rows_once(OzOperand A, int M, int s, int Kpad,
+                                                            int8_t* __restrict__ out, double* __restrict__ rscale) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* rows = reinterpret_cast<cplx*>(smraw);
+  __shared__ double smax[8][R];
+  __shared__ int sexp[R];
+  const int inst = blockIdx.y;
+  const int m0 = blockIdx.x * R;
+  const int Kc = A.K1 + A.K2;
+  const OzLine V = oz_view(A, inst);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  {
+    const int r = threadIdx.x & (R - 1);
+    const bool ok = m0 + r < M;
+    for (int c = threadIdx.x / R; c < Kc; c += 256 / R)
+      oz_cp_async16(rows + oz_at<R>(r, c), ok ? &oz_a(V, m0 + r, c) : V.p1, ok);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    double mx = 0.0;  // of the entries this thread copied
+    for (int c = threadIdx.x / R; c < Kc; c += 256 / R) mx = oz_absmax(mx, rows[oz_at<R>(r, c)]);
+#pragma unroll
+    for (int o = 16; o >= R; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane < R) smax[w][lane] = mx;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
+  if (threadIdx.x < R) {
     double mx = 0.0;
     for (int i = 0; i < 8; i++) mx = fmax(mx, smax[i][threadIdx.x]);
     const int e = oz_exponent(mx);
@@ -147,146 +236,183 @@ __global__ void __launch_bounds__(256, 3) k_oz_split_rows(OzOperand A, int M, in
   __syncthreads();
   const size_t slice_stride = (size_t)M * Kpad;
   int8_t* base = out + (size_t)inst * s * slice_stride;
+  const int r = (threadIdx.x >> 3) & (R - 1), m = m0 + r;
+  if (m < M) {
+    const OzScale sc = oz_scale(sexp[r], s);
+#pragma unroll 1
+    for (int k = 8 * ((threadIdx.x & 7) + 8 * (threadIdx.x / (8 * R))); k < Kc; k += 8 * (256 / R))
+      oz_row_slices([&](int c) { return rows[oz_at<R>(r, k + c)]; }, sc, k, Kc, s, slice_stride,
+                    base + (size_t)m * Kpad);
+  }
+  oz_row_padding<R>(base, m0, M, Kc, s, Kpad, slice_stride);
+}
+
+// Rows of A' that are too long for that: one CTA per 32 rows of one instance.
+// Pass 1 finds each row's scale (a warp per 8 columns at a time, eight loads
+// in flight per thread); pass 2 brings 32 x 64 complex tiles into two
+// shared-memory buffers by cp.async, two tiles ahead of the conversion, and
+// writes each row's slices as 8-byte runs.  Element (row r, column c) of a tile
+// stands at 32 c + ((r + c / 8) & 31), so that neither the copies (rows
+// fastest) nor the eight lanes of a quarter warp (one row, columns 8 apart)
+// meet on a bank.  Bound by HBM: A is read twice (the second read misses L2).
+constexpr int OZ_RT = 64;  // columns per staged tile of the row slicer
+constexpr size_t kOzRowsSmem = (size_t)2 * OZ_RT * 32 * sizeof(cplx);
+__global__ void __launch_bounds__(256, 3) k_oz_split_rows(OzOperand A, int M, int s, int Kpad, int8_t* __restrict__ out,
+                                                       double* __restrict__ rscale) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cplx* tiles = reinterpret_cast<cplx*>(smraw);
+  const int inst = blockIdx.y;
+  const int m0 = blockIdx.x * 32;
+  const int Kc = A.K1 + A.K2;
+  const OzLine V = oz_view(A, inst);
+  __shared__ double smax[8][33];
+  __shared__ int sexp[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  {
+    const int m = m0 + lane;
+    double mx[8] = {};
+    if (m < M) {
+      int k = w;
+      for (; k + 56 < Kc; k += 64) {
+        cplx v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = oz_a(V, m, k + 8 * j);
+#pragma unroll
+        for (int j = 0; j < 8; j++) mx[j] = oz_absmax(mx[j], v[j]);
+      }
+      for (; k < Kc; k += 8) {
+        mx[0] = oz_absmax(mx[0], oz_a(V, m, k));
+      }
+    }
+#pragma unroll
+    for (int j = 4; j > 0; j >>= 1)
+      for (int x = 0; x < j; x++) mx[x] = fmax(mx[x], mx[x + j]);
+    smax[w][lane] = mx[0];
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double mx = 0.0;
+    for (int i = 0; i < 8; i++) mx = fmax(mx, smax[i][threadIdx.x]);
+    const int e = oz_exponent(mx);
+    sexp[threadIdx.x] = e;
+    const int m = m0 + threadIdx.x;
+    if (m < M) rscale[(size_t)inst * M + m] = ldexp(1.0, e);
+  }
+  const int ntile = (Kc + OZ_RT - 1) / OZ_RT;
+  auto load = [&](int t) {
+    if (t < ntile) {
+      cplx* d = tiles + (size_t)(t & 1) * OZ_RT * 32;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int c = w + 8 * j, k = t * OZ_RT + c;
+        const bool ok = m0 + lane < M && k < Kc;
+        oz_cp_async16(d + 32 * c + ((lane + (c >> 3)) & 31), ok ? &oz_a(V, m0 + lane, k) : V.p1, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  load(0);
+  load(1);
+  __syncthreads();
+  const size_t slice_stride = (size_t)M * Kpad;
+  int8_t* base = out + (size_t)inst * s * slice_stride;
   // thread -> (row rr, 8 consecutive columns 8 cg .. 8 cg + 7): 8 groups x 32 rows
   const int cg = threadIdx.x & 7, rr = threadIdx.x >> 3;
   const int m = m0 + rr;
-  const int e = sexp[rr];
-  const bool vec = (Kc & 7) == 0;
-  for (int k0 = 0; k0 < Kc; k0 += OZ_RT) {
-    // load a 32 x 64 tile, rows fastest: eight independent loads per thread
-    cplx v[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int x = threadIdx.x + 256 * j;
-      const int r = x & 31, c = x >> 5;
-      const int mm = m0 + r, k = k0 + c;
-      v[j] = (mm < M && k < Kc) ? oz_a(V, mm, k) : cmk(0.0, 0.0);
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int x = threadIdx.x + 256 * j;
-      tile[x >> 5][x & 31] = v[j];
-    }
+  const OzScale sc = oz_scale(sexp[rr], s);
+  for (int t = 0; t < ntile; t++) {
+    asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();
-    const int k = k0 + cg * 8;
+    const cplx* tile = tiles + (size_t)(t & 1) * OZ_RT * 32 + 256 * cg + ((rr + cg) & 31);
+    const int k = t * OZ_RT + cg * 8;
     if (m < M && k < Kc) {
-      uint32_t lre[8], hre[8], lim[8], him[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) lre[i] = hre[i] = lim[i] = him[i] = 0u;
-      // column c = (j + cg) & 7 at step j: the eight lanes of a quarter warp
-      // (cg = 0..7, one row) then read eight different banks
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int c = (j + cg) & 7;
-        const cplx x = (k + c < Kc) ? tile[cg * 8 + c][rr] : cmk(0.0, 0.0);
-        const long long tr = oz_fixed(x.x, e, s), ti = oz_fixed(x.y, e, s);
-        const int sh = 8 * (c & 3);
-        const bool lo = c < 4;
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (i < s) {
-            const uint32_t dr = oz_digit(tr, i, s) << sh, di = oz_digit(ti, i, s) << sh;
-            lre[i] |= lo ? dr : 0u;
-            hre[i] |= lo ? 0u : dr;
-            lim[i] |= lo ? di : 0u;
-            him[i] |= lo ? 0u : di;
-          }
-      }
-      int8_t* row = base + (size_t)m * Kpad;
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        if (i >= s) continue;
-        int8_t* dst = row + (size_t)i * slice_stride;
-        if (vec && k + 7 < Kc) {
-          *reinterpret_cast<uint2*>(dst + k) = make_uint2(lre[i], hre[i]);
-          *reinterpret_cast<uint2*>(dst + Kc + k) = make_uint2(lim[i], him[i]);
-        } else {
-          for (int c = 0; c < 8 && k + c < Kc; c++) {
-            dst[k + c] = (int8_t)((c < 4 ? lre[i] : hre[i]) >> (8 * (c & 3)));
-            dst[Kc + k + c] = (int8_t)((c < 4 ? lim[i] : him[i]) >> (8 * (c & 3)));
-          }
-        }
-      }
+      oz_row_slices([&](int c) { return tile[32 * c]; }, sc, k, Kc, s, slice_stride, base + (size_t)m * Kpad);
     }
     __syncthreads();
+    load(t + 2);
   }
-  // zero the K padding [2 Kc, Kpad) of this CTA's rows
-  const int pad = Kpad - 2 * Kc;
-  for (int x = threadIdx.x; x < 32 * pad * s; x += 256) {
-    const int b = x % pad, r = (x / pad) % 32, i = x / (pad * 32);
-    if (m0 + r < M) base[(size_t)i * slice_stride + (size_t)(m0 + r) * Kpad + 2 * Kc + b] = 0;
-  }
+  oz_row_padding<32>(base, m0, M, Kc, s, Kpad, slice_stride);
 }
 
 // Columns of B': one warp per complex column j of B (K1 + K2 long); writes
-// rows 2j and 2j+1 of every slice.  out: [inst][s][2N][Kpad].  The column
-// is read twice (scale, then slices); the second read hits L1.
+// rows 2j and 2j+1 of every slice.  out: [inst][s][2N][Kpad].  STAGED: the
+// warp's column is brought into its own part of shared memory by cp.async, all
+// of it in flight at once, and read there for the scale and for the slices;
+// entry k stands at k ^ ((k >> 3) & 3), so that the eight lanes of a quarter
+// warp (four entries each) meet on no bank.  Otherwise the column is read
+// twice from global memory.  32 x 576 x 576 in six slices, 425 MB: 81 us
+// (5.2 TB/s), 127 before with two reads from global memory and the digits taken
+// one by one.
+template <bool STAGED>
 __global__ void __launch_bounds__(256) k_oz_split_cols(OzOperand B, int N, int s, int Kpad, int8_t* __restrict__ out,
                                                        double* __restrict__ cscale) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int inst = blockIdx.y;
-  const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int w = threadIdx.x >> 5;
+  const int j = blockIdx.x * (blockDim.x >> 5) + w;
   const int lane = threadIdx.x & 31;
   if (j >= N) return;
   const int Kc = B.K1 + B.K2;
   const OzLine V = oz_view(B, inst);
-  double mx0 = 0.0, mx1 = 0.0, mx2 = 0.0, mx3 = 0.0;
-  {
-    int k = lane;
-    for (; k + 96 < Kc; k += 128) {
-      const cplx v0 = oz_b(V, k, j), v1 = oz_b(V, k + 32, j), v2 = oz_b(V, k + 64, j), v3 = oz_b(V, k + 96, j);
-      mx0 = fmax(mx0, fmax(fabs(v0.x), fabs(v0.y)));
-      mx1 = fmax(mx1, fmax(fabs(v1.x), fabs(v1.y)));
-      mx2 = fmax(mx2, fmax(fabs(v2.x), fabs(v2.y)));
-      mx3 = fmax(mx3, fmax(fabs(v3.x), fabs(v3.y)));
-    }
-    for (; k < Kc; k += 32) {
-      const cplx v = oz_b(V, k, j);
-      mx0 = fmax(mx0, fmax(fabs(v.x), fabs(v.y)));
-    }
+  cplx* col = reinterpret_cast<cplx*>(smraw) + (size_t)w * ((Kc + 3) & ~3);
+  double mx = 0.0;
+  if constexpr (STAGED) {
+    for (int k = lane; k < ((Kc + 3) & ~3); k += 32)
+      oz_cp_async16(col + (k ^ ((k >> 3) & 3)), k < Kc ? &oz_b(V, k, j) : V.p1, k < Kc);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+    for (int k = lane; k < Kc; k += 32) mx = oz_absmax(mx, col[k ^ ((k >> 3) & 3)]);
+  } else {
+    for (int k = lane; k < Kc; k += 32) mx = oz_absmax(mx, oz_b(V, k, j));
   }
-  const double mx = warp_max(fmax(fmax(mx0, mx1), fmax(mx2, mx3)));
+  mx = warp_max(mx);
   const int e = oz_exponent(mx);
   if (lane == 0) cscale[(size_t)inst * N + j] = ldexp(1.0, e);
+  const OzScale sc = oz_scale(e, s);
   const size_t slice_stride = (size_t)2 * N * Kpad;
   int8_t* r0 = out + (size_t)inst * s * slice_stride + (size_t)(2 * j) * Kpad;
   int8_t* r1 = r0 + Kpad;
   const bool vec = (Kc & 3) == 0;
+#pragma unroll 1
   for (int k = lane * 4; k < Kc; k += 128) {
     cplx v[4];
 #pragma unroll
-    for (int c = 0; c < 4; c++) v[c] = k + c < Kc ? oz_b(V, k + c, j) : cmk(0.0, 0.0);
-    uint32_t wre[8], wim[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) wre[i] = wim[i] = 0u;
+    for (int c = 0; c < 4; c++) {
+      if constexpr (STAGED)
+        v[c] = col[(k + c) ^ ((k >> 3) & 3)];
+      else
+        v[c] = k + c < Kc ? oz_b(V, k + c, j) : cmk(0.0, 0.0);
+    }
+    uint32_t rl[4], rh[4], il[4], ih[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const long long tr = oz_fixed(v[c].x, e, s), ti = oz_fixed(v[c].y, e, s);
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (i < s) {
-          wre[i] |= oz_digit(tr, i, s) << (8 * c);
-          wim[i] |= oz_digit(ti, i, s) << (8 * c);
-        }
+      oz_digits(v[c].x, sc, rl[c], rh[c]);
+      oz_digits(v[c].y, sc, il[c], ih[c]);
     }
+    oz_transpose4(rl[0], rl[1], rl[2], rl[3]);
+    oz_transpose4(rh[0], rh[1], rh[2], rh[3]);
+    oz_transpose4(il[0], il[1], il[2], il[3]);
+    oz_transpose4(ih[0], ih[1], ih[2], ih[3]);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      if (i >= s) continue;
-      int8_t* d0 = r0 + (size_t)i * slice_stride;
-      int8_t* d1 = r1 + (size_t)i * slice_stride;
+    for (int d = 0; d < 8; d++) {
+      if (d >= s) continue;
+      const uint32_t wre = d < 4 ? rl[d & 3] : rh[d & 3], wim = d < 4 ? il[d & 3] : ih[d & 3];
+      int8_t* d0 = r0 + (size_t)(s - 1 - d) * slice_stride;
+      int8_t* d1 = r1 + (size_t)(s - 1 - d) * slice_stride;
       // the slices of -Im are the negated slices of Im (truncation is odd):
       // a byte-wise negation of the packed digits
-      const uint32_t wnim = __vneg4(wim[i]);
+      const uint32_t wnim = __vneg4(wim);
       if (vec && k + 3 < Kc) {
-        *reinterpret_cast<uint32_t*>(d0 + k) = wre[i];
+        *reinterpret_cast<uint32_t*>(d0 + k) = wre;
         *reinterpret_cast<uint32_t*>(d0 + Kc + k) = wnim;
-        *reinterpret_cast<uint32_t*>(d1 + k) = wim[i];
-        *reinterpret_cast<uint32_t*>(d1 + Kc + k) = wre[i];
+        *reinterpret_cast<uint32_t*>(d1 + k) = wim;
+        *reinterpret_cast<uint32_t*>(d1 + Kc + k) = wre;
       } else {
         for (int c = 0; c < 4 && k + c < Kc; c++) {
-          d0[k + c] = (int8_t)(wre[i] >> (8 * c));
+          d0[k + c] = (int8_t)(wre >> (8 * c));
           d0[Kc + k + c] = (int8_t)(wnim >> (8 * c));
-          d1[k + c] = (int8_t)(wim[i] >> (8 * c));
-          d1[Kc + k + c] = (int8_t)(wre[i] >> (8 * c));
+          d1[k + c] = (int8_t)(wim >> (8 * c));
+          d1[Kc + k + c] = (int8_t)(wre >> (8 * c));
         }
       }
     }
@@ -1099,13 +1225,39 @@ int oz_run(OzRun& R, cudaStream_t stream, long long* launches) {
   if ((long long)batch * s * std::max(M, 2 * N) >= (1LL << 31)) return TUPS_ERR_BADDIM;
   // rows of the split kernels
   {
-    dim3 g((M + 31) / 32, batch);
-    k_oz_split_rows<<<g, 256, 0, stream>>>(R.A, M, s, Kpad, R.a_slices, R.rscale);
+    cudaError_t e;
+    auto rows = [&](auto* kernel, int nr, size_t smem) {
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess)
+        kernel<<<dim3((M + nr - 1) / nr, batch), 256, smem, stream>>>(R.A, M, s, Kpad, R.a_slices, R.rscale);
+    };
+    const size_t entry = (size_t)((K + 7) & ~7) * sizeof(cplx);
+    // whole rows while three CTAs of them share an SM (K' = 576: 68 us against 93 for
+    // the streamed rows, 4 of them at 1152: 131 against 179); longer ones are
+    // streamed (2304: 182 against 219 for 4 rows of 147 KB, one CTA per SM)
+    if (8 * entry <= kOzLinesSmem)
+      rows(k_oz_split_rows_once<8>, 8, 8 * entry);
+    else if (4 * entry <= kOzLinesSmem)
+      rows(k_oz_split_rows_once<4>, 4, 4 * entry);
+    else
+      rows(k_oz_split_rows, 32, kOzRowsSmem);
+    if (e != cudaSuccess) return oz_fail("slice kernel attribute", e);
     if (launches) (*launches)++;
-    dim3 gc((N + 7) / 8, batch);
-    k_oz_split_cols<<<gc, 256, 0, stream>>>(R.B, N, s, Kpad, R.b_slices, R.cscale);
+    // as many columns per CTA as fit; a column beyond that is read twice
+    const size_t line = (size_t)((K + 3) & ~3) * sizeof(cplx);
+    const bool staged = line <= kOzLinesSmem;
+    int cols = 8;
+    while (staged && cols > 1 && cols * line > kOzLinesSmem) cols /= 2;
+    dim3 gc((N + cols - 1) / cols, batch);
+    if (staged) {
+      e = cudaFuncSetAttribute(k_oz_split_cols<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOzLinesSmem);
+      if (e != cudaSuccess) return oz_fail("slice kernel attribute", e);
+      k_oz_split_cols<true><<<gc, 32 * cols, cols * line, stream>>>(R.B, N, s, Kpad, R.b_slices, R.cscale);
+    } else {
+      k_oz_split_cols<false><<<gc, 256, 0, stream>>>(R.B, N, s, Kpad, R.b_slices, R.cscale);
+    }
     if (launches) (*launches)++;
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return oz_fail("slice kernels launch", e);
   }
   OzGemm P;

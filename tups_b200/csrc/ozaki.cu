@@ -33,7 +33,8 @@ namespace tups {
 
 constexpr int OZ_BM = 128;       // rows per tile (TMEM lanes)
 constexpr int OZ_BK = 128;       // K bytes per pipeline stage
-constexpr int OZ_STAGES = 6;     // 6 x (16 KB of A + <= 16 KB of B) in flight
+constexpr int OZ_STAGES = 7;     // 7 x (16 KB of A + <= 16 KB of B) in flight
+constexpr uint32_t OZ_STAGE_BYTES = 2 * OZ_BM * OZ_BK;
 constexpr int OZ_SLICE_BITS = 7;
 
 // ---- splitting ---------------------------------------------------------------
@@ -453,6 +454,7 @@ constexpr long long OZ_WAIT_CYCLES = 4000000000LL;
 // `limit` SM cycles pass, in which case the abort flag is set
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           bool honor_abort = true, long long limit = OZ_WAIT_CYCLES) {
+  if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   for (uint32_t it = 0;; it++) {
     if (mbar_try(bar, parity)) return true;
@@ -515,15 +517,39 @@ __device__ __forceinline__ uint64_t oz_desc(uint32_t saddr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+// one lane of a converged warp, and a value that every lane has, in the form
+// that lets the compiler keep control flow and operands warp-uniform
+__device__ __forceinline__ bool oz_elect() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ uint32_t oz_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // ---- the GEMM ----------------------------------------------------------------------
 // Persistent: each CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... of
 // the list (instance, row tile, column tile), instance outermost.  Per tile
-// and diagonal d the MMA warp accumulates the slice products (i, d - i) over
-// K into one of OZ_NBUF TMEM buffers; the eight drain warps (two per TMEM
-// lane quarter, each owning half of the tile's columns) fold the finished
-// buffer into FP64 registers, acc += 2^(-7(d+2)) D_d, while the MMAs of the
-// next diagonals proceed; after the last diagonal they apply the row and
-// column scales and the epilogue, and the next tile starts.
+// the diagonals i + j = d of slice products go two at a time, d1 - 1 and d1 (d
+// = 0 alone where s is odd), each into its own of OZ_NBUF TMEM buffers: a
+// stage holds the K chunk of A_i and of B_(d1-i), i = 0 .. d1, and serves
+// A_i B_(d1-i) and, with the A of the stage before it, A_(i-1) B_(d1-i), so
+// that an operand tile is loaded for two products (but the first and the last).
+// The eight drain warps (two per TMEM lane quarter, each owning half of the
+// tile's columns) fold the finished buffers into FP64 registers, acc +=
+// 2^(-7(d+2)) D_d, while the MMAs of the next diagonals proceed; after the last
+// diagonal they apply the row and column scales and the epilogue, and the next
+// tile starts.
+//
+// What bounds it: the instructions of the one issuing thread came first (a wait
+// and a commit per product and descriptors in divergent code: 600 cycles per
+// product of 128 x 128 x 128, of which the MMAs need 256), then the drain
+// (tcgen05.ld latency under the MMAs, FP64 conversions, one column's reads
+// waiting for the last one's writes).  32 x 576^3 in six slices (1.03 P int8
+// operations, 576 rows in 640): 637 us with a stage per product; 650 with two
+// diagonals per stage; 490 with one wait and one commit per two products; 430
+// with a warp-uniform schedule and one elected lane; 397 with the drain in loads of
+// 16 columns, FP64 conversions by addition and four columns' reads ahead (2.6
+// POPS).
 enum { OZ_EPI_ZGEMM = 0, OZ_EPI_BSE = 1, OZ_EPI_SUB = 2 };
 
 constexpr int OZ_NBUF = 4;            // TMEM accumulator buffers
@@ -555,10 +581,74 @@ struct OzGemm {
   int stall_test;         // 1: the MMA warp first waits on a barrier nothing signals
 };
 
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, int32_t* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr));
+// acc += w D of one TMEM lane's `half` columns at tb (up to 8 more of the 512
+// columns are read and left unused).  Loads of 16 columns: under the MMAs a
+// load's latency, several hundred cycles, and not its width is what counts; 32
+// would take the registers that the sums need.  An int32 v becomes exact in FP64 as the low word of
+// 2^52 + 2^31 + v, one addition at the full FP64 rate where the conversion
+// instruction has a quarter of it.
+__device__ __forceinline__ void oz_fold(uint32_t tb, int half, double w, double* acc) {
+#pragma unroll
+  for (int c = 0; c < OZ_HALF; c += 16) {
+    if (c < half) {
+      int32_t v[16];
+      tc_ld16(tb + (uint32_t)c, v);
+#pragma unroll
+      for (int e = 0; e < 16; e++)
+        acc[c + e] = fma(__hiloint2double(0x43300000, v[e] ^ (int)0x80000000) - 4503601774854144.0, w, acc[c + e]);
+    }
+  }
+}
+
+// scales and epilogue of one row m: acc[0 .. half) are the real columns np0 ..,
+// lane l of the warp holds the column scale of complex column np0 / 2 + l.  The
+// reads of four columns go out before their writes, which could alias the next.
+__device__ __forceinline__ void oz_epilogue(const OzGemm& P, int inst, int m, int np0, int half, const double* acc,
+                                            double rs, double cs) {
+  const bool mok = m < P.M;
+  const int jc0 = np0 >> 1, nj = min(half >> 1, P.N - jc0);
+  const int r = inst & 3, q = P.q_begin + (inst >> 2);
+  const cplx* rd1 = nullptr;
+  cplx* out;
+  size_t ld = P.M;
+  double sr = 1.0;
+  if (P.epi == OZ_EPI_BSE) {
+    const size_t o = (size_t)P.M * P.M * q;
+    rd1 = (r == 0 ? P.F[0] : r == 1 ? P.F[1] : r == 2 ? P.F[2] : P.F[3]) + o;
+    out = (r == 0 ? P.G[0] : r == 1 ? P.G[1] : r == 2 ? P.G[2] : P.G[3]) + o;
+    sr = r == 0 ? P.scale[0] : r == 1 ? P.scale[1] : r == 2 ? P.scale[2] : P.scale[3];
+  } else if (P.epi == OZ_EPI_SUB) {
+    out = P.C + (size_t)inst * P.c_stride;
+    ld = P.ldc;
+  } else {
+    out = P.C + (size_t)inst * P.M * P.N;
+  }
+#pragma unroll
+  for (int c0 = 0; c0 < OZ_HALF / 2; c0 += 4) {
+    if (c0 >= nj) continue;
+    cplx f[4], g[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const size_t ix = m + ld * (jc0 + c0 + c);
+      const bool ok = mok && c0 + c < nj;
+      f[c] = ok && P.epi == OZ_EPI_BSE ? rd1[ix] : cmk(0.0, 0.0);
+      g[c] = ok && P.epi != OZ_EPI_ZGEMM ? out[ix] : cmk(0.0, 0.0);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const size_t ix = m + ld * (jc0 + c0 + c);
+      const double sc = rs * __shfl_sync(0xffffffffu, cs, c0 + c);
+      const double cre = acc[2 * (c0 + c)] * sc, cim = acc[2 * (c0 + c) + 1] * sc;
+      if (!mok || c0 + c >= nj) continue;
+      if (P.epi == OZ_EPI_ZGEMM)
+        out[ix] = cmk(cre, cim);
+      else if (P.epi == OZ_EPI_SUB)
+        out[ix] = cmk(g[c].x - cre, g[c].y - cim);
+      else
+        out[ix] = cmk(__dadd_rn(__dmul_rn(sr, cre), __dmul_rn(P.omf, __dsub_rn(f[c].x, g[c].x))),
+                      __dadd_rn(__dmul_rn(sr, cim), __dmul_rn(P.omf, __dsub_rn(f[c].y, g[c].y))));
+    }
+  }
 }
 
 __global__ void __launch_bounds__(OZ_THREADS2, 1)
@@ -570,12 +660,12 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
   __shared__ volatile int abort_sh;
   __shared__ int issued_sh, consumed_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)oz_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int Np = 2 * P.N;
   const uint32_t a_bytes = OZ_BM * OZ_BK, b_bytes = (uint32_t)P.n_tile * OZ_BK;
   const uint32_t dyn = (oz_smem(oz_dyn) + 1023u) & ~1023u;
-  auto sA = [&](int st) { return dyn + (uint32_t)st * (a_bytes + b_bytes); };
-  auto sB = [&](int st) { return dyn + (uint32_t)st * (a_bytes + b_bytes) + a_bytes; };
+  auto slot_a = [&](int st) { return dyn + (uint32_t)st * OZ_STAGE_BYTES; };
+  auto slot_b = [&](int st) { return dyn + (uint32_t)st * OZ_STAGE_BYTES + OZ_BM * OZ_BK; };
   const int per_inst = P.m_tiles * P.n_tiles;
 
   if (threadIdx.x == 0) {
@@ -602,7 +692,7 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_sh;
+  const uint32_t tmem = oz_uniform(tmem_base_sh);
 
   if (warp == OZ_DRAIN_WARPS + 1) {
     // ---- TMA producer ----
@@ -614,77 +704,95 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
       for (int t = blockIdx.x; t < P.tiles && ok; t += gridDim.x) {
         const int inst = t / per_inst, rem = t % per_inst;
         const int m0 = (rem % P.m_tiles) * OZ_BM, n0 = (rem / P.m_tiles) * P.n_tile;
-        for (int d = 0; d < P.s && ok; d++)
-          for (int i = 0; i <= d && ok; i++) {
-            const int ya = (inst * P.s + i) * P.M + m0;
-            const int yb = (inst * P.s + (d - i)) * Np + n0;
-            for (int kc = 0; kc < P.kchunks; kc++) {
+        // steps (d1 - 1, d1): stages (A_i, B_(d1 - i)), i = 0 .. d1
+        for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2)
+          for (int kc = 0; kc < P.kchunks && ok; kc++)
+            for (int i = 0; i <= d1; i++) {
               if (!mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_sh, true, P.wait_cycles)) {
                 ok = false;
                 break;
               }
               mbar_expect_tx(&full_bar[stage], a_bytes + b_bytes);
-              tma_load_2d(sA(stage), &tmA, kc * OZ_BK, ya, &full_bar[stage]);
-              tma_load_2d(sB(stage), &tmB, kc * OZ_BK, yb, &full_bar[stage]);
+              tma_load_2d(slot_b(stage), &tmB, kc * OZ_BK, (inst * P.s + d1 - i) * Np + n0, &full_bar[stage]);
+              tma_load_2d(slot_a(stage), &tmA, kc * OZ_BK, (inst * P.s + i) * P.M + m0, &full_bar[stage]);
               issued++;
               if (++stage == OZ_STAGES) {
                 stage = 0;
                 phase ^= 1u;
               }
             }
-          }
       }
       issued_sh = issued;
     }
   } else if (warp == OZ_DRAIN_WARPS) {
     // ---- MMA issuer ----
-    if (lane == 0) {
+    // the whole warp walks the schedule, so that it is uniform; one lane issues
+    {
+      const bool el = oz_elect();
+      auto wait = [&](uint64_t* bar, uint32_t ph) {
+        return __all_sync(0xffffffffu, mbar_wait(bar, ph, &abort_sh, true, P.wait_cycles)) != 0;
+      };
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.n_tile >> 3) << 17) |
                              ((uint32_t)(OZ_BM >> 4) << 24);
+      const uint64_t desc0 = oz_desc(dyn);  // of stage 0's A; the address counts 16 bytes
       int stage = 0;
       uint32_t phase = 0;
       int consumed = 0;
       int nacc = 0;  // accumulations issued so far (one per tile and diagonal)
       bool ok = true;
       // failure-path test: a wait that can only run out, before any MMA
-      if (P.stall_test) ok = mbar_wait(&never_bar, 0, &abort_sh, true, P.wait_cycles);
+      if (P.stall_test) ok = wait(&never_bar, 0);
       for (int t = blockIdx.x; t < P.tiles && ok; t += gridDim.x)
-        for (int d = 0; d < P.s && ok; d++, nacc++) {
-          const int buf = nacc % OZ_NBUF;
-          if (nacc >= OZ_NBUF &&
-              !mbar_wait(&acce_bar[buf], (uint32_t)((nacc - OZ_NBUF) / OZ_NBUF) & 1u, &abort_sh, true,
-                         P.wait_cycles)) {
-            ok = false;
-            break;
+        for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2) {
+          const int nb = d1 > 0 ? 2 : 1;  // diagonals of this step
+          for (int b = 0; b < nb && ok; b++) {
+            const int n = nacc + b;
+            if (n >= OZ_NBUF)
+              ok = wait(&acce_bar[n % OZ_NBUF], (uint32_t)((n - OZ_NBUF) / OZ_NBUF) & 1u);
           }
           tc_fence_after();
-          const uint32_t dtm = tmem + (uint32_t)(buf * OZ_MAX_NT);
-          uint32_t accum = 0;
-          for (int i = 0; i <= d && ok; i++)
-            for (int kc = 0; kc < P.kchunks; kc++) {
-              if (!mbar_wait(&full_bar[stage], phase, &abort_sh, true, P.wait_cycles)) {
+          const uint32_t dt1 = tmem + (uint32_t)((nacc + nb - 1) % OZ_NBUF * OZ_MAX_NT);
+          const uint32_t dt0 = tmem + (uint32_t)(nacc % OZ_NBUF * OZ_MAX_NT);
+          for (int kc = 0; kc < P.kchunks && ok; kc++) {
+            uint64_t da = 0;
+            int prev = 0;
+            for (int i = 0; i <= d1; i++) {
+              if (!wait(&full_bar[stage], phase)) {
                 ok = false;
                 break;
               }
               consumed++;
               tc_fence_after();
-              const uint64_t da = oz_desc(sA(stage)), db = oz_desc(sB(stage));
+              const uint64_t db = desc0 + (uint32_t)(stage * (int)(OZ_STAGE_BYTES >> 4)) + (OZ_BM * OZ_BK >> 4);
+              if (i > 0 && el) {  // A_(i-1) B_(d1-i): diagonal d1 - 1
 #pragma unroll
-              for (int kk = 0; kk < OZ_BK / 32; kk++) {
-                tc_mma_i8(dtm, da + 2 * kk, db + 2 * kk, idesc, accum);
-                accum = 1;
+                for (int kk = 0; kk < OZ_BK / 32; kk++)
+                  tc_mma_i8(dt0, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || i > 1 || kk > 0);
+                tc_commit(&empty_bar[prev]);
               }
-              tc_commit(&empty_bar[stage]);
+              da = desc0 + (uint32_t)(stage * (int)(OZ_STAGE_BYTES >> 4));
+              if (el) {
+#pragma unroll
+                for (int kk = 0; kk < OZ_BK / 32; kk++)
+                  tc_mma_i8(dt1, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || i > 0 || kk > 0);
+              }
+              prev = stage;
               if (++stage == OZ_STAGES) {
                 stage = 0;
                 phase ^= 1u;
               }
             }
-          if (ok) tc_commit(&accf_bar[buf]);
+            if (ok && el) tc_commit(&empty_bar[prev]);
+          }
+          for (int b = 0; b < nb && ok; b++, nacc++)
+            if (el) tc_commit(&accf_bar[nacc % OZ_NBUF]);
         }
-      consumed_sh = consumed;
-      tc_commit(&done_bar);
-      mbar_wait(&done_bar, 0, &abort_sh, false);
+      if (el) {
+        consumed_sh = consumed;
+        tc_commit(&done_bar);
+        mbar_wait(&done_bar, 0, &abort_sh, false);
+      }
+      __syncwarp();
     }
   } else {
     // ---- drain: warp w reads TMEM lanes 32 (w % 4) .. + 31 and columns
@@ -699,7 +807,10 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
       const int inst = t / per_inst, rem = t % per_inst;
       const int m0 = (rem % P.m_tiles) * OZ_BM, n0 = (rem / P.m_tiles) * P.n_tile;
       const int m = m0 + row;
-      const bool mok = m < P.M;
+      const int np0 = n0 + h * half;
+      // the scales, long before their use
+      const double rs = m < P.M ? __ldg(P.rscale + (size_t)inst * P.M + m) : 0.0;
+      const double cs = 2 * lane < half && (np0 >> 1) + lane < P.N ? __ldg(P.cscale + (size_t)inst * P.N + (np0 >> 1) + lane) : 0.0;
 #pragma unroll
       for (int c = 0; c < OZ_HALF; c++) acc[c] = 0.0;
       for (int d = 0; d < P.s; d++, nacc++) {
@@ -711,61 +822,12 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
         tc_fence_after();
         const double w = ldexp(1.0, -OZ_SLICE_BITS * (d + 2));
         const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * OZ_MAX_NT + h * half);
-#pragma unroll
-        for (int c = 0; c < OZ_HALF; c += 8) {
-          if (c < half) {
-            int32_t v[8];
-            tc_ld8(tb + (uint32_t)c, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int e = 0; e < 8; e++) acc[c + e] = fma((double)v[e], w, acc[c + e]);
-          }
-        }
+        oz_fold(tb, half, w, acc);
         tc_fence_before();
         mbar_arrive(&acce_bar[buf]);
       }
       if (!ok) break;
-      if (!mok) continue;
-      // scales and the epilogue; complex column jc = (n0 + h half + c) / 2
-      const double rs = P.rscale[(size_t)inst * P.M + m];
-      cplx* Cq = nullptr;
-      const cplx* Fq = nullptr;
-      cplx* Gq = nullptr;
-      int r = 0;
-      if (P.epi == OZ_EPI_BSE) {
-        const int q = P.q_begin + inst / 4;
-        r = inst % 4;
-        Fq = P.F[r] + (size_t)P.M * P.M * q;
-        Gq = P.G[r] + (size_t)P.M * P.M * q;
-      } else if (P.epi == OZ_EPI_SUB) {
-        Cq = P.C + (size_t)inst * P.c_stride;
-      } else {
-        Cq = P.C + (size_t)inst * P.M * P.N;
-      }
-#pragma unroll
-      for (int c = 0; c < OZ_HALF; c += 2) {
-        const int np = n0 + h * half + c;
-        if (c < half && np < Np) {
-          const int jc = np >> 1;
-          const double sc = rs * P.cscale[(size_t)inst * P.N + jc];
-          const double cre = acc[c] * sc, cim = acc[c + 1] * sc;
-          if (P.epi == OZ_EPI_SUB) {
-            const size_t ix = m + (size_t)P.ldc * jc;
-            const cplx c0 = Cq[ix];
-            Cq[ix] = cmk(c0.x - cre, c0.y - cim);
-            continue;
-          }
-          const size_t idx = m + (size_t)P.M * jc;
-          if (P.epi == OZ_EPI_ZGEMM) {
-            Cq[idx] = cmk(cre, cim);
-          } else {
-            const cplx f = Fq[idx], g = Gq[idx];
-            const double sr = P.scale[r];
-            Gq[idx] = cmk(__dadd_rn(__dmul_rn(sr, cre), __dmul_rn(P.omf, __dsub_rn(f.x, g.x))),
-                          __dadd_rn(__dmul_rn(sr, cim), __dmul_rn(P.omf, __dsub_rn(f.y, g.y))));
-          }
-        }
-      }
+      oz_epilogue(P, inst, m, np0, half, acc, rs, cs);
     }
   }
 
@@ -803,7 +865,7 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
 // barriers by multicast commits; each CTA's drain warps read their own TMEM
 // rows and arrive on the leader's accumulator-empty barrier.  Only the
 // tensor maps of this GPU's own memory are read, and no copy multicasts.
-constexpr int OZ2_STAGES = 8;  // 8 x (16 KB of A + <= 8 KB of B)
+constexpr int OZ2_STAGES = 14;  // 14 x one operand tile (16 KB of A or <= 8 KB of B)
 
 __device__ __forceinline__ uint32_t oz_cluster_rank() {
   uint32_t r;
@@ -892,8 +954,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
   const int NT = P.n_tile, HB = NT >> 1;  // B' rows staged by each CTA
   const uint32_t a_bytes = OZ_BM * OZ_BK, b_bytes = (uint32_t)HB * OZ_BK;
   const uint32_t dyn = (oz_smem(oz_dyn) + 1023u) & ~1023u;
-  auto sA = [&](int st) { return dyn + (uint32_t)st * (a_bytes + b_bytes); };
-  auto sB = [&](int st) { return dyn + (uint32_t)st * (a_bytes + b_bytes) + a_bytes; };
+  auto slot = [&](int st) { return dyn + (uint32_t)st * a_bytes; };
   const int per_inst = P.m_tiles * P.n_tiles;
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
 
@@ -936,27 +997,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
         const int inst = t / per_inst, rem = t % per_inst;
         const int m0 = (rem % P.m_tiles) * (2 * OZ_BM) + (int)crank * OZ_BM;
         const int n0 = (rem / P.m_tiles) * NT + (int)crank * HB;
-        for (int d = 0; d < P.s && ok; d++)
-          for (int i = 0; i <= d && ok; i++) {
-            const int ya = (inst * P.s + i) * P.M + m0;
-            const int yb = (inst * P.s + (d - i)) * Np + n0;
-            for (int kc = 0; kc < P.kchunks; kc++) {
+        for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2)
+          for (int kc = 0; kc < P.kchunks && ok; kc++)
+            for (int x = 0; x < 2 * d1 + 2; x++) {
               if (!mbar_wait_cl(&empty_bar[stage], phase ^ 1u, &abort_sh, true, P.wait_cycles)) {
                 ok = false;
                 break;
               }
               // the leader's stage-full barrier counts both CTAs' bytes
-              if (leader) mbar_expect_tx(&full_bar[stage], 2 * (a_bytes + b_bytes));
               const uint32_t fb = oz_mapa(oz_smem(&full_bar[stage]), 0);
-              tma_load_2d_pair(sA(stage), &tmA, kc * OZ_BK, ya, fb);
-              tma_load_2d_pair(sB(stage), &tmB, kc * OZ_BK, yb, fb);
+              if (leader) mbar_expect_tx(&full_bar[stage], 2 * (x & 1 ? a_bytes : b_bytes));
+              if (x & 1)
+                tma_load_2d_pair(slot(stage), &tmA, kc * OZ_BK, (inst * P.s + (x >> 1)) * P.M + m0, fb);
+              else
+                tma_load_2d_pair(slot(stage), &tmB, kc * OZ_BK, (inst * P.s + d1 - (x >> 1)) * Np + n0, fb);
               issued++;
               if (++stage == OZ2_STAGES) {
                 stage = 0;
                 phase ^= 1u;
               }
             }
-          }
       }
       issued_sh = issued;
     }
@@ -972,38 +1032,44 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
       bool ok = true;
       if (P.stall_test) ok = mbar_wait(&never_bar, 0, &abort_sh, true, P.wait_cycles);
       for (int t = cid; t < P.tiles && ok; t += ncl)
-        for (int d = 0; d < P.s && ok; d++, nacc++) {
-          const int buf = nacc % OZ_NBUF;
-          if (nacc >= OZ_NBUF &&
-              !mbar_wait_cl(&acce_bar[buf], (uint32_t)((nacc - OZ_NBUF) / OZ_NBUF) & 1u, &abort_sh, true,
-                            P.wait_cycles)) {
-            ok = false;
-            break;
+        for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2) {
+          const int nb = d1 > 0 ? 2 : 1;
+          for (int b = 0; b < nb && ok; b++) {
+            const int n = nacc + b;
+            if (n >= OZ_NBUF)
+              ok = mbar_wait_cl(&acce_bar[n % OZ_NBUF], (uint32_t)((n - OZ_NBUF) / OZ_NBUF) & 1u, &abort_sh, true,
+                                P.wait_cycles);
           }
           tc_fence_after();
-          const uint32_t dtm = tmem + (uint32_t)(buf * OZ_MAX_NT);
-          uint32_t accum = 0;
-          for (int i = 0; i <= d && ok; i++)
-            for (int kc = 0; kc < P.kchunks; kc++) {
-              if (!mbar_wait_cl(&full_bar[stage], phase, &abort_sh, true, P.wait_cycles)) {
-                ok = false;
-                break;
-              }
-              consumed++;
-              tc_fence_after();
-              const uint64_t da = oz_desc(sA(stage)), db = oz_desc(sB(stage));
-#pragma unroll
-              for (int kk = 0; kk < OZ_BK / 32; kk++) {
-                tc_mma_i8_pair(dtm, da + 2 * kk, db + 2 * kk, idesc, accum);
-                accum = 1;
-              }
-              tc_commit_pair(&empty_bar[stage], 0x3);
-              if (++stage == OZ2_STAGES) {
-                stage = 0;
-                phase ^= 1u;
-              }
+          const uint32_t dt0 = tmem + (uint32_t)((nacc + nb - 1) % OZ_NBUF * OZ_MAX_NT);
+          const uint32_t dt1 = tmem + (uint32_t)(nacc % OZ_NBUF * OZ_MAX_NT);
+          auto next = [&](int& st) {
+            if (!mbar_wait_cl(&full_bar[stage], phase, &abort_sh, true, P.wait_cycles)) return false;
+            consumed++;
+            st = stage;
+            if (++stage == OZ2_STAGES) {
+              stage = 0;
+              phase ^= 1u;
             }
-          if (ok) tc_commit_pair(&accf_bar[buf], 0x3);
+            return true;
+          };
+          for (int kc = 0; kc < P.kchunks && ok; kc++) {
+            int cur, nxt;
+            if (!(ok = next(cur))) break;
+            for (int x = 0; x <= 2 * d1; x++) {
+              if (!(ok = next(nxt))) break;
+              tc_fence_after();
+              const uint64_t da = oz_desc(slot(x & 1 ? cur : nxt)), db = oz_desc(slot(x & 1 ? nxt : cur));
+              const uint32_t dtm = x & 1 ? dt1 : dt0;
+#pragma unroll
+              for (int kk = 0; kk < OZ_BK / 32; kk++)
+                tc_mma_i8_pair(dtm, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || x > 1 || kk > 0);
+              tc_commit_pair(&empty_bar[cur], 0x3);
+              cur = nxt;
+            }
+            if (ok) tc_commit_pair(&empty_bar[cur], 0x3);
+          }
+          for (int b = 0; b < nb && ok; b++, nacc++) tc_commit_pair(&accf_bar[nacc % OZ_NBUF], 0x3);
         }
       consumed_sh = consumed;
       tc_commit_pair(&done_bar, 0x1);
@@ -1023,7 +1089,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
       const int m0 = (rem % P.m_tiles) * (2 * OZ_BM) + (int)crank * OZ_BM;
       const int n0 = (rem / P.m_tiles) * NT;
       const int m = m0 + row;
-      const bool mok = m < P.M;
+      const int np0 = n0 + h * half;
+      // the scales, long before their use
+      const double rs = m < P.M ? __ldg(P.rscale + (size_t)inst * P.M + m) : 0.0;
+      const double cs = 2 * lane < half && (np0 >> 1) + lane < P.N ? __ldg(P.cscale + (size_t)inst * P.N + (np0 >> 1) + lane) : 0.0;
 #pragma unroll
       for (int c = 0; c < OZ_HALF; c++) acc[c] = 0.0;
       for (int d = 0; d < P.s; d++, nacc++) {
@@ -1035,62 +1104,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
         tc_fence_after();
         const double w = ldexp(1.0, -OZ_SLICE_BITS * (d + 2));
         const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * OZ_MAX_NT + h * half);
-#pragma unroll
-        for (int c = 0; c < OZ_HALF; c += 8) {
-          if (c < half) {
-            int32_t v[8];
-            tc_ld8(tb + (uint32_t)c, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int e = 0; e < 8; e++) acc[c + e] = fma((double)v[e], w, acc[c + e]);
-          }
-        }
+        oz_fold(tb, half, w, acc);
         tc_fence_before();
         mbar_arrive_remote(acce_leader0 + (uint32_t)(buf * sizeof(uint64_t)));
       }
       if (!ok) break;
-      if (!mok) continue;
-      const double rs = P.rscale[(size_t)inst * P.M + m];
-      cplx* Cq = nullptr;
-      const cplx* Fq = nullptr;
-      cplx* Gq = nullptr;
-      int r = 0;
-      if (P.epi == OZ_EPI_BSE) {
-        const int q = P.q_begin + inst / 4;
-        r = inst % 4;
-        const cplx* Fr = r == 0 ? P.F[0] : r == 1 ? P.F[1] : r == 2 ? P.F[2] : P.F[3];
-        cplx* Gr = r == 0 ? P.G[0] : r == 1 ? P.G[1] : r == 2 ? P.G[2] : P.G[3];
-        Fq = Fr + (size_t)P.M * P.M * q;
-        Gq = Gr + (size_t)P.M * P.M * q;
-      } else if (P.epi == OZ_EPI_SUB) {
-        Cq = P.C + (size_t)inst * P.c_stride;
-      } else {
-        Cq = P.C + (size_t)inst * P.M * P.N;
-      }
-      const double sr = r == 0 ? P.scale[0] : r == 1 ? P.scale[1] : r == 2 ? P.scale[2] : P.scale[3];
-#pragma unroll
-      for (int c = 0; c < OZ_HALF; c += 2) {
-        const int np = n0 + h * half + c;
-        if (c < half && np < Np) {
-          const int jc = np >> 1;
-          const double sc = rs * P.cscale[(size_t)inst * P.N + jc];
-          const double cre = acc[c] * sc, cim = acc[c + 1] * sc;
-          if (P.epi == OZ_EPI_SUB) {
-            const size_t ix = m + (size_t)P.ldc * jc;
-            const cplx c0 = Cq[ix];
-            Cq[ix] = cmk(c0.x - cre, c0.y - cim);
-            continue;
-          }
-          const size_t idx = m + (size_t)P.M * jc;
-          if (P.epi == OZ_EPI_ZGEMM) {
-            Cq[idx] = cmk(cre, cim);
-          } else {
-            const cplx f = Fq[idx], g = Gq[idx];
-            Gq[idx] = cmk(__dadd_rn(__dmul_rn(sr, cre), __dmul_rn(P.omf, __dsub_rn(f.x, g.x))),
-                          __dadd_rn(__dmul_rn(sr, cim), __dmul_rn(P.omf, __dsub_rn(f.y, g.y))));
-          }
-        }
-      }
+      oz_epilogue(P, inst, m, np0, half, acc, rs, cs);
     }
   }
 
@@ -1176,9 +1195,8 @@ int oz_n_tile(int N) {
   return best;
 }
 
-size_t oz_smem_bytes(int n_tile) {
-  size_t s = (size_t)OZ_STAGES * (OZ_BM * OZ_BK + (size_t)n_tile * OZ_BK) + 1024;
-  return std::max<size_t>(s, 120 * 1024);  // one CTA per SM: the CTA owns all 512 TMEM columns
+size_t oz_smem_bytes() {  // > half of the SM's: the CTA owns all 512 TMEM columns
+  return (size_t)OZ_STAGES * OZ_STAGE_BYTES + 1024;
 }
 
 OzWork oz_work_layout(int batch, int M, int N, int K, int s) {
@@ -1307,7 +1325,7 @@ int oz_run(OzRun& R, cudaStream_t stream, long long* launches) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaError_t e;
   if (pairs) {
-    const size_t smem = (size_t)OZ2_STAGES * (OZ_BM * OZ_BK + (size_t)(P.n_tile / 2) * OZ_BK) + 1024;
+    const size_t smem = (size_t)OZ2_STAGES * OZ_BM * OZ_BK + 1024;
     e = cudaFuncSetAttribute(k_oz_gemm2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return oz_fail("k_oz_gemm2 shared memory attribute", e);
     const int grid = 2 * std::max(1, std::min(P.tiles, sms / 2));
@@ -1316,7 +1334,7 @@ int oz_run(OzRun& R, cudaStream_t stream, long long* launches) {
     e = cudaGetLastError();
     return e == cudaSuccess ? TUPS_OK : oz_fail("k_oz_gemm2 launch", e);
   }
-  const size_t smem = oz_smem_bytes(P.n_tile);
+  const size_t smem = oz_smem_bytes();
   e = cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return oz_fail("k_oz_gemm shared memory attribute", e);
   const int grid = std::max(1, std::min(P.tiles, sms));

@@ -865,7 +865,8 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
 // barriers by multicast commits; each CTA's drain warps read their own TMEM
 // rows and arrive on the leader's accumulator-empty barrier.  Only the
 // tensor maps of this GPU's own memory are read, and no copy multicasts.
-constexpr int OZ2_STAGES = 14;  // 14 x one operand tile (16 KB of A or <= 8 KB of B)
+constexpr int OZ2_STAGES = 9;  // 9 x (16 KB of A + <= 8 KB of B)
+constexpr uint32_t OZ2_STAGE_BYTES = OZ_BM * OZ_BK + OZ_HALF * OZ_BK;
 
 __device__ __forceinline__ uint32_t oz_cluster_rank() {
   uint32_t r;
@@ -895,6 +896,7 @@ __device__ __forceinline__ bool mbar_try_cl(uint64_t* bar, uint32_t parity) {
 // bounded wait with cluster-scope acquire (barriers that other CTAs signal)
 __device__ __forceinline__ bool mbar_wait_cl(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                              bool honor_abort = true, long long limit = OZ_WAIT_CYCLES) {
+  if (mbar_try_cl(bar, parity)) return true;
   const long long t0 = clock64();
   for (uint32_t it = 0;; it++) {
     if (mbar_try_cl(bar, parity)) return true;
@@ -947,14 +949,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
   __shared__ volatile int abort_sh;
   __shared__ int issued_sh, consumed_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)oz_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t crank = oz_cluster_rank();
   const bool leader = crank == 0;
   const int Np = 2 * P.N;
   const int NT = P.n_tile, HB = NT >> 1;  // B' rows staged by each CTA
   const uint32_t a_bytes = OZ_BM * OZ_BK, b_bytes = (uint32_t)HB * OZ_BK;
   const uint32_t dyn = (oz_smem(oz_dyn) + 1023u) & ~1023u;
-  auto slot = [&](int st) { return dyn + (uint32_t)st * a_bytes; };
+  auto slot_a = [&](int st) { return dyn + (uint32_t)st * OZ2_STAGE_BYTES; };
+  auto slot_b = [&](int st) { return dyn + (uint32_t)st * OZ2_STAGE_BYTES + OZ_BM * OZ_BK; };
   const int per_inst = P.m_tiles * P.n_tiles;
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
 
@@ -984,7 +987,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
   // both CTAs' barriers exist before either CTA signals the other's
   oz_cluster_sync();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_sh;
+  const uint32_t tmem = oz_uniform(tmem_base_sh);
 
   if (warp == OZ_DRAIN_WARPS + 1) {
     // ---- TMA producer (both CTAs): own rows of A, own half of B' ----
@@ -999,18 +1002,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
         const int n0 = (rem / P.m_tiles) * NT + (int)crank * HB;
         for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2)
           for (int kc = 0; kc < P.kchunks && ok; kc++)
-            for (int x = 0; x < 2 * d1 + 2; x++) {
+            for (int i = 0; i <= d1; i++) {
               if (!mbar_wait_cl(&empty_bar[stage], phase ^ 1u, &abort_sh, true, P.wait_cycles)) {
                 ok = false;
                 break;
               }
               // the leader's stage-full barrier counts both CTAs' bytes
+              if (leader) mbar_expect_tx(&full_bar[stage], 2 * (a_bytes + b_bytes));
               const uint32_t fb = oz_mapa(oz_smem(&full_bar[stage]), 0);
-              if (leader) mbar_expect_tx(&full_bar[stage], 2 * (x & 1 ? a_bytes : b_bytes));
-              if (x & 1)
-                tma_load_2d_pair(slot(stage), &tmA, kc * OZ_BK, (inst * P.s + (x >> 1)) * P.M + m0, fb);
-              else
-                tma_load_2d_pair(slot(stage), &tmB, kc * OZ_BK, (inst * P.s + d1 - (x >> 1)) * Np + n0, fb);
+              tma_load_2d_pair(slot_b(stage), &tmB, kc * OZ_BK, (inst * P.s + d1 - i) * Np + n0, fb);
+              tma_load_2d_pair(slot_a(stage), &tmA, kc * OZ_BK, (inst * P.s + i) * P.M + m0, fb);
               issued++;
               if (++stage == OZ2_STAGES) {
                 stage = 0;
@@ -1022,58 +1023,73 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
     }
   } else if (warp == OZ_DRAIN_WARPS) {
     // ---- MMA issuer: the leader only ----
-    if (lane == 0 && leader) {
+    // the whole warp walks the schedule, so that it is uniform; one lane issues
+    if (leader) {
+      const bool el = oz_elect();
+      auto wait = [&](uint64_t* bar, uint32_t ph) {
+        return __all_sync(0xffffffffu, mbar_wait_cl(bar, ph, &abort_sh, true, P.wait_cycles)) != 0;
+      };
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) |
                              ((uint32_t)((2 * OZ_BM) >> 4) << 24);
+      const uint64_t desc0 = oz_desc(dyn);  // of stage 0's A; the address counts 16 bytes
       int stage = 0;
       uint32_t phase = 0;
       int consumed = 0;
-      int nacc = 0;
+      int nacc = 0;  // accumulations issued so far (one per tile and diagonal)
       bool ok = true;
-      if (P.stall_test) ok = mbar_wait(&never_bar, 0, &abort_sh, true, P.wait_cycles);
+      // failure-path test: a wait that can only run out, before any MMA
+      if (P.stall_test) ok = wait(&never_bar, 0);
       for (int t = cid; t < P.tiles && ok; t += ncl)
         for (int d1 = (P.s & 1) ? 0 : 1; d1 < P.s && ok; d1 += 2) {
-          const int nb = d1 > 0 ? 2 : 1;
+          const int nb = d1 > 0 ? 2 : 1;  // diagonals of this step
           for (int b = 0; b < nb && ok; b++) {
             const int n = nacc + b;
             if (n >= OZ_NBUF)
-              ok = mbar_wait_cl(&acce_bar[n % OZ_NBUF], (uint32_t)((n - OZ_NBUF) / OZ_NBUF) & 1u, &abort_sh, true,
-                                P.wait_cycles);
+              ok = wait(&acce_bar[n % OZ_NBUF], (uint32_t)((n - OZ_NBUF) / OZ_NBUF) & 1u);
           }
           tc_fence_after();
-          const uint32_t dt0 = tmem + (uint32_t)((nacc + nb - 1) % OZ_NBUF * OZ_MAX_NT);
-          const uint32_t dt1 = tmem + (uint32_t)(nacc % OZ_NBUF * OZ_MAX_NT);
-          auto next = [&](int& st) {
-            if (!mbar_wait_cl(&full_bar[stage], phase, &abort_sh, true, P.wait_cycles)) return false;
-            consumed++;
-            st = stage;
-            if (++stage == OZ2_STAGES) {
-              stage = 0;
-              phase ^= 1u;
-            }
-            return true;
-          };
+          const uint32_t dt1 = tmem + (uint32_t)((nacc + nb - 1) % OZ_NBUF * OZ_MAX_NT);
+          const uint32_t dt0 = tmem + (uint32_t)(nacc % OZ_NBUF * OZ_MAX_NT);
           for (int kc = 0; kc < P.kchunks && ok; kc++) {
-            int cur, nxt;
-            if (!(ok = next(cur))) break;
-            for (int x = 0; x <= 2 * d1; x++) {
-              if (!(ok = next(nxt))) break;
+            uint64_t da = 0;
+            int prev = 0;
+            for (int i = 0; i <= d1; i++) {
+              if (!wait(&full_bar[stage], phase)) {
+                ok = false;
+                break;
+              }
+              consumed++;
               tc_fence_after();
-              const uint64_t da = oz_desc(slot(x & 1 ? cur : nxt)), db = oz_desc(slot(x & 1 ? nxt : cur));
-              const uint32_t dtm = x & 1 ? dt1 : dt0;
+              const uint64_t db = desc0 + (uint32_t)(stage * (int)(OZ2_STAGE_BYTES >> 4)) + (OZ_BM * OZ_BK >> 4);
+              if (i > 0 && el) {  // A_(i-1) B_(d1-i): diagonal d1 - 1
 #pragma unroll
-              for (int kk = 0; kk < OZ_BK / 32; kk++)
-                tc_mma_i8_pair(dtm, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || x > 1 || kk > 0);
-              tc_commit_pair(&empty_bar[cur], 0x3);
-              cur = nxt;
+                for (int kk = 0; kk < OZ_BK / 32; kk++)
+                  tc_mma_i8_pair(dt0, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || i > 1 || kk > 0);
+                tc_commit_pair(&empty_bar[prev], 0x3);
+              }
+              da = desc0 + (uint32_t)(stage * (int)(OZ2_STAGE_BYTES >> 4));
+              if (el) {
+#pragma unroll
+                for (int kk = 0; kk < OZ_BK / 32; kk++)
+                  tc_mma_i8_pair(dt1, da + 2 * kk, db + 2 * kk, idesc, kc > 0 || i > 0 || kk > 0);
+              }
+              prev = stage;
+              if (++stage == OZ2_STAGES) {
+                stage = 0;
+                phase ^= 1u;
+              }
             }
-            if (ok) tc_commit_pair(&empty_bar[cur], 0x3);
+            if (ok && el) tc_commit_pair(&empty_bar[prev], 0x3);
           }
-          for (int b = 0; b < nb && ok; b++, nacc++) tc_commit_pair(&accf_bar[nacc % OZ_NBUF], 0x3);
+          for (int b = 0; b < nb && ok; b++, nacc++)
+            if (el) tc_commit_pair(&accf_bar[nacc % OZ_NBUF], 0x3);
         }
-      consumed_sh = consumed;
-      tc_commit_pair(&done_bar, 0x1);
-      mbar_wait_cl(&done_bar, 0, &abort_sh, false);
+      if (el) {
+        consumed_sh = consumed;
+        tc_commit_pair(&done_bar, 0x1);
+        mbar_wait_cl(&done_bar, 0, &abort_sh, false);
+      }
+      __syncwarp();
     }
   } else {
     // ---- drain (both CTAs): own TMEM lanes = own 128 rows of the pair tile ----
@@ -1325,7 +1341,7 @@ int oz_run(OzRun& R, cudaStream_t stream, long long* launches) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaError_t e;
   if (pairs) {
-    const size_t smem = (size_t)OZ2_STAGES * OZ_BM * OZ_BK + 1024;
+    const size_t smem = (size_t)OZ2_STAGES * OZ2_STAGE_BYTES + 1024;
     e = cudaFuncSetAttribute(k_oz_gemm2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return oz_fail("k_oz_gemm2 shared memory attribute", e);
     const int grid = 2 * std::max(1, std::min(P.tiles, sms / 2));

@@ -549,7 +549,9 @@ __device__ __forceinline__ uint32_t oz_uniform(uint32_t v) { return __shfl_sync(
 // diagonals per stage; 490 with one wait and one commit per two products; 430
 // with a warp-uniform schedule and one elected lane; 397 with the drain in loads of
 // 16 columns, FP64 conversions by addition and four columns' reads ahead (2.6
-// POPS).
+// POPS).  Then it is near what shared memory gives: 16 KB of copies and 32 KB
+// of operand reads per product, 384 cycles at 128 bytes per cycle, 367 measured;
+// the drain runs four times slower under the MMAs than alone for the same reason.
 enum { OZ_EPI_ZGEMM = 0, OZ_EPI_BSE = 1, OZ_EPI_SUB = 2 };
 
 constexpr int OZ_NBUF = 4;            // TMEM accumulator buffers
@@ -600,57 +602,75 @@ __device__ __forceinline__ void oz_fold(uint32_t tb, int half, double w, double*
   }
 }
 
+// where the epilogue of an instance reads and writes
+struct OzOut {
+  const cplx* in;  // F (BSE only)
+  cplx* out;
+  size_t ld;
+  double scale;
+};
+template <int EPI>
+__device__ __forceinline__ OzOut oz_out(const OzGemm& P, int inst) {
+  OzOut o = {nullptr, nullptr, (size_t)P.M, 1.0};
+  if constexpr (EPI == OZ_EPI_BSE) {
+    const int r = inst & 3;
+    const size_t at = (size_t)P.M * P.M * (P.q_begin + (inst >> 2));
+    o.in = (r == 0 ? P.F[0] : r == 1 ? P.F[1] : r == 2 ? P.F[2] : P.F[3]) + at;
+    o.out = (r == 0 ? P.G[0] : r == 1 ? P.G[1] : r == 2 ? P.G[2] : P.G[3]) + at;
+    o.scale = r == 0 ? P.scale[0] : r == 1 ? P.scale[1] : r == 2 ? P.scale[2] : P.scale[3];
+  } else if constexpr (EPI == OZ_EPI_SUB) {
+    o.out = P.C + (size_t)inst * P.c_stride;
+    o.ld = P.ldc;
+  } else {
+    o.out = P.C + (size_t)inst * P.M * P.N;
+  }
+  return o;
+}
+
 // scales and epilogue of one row m: acc[0 .. half) are the real columns np0 ..,
 // lane l of the warp holds the column scale of complex column np0 / 2 + l.  The
-// reads of four columns go out before their writes, which could alias the next.
+// reads of four columns go out together, before writes that they could alias;
+// rows and columns beyond the matrix read its last ones and write nothing.
+template <int EPI>
 __device__ __forceinline__ void oz_epilogue(const OzGemm& P, int inst, int m, int np0, int half, const double* acc,
                                             double rs, double cs) {
-  const bool mok = m < P.M;
   const int jc0 = np0 >> 1, nj = min(half >> 1, P.N - jc0);
-  const int r = inst & 3, q = P.q_begin + (inst >> 2);
-  const cplx* rd1 = nullptr;
-  cplx* out;
-  size_t ld = P.M;
-  double sr = 1.0;
-  if (P.epi == OZ_EPI_BSE) {
-    const size_t o = (size_t)P.M * P.M * q;
-    rd1 = (r == 0 ? P.F[0] : r == 1 ? P.F[1] : r == 2 ? P.F[2] : P.F[3]) + o;
-    out = (r == 0 ? P.G[0] : r == 1 ? P.G[1] : r == 2 ? P.G[2] : P.G[3]) + o;
-    sr = r == 0 ? P.scale[0] : r == 1 ? P.scale[1] : r == 2 ? P.scale[2] : P.scale[3];
-  } else if (P.epi == OZ_EPI_SUB) {
-    out = P.C + (size_t)inst * P.c_stride;
-    ld = P.ldc;
-  } else {
-    out = P.C + (size_t)inst * P.M * P.N;
-  }
+  const OzOut o = oz_out<EPI>(P, inst);
+  const size_t ld = o.ld;
+  cplx* out = o.out + ld * jc0;
+  const cplx* in = EPI == OZ_EPI_BSE ? o.in + ld * jc0 : nullptr;
+  const double sr = o.scale;
+  const int mr = min(m, P.M - 1);
 #pragma unroll
   for (int c0 = 0; c0 < OZ_HALF / 2; c0 += 4) {
     if (c0 >= nj) continue;
     cplx f[4], g[4];
+    if constexpr (EPI != OZ_EPI_ZGEMM) {
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const size_t ix = m + ld * (jc0 + c0 + c);
-      const bool ok = mok && c0 + c < nj;
-      f[c] = ok && P.epi == OZ_EPI_BSE ? rd1[ix] : cmk(0.0, 0.0);
-      g[c] = ok && P.epi != OZ_EPI_ZGEMM ? out[ix] : cmk(0.0, 0.0);
+      for (int c = 0; c < 4; c++) {
+        const size_t ix = mr + ld * min(c0 + c, nj - 1);
+        if constexpr (EPI == OZ_EPI_BSE) f[c] = in[ix];
+        g[c] = out[ix];
+      }
     }
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const size_t ix = m + ld * (jc0 + c0 + c);
       const double sc = rs * __shfl_sync(0xffffffffu, cs, c0 + c);
       const double cre = acc[2 * (c0 + c)] * sc, cim = acc[2 * (c0 + c) + 1] * sc;
-      if (!mok || c0 + c >= nj) continue;
-      if (P.epi == OZ_EPI_ZGEMM)
-        out[ix] = cmk(cre, cim);
-      else if (P.epi == OZ_EPI_SUB)
-        out[ix] = cmk(g[c].x - cre, g[c].y - cim);
+      cplx v;
+      if constexpr (EPI == OZ_EPI_ZGEMM)
+        v = cmk(cre, cim);
+      else if constexpr (EPI == OZ_EPI_SUB)
+        v = cmk(g[c].x - cre, g[c].y - cim);
       else
-        out[ix] = cmk(__dadd_rn(__dmul_rn(sr, cre), __dmul_rn(P.omf, __dsub_rn(f[c].x, g[c].x))),
-                      __dadd_rn(__dmul_rn(sr, cim), __dmul_rn(P.omf, __dsub_rn(f[c].y, g[c].y))));
+        v = cmk(__dadd_rn(__dmul_rn(sr, cre), __dmul_rn(P.omf, __dsub_rn(f[c].x, g[c].x))),
+                __dadd_rn(__dmul_rn(sr, cim), __dmul_rn(P.omf, __dsub_rn(f[c].y, g[c].y))));
+      if (m < P.M && c0 + c < nj) out[m + ld * (c0 + c)] = v;
     }
   }
 }
 
+template <int EPI>
 __global__ void __launch_bounds__(OZ_THREADS2, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OzGemm P) {
   extern __shared__ uint8_t oz_dyn[];
@@ -827,7 +847,7 @@ __global__ void __launch_bounds__(OZ_THREADS2, 1)
         mbar_arrive(&acce_bar[buf]);
       }
       if (!ok) break;
-      oz_epilogue(P, inst, m, np0, half, acc, rs, cs);
+      oz_epilogue<EPI>(P, inst, m, np0, half, acc, rs, cs);
     }
   }
 
@@ -940,6 +960,7 @@ __device__ __forceinline__ void tc_mma_i8_pair(uint32_t d_tmem, uint64_t adesc, 
 }
 
 // P.m_tiles counts 256-row pair tiles here
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
     k_oz_gemm2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OzGemm P) {
   extern __shared__ uint8_t oz_dyn[];
@@ -1125,7 +1146,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS2, 1)
         mbar_arrive_remote(acce_leader0 + (uint32_t)(buf * sizeof(uint64_t)));
       }
       if (!ok) break;
-      oz_epilogue(P, inst, m, np0, half, acc, rs, cs);
+      oz_epilogue<EPI>(P, inst, m, np0, half, acc, rs, cs);
     }
   }
 
@@ -1342,19 +1363,21 @@ int oz_run(OzRun& R, cudaStream_t stream, long long* launches) {
   cudaError_t e;
   if (pairs) {
     const size_t smem = (size_t)OZ2_STAGES * OZ2_STAGE_BYTES + 1024;
-    e = cudaFuncSetAttribute(k_oz_gemm2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto* kernel = P.epi == OZ_EPI_BSE ? k_oz_gemm2<OZ_EPI_BSE> : P.epi == OZ_EPI_SUB ? k_oz_gemm2<OZ_EPI_SUB> : k_oz_gemm2<OZ_EPI_ZGEMM>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return oz_fail("k_oz_gemm2 shared memory attribute", e);
     const int grid = 2 * std::max(1, std::min(P.tiles, sms / 2));
-    k_oz_gemm2<<<grid, OZ_THREADS2, smem, stream>>>(ta, tb, P);
+    kernel<<<grid, OZ_THREADS2, smem, stream>>>(ta, tb, P);
     if (launches) (*launches)++;
     e = cudaGetLastError();
     return e == cudaSuccess ? TUPS_OK : oz_fail("k_oz_gemm2 launch", e);
   }
   const size_t smem = oz_smem_bytes();
-  e = cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto* kernel = P.epi == OZ_EPI_BSE ? k_oz_gemm<OZ_EPI_BSE> : P.epi == OZ_EPI_SUB ? k_oz_gemm<OZ_EPI_SUB> : k_oz_gemm<OZ_EPI_ZGEMM>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return oz_fail("k_oz_gemm shared memory attribute", e);
   const int grid = std::max(1, std::min(P.tiles, sms));
-  k_oz_gemm<<<grid, OZ_THREADS2, smem, stream>>>(ta, tb, P);
+  kernel<<<grid, OZ_THREADS2, smem, stream>>>(ta, tb, P);
   if (launches) (*launches)++;
   e = cudaGetLastError();
   return e == cudaSuccess ? TUPS_OK : oz_fail("k_oz_gemm launch", e);

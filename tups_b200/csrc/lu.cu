@@ -399,21 +399,16 @@ __global__ void __launch_bounds__(256) k_lu_phi(const cplx* __restrict__ Gam, cp
     F[e] = tups::csub(F[e], G[e]);
 }
 
-// opt-in shared-memory sizes, once per device
-bool lu_prepare(int dev) {
-  static bool done[64] = {};
-  if (dev >= 0 && dev < 64 && done[dev]) return true;
+// opt-in shared-memory sizes on the current device
+bool lu_prepare() {
   const int ps = (int)sizeof(LuPanelShared), rs = (int)kRowsSmem;
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (cudaFuncSetAttribute(k_lu_panel<0>, attr, ps) != cudaSuccess ||
-      cudaFuncSetAttribute(k_lu_panel<1>, attr, ps) != cudaSuccess ||
-      cudaFuncSetAttribute(k_lu_panel<2>, attr, ps) != cudaSuccess ||
-      cudaFuncSetAttribute(k_lu_invert, attr, (int)kInvertSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_lu_rows<false>, attr, rs) != cudaSuccess ||
-      cudaFuncSetAttribute(k_lu_rows<true>, attr, rs) != cudaSuccess)
-    return false;
-  if (dev >= 0 && dev < 64) done[dev] = true;
-  return true;
+  return cudaFuncSetAttribute(k_lu_panel<0>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_lu_panel<1>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_lu_panel<2>, attr, ps) == cudaSuccess &&
+         cudaFuncSetAttribute(k_lu_invert, attr, (int)kInvertSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(k_lu_rows<false>, attr, rs) == cudaSuccess &&
+         cudaFuncSetAttribute(k_lu_rows<true>, attr, rs) == cudaSuccess;
 }
 
 }  // namespace
@@ -439,8 +434,7 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
   std::vector<LuDesc> queued(n_inst);
   for (int i = 0; i < n_inst; i++) queued[i] = desc[order[i]];
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || !lu_prepare(dev) ||
+  if (!lu_prepare() ||
       cudaMemcpyToSymbolAsync(g_lu_desc, queued.data(), n_inst * sizeof(LuDesc), 0, cudaMemcpyHostToDevice, st) !=
           cudaSuccess) {
     cudaGetLastError();

@@ -152,11 +152,13 @@ __global__ void __launch_bounds__(Tile::NT, MINB) k_bse_gemm(BsePtrs P, const cp
   Tile t;
   t.run(BseSource<BK>{A + n2 * inst, Fq, B + n2 * inst, Nz, m0, n0}, reinterpret_cast<cplx*>(smraw), Nz - m0, Nz - n0);
   // epilogue: Phi = s * C + (1-f) (F - Gamma), written over Gamma
-  t.each(Nz - m0, Nz - n0, [&](int row, int col, cplx c) {
-    const size_t idx = (m0 + row) + (size_t)Nz * (n0 + col);
-    const cplx f = Fq[idx], g = Gq[idx];
-    Gq[idx] = cmk(s * c.x + one_minus_f * (f.x - g.x), s * c.y + one_minus_f * (f.y - g.y));
-  });
+  const auto at = [&](int row, int col) { return (m0 + row) + (size_t)Nz * (n0 + col); };
+  t.each(
+      Nz - m0, Nz - n0, [&](int row, int col) { return ZgPair{Fq[at(row, col)], Gq[at(row, col)]}; },
+      [&](int row, int col, cplx c, const ZgPair& v) {
+        Gq[at(row, col)] =
+            cmk(s * c.x + one_minus_f * (v.a.x - v.b.x), s * c.y + one_minus_f * (v.a.y - v.b.y));
+      });
 }
 
 template <int TM, int TN, int WM, int WN, int BK, int ST, int MINB>

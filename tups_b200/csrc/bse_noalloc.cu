@@ -147,11 +147,13 @@ __global__ void __launch_bounds__(NaTile::NT, NB_PER_SM) k_noalloc_gemm(cplx* __
   NaTile t;
   t.run(tups::BseSource<NB_BK>{A + n2 * li, Fi, B + n2 * li, Nz, m0, n0}, reinterpret_cast<cplx*>(smraw), Nz - m0,
         Nz - n0);
-  t.each(Nz - m0, Nz - n0, [&](int row, int col, cplx c) {
-    const size_t e = (m0 + row) + (size_t)Nz * (n0 + col);
-    const cplx f = Fi[e], g = Gi[e];
-    Gi[e] = tups::cmk(s * c.x + one_minus_f * (f.x - g.x), s * c.y + one_minus_f * (f.y - g.y));
-  });
+  const auto at = [&](int row, int col) { return (m0 + row) + (size_t)Nz * (n0 + col); };
+  t.each(
+      Nz - m0, Nz - n0, [&](int row, int col) { return tups::ZgPair{Fi[at(row, col)], Gi[at(row, col)]}; },
+      [&](int row, int col, cplx c, const tups::ZgPair& v) {
+        Gi[at(row, col)] =
+            tups::cmk(s * c.x + one_minus_f * (v.a.x - v.b.x), s * c.y + one_minus_f * (v.a.y - v.b.y));
+      });
 }
 
 }  // namespace

@@ -376,16 +376,25 @@ __global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cpl
       }
     }
   }
+  // the old entries all go out before the first write, which could alias them
+  // (one after another they kept the kernel waiting: 96 instances 10.2 -> 9.3 ms)
+  cplx old[2][4];
 #pragma unroll
   for (int j = 0; j < 2; j++)
 #pragma unroll
     for (int x = 0; x < 4; x++) {
       const int row = m0 + wm0 + gid + (x >= 2 ? 8 : 0), col = n0 + wn0 + j * 8 + 2 * tig + (x & 1);
-      if (row < rows && col < width) {
-        cplx* c = rhs_column(A, F, n, right, col) + first + row;
-        const cplx v = *c;
-        *c = cmk(v.x - (p1[j][x] - p2[j][x]), v.y - (p3[j][x] - p1[j][x] - p2[j][x]));
-      }
+      old[j][x] = rhs_column(A, F, n, right, min(col, width - 1))[first + min(row, rows - 1)];
+    }
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int row = m0 + wm0 + gid + (x >= 2 ? 8 : 0), col = n0 + wn0 + j * 8 + 2 * tig + (x & 1);
+      const cplx v = old[j][x];
+      if (row < rows && col < width)
+        rhs_column(A, F, n, right, col)[first + row] =
+            cmk(v.x - (p1[j][x] - p2[j][x]), v.y - (p3[j][x] - p1[j][x] - p2[j][x]));
     }
 }
 

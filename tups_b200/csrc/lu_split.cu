@@ -196,10 +196,10 @@ __global__ void __launch_bounds__(LsTile::NT, 5) k_ls_mid(cplx* __restrict__ Ag,
   LsTile t;
   t.run(LsSource{A + j1 + m0 + (size_t)n * J0, A + J0 + (size_t)n * j1, n, j1 - J0, n0}, reinterpret_cast<cplx*>(smraw),
         rows, cols);
-  t.each(rows, cols, [&](int row, int col, cplx v) {
-    cplx* c = A + (j1 + m0 + row) + (size_t)n * (j1 + n0 + col);
-    *c = csub(*c, v);
-  });
+  cplx* C = A + (j1 + m0) + (size_t)n * (j1 + n0);
+  t.each(
+      rows, cols, [&](int row, int col) { return C[row + (size_t)n * col]; },
+      [&](int row, int col, cplx v, cplx c) { C[row + (size_t)n * col] = csub(c, v); });
 }
 
 // U_bb^{-1} over the upper 64 x 64 diagonal triangles, off the chain of panels
@@ -412,12 +412,14 @@ __global__ void __launch_bounds__(RsTile::NT, 3) k_ls_resid(const LsDesc* __rest
   t.run(LsSource{G + m0, Yg + n2 * i, n, n, n0}, reinterpret_cast<cplx*>(smraw), n - m0, n - n0);
   const double s = desc[i].scale;
   double mx = 0.0;
-  t.each(n - m0, n - n0, [&](int row, int col, cplx c) {
-    const size_t e = (m0 + row) + (size_t)n * (n0 + col);
-    const cplx g = G[e], x = X[e], v = cmk((g.x - x.x) + s * c.x, (g.y - x.y) + s * c.y);
-    R[e] = v;
-    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
-  });
+  const auto at = [&](int row, int col) { return (m0 + row) + (size_t)n * (n0 + col); };
+  t.each(
+      n - m0, n - n0, [&](int row, int col) { return ZgPair{G[at(row, col)], X[at(row, col)]}; },
+      [&](int row, int col, cplx c, const ZgPair& in) {
+        const cplx v = cmk((in.a.x - in.b.x) + s * c.x, (in.a.y - in.b.y) + s * c.y);
+        R[at(row, col)] = v;
+        mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+      });
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) atomic_max_nonneg(&rmax[i], mx);
 }

@@ -46,6 +46,10 @@ __device__ __forceinline__ void zg_dmma(double* c, const double* a, const double
 // 64-column LU update: 5 CTAs per SM 6.4 ms, 3 with AHEAD 9.6).
 //
 // WM x WN warps of 16 TM x 8 TN
+struct ZgPair {
+  cplx a, b;
+};
+
 template <int TM, int TN, int WM, int WN, int BK, int ST, bool M3, bool AHEAD = true>
 struct ZgemmTile {
   static constexpr int BM = 16 * TM * WM, BN = 8 * TN * WN, NW = WM * WN, NT = 32 * NW;
@@ -218,6 +222,34 @@ struct ZgemmTile {
           if (row < rows && col < cols)
             f(row, col, M3 ? cmk(p1[i][j][e] - p2[i][j][e], p3[M3 ? i : 0][M3 ? j : 0][e] - p1[i][j][e] - p2[i][j][e])
                            : cmk(p1[i][j][e], p2[i][j][e]));
+        }
+  }
+
+  // the same with what f reads: get(row, col) of all of this thread's entries
+  // goes out before the first f writes.  The writes could alias the reads, so
+  // that otherwise each entry's reads wait for memory in turn.  Entries
+  // outside the matrix get its last row or column and see no f.
+  template <class G, class F>
+  __device__ __forceinline__ void each(int rows, int cols, G get, F f) const {
+    decltype(get(0, 0)) in[TM][TN][4];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          in[i][j][e] = get(min(wm0 + 16 * i + gid + (e >= 2 ? 8 : 0), rows - 1),
+                            min(wn0 + 8 * j + 2 * tig + (e & 1), cols - 1));
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int row = wm0 + 16 * i + gid + (e >= 2 ? 8 : 0), col = wn0 + 8 * j + 2 * tig + (e & 1);
+          if (row < rows && col < cols)
+            f(row, col, M3 ? cmk(p1[i][j][e] - p2[i][j][e], p3[M3 ? i : 0][M3 ? j : 0][e] - p1[i][j][e] - p2[i][j][e])
+                           : cmk(p1[i][j][e], p2[i][j][e]), in[i][j][e]);
         }
   }
 };

@@ -142,3 +142,141 @@ def test_batched_lu_at_block_edges(gpu_lib):
     ref = LU.bse_lu(g, inst.chi[0], 1.0)
     cond = np.linalg.cond(np.eye(n) - g)
     assert np.abs(solve(inst)[0] - ref).max() <= 4 * n * 2.3e-16 * cond * np.abs(ref).max()
+
+
+def _unit_chi_instances(mats):
+    """A x = (I - A) for each matrix A: Gamma = I - A with one form factor and chi = 1."""
+    from tups_b200.bse_batched import Instances
+    n = np.array([a.shape[0] for a in mats], dtype=np.int32)
+    return Instances(n=n, nl=np.ones(len(mats), dtype=np.int32), scale=np.ones(len(mats)),
+                     gamma=[np.asfortranarray(np.eye(a.shape[0]) - a) for a in mats],
+                     chi=[np.ones((1, 1, k), dtype=np.complex128, order="F") for k in n],
+                     q=np.zeros((len(mats), 3), dtype=np.int32))
+
+
+def _residual_over_factors(g, x):
+    """max |Gamma - A X| / (|L| |U| |X|) with LAPACK's factors of A = 1 - Gamma."""
+    import scipy.linalg as sl
+    n = g.shape[0]
+    a = np.eye(n) - g
+    lu, piv = sl.lu_factor(a)
+    p = np.arange(n)
+    for i, k in enumerate(piv):
+        p[[i, k]] = p[[k, i]]
+    low, up = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+    r = np.abs(g.astype(np.clongdouble) - a.astype(np.clongdouble) @ x)[p].astype(float)
+    return (r / np.maximum(np.abs(low) @ (np.abs(up) @ np.abs(x)), 1e-300)).max()
+
+
+def _hard_matrices(n):
+    rng = np.random.default_rng(n)
+    z = lambda: rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    u, v = (np.linalg.qr(z())[0] for _ in range(2))
+    s = np.logspace(6, -6, n)
+    h = z()
+    w, q = np.linalg.eigh(h + h.conj().T)
+    w *= 0.9 / np.abs(w).max()
+    w[-1] = 1.0 - 1e-8
+    return [z(), z() * s[None, :], z() * s[:, None], z() * np.sqrt(s)[:, None] / np.sqrt(s)[None, :],
+            (u * np.logspace(0, -6, n)) @ v, (u * np.logspace(0, -10, n)) @ v, np.eye(n) - (q * w) @ q.conj().T]
+
+
+# The factorisation and the two triangular solves each leave a residual of sums of n complex products, 2 sqrt(2)
+# units of rounding each, that add up as their square root: 3 x 2.83 sqrt(n) units of |L| |U| |X|
+def _residual_bound(n):
+    return 8.5 * np.sqrt(n) * 1.11e-16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [50, 130, 300])
+def test_batched_lu_is_backward_stable(gpu_lib, n):
+    """Condition numbers of 1e6 and 1e10, rows and columns over twelve decades, 1 - Gamma chi next to singular: the
+    residual stays that of substitution with the factors."""
+    from tups_b200.bse_batched import solve
+    inst = _unit_chi_instances(_hard_matrices(n))
+    for i, x in enumerate(solve(inst)):
+        r = _residual_over_factors(inst.gamma[i], x)
+        assert r <= _residual_bound(n), (i, r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [50, 128])
+def test_unsplit_blocks_of_the_split_lu_are_backward_stable(gpu_lib, n):
+    """Up to 128 columns nothing runs on int8 slices: the same bound without a correction."""
+    from tups_b200.bse_batched import solve_split
+    inst = _unit_chi_instances(_hard_matrices(n))
+    for i, x in enumerate(solve_split(inst, slices=8, max_refine=0)[0]):
+        r = _residual_over_factors(inst.gamma[i], x)
+        assert r <= _residual_bound(n), (i, r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [64, 129, 300])
+def test_batched_lu_keeps_small_imaginary_parts(gpu_lib, n):
+    """A real to 1e-8: the imaginary part of the solution has the relative error of the real one (4 n eps cond,
+    cond(A) of the real part), since every product of the imaginary parts' sums is small."""
+    from tups_b200.bse_batched import solve
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1e-8j * rng.standard_normal((n, n))
+    inst = _unit_chi_instances([a])
+    g = inst.gamma[0]
+    a = np.eye(n) - g
+    ref = LU.bse_lu(g, inst.chi[0], 1.0).astype(np.clongdouble)
+    for _ in range(3):
+        r = g.astype(np.clongdouble) - a.astype(np.clongdouble) @ ref
+        ref += np.linalg.solve(a, r.real.astype(float)) + 1j * np.linalg.solve(a, r.imag.astype(float))
+    err = np.abs((solve(inst)[0] - ref).imag).max() / np.abs(ref.imag).max()
+    assert err <= 4 * n * 2.3e-16 * np.linalg.cond(a), err
+
+
+def _edge_instances(sizes, seed):
+    """One form factor, chi diagonal in the frequency; |Gamma chi|_2 <= 0.9, so |A^-1|_2 <= 10."""
+    from tups_b200.bse_batched import Instances
+    rng = np.random.default_rng(seed)
+    gam, chi = [], []
+    for n in sizes:
+        c = rng.standard_normal((1, 1, n)) + 1j * rng.standard_normal((1, 1, n))
+        g = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        g *= 0.9 / (3.0 * np.sqrt(n) * np.abs(c).max())
+        gam.append(np.asfortranarray(g))
+        chi.append(np.asfortranarray(c))
+    return Instances(n=np.array(sizes, dtype=np.int32), nl=np.ones(len(sizes), dtype=np.int32),
+                     scale=np.ones(len(sizes)), gamma=gam, chi=chi, q=np.zeros((len(sizes), 3), dtype=np.int32))
+
+
+@pytest.mark.gpu
+def test_split_lu_at_block_edges(gpu_lib):
+    """Remainders of 1, 63, 64, 65 and 127 in a block of 128, fewer than 64 rows, and the row counts past which a
+    panel takes two rows per thread and past which it stays in global memory; two instances of some sizes."""
+    from tups_b200.bse_batched import solve_split
+    sizes = [1, 7, 33, 63, 64, 65, 65, 127, 128, 129, 129, 191, 192, 193, 255, 257, 513, 577, 1089]
+    inst = _edge_instances(sizes, 31)
+    tol = 1e-12
+    out, info = solve_split(inst, slices=6, tol=tol, max_refine=8)
+    assert np.all(info["residual"] <= tol)
+    for i, x in enumerate(out):
+        g = inst.gamma[i]
+        ref = LU.bse_lu(g, inst.chi[i], 1.0)
+        # a column of the residual is at most sqrt(n) tol max|Gamma|, and the oracle's own error is far below
+        assert np.abs(x - ref).max() <= 11 * np.sqrt(sizes[i]) * tol * np.abs(g).max(), sizes[i]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [130, 200, 600])
+def test_split_lu_interchanges_far_from_the_diagonal(gpu_lib, n):
+    """Every pivot far below its diagonal entry, by another distance in each of three instances of one group."""
+    from tups_b200.bse_batched import solve_split
+    rng = np.random.default_rng(n)
+    mats = []
+    for shift in (n // 2 + 2, 1, n - 70):
+        a = 0.01 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+        a[(np.arange(n) + shift) % n, np.arange(n)] += 5.0 + rng.uniform(0.0, 1.0, n)
+        mats.append(a)
+    inst = _unit_chi_instances(mats)
+    tol = 1e-12
+    out, info = solve_split(inst, slices=6, tol=tol, max_refine=8)
+    assert np.all(info["residual"] <= tol)
+    for i, x in enumerate(out):
+        g = inst.gamma[i]
+        # |A^-1| is at most 1 / (5 - 0.02)
+        assert np.abs(x - LU.bse_lu(g, inst.chi[i], 1.0)).max() <= 0.25 * np.sqrt(n) * tol * np.abs(g).max(), i

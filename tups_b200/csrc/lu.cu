@@ -7,13 +7,11 @@
 // Right-looking LU with partial pivoting of [A | Gamma], A = I - c Gamma chi,
 // in blocks of 64 columns, every step one launch over all instances that
 // still have a block:
-//   k_lu_panel   one CTA per instance factors the block's columns and inverts
-//                its unit lower 64 x 64 diagonal factor in place,
+//   k_lu_panel   one CTA per instance factors the block's columns,
 //   k_lu_rows    column tiles: the block's row interchanges, then
 //                U12 = L11^{-1} P A12 (and the same of the right-hand sides),
 //   k_lu_update  32 x 32 tiles of [A22 | F2] -= L21 U12,
-// then, with the upper diagonal factors inverted (k_lu_invert), back
-// substitution from each instance's last block:
+// then back substitution from each instance's last block:
 //   k_lu_rows    X_b = U_bb^{-1} F_b,      k_lu_update   F_above -= U_above,b X_b.
 // The forward substitution of the right-hand sides is part of the update, so
 // rows of L left of the block are never interchanged.  The products run on the
@@ -35,7 +33,6 @@ namespace {
 using tups::cplx;
 using tups::cmk;
 using tups::lud::dmma8;
-using tups::lud::kInvLd;
 using tups::lud::kPanelCols;
 using tups::lud::kPanelRows;
 using tups::lud::kPanelThreads;
@@ -122,8 +119,7 @@ struct LuPanelShared {
 };
 
 // Columns [j0, j0 + 64) of every instance (one CTA each): two 32-column panels
-// with a 32-wide update between them, the interchange map, and the unit lower
-// diagonal factor replaced by its inverse (nothing later needs the factor).
+// with a 32-wide update between them, and the interchange map.
 // RPT: rows per thread in registers, 0 = columns in global memory.
 // A serial chain of column steps: bound by barrier and FP64 latency, not by
 // bandwidth; its SMs' FP64 pipes idle between the steps.
@@ -183,21 +179,6 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_lu_panel(cplx* __restrict_
   if (tid == 0) map.count = S.moved;
 }
 
-// U_bb^{-1} over U_bb for every diagonal block of every instance, off the
-// chain of panels: the back substitution reads nothing else of them
-__global__ void __launch_bounds__(256) k_lu_invert(cplx* __restrict__ Aw) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx* M = reinterpret_cast<cplx*>(smraw);
-  const LuDesc d = g_lu_desc[blockIdx.y];
-  const int n = d.n, j0 = blockIdx.x * NB, jb = min(NB, n - j0);
-  if (j0 >= n) return;
-  cplx* A = Aw + d.g_off;
-  tups::lud::load_triangle<true>(A, n, j0, jb, M);
-  tups::lud::invert_triangle<true>(M, M + NB * kInvLd);
-  tups::lud::store_triangle<true>(A, n, j0, jb, M);
-}
-constexpr size_t kInvertSmem = ((size_t)NB * kInvLd + kPanelCols * kPanelCols) * sizeof(cplx);
-
 // column c of [A right of the block | F] (forward) or of F (backward)
 __device__ __forceinline__ cplx* rhs_column(cplx* A, cplx* F, int n, int right, int c) {
   return c < right ? A + (size_t)n * (n - right + c) : F + (size_t)n * (c - right);
@@ -210,12 +191,12 @@ __device__ __forceinline__ int block_start(int n, int step) {
   return BACK ? ((n + NB - 1) / NB - 1 - step) * NB : step * NB;
 }
 
-// ---- block row: X[block, tile] = T (P X)[block, tile], T = L11^{-1} or U_bb^{-1} ----
+// ---- block row: X[block, tile] = T^{-1} (P X)[block, tile], T = L11 or U_bb -------
 // 32 columns per CTA, a warp per 8 of them and all 64 rows, so the triangle's
-// skipped 16 x 16 blocks shorten every warp alike.  The interchanges are a
-// gather: all reads of the tile end before its first write.
+// shape shortens every warp alike.  The interchanges are a gather: all reads of
+// the tile end before its first write.
 constexpr int RW_BN = 32, RW_THREADS = 4 * RW_BN, RW_LDL = NB + 2, RW_LDB = NB + 4;
-constexpr size_t kRowsSmem = ((size_t)NB * RW_LDL + RW_BN * RW_LDB) * sizeof(cplx);
+constexpr size_t kRowsSmem = ((size_t)NB * RW_LDL + RW_BN * RW_LDB + NB) * sizeof(cplx);
 
 __device__ __forceinline__ void lu_cp_async16(void* sdst, const void* gsrc, bool valid) {
   unsigned sz = valid ? 16u : 0u;
@@ -228,6 +209,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) k_lu_rows(cplx* __restrict__ Aw
   extern __shared__ __align__(16) unsigned char smraw[];
   cplx* sL = reinterpret_cast<cplx*>(smraw);  // [k][m]
   cplx* sB = sL + NB * RW_LDL;                // [col][k]
+  cplx* sI = sB + RW_BN * RW_LDB;             // reciprocals of U_bb's diagonal
   const int inst = blockIdx.y;
   const LuDesc d = g_lu_desc[inst];
   const int n = d.n, j0 = block_start<BACK>(n, step), jb = min(NB, n - j0), je = j0 + jb;
@@ -236,7 +218,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) k_lu_rows(cplx* __restrict__ Aw
   cplx* A = Aw + d.g_off;
   cplx* F = Fout + d.g_off;
   const LuMap& map = g_lu_map[inst];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kStep = RW_THREADS / NB;
   const int tm = tid % NB, tc = tid / NB;  // this thread's row and first column of both operands
   const int srow = BACK ? j0 + tm : map.src[tm];
@@ -265,48 +247,30 @@ __global__ void __launch_bounds__(RW_THREADS, 2) k_lu_rows(cplx* __restrict__ Aw
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
-  if (!BACK) {
-    if (tid < NB) sL[tid * RW_LDL + tid] = cmk(1.0, 0.0);
-    if (tm < cnt) {
-#pragma unroll
-      for (int i = 0; i < RW_BN / kStep; i++) {
-        const int c = c0 + tc + kStep * i;
-        if (c < width) rhs_column(A, F, n, right, c)[mv >> 6] = v[i];
-      }
-    }
+  if (BACK) {
+    if (tid < NB) sI[tid] = tups::lud::diagonal_reciprocal(sL[tid * RW_LDL + tid]);
     __syncthreads();
-  }
-  double re[4][4] = {}, im[4][4] = {};
-  const cplx* b = sB + (warp * 8 + gid) * RW_LDB;
+  } else if (tm < cnt) {
 #pragma unroll
-  for (int k8 = 0; k8 < NB; k8 += 8) {
-    const cplx b0 = b[k8 + tig], b1 = b[k8 + tig + 4];
-    const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      if (BACK ? k8 < 16 * t : k8 >= 16 * (t + 1)) continue;
-      const cplx* l = sL + (k8 + tig) * RW_LDL + 16 * t + gid;
-      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * RW_LDL], a3 = l[4 * RW_LDL + 8];
-      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
-      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
-      dmma8(re[t], ar, br);
-      dmma8(re[t], an, bi);
-      dmma8(im[t], ar, bi);
-      dmma8(im[t], ai, br);
+    for (int i = 0; i < RW_BN / kStep; i++) {
+      const int c = c0 + tc + kStep * i;
+      if (c < width) rhs_column(A, F, n, right, c)[mv >> 6] = v[i];
     }
   }
+  cplx* x = sB + warp * 8 * RW_LDB;
+  tups::lud::solve_triangle<BACK>(sL, RW_LDL, sI, x, RW_LDB);
 #pragma unroll
-  for (int t = 0; t < 4; t++)
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      const int m = 16 * t + gid + (x >= 2 ? 8 : 0), c = c0 + warp * 8 + 2 * tig + (x & 1);
-      if (m < jb && c < width) rhs_column(A, F, n, right, c)[j0 + m] = cmk(re[t][x], im[t][x]);
-    }
+  for (int i = 0; i < NB / 4; i++) {
+    const int m = lane + 32 * (i & 1), j = i >> 1, c = c0 + warp * 8 + j;
+    if (m < jb && c < width) rhs_column(A, F, n, right, c)[j0 + m] = x[j * RW_LDB + m];
+  }
 }
 
 // ---- update: C -= L21 U12 (forward), F_above -= U_above,b X_b (backward) -----------
 // 32 x 32 complex tiles, 4 warps of 16 x 16, K = 64 in two cp.async stages of
-// 16, three real tensor-core products per complex one (as the BSE GEMM).
+// 16, four real tensor-core products per complex one: with three the error of
+// an imaginary part is that of the real parts' products, 1e-7 of it where the
+// matrix is real to 1e-8.
 constexpr int UP_BM = 32, UP_BN = 32, UP_BK = 16, UP_LDL = UP_BM + 2, UP_LDR = UP_BK + 4;
 
 template <bool BACK>
@@ -351,7 +315,7 @@ __global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cpl
       lu_cp_async16(&sR[st][bc + 8 * i][bk], k0 + bk < K ? pb[i] + k0 + bk : pb[i], okc[i] && k0 + bk < K);
     asm volatile("cp.async.commit_group;\n" ::);
   };
-  double p1[2][4] = {}, p2[2][4] = {}, p3[2][4] = {};
+  double re[2][4] = {}, im[2][4] = {};
   load(0, 0);
   for (int kt = 0; kt < ktiles; kt++) {
     const int cur = kt & 1;
@@ -364,20 +328,21 @@ __global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cpl
       const cplx v0 = sL[cur][k8 + tig][mb], v1 = sL[cur][k8 + tig][mb + 8];
       const cplx v2 = sL[cur][k8 + tig + 4][mb], v3 = sL[cur][k8 + tig + 4][mb + 8];
       const double are[4] = {v0.x, v1.x, v2.x, v3.x}, aim[4] = {v0.y, v1.y, v2.y, v3.y};
-      const double asum[4] = {v0.x + v0.y, v1.x + v1.y, v2.x + v2.y, v3.x + v3.y};
+      const double aneg[4] = {-v0.y, -v1.y, -v2.y, -v3.y};
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const int nb = wn0 + j * 8 + gid;
         const cplx w0 = sR[cur][nb][k8 + tig], w1 = sR[cur][nb][k8 + tig + 4];
-        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y}, bsum[2] = {w0.x + w0.y, w1.x + w1.y};
-        dmma8(p1[j], are, bre);
-        dmma8(p2[j], aim, bim);
-        dmma8(p3[j], asum, bsum);
+        const double bre[2] = {w0.x, w1.x}, bim[2] = {w0.y, w1.y};
+        dmma8(re[j], are, bre);
+        dmma8(re[j], aneg, bim);
+        dmma8(im[j], are, bim);
+        dmma8(im[j], aim, bre);
       }
     }
   }
   // the old entries all go out before the first write, which could alias them
-  // (one after another they kept the kernel waiting: 96 instances 10.2 -> 9.3 ms)
+  // (one after another they kept the kernel waiting: 0.9 ms over 96 instances of n = 64..832)
   cplx old[2][4];
 #pragma unroll
   for (int j = 0; j < 2; j++)
@@ -394,7 +359,7 @@ __global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cpl
       const cplx v = old[j][x];
       if (row < rows && col < width)
         rhs_column(A, F, n, right, col)[first + row] =
-            cmk(v.x - (p1[j][x] - p2[j][x]), v.y - (p3[j][x] - p1[j][x] - p2[j][x]));
+            cmk(v.x - re[j][x], v.y - im[j][x]);
     }
 }
 
@@ -415,7 +380,6 @@ bool lu_prepare() {
   return cudaFuncSetAttribute(k_lu_panel<0>, attr, ps) == cudaSuccess &&
          cudaFuncSetAttribute(k_lu_panel<1>, attr, ps) == cudaSuccess &&
          cudaFuncSetAttribute(k_lu_panel<2>, attr, ps) == cudaSuccess &&
-         cudaFuncSetAttribute(k_lu_invert, attr, (int)kInvertSmem) == cudaSuccess &&
          cudaFuncSetAttribute(k_lu_rows<false>, attr, rs) == cudaSuccess &&
          cudaFuncSetAttribute(k_lu_rows<true>, attr, rs) == cudaSuccess;
 }
@@ -471,7 +435,6 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
     k_lu_rows<false><<<dim3((unsigned)((width + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);
     if (below > 0) k_lu_update<false><<<dim3(tiles(below, width), live), 128, 0, st>>>(A, F, step);
   }
-  k_lu_invert<<<dim3((unsigned)((nmax + NB - 1) / NB), n_inst), 256, kInvertSmem, st>>>(A);
   live = n_inst;
   for (int step = 0; step * NB < nmax; step++) {
     while (queued[live - 1].n <= step * NB) live--;

@@ -1,6 +1,6 @@
 // Device pieces shared by the batched LU kernels (lu.cu, lu_split.cu):
 // the factorisation of a block of 64 columns by one CTA as two 32-column
-// panels, and the inversion of its 64 x 64 triangles.
+// panels, and the solves with its 64 x 64 triangles.
 #pragma once
 
 #include "tups_device.cuh"
@@ -396,113 +396,17 @@ static __device__ void panel_factor_global(cplx* __restrict__ A, int n, int h0, 
 }
 
 // ---- one block of 64 columns by one CTA ------------------------------------------
-constexpr int kBlock = 2 * kPanelCols, kInvLd = kBlock + 1;
+constexpr int kBlock = 2 * kPanelCols;
 
 struct BlockShared {
   PanelShared p;
   int orig[kPanelRows];  // where a row's content stood before the block
-  union {
-    HalfShared half;
-    struct {
-      cplx M[kBlock * kInvLd], T[kPanelCols * kPanelCols];  // [col][row]
-    };
-  };
+  HalfShared half;
 };
 
-// M <- M^{-1}, a 64 x 64 triangle (unit lower, or UP: upper) in shared memory
-// with the pitch kInvLd: 16 x 16 diagonal blocks by substitution, one thread
-// per column, then merged pairwise, inv([X 0; Y Z]) = [X' 0; -Z' Y X' Z'] and
-// its mirror.  A zero pivot divides by one (its instance is reported
-// singular).  T: 1024 complex of scratch.  At least 64 threads.
-template <bool UP>
-static __device__ void invert_triangle(cplx* __restrict__ M, cplx* __restrict__ T) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid < 64) {
-    const int b = tid & 48, c = tid & 15;
-    const cplx* D = M + b * kInvLd + b;
-    cplx x[16];
-#pragma unroll
-    for (int r = 0; r < 16; r++) x[r] = cmk(r == c ? 1.0 : 0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const int k = UP ? 15 - i : i;
-      if (UP) {
-        const cplx u = D[k * kInvLd + k];
-        if (u.x != 0.0 || u.y != 0.0) x[k] = cmul(x[k], crecip1(u));
-      }
-#pragma unroll
-      for (int r = 0; r < 16; r++)
-        if (UP ? r < k : r > k) x[r] = cfnma(D[k * kInvLd + r], x[k], x[r]);
-    }
-    __syncwarp();  // a 16-column block belongs to half a warp
-#pragma unroll
-    for (int r = 0; r < 16; r++) M[(b + c) * kInvLd + b + r] = x[r];
-  }
-  __syncthreads();
-  // Y is s x s; a warp per 16 x 8 tile of a product
-  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5, gid = lane >> 2, tig = lane & 3;
-  auto product = [&](const cplx* L, int ldl, const cplx* R, int ldr, int s, int m0, int c0, double* re, double* im) {
-    for (int k8 = 0; k8 < s; k8 += 8) {
-      const cplx* l = L + (k8 + tig) * ldl + m0 + gid;
-      const cplx* r = R + (c0 + gid) * ldr + k8 + tig;
-      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * ldl], a3 = l[4 * ldl + 8], b0 = r[0], b1 = r[4];
-      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
-      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y}, br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
-      dmma8(re, ar, br);
-      dmma8(im, ar, bi);
-      dmma8(re, an, bi);
-      dmma8(im, ai, br);
-    }
-  };
-  for (int s = 16; s < kBlock; s *= 2) {
-    const int per = s / 16 * (s / 8), tiles = kBlock / (2 * s) * per;
-    for (int pass = 0; pass < 2; pass++) {
-      // pass 0: T = Y X' (lower) or Y Z' (upper); pass 1: Y = -Z' T or -X' T
-      for (int t = warp; t < tiles; t += nw) {
-        const int b = t / per * 2 * s, m0 = t % per % (s / 16) * 16, c0 = t % per / (s / 16) * 8;
-        const int y0 = UP ? b : b + s, x0 = UP ? b + s : b;  // first row and column of Y
-        cplx* Y = M + x0 * kInvLd + y0;
-        cplx* Tp = T + t / per * s * s;  // [c][r]
-        double re[4] = {}, im[4] = {};
-        if (pass == 0) product(Y, kInvLd, M + x0 * kInvLd + x0, kInvLd, s, m0, c0, re, im);
-        else product(M + y0 * kInvLd + y0, kInvLd, Tp, s, s, m0, c0, re, im);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + 2 * tig + (e & 1);
-          if (pass == 0) Tp[c * s + r] = cmk(re[e], im[e]);
-          else Y[c * kInvLd + r] = cmk(-re[e], -im[e]);
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// the triangle of the diagonal block at (j0, j0), identity past jb, into M
-template <bool UP>
-static __device__ void load_triangle(const cplx* __restrict__ A, int n, int j0, int jb, cplx* __restrict__ M) {
-  for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
-    const int r = e % kBlock, c = e / kBlock;
-    const bool in = r < jb && c < jb && (UP ? r <= c : r > c);
-    M[c * kInvLd + r] = in ? A[j0 + r + (size_t)n * (j0 + c)] : cmk(r == c ? 1.0 : 0.0, 0.0);
-  }
-  __syncthreads();
-}
-
-template <bool UP>
-static __device__ void store_triangle(cplx* __restrict__ A, int n, int j0, int jb, const cplx* __restrict__ M) {
-  for (int e = threadIdx.x; e < kBlock * kBlock; e += blockDim.x) {
-    const int r = e % kBlock, c = e / kBlock;
-    if (r < jb && c < jb && (UP ? r <= c : r > c)) A[j0 + r + (size_t)n * (j0 + c)] = M[c * kInvLd + r];
-  }
-}
-
-
 // Columns [j0, j0 + jb), jb <= 64, rows j0 .. n-1: two 32-column panels with a
-// 32-wide update between them, then the unit lower diagonal factor replaced by
-// its inverse (nothing later needs the factor).  RPT: rows per thread in
-// registers, 0 = columns in global memory.  Interchanges as panel_factor's.
-// Ends with a barrier.
+// 32-wide update between them.  RPT: rows per thread in registers, 0 = columns
+// in global memory.  Interchanges as panel_factor's.  Ends with a barrier.
 template <int RPT, int COLS, class Track>
 static __device__ void block_factor(cplx* __restrict__ A, int n, int j0, int jb, int ca, int cb, int* __restrict__ ipiv,
                                     int* __restrict__ status, BlockShared& S, Track track) {
@@ -515,10 +419,87 @@ static __device__ void block_factor(cplx* __restrict__ A, int n, int j0, int jb,
     if constexpr (RPT > 0) panel_factor<RPT, COLS>(A, n, h0, kb, ca, cb, ipiv, status, S.p, track);
     else panel_factor_global(A, n, h0, kb, ca, cb, ipiv, status, S.p, track);
   }
-  load_triangle<false>(A, n, j0, jb, S.M);
-  invert_triangle<false>(S.M, S.T);
-  store_triangle<false>(A, n, j0, jb, S.M);
-  __syncthreads();
+}
+
+// ---- solves with a 64 x 64 triangle ------------------------------------------------
+//
+// X <- T^{-1} X for one warp's 8 columns, 64 rows each in shared memory
+// (column c at X + c ldx): T, [column][row] with the pitch ldt, is unit lower
+// (entries above and on the diagonal are not read) or, UP, upper with the
+// reciprocals of its diagonal in inv.  Blocks of 16 rows: what the rows solved
+// before contribute goes through the FP64 tensor cores (four real products per
+// complex one), the block itself by substitution, four lanes per column with
+// the rows interleaved over them.
+//
+// Products with explicit inverses of the triangles instead were faster (with
+// three real products per complex one in the updates besides, 96 instances of
+// n = 64..832 9.3 ms against 10.4), but their error grows with the triangle's
+// condition: the residuals of well-conditioned systems were three to ten times
+// those of substitution, a thousand units of |L| |U| |X| against eleven for rows
+// that spread over twelve decades.
+template <bool UP>
+static __device__ __forceinline__ void solve_triangle(const cplx* __restrict__ T, int ldt, const cplx* __restrict__ inv,
+                                                      cplx* X, int ldx) {
+  const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+#pragma unroll 1
+  for (int b = 0; b < kBlock / 16; b++) {
+    const int r0 = 16 * (UP ? kBlock / 16 - 1 - b : b);
+    if (b > 0) {
+      double re[4], im[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const cplx v = X[(2 * tig + (e & 1)) * ldx + r0 + gid + (e >= 2 ? 8 : 0)];
+        re[e] = v.x;
+        im[e] = v.y;
+      }
+      for (int k8 = UP ? r0 + 16 : 0; k8 < (UP ? kBlock : r0); k8 += 8) {
+        const cplx* l = T + (k8 + tig) * ldt + r0 + gid;
+        const cplx a0 = l[0], a1 = l[8], a2 = l[4 * ldt], a3 = l[4 * ldt + 8];
+        const double ar[4] = {-a0.x, -a1.x, -a2.x, -a3.x}, an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+        const double ai[4] = {a0.y, a1.y, a2.y, a3.y};
+        const cplx b0 = X[gid * ldx + k8 + tig], b1 = X[gid * ldx + k8 + tig + 4];
+        const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y};
+        dmma8(re, ar, br);
+        dmma8(re, ai, bi);
+        dmma8(im, ar, bi);
+        dmma8(im, an, br);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        X[(2 * tig + (e & 1)) * ldx + r0 + gid + (e >= 2 ? 8 : 0)] = cmk(re[e], im[e]);
+      __syncwarp();
+    }
+    cplx x[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) x[i] = X[gid * ldx + r0 + tig + 4 * i];
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+      const int k = UP ? 15 - c : c;
+      cplx xk = cmk(__shfl_sync(0xffffffffu, x[k >> 2].x, (lane & ~3) | (k & 3)),
+                    __shfl_sync(0xffffffffu, x[k >> 2].y, (lane & ~3) | (k & 3)));
+      if (UP) {
+        xk = cmul(xk, inv[r0 + k]);
+        if (tig == (k & 3)) x[k >> 2] = xk;
+      }
+      const cplx* l = T + (r0 + k) * ldt + r0 + tig;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (UP ? i > k >> 2 : i < k >> 2) continue;
+        const bool mine = i != k >> 2 || (UP ? tig < (k & 3) : tig > (k & 3));
+        const cplx y = cfnma(l[4 * i], xk, x[i]);
+        if (mine) x[i] = y;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) X[gid * ldx + r0 + tig + 4 * i] = x[i];
+    __syncwarp();
+  }
+}
+
+// reciprocal of a diagonal entry of U; a zero pivot divides by one (its
+// instance is reported singular)
+static __device__ __forceinline__ cplx diagonal_reciprocal(cplx u) {
+  return u.x == 0.0 && u.y == 0.0 ? cmk(1.0, 0.0) : crecip1(u);
 }
 
 }  // namespace lud

@@ -13,9 +13,9 @@
 //    tiles between them; the trailing update A22 -= L21 U12 (K = 128) runs on
 //    the int8 tensor cores as an Ozaki split GEMM with s slices (ozaki.cu),
 //    so the factors are those of a matrix within about 10^(1.1-2s) of A.
-//  * X = U^{-1} L^{-1} P Gamma: 128-row diagonal blocks in FP64 through the
-//    inverses of their 64 x 64 triangles (FP64 tensor cores), the off-diagonal
-//    updates on the int8 path.
+//  * X = U^{-1} L^{-1} P Gamma: 128-row diagonal blocks in FP64 (their 64 x 64
+//    triangles by blocked substitution), the off-diagonal updates on the int8
+//    path.
 //  * Refinement: R = Gamma - A X = Gamma - X + c Gamma (chi X) in FP64 (the
 //    GEMM on the FP64 tensor cores, three real products per complex one);
 //    stop when max|R| <= tol max|Gamma| for every instance of the group (or
@@ -94,21 +94,23 @@ __global__ void __launch_bounds__(LS_THREADS) k_ls_form(const LsDesc* __restrict
 // ---- 128-column block ------------------------------------------------------------
 using lud::BlockShared;
 using lud::kBlock;
-using lud::kInvLd;
 using lud::kPanelRows;
 using lud::kPanelThreads;
 
+constexpr int LS_LDT = kBlock + 2, LS_LDX = kBlock + 4;
+
 struct LsPanelShared {
   BlockShared b;
-  cplx x[32 * (kBlock + 4)];  // [column][row]: columns of the block right of the panel
+  cplx t[kBlock * LS_LDT];  // [column][row] of L11
+  cplx x[kBlock * LS_LDX];  // [column][row]: the block's columns right of the panel
 };
 
 // Columns [j0, j0 + 64) of the block [J0, JE), one CTA per instance: the panel
-// with its interchanges on all the block's columns, L11^{-1} over L11, and for
-// the first panel U12 = L11^{-1} A12 of the block's other columns (32 at a time,
-// 16 x 8 warp tiles).  worig[r]: the row whose content, as it stood before the
-// block, row r now holds.  With the block's last panel the instance's whole
-// permutation follows: perm'[r] = perm[worig[r]].  RPT as in block_factor.
+// with its interchanges on all the block's columns and for the first panel U12
+// = L11^{-1} A12 of the block's other columns, a warp per 8 of them.
+// worig[r]: the row whose content, as it stood before the block, row r now
+// holds.  With the block's last panel the instance's whole permutation
+// follows: perm'[r] = perm[worig[r]].  RPT as in block_factor.
 template <int RPT>
 __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict__ Ag, int* __restrict__ ipiv_all,
                                                                int* __restrict__ worig_all, int* __restrict__ wtmp_all,
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict_
                                                                int n, int j0, int J0, int JE) {
   extern __shared__ __align__(16) unsigned char smraw[];
   LsPanelShared& S = *reinterpret_cast<LsPanelShared*>(smraw);
-  const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i = blockIdx.x, tid = threadIdx.x;
   const int jb = min(kBlock, JE - j0), je = j0 + jb;
   cplx* A = Ag + (size_t)n * n * i;
   int* worig = worig_all + (size_t)n * i;
@@ -143,40 +145,24 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict_
     for (int r = J0 + tid; r < n; r += kPanelThreads) perm[r] = tmp[r];
     return;
   }
-  // L11^{-1} is still in S.b.M (unit diagonal included)
-  const int gid = lane >> 2, tig = lane & 3, cn = (warp & 3) * 8;
-  for (int c0 = je; c0 < JE; c0 += 32) {
-    for (int e = tid; e < 32 * kBlock; e += kPanelThreads) {
-      const int r = e % kBlock, c = e / kBlock;
-      S.x[c * (kBlock + 4) + r] = c0 + c < JE ? A[j0 + r + (size_t)n * (c0 + c)] : cmk(0.0, 0.0);
-    }
-    __syncthreads();
-    for (int m0 = (warp >> 2) * 16; m0 < kBlock; m0 += kPanelThreads / 128 * 16) {
-      double re[4] = {}, im[4] = {};
-      for (int k8 = 0; k8 < m0 + 16; k8 += 8) {
-        const cplx* l = S.b.M + (k8 + tig) * kInvLd + m0 + gid;
-        const cplx a0 = l[0], a1 = l[8], a2 = l[4 * kInvLd], a3 = l[4 * kInvLd + 8];
-        const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
-        const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
-        const cplx* x = S.x + (cn + gid) * (kBlock + 4) + k8 + tig;
-        const double br[2] = {x[0].x, x[4].x}, bi[2] = {x[0].y, x[4].y};
-        lud::dmma8(re, ar, br);
-        lud::dmma8(re, an, bi);
-        lud::dmma8(im, ar, bi);
-        lud::dmma8(im, ai, br);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int r = m0 + gid + (e >= 2 ? 8 : 0), c = c0 + cn + 2 * tig + (e & 1);
-        if (c < JE) A[j0 + r + (size_t)n * c] = cmk(re[e], im[e]);
-      }
-    }
-    __syncthreads();
+  const int warp = tid >> 5;
+  for (int e = tid; e < kBlock * kBlock; e += kPanelThreads) {
+    const int r = e % kBlock, c = e / kBlock;
+    S.t[c * LS_LDT + r] = A[j0 + r + (size_t)n * (j0 + c)];
+    S.x[c * LS_LDX + r] = je + c < JE ? A[j0 + r + (size_t)n * (je + c)] : cmk(0.0, 0.0);
+  }
+  __syncthreads();
+  if (8 * warp < JE - je) lud::solve_triangle<false>(S.t, LS_LDT, nullptr, S.x + 8 * warp * LS_LDX, LS_LDX);
+  __syncthreads();
+  for (int e = tid; e < kBlock * (JE - je); e += kPanelThreads) {
+    const int r = e % kBlock, c = e / kBlock;
+    A[j0 + r + (size_t)n * (je + c)] = S.x[c * LS_LDX + r];
   }
 }
 
-// A[j1.., j1..JE) -= A[j1.., J0..j1) A[J0..j1, j1..JE): the block's second panel
-using LsTile = ZgemmTile<1, 2, 2, 2, 16, 2, true, false>;
+// A[j1.., j1..JE) -= A[j1.., J0..j1) A[J0..j1, j1..JE): the block's second panel;
+// four real products per complex one, as the FP64 form's update (lu.cu)
+using LsTile = ZgemmTile<1, 2, 2, 2, 16, 2, false, false>;
 
 struct LsSource {
   const cplx *l, *r;
@@ -202,29 +188,15 @@ __global__ void __launch_bounds__(LsTile::NT, 5) k_ls_mid(cplx* __restrict__ Ag,
       [&](int row, int col, cplx v, cplx c) { C[row + (size_t)n * col] = csub(c, v); });
 }
 
-// U_bb^{-1} over the upper 64 x 64 diagonal triangles, off the chain of panels
-__global__ void __launch_bounds__(256) k_ls_invert(cplx* __restrict__ Ag, int n) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx* M = reinterpret_cast<cplx*>(smraw);
-  const int j0 = blockIdx.x * kBlock, jb = min(kBlock, n - j0);
-  cplx* A = Ag + (size_t)n * n * blockIdx.y;
-  lud::load_triangle<true>(A, n, j0, jb, M);
-  lud::invert_triangle<true>(M, M + kBlock * kInvLd);
-  lud::store_triangle<true>(A, n, j0, jb, M);
-}
-constexpr size_t kLsInvertSmem = ((size_t)kBlock * kInvLd + lud::kPanelCols * lud::kPanelCols) * sizeof(cplx);
-
 // ---- solves with a 128-row diagonal block [j0, j0 + jb) on LT_COLS columns per CTA ----
-// T is the block's unit lower (or, BACK, upper) triangle; its 64 x 64 diagonal
-// triangles hold their inverses, so X = T^{-1} X is three products per tile,
-// lower: X1 = I1 X1, X2 -= L21 X1, X2 = I2 X2.  A warp takes 8 columns and two
-// of the four 16-row strips, the first with the last, so that the triangles'
-// skipped strips cost every warp the same.
+// T is the block's unit lower (or, BACK, upper) triangle, in 64 x 64 parts: X =
+// T^{-1} X is, lower, X1 = L11^{-1} X1, X2 -= L21 X1, X2 = L22^{-1} X2.  A warp
+// takes 8 columns through all of it.
 // ROWS: the columns of A outside the block first take the block's interchanges
 // (worig), all reads of a tile before its first write; those left of the
 // block take nothing else.
-constexpr int LT_COLS = 16, LT_LDL = kBlock + 2, LT_LDX = LS_NB + 4;
-constexpr size_t kTriSmem = ((size_t)kBlock * LT_LDL + LT_COLS * LT_LDX) * sizeof(cplx);
+constexpr int LT_COLS = 32, LT_LDX = LS_NB + 4;
+constexpr size_t kTriSmem = ((size_t)kBlock * LS_LDT + LT_COLS * LT_LDX + kBlock) * sizeof(cplx);
 enum { TRI_ROWS = 0, TRI_FWD = 1, TRI_BACK = 2 };
 
 __device__ __forceinline__ void ls_cp_async16(void* sdst, const void* gsrc, bool valid) {
@@ -233,65 +205,72 @@ __device__ __forceinline__ void ls_cp_async16(void* sdst, const void* gsrc, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz));
 }
 
-// out = sgn (x + ...): KIND 0 lower triangle (unit diagonal implied), 1 upper
-// triangle, 2 full block; rows r0.. (64) of the tile from rows k0.. (64) of it;
-// KIND 2 subtracts from the tile, the triangles replace it
+// one 64 x 64 part, A's rows row.. (nr of them) and columns col.. (nk): KIND 0
+// unit lower, 1 upper: the tile's rows r0.. become T^{-1} of themselves; 2: minus
+// the part times the tile's rows k0..
 template <int KIND>
 __device__ __forceinline__ void tri_stage(const cplx* __restrict__ A, int n, int row, int col, int nr, int nk, cplx* sL,
-                                          cplx* sX, int r0, int k0) {
+                                          cplx* sI, cplx* sX, int r0, int k0) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
+  __syncthreads();  // every warp is done with the part before
 #pragma unroll 8
   for (int i = 0; i < kBlock * kBlock / 128; i++) {
     const int m = tid % kBlock, k = tid / kBlock + 2 * i;
-    const bool in = m < nr && k < nk && (KIND == 0 ? m > k : KIND == 1 ? m <= k : true);
-    ls_cp_async16(sL + k * LT_LDL + m, in ? A + row + m + (size_t)n * (col + k) : A, in);
+    const bool in = m < nr && k < nk;
+    ls_cp_async16(sL + k * LS_LDT + m, in ? A + row + m + (size_t)n * (col + k) : A, in);
   }
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  if (KIND == 0) {
-    if (tid < kBlock) sL[tid * LT_LDL + tid] = cmk(1.0, 0.0);
+  cplx* X = sX + warp * 8 * LT_LDX;
+  if (KIND == 1) {
+    if (tid < kBlock) sI[tid] = lud::diagonal_reciprocal(sL[tid * LS_LDT + tid]);
     __syncthreads();
   }
-  const int cn = (warp & 1) * 8;
-  double re[2][4] = {}, im[2][4] = {};
-  const cplx* x = sX + (cn + gid) * LT_LDX + k0 + tig;
-#pragma unroll
-  for (int u = 0; u < 2; u++) {
-    const int t = u == 0 ? warp >> 1 : 3 - (warp >> 1);
-    const int ka = KIND == 1 ? 16 * t : 0, kz = KIND == 0 ? 16 * (t + 1) : kBlock;
-    for (int k8 = ka; k8 < kz; k8 += 8) {
-      const cplx* l = sL + (k8 + tig) * LT_LDL + 16 * t + gid;
-      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * LT_LDL], a3 = l[4 * LT_LDL + 8];
-      const double ar[4] = {a0.x, a1.x, a2.x, a3.x}, ai[4] = {a0.y, a1.y, a2.y, a3.y};
-      const double an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
-      const double br[2] = {x[k8].x, x[k8 + 4].x}, bi[2] = {x[k8].y, x[k8 + 4].y};
-      lud::dmma8(re[u], ar, br);
-      lud::dmma8(re[u], an, bi);
-      lud::dmma8(im[u], ar, bi);
-      lud::dmma8(im[u], ai, br);
-    }
+  if (KIND < 2) {
+    lud::solve_triangle<KIND == 1>(sL, LS_LDT, sI, X + r0, LT_LDX);
+    return;
   }
-  __syncthreads();  // every warp has read the tile and the operand
+  double re[4][4], im[4][4];
+  auto at = [&](int t, int e) { return X + (2 * tig + (e & 1)) * LT_LDX + r0 + 16 * t + gid + (e >= 2 ? 8 : 0); };
 #pragma unroll
-  for (int u = 0; u < 2; u++) {
-    const int t = u == 0 ? warp >> 1 : 3 - (warp >> 1);
+  for (int t = 0; t < 4; t++)
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      cplx* d = sX + (cn + 2 * tig + (e & 1)) * LT_LDX + r0 + 16 * t + gid + (e >= 2 ? 8 : 0);
-      *d = KIND == 2 ? cmk(d->x - re[u][e], d->y - im[u][e]) : cmk(re[u][e], im[u][e]);
+      re[t][e] = at(t, e)->x;
+      im[t][e] = at(t, e)->y;
+    }
+  const cplx* x = X + gid * LT_LDX + k0 + tig;
+#pragma unroll 2
+  for (int k8 = 0; k8 < kBlock; k8 += 8) {
+    const double br[2] = {x[k8].x, x[k8 + 4].x}, bi[2] = {x[k8].y, x[k8 + 4].y};
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const cplx* l = sL + (k8 + tig) * LS_LDT + 16 * t + gid;
+      const cplx a0 = l[0], a1 = l[8], a2 = l[4 * LS_LDT], a3 = l[4 * LS_LDT + 8];
+      const double ar[4] = {-a0.x, -a1.x, -a2.x, -a3.x}, an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
+      const double ai[4] = {a0.y, a1.y, a2.y, a3.y};
+      lud::dmma8(re[t], ar, br);
+      lud::dmma8(re[t], ai, bi);
+      lud::dmma8(im[t], ar, bi);
+      lud::dmma8(im[t], an, br);
     }
   }
-  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < 4; t++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) *at(t, e) = cmk(re[t][e], im[t][e]);
+  __syncwarp();
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128, 2) k_ls_tri(const cplx* __restrict__ Ag, cplx* Xg, const int* __restrict__ worig_all,
+__global__ void __launch_bounds__(128, 1) k_ls_tri(const cplx* __restrict__ Ag, cplx* Xg, const int* __restrict__ worig_all,
                                                    int n, int j0, int jb) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_moved[LS_NB];
   __shared__ int s_cnt;
   cplx* sL = reinterpret_cast<cplx*>(smraw);  // [k][m]
-  cplx* sX = sL + kBlock * LT_LDL;            // [column][row]
+  cplx* sX = sL + kBlock * LS_LDT;            // [column][row]
+  cplx* sI = sX + LT_COLS * LT_LDX;
   const int i = blockIdx.y, tid = threadIdx.x, je = j0 + jb;
   const cplx* A = Ag + (size_t)n * n * i;
   cplx* X = Xg + (size_t)n * n * i;
@@ -335,31 +314,26 @@ __global__ void __launch_bounds__(128, 2) k_ls_tri(const cplx* __restrict__ Ag, 
   // solves all its columns and stores the right ones
   const bool solve = MODE != TRI_ROWS || c0 + nc > j0;
   const int b1 = min(jb, kBlock), b2 = jb - b1;
-  if (!solve) {
-#pragma unroll
-    for (int c = 0; c < LT_COLS; c++)
-      if (tid < jb && c < nc) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
-    return;
-  }
   if (MODE == TRI_ROWS && c0 < j0) {
 #pragma unroll
     for (int c = 0; c < LT_COLS; c++)
-      if (tid < jb && c0 + c < j0) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
-    __syncthreads();
+      if (tid < jb && c < nc && c0 + c < j0) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
   }
+  if (!solve) return;
   if (MODE == TRI_BACK) {
     if (b2 > 0) {
-      tri_stage<1>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sX, kBlock, kBlock);
-      tri_stage<2>(A, n, j0, j0 + kBlock, b1, b2, sL, sX, 0, kBlock);
+      tri_stage<1>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sI, sX, kBlock, kBlock);
+      tri_stage<2>(A, n, j0, j0 + kBlock, b1, b2, sL, sI, sX, 0, kBlock);
     }
-    tri_stage<1>(A, n, j0, j0, b1, b1, sL, sX, 0, 0);
+    tri_stage<1>(A, n, j0, j0, b1, b1, sL, sI, sX, 0, 0);
   } else {
-    tri_stage<0>(A, n, j0, j0, b1, b1, sL, sX, 0, 0);
+    tri_stage<0>(A, n, j0, j0, b1, b1, sL, sI, sX, 0, 0);
     if (b2 > 0) {
-      tri_stage<2>(A, n, j0 + kBlock, j0, b2, b1, sL, sX, kBlock, 0);
-      tri_stage<0>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sX, kBlock, kBlock);
+      tri_stage<2>(A, n, j0 + kBlock, j0, b2, b1, sL, sI, sX, kBlock, 0);
+      tri_stage<0>(A, n, j0 + kBlock, j0 + kBlock, b2, b2, sL, sI, sX, kBlock, kBlock);
     }
   }
+  __syncthreads();
 #pragma unroll
   for (int c = 0; c < LT_COLS; c++)
     if (tid < jb && c < nc && (MODE != TRI_ROWS || c0 + c >= j0)) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
@@ -538,7 +512,6 @@ bool ls_prepare() {
          cudaFuncSetAttribute(k_ls_tri<TRI_ROWS>, attr, ts) == cudaSuccess &&
          cudaFuncSetAttribute(k_ls_tri<TRI_FWD>, attr, ts) == cudaSuccess &&
          cudaFuncSetAttribute(k_ls_tri<TRI_BACK>, attr, ts) == cudaSuccess &&
-         cudaFuncSetAttribute(k_ls_invert, attr, (int)kLsInvertSmem) == cudaSuccess &&
          cudaFuncSetAttribute(k_ls_mid, attr, (int)LsTile::kSmem) == cudaSuccess &&
          cudaFuncSetAttribute(k_ls_resid, attr, (int)RsTile::kSmem) == cudaSuccess;
 }
@@ -637,7 +610,6 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
         if (rc) return rc;
       }
     }
-    k_ls_invert<<<dim3((nn + kBlock - 1) / kBlock, b), 256, kLsInvertSmem, st>>>(Ag, nn);
     if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
     int rc = ls_solve(st, Ag, Gg, Xg, perm, ozw, b, nn, slices, ozstat, &launches);
     if (rc) return rc;

@@ -43,6 +43,21 @@ def test_bisection_cap_reports_error(gpu_lib):
     sol.close()
 
 
+@pytest.mark.parametrize("entry", ["tups_iteration", "tups_iteration_readout"])
+def test_bisection_cap_leaves_the_info_untouched(gpu_lib, entry):
+    """An iteration that ends at the bisection's step cap returns MU_NOCONV and writes nothing into the caller's
+    struct."""
+    import ctypes as C
+    from tups_b200 import Solver
+    from tups_b200._lib import tups_conv_info
+    sol = Solver(_params(U=0.0, nParticle=0.9))
+    ci = tups_conv_info()
+    C.memset(C.byref(ci), 0xA5, C.sizeof(ci))
+    assert getattr(gpu_lib, entry)(sol._ctx, 0, C.byref(ci)) == -3   # TUPS_ERR_MU_NOCONV
+    assert bytes(ci) == b"\xa5" * C.sizeof(ci)
+    sol.close()
+
+
 def test_nan_in_sigma_is_detected(gpu_lib):
     from tups_b200 import Solver, TupsError
     sol = Solver(_params())

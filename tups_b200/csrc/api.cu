@@ -497,8 +497,10 @@ static int iteration_impl(tups_ctx* ctx, int ite, tups_conv_info* info, bool wit
   TRY(tups::launch_pae(ctx));
   tups::phase_end(ctx, TUPS_PHASE_PAE);
   if (!ctx->p.oneshot || ite == ctx->p.ite_max - 1) TRY(sde_async(ctx));
-  tups_conv_info ci;
-  int rc = conv_impl(ctx, &ci, true);
+  // an error before the check's decision (bisection cap, launch) leaves info as it was
+  tups_conv_info ci{};
+  if (info) ci = *info;
+  const int rc = conv_impl(ctx, &ci, true);
   if (info) *info = ci;
   if (rc) return rc;
   if (ite % 5 == 0 || ite == ctx->p.ite_max - 1 || ci.converged) {

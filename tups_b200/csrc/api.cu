@@ -33,8 +33,7 @@ int read_scalars(tups_ctx* ctx, double* out) {
 int status_of(tups_ctx* ctx, const double* sc) {
   int st = (int)sc[tups::S_STATUS];
   if (st != 0) {
-    double z = 0.0;
-    cudaMemcpy(ctx->s.scal + tups::S_STATUS, &z, sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemsetAsync(ctx->s.scal + tups::S_STATUS, 0, sizeof(double), ctx->stream);
     if (st == TUPS_ERR_MU_NOCONV)
       return tups::set_error(ctx, st, "mu bisection exceeded " + std::to_string(kMuMaxSteps) + " steps");
     return tups::set_error(ctx, st, "device routine reported an error");
@@ -168,14 +167,32 @@ extern "C" int tups_calc_PhiR(tups_ctx* ctx, int ite) {
   return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "calc_PhiR");
 }
 
-static int calc_M(tups_ctx* ctx, int which) {
+extern "C" int tups_calculate_expSqR(tups_ctx* ctx) {
   if (!ctx) return TUPS_ERR_BADARG;
   TRY(set_dev(ctx));
+  TRY(tups::upload_expSqR(ctx));
+  return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "calculate_expSqR");
+}
+
+extern "C" int tups_calculate_expqSR(tups_ctx* ctx) {
+  if (!ctx) return TUPS_ERR_BADARG;
+  TRY(set_dev(ctx));
+  TRY(tups::upload_expqSR(ctx));
+  return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "calculate_expqSR");
+}
+
+static int m_async(tups_ctx* ctx, int which) {
   tups::phase_begin(ctx, TUPS_PHASE_M);
   TRY(tups::launch_M(ctx, which));
   tups::phase_end(ctx, TUPS_PHASE_M);
   ctx->have_M = true;
   return TUPS_OK;
+}
+static int calc_M(tups_ctx* ctx, int which) {
+  if (!ctx) return TUPS_ERR_BADARG;
+  TRY(set_dev(ctx));
+  TRY(m_async(ctx, which));
+  return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "calc_M");
 }
 extern "C" int tups_calc_M_phbar_to_ph(tups_ctx* ctx) { return calc_M(ctx, 0); }
 extern "C" int tups_calc_M_pp_to_ph(tups_ctx* ctx) { return calc_M(ctx, 1); }
@@ -449,8 +466,7 @@ static int iteration_graph(tups_ctx* ctx, int ite, tups_conv_info* info) {
   TRY(read_scalars(ctx, sc));
   const int st = (int)sc[tups::S_STATUS];
   if (st != 0) {
-    double z = 0.0;
-    cudaMemcpy(ctx->s.scal + tups::S_STATUS, &z, sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemsetAsync(ctx->s.scal + tups::S_STATUS, 0, sizeof(double), ctx->stream);
     return tups::set_error(ctx, st, st == TUPS_ERR_MU_NOCONV ? "mu bisection exceeded its step cap"
                                                              : "device routine reported an error");
   }
@@ -484,15 +500,15 @@ static int iteration_impl(tups_ctx* ctx, int ite, tups_conv_info* info, bool wit
   TRY(green_async(ctx, 0));
   TRY(bse_async(ctx));
   if (ite == 0 || !ctx->have_exp) {
-    TRY(tups_calculate_expSqR(ctx));
-    TRY(tups_calculate_expqSR(ctx));
+    TRY(tups::upload_expSqR(ctx));
+    TRY(tups::upload_expqSR(ctx));
   }
   tups::phase_begin(ctx, TUPS_PHASE_PHIR);
   TRY(tups::launch_phir(ctx));
   tups::phase_end(ctx, TUPS_PHASE_PHIR);
   ctx->have_phir = true;
   if (ite == 0 || !ctx->have_M)
-    for (int w = 0; w < 4; w++) TRY(calc_M(ctx, w));
+    for (int w = 0; w < 4; w++) TRY(m_async(ctx, w));
   tups::phase_begin(ctx, TUPS_PHASE_PAE);
   TRY(tups::launch_pae(ctx));
   tups::phase_end(ctx, TUPS_PHASE_PAE);

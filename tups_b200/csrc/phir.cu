@@ -398,7 +398,7 @@ int launch_M(tups_ctx* ctx, int which) {
     int rc = cuda_check(ctx, cudaMalloc(&p, tab.size() * sizeof(int)), "M tables");
     if (rc) return rc;
     ctx->allocations.push_back(p);
-    rc = cuda_check(ctx, cudaMemcpy(p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice), "M tables");
+    rc = upload(ctx, p, tab.data(), tab.size() * sizeof(int), "M tables");
     if (rc) return rc;
     ctx->t.ibz_xy = (int*)p;
   }
@@ -430,8 +430,7 @@ void sym_op(int s, int ix, int iy, int N, int* ox, int* oy) {
 }  // namespace
 
 // expSqR(Q, R, sym) = e^{i S(Q).R} for sym in the star of Q, else 0
-extern "C" int tups_calculate_expSqR(tups_ctx* ctx) {
-  if (!ctx) return TUPS_ERR_BADARG;
+int tups::upload_expSqR(tups_ctx* ctx) {
   const auto& d = ctx->d;
   const int nh = d.Nf / 2;
   std::vector<cplx> v((size_t)d.NIBZ * d.NR * tups::NS, make_double2(0.0, 0.0));
@@ -448,15 +447,13 @@ extern "C" int tups_calculate_expSqR(tups_ctx* ctx) {
       }
     }
   }
-  int rc = tups::cuda_check(ctx, cudaMemcpy(ctx->t.expSqR, v.data(), v.size() * sizeof(cplx), cudaMemcpyHostToDevice),
-                            "expSqR");
+  const int rc = upload(ctx, ctx->t.expSqR, v.data(), v.size() * sizeof(cplx), "expSqR");
   if (rc == TUPS_OK) ctx->have_exp = true;
   return rc;
 }
 
 // expqSR(k, R, sym) = e^{-i k.S(R)} for sym in the star of R, k index (ky-1)*Nx+kx
-extern "C" int tups_calculate_expqSR(tups_ctx* ctx) {
-  if (!ctx) return TUPS_ERR_BADARG;
+int tups::upload_expqSR(tups_ctx* ctx) {
   const auto& d = ctx->d;
   const int nh = d.Nf / 2;
   std::vector<cplx> v((size_t)d.Nc * d.NR * tups::NS, make_double2(0.0, 0.0));
@@ -474,6 +471,5 @@ extern "C" int tups_calculate_expqSR(tups_ctx* ctx) {
         }
     }
   }
-  return tups::cuda_check(ctx, cudaMemcpy(ctx->t.expqSR, v.data(), v.size() * sizeof(cplx), cudaMemcpyHostToDevice),
-                          "expqSR");
+  return upload(ctx, ctx->t.expqSR, v.data(), v.size() * sizeof(cplx), "expqSR");
 }

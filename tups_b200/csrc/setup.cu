@@ -38,6 +38,10 @@ int cuda_check(tups_ctx* ctx, cudaError_t e, const char* what) {
                    std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+int upload(tups_ctx* ctx, void* dst, const void* src, size_t bytes, const char* what) {
+  return cuda_check(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream), what);
+}
+
 int after_launch(tups_ctx* ctx, const char* name) {
   ctx->launches++;
   return cuda_check(ctx, cudaGetLastError(), name);
@@ -385,8 +389,7 @@ template <typename T>
 int upload(tups_ctx* ctx, T** ptr, const std::vector<T>& v) {
   int rc = dalloc(ctx, ptr, v.size());
   if (rc) return rc;
-  return tups::cuda_check(ctx, cudaMemcpy(*ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice),
-                          "upload");
+  return tups::upload(ctx, *ptr, v.data(), v.size() * sizeof(T), "upload");
 }
 
 }  // namespace
@@ -765,14 +768,10 @@ static int init_state(tups_ctx* ctx) {
     for (int k = 0; k < d.Nc; k++)
       for (int nu = 0; nu < d.Nf; nu++) sig[(size_t)k * d.Nf + nu] = make_double2(0.0, im[nu]);
   }
-  TRY(tups::cuda_check(ctx, cudaMemcpy(s.Sigma, sig.data(), sig.size() * sizeof(cplx), cudaMemcpyHostToDevice),
-                       "init Sigma"));
-  TRY(tups::cuda_check(ctx, cudaMemcpy(s.SigmaOld, sig.data(), sig.size() * sizeof(cplx), cudaMemcpyHostToDevice),
-                       "init SigmaOld"));
-  std::vector<double> sc(tups::S_COUNT, 0.0);
-  TRY(tups::cuda_check(ctx, cudaMemcpy(s.scal, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice),
-                       "init scalars"));
-  return TUPS_OK;
+  TRY(tups::upload(ctx, s.Sigma, sig.data(), sig.size() * sizeof(cplx), "init Sigma"));
+  TRY(tups::upload(ctx, s.SigmaOld, sig.data(), sig.size() * sizeof(cplx), "init SigmaOld"));
+  TRY(tups::cuda_check(ctx, cudaMemsetAsync(s.scal, 0, tups::S_COUNT * sizeof(double), ctx->stream), "init scalars"));
+  return tups::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "init state");
 }
 
 namespace tups {

@@ -252,6 +252,11 @@ int exchange(tups_ctx* ctx, int what, double* dev, size_t n, int op);
 // the ibz rows of this context's slots (local slot q -> global slot slot0 + q)
 inline const int* ibz_local(const tups_ctx* ctx) { return ctx->t.ibz + 3 * (size_t)ctx->slot0; }
 int cuda_check(tups_ctx* ctx, cudaError_t e, const char* what);
+// Host data into device memory in the order of the context's stream, which does
+// not wait for the legacy stream: a plain cudaMemcpy from pageable memory may
+// return before the data has landed, and a kernel launched next could read what
+// was there before.  The host buffer is free again on return.
+int upload(tups_ctx* ctx, void* dst, const void* src, size_t bytes, const char* what);
 // record a kernel launch and check for launch errors
 int after_launch(tups_ctx* ctx, const char* name);
 
@@ -259,6 +264,9 @@ int after_launch(tups_ctx* ctx, const char* name);
 int launch_bisection(tups_ctx* ctx, int cal_chi, int max_steps);
 // G(r, tau), G(k, nu) and Sigma_H for the mu of launch_bisection
 int launch_green(tups_ctx* ctx);
+// phase tables of Phi(R) and of the crossing tensors
+int upload_expSqR(tups_ctx* ctx);
+int upload_expqSR(tups_ctx* ctx);
 int launch_chi(tups_ctx* ctx, int q_begin, int q_count);
 int launch_bse_chunk(tups_ctx* ctx, int q_begin, int q_count);
 // slices the next BSE call will use (0 = FP64), see bse.cu

@@ -280,3 +280,21 @@ def test_split_lu_interchanges_far_from_the_diagonal(gpu_lib, n):
         g = inst.gamma[i]
         # |A^-1| is at most 1 / (5 - 0.02)
         assert np.abs(x - LU.bse_lu(g, inst.chi[i], 1.0)).max() <= 0.25 * np.sqrt(n) * tol * np.abs(g).max(), i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1e-40, 1e-158, 1e-250, 1e-300])
+def test_pivots_of_any_magnitude(gpu_lib, t):
+    """A = 1 - Gamma with pivots of t, whose square is far below the smallest double: the first columns hold nothing
+    but -t, one row off the diagonal, and X = A^-1 Gamma comes out in closed form."""
+    from tups_b200.bse_batched import solve, solve_split
+    n, m = 70, 5
+    a = 2.0 * np.eye(n, dtype=np.complex128)
+    a[:m, :m] = -t * (1.0 + 0.5j) * np.roll(np.eye(m), 1, axis=0)
+    inst = _unit_chi_instances([a])
+    want = -0.5 * np.eye(n, dtype=np.complex128)
+    want[:m, :m] = np.roll(np.eye(m), -1, axis=0) / (-t * (1.0 + 0.5j)) - np.eye(m)  # A^-1 - 1
+    for got in (solve(inst)[0], solve_split(inst, slices=8, max_refine=0)[0][0]):
+        big = np.abs(want) > 0.0
+        assert np.all(got[~big] == 0.0)
+        assert np.abs(got[big] / want[big] - 1.0).max() <= 8 * 2.3e-16

@@ -52,10 +52,18 @@ static __device__ __forceinline__ cplx cfnma(cplx a, cplx b, cplx acc) {
   return acc;
 }
 
-// 1/z with one reciprocal
+// 1/z with one reciprocal.  Where |z|^2 would leave the normal range, z is
+// scaled by the power of two of its larger part first.
 static __device__ __forceinline__ cplx crecip1(cplx z) {
-  const double q = __drcp_rn(z.x * z.x + z.y * z.y);
-  return cmk(z.x * q, -z.y * q);
+  const double d = z.x * z.x + z.y * z.y;
+  if (d > 1e-290 && d < 1e290) {
+    const double q = __drcp_rn(d);
+    return cmk(z.x * q, -z.y * q);
+  }
+  const int e = min(max(max(__double2hiint(fabs(z.x)), __double2hiint(fabs(z.y))) >> 20, 1), 2045);
+  const double s = __hiloint2double((2046 - e) << 20, 0), x = z.x * s, y = z.y * s;
+  const double q = __drcp_rn(x * x + y * y);
+  return cmk(x * q * s, -y * q * s);
 }
 
 // larger |re| + |im| <=> larger key; NaN below every number

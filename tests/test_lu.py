@@ -298,3 +298,17 @@ def test_pivots_of_any_magnitude(gpu_lib, t):
         big = np.abs(want) > 0.0
         assert np.all(got[~big] == 0.0)
         assert np.abs(got[big] / want[big] - 1.0).max() <= 8 * 2.3e-16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("split", [False, True])
+def test_small_instances_are_solved_whole(gpu_lib, split):
+    """Up to 32 rows an instance is one CTA's: the residual bound of the blocks, in a batch where larger instances
+    stand before and between them."""
+    from tups_b200.bse_batched import solve, solve_split
+    mats = [m for n in (40, 32, 5, 31, 33, 2, 20) for m in _hard_matrices(n)] + [np.full((1, 1), 3.0 - 2.0j)]
+    inst = _unit_chi_instances(mats)
+    out = solve_split(inst, slices=8, max_refine=0)[0] if split else solve(inst)
+    for i, x in enumerate(out):
+        r = _residual_over_factors(inst.gamma[i], x)
+        assert r <= _residual_bound(mats[i].shape[0]), (i, mats[i].shape[0], r)

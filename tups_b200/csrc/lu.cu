@@ -17,6 +17,7 @@
 // rows of L left of the block are never interchanged.  The products run on the
 // FP64 tensor cores.  One CTA per instance for the whole solve, which this
 // replaces, left most SMs idle and its largest instance alone at the end.
+// Instances of up to 32 rows take one kernel for all of it (k_lu_small).
 //
 // Caller-owned buffers only; the instance table and the interchange maps live
 // in static device arrays.
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) k_lu_rows(cplx* __restrict__ Aw
     }
   }
   cplx* x = sB + warp * 8 * RW_LDB;
-  tups::lud::solve_triangle<BACK>(sL, RW_LDL, sI, x, RW_LDB);
+  tups::lud::solve_triangle<BACK>(sL, RW_LDL, sI, x, RW_LDB, jb);
 #pragma unroll
   for (int i = 0; i < NB / 4; i++) {
     const int m = lane + 32 * (i & 1), j = i >> 1, c = c0 + warp * 8 + j;
@@ -363,6 +364,16 @@ __global__ void __launch_bounds__(128, 5) k_lu_update(cplx* __restrict__ Aw, cpl
     }
 }
 
+// the instances of up to kSmall rows (the last of the queue, from `first` on): a CTA each
+__global__ void __launch_bounds__(tups::lud::kSmallThreads) k_lu_small(cplx* __restrict__ Aw, cplx* __restrict__ Fout,
+                                                                       int* __restrict__ piv_all, int first) {
+  __shared__ tups::lud::SmallShared S;
+  const int inst = first + blockIdx.x;
+  const LuDesc& d = g_lu_desc[inst];
+  cplx* F = Fout + d.g_off;
+  tups::lud::small_solve(Aw + d.g_off, F, F, d.n, piv_all + d.p_off, &g_lu_status[inst], S);
+}
+
 // F -= Gamma
 __global__ void __launch_bounds__(256) k_lu_phi(const cplx* __restrict__ Gam, cplx* __restrict__ Fout) {
   const LuDesc& d = g_lu_desc[blockIdx.y];
@@ -423,8 +434,12 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
   };
   // grid rows of at most 65535 instances (n_inst <= 16384)
   k_lu_form<<<dim3(eg, n_inst), 256, 0, st>>>(G, reinterpret_cast<const cplx*>(chi), F, A);
-  int live = n_inst;
-  for (int step = 0; step * NB < nmax; step++) {
+  // instances of up to 32 rows, the last of the queue, whole; the others by blocks
+  int large = n_inst;
+  while (large > 0 && queued[large - 1].n <= tups::lud::kSmall) large--;
+  if (large < n_inst) k_lu_small<<<n_inst - large, tups::lud::kSmallThreads, 0, st>>>(A, F, ipiv, large);
+  int live = large;
+  for (int step = 0; large > 0 && step * NB < nmax; step++) {
     const int j0 = step * NB;
     while (queued[live - 1].n <= j0) live--;
     const int rows = nmax - j0, below = std::max(0, rows - NB);
@@ -435,8 +450,8 @@ extern "C" int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, cons
     k_lu_rows<false><<<dim3((unsigned)((width + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);
     if (below > 0) k_lu_update<false><<<dim3(tiles(below, width), live), 128, 0, st>>>(A, F, step);
   }
-  live = n_inst;
-  for (int step = 0; step * NB < nmax; step++) {
+  live = large;
+  for (int step = 0; large > 0 && step * NB < nmax; step++) {
     while (queued[live - 1].n <= step * NB) live--;
     const int above = ((nmax + NB - 1) / NB - 1 - step) * NB;
     k_lu_rows<true><<<dim3((unsigned)((nmax + RW_BN - 1) / RW_BN), live), RW_THREADS, kRowsSmem, st>>>(A, F, step);

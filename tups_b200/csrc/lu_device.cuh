@@ -431,8 +431,8 @@ static __device__ void block_factor(cplx* __restrict__ A, int n, int j0, int jb,
 
 // ---- solves with a 64 x 64 triangle ------------------------------------------------
 //
-// X <- T^{-1} X for one warp's 8 columns, 64 rows each in shared memory
-// (column c at X + c ldx): T, [column][row] with the pitch ldt, is unit lower
+// X <- T^{-1} X for one warp's 8 columns, `rows` <= 64 rows each in shared
+// memory (column c at X + c ldx; the rest of the last 16 rows is zero): T, [column][row] with the pitch ldt, is unit lower
 // (entries above and on the diagonal are not read) or, UP, upper with the
 // reciprocals of its diagonal in inv.  Blocks of 16 rows: what the rows solved
 // before contribute goes through the FP64 tensor cores (four real products per
@@ -447,11 +447,11 @@ static __device__ void block_factor(cplx* __restrict__ A, int n, int j0, int jb,
 // that spread over twelve decades.
 template <bool UP>
 static __device__ __forceinline__ void solve_triangle(const cplx* __restrict__ T, int ldt, const cplx* __restrict__ inv,
-                                                      cplx* X, int ldx) {
-  const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+                                                      cplx* X, int ldx, int rows) {
+  const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, nb = (rows + 15) / 16;
 #pragma unroll 1
-  for (int b = 0; b < kBlock / 16; b++) {
-    const int r0 = 16 * (UP ? kBlock / 16 - 1 - b : b);
+  for (int b = 0; b < nb; b++) {
+    const int r0 = 16 * (UP ? nb - 1 - b : b);
     if (b > 0) {
       double re[4], im[4];
 #pragma unroll
@@ -460,7 +460,7 @@ static __device__ __forceinline__ void solve_triangle(const cplx* __restrict__ T
         re[e] = v.x;
         im[e] = v.y;
       }
-      for (int k8 = UP ? r0 + 16 : 0; k8 < (UP ? kBlock : r0); k8 += 8) {
+      for (int k8 = UP ? r0 + 16 : 0; k8 < (UP ? 16 * nb : r0); k8 += 8) {
         const cplx* l = T + (k8 + tig) * ldt + r0 + gid;
         const cplx a0 = l[0], a1 = l[8], a2 = l[4 * ldt], a3 = l[4 * ldt + 8];
         const double ar[4] = {-a0.x, -a1.x, -a2.x, -a3.x}, an[4] = {-a0.y, -a1.y, -a2.y, -a3.y};
@@ -501,6 +501,70 @@ static __device__ __forceinline__ void solve_triangle(const cplx* __restrict__ T
 #pragma unroll
     for (int i = 0; i < 4; i++) X[gid * ldx + r0 + tig + 4 * i] = x[i];
     __syncwarp();
+  }
+}
+
+// ---- whole instances of up to 32 rows ------------------------------------------------
+//
+// X = A^{-1} Y by one CTA: [A | Y] in shared memory, columns with a lane per
+// row, so a column step is one search by every warp on its own, one barrier,
+// and a rank-1 update of the columns right of it that takes the interchange
+// along; L is not kept.  Pivots, status and zero pivots as in panel_factor.
+// X may be Y.  16384 instances of n = 5, 16, 32 (with the forming of A): 0.97,
+// 2.7, 7.9 ms with one CTA per instance on global memory, 2.2, 3.2, 6.0 by blocks
+// of 64 columns, 0.42, 0.95, 2.7 here.
+constexpr int kSmall = 32, kSmallThreads = 128;
+
+struct SmallShared {
+  cplx m[2 * kSmall][kSmall + 1];  // [column][row]
+  cplx inv[kSmall];                // reciprocals of U's diagonal, one for a zero
+};
+
+static __device__ void small_solve(const cplx* __restrict__ A, const cplx* Y, cplx* X, int n, int* __restrict__ ipiv,
+                                   int* __restrict__ status, SmallShared& S) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kSmallThreads / 32;
+  for (int j = warp; j < 2 * n; j += kWarps)
+    if (lane < n) S.m[j][lane] = j < n ? A[lane + (size_t)n * j] : Y[lane + (size_t)n * (j - n)];
+  __syncthreads();
+  const cplx zero = cmk(0.0, 0.0);
+  for (int c = 0; c < n; c++) {
+    cplx a = lane < n ? S.m[c][lane] : zero;
+    const bool in = lane >= c && lane < n;
+    const unsigned long long key = in ? pivot_key(a) : 0ull;
+    unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    int p = in ? lane : 0x7fffffff;
+    warp_argmax(hi, lo, p);
+    const bool singular = hi == 0u && lo == 1u;  // the key of 0.0
+    auto exchanged = [&](cplx v) {
+      const int from = lane == c ? p : lane == p ? c : lane;
+      return cmk(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from));
+    };
+    a = exchanged(a);
+    const cplx pv = cmk(__shfl_sync(0xffffffffu, a.x, c), __shfl_sync(0xffffffffu, a.y, c));
+    const cplx inv = singular ? zero : crecip1(pv);
+    const cplx l = lane > c ? cmul(a, inv) : zero;
+    for (int j = c + 1 + warp; j < 2 * n; j += kWarps) {
+      cplx x = exchanged(lane < n ? S.m[j][lane] : zero);
+      const cplx u = cmk(__shfl_sync(0xffffffffu, x.x, c), __shfl_sync(0xffffffffu, x.y, c));
+      if (lane > c) x = cfnma(l, u, x);
+      if (lane < n) S.m[j][lane] = x;
+    }
+    if (threadIdx.x == 0) {
+      ipiv[c] = p;
+      S.inv[c] = singular ? cmk(1.0, 0.0) : inv;
+      if (singular && *status == 0) *status = c + 1;
+    }
+    __syncthreads();
+  }
+  for (int j = n + warp; j < 2 * n; j += kWarps) {
+    cplx x = lane < n ? S.m[j][lane] : zero;
+    for (int c = n - 1; c >= 0; c--) {
+      const cplx v = cmul(cmk(__shfl_sync(0xffffffffu, x.x, c), __shfl_sync(0xffffffffu, x.y, c)), S.inv[c]);
+      if (lane == c) x = v;
+      if (lane < c) x = cfnma(S.m[c][lane], v, x);
+    }
+    if (lane < n) X[lane + (size_t)n * (j - n)] = x;
   }
 }
 

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict_
     S.x[c * LS_LDX + r] = je + c < JE ? A[j0 + r + (size_t)n * (je + c)] : cmk(0.0, 0.0);
   }
   __syncthreads();
-  if (8 * warp < JE - je) lud::solve_triangle<false>(S.t, LS_LDT, nullptr, S.x + 8 * warp * LS_LDX, LS_LDX);
+  if (8 * warp < JE - je) lud::solve_triangle<false>(S.t, LS_LDT, nullptr, S.x + 8 * warp * LS_LDX, LS_LDX, kBlock);
   __syncthreads();
   for (int e = tid; e < kBlock * (JE - je); e += kPanelThreads) {
     const int r = e % kBlock, c = e / kBlock;
@@ -227,7 +227,7 @@ __device__ __forceinline__ void tri_stage(const cplx* __restrict__ A, int n, int
     __syncthreads();
   }
   if (KIND < 2) {
-    lud::solve_triangle<KIND == 1>(sL, LS_LDT, sI, X + r0, LT_LDX);
+    lud::solve_triangle<KIND == 1>(sL, LS_LDT, sI, X + r0, LT_LDX, nr);
     return;
   }
   double re[4][4], im[4][4];
@@ -337,6 +337,15 @@ __global__ void __launch_bounds__(128, 1) k_ls_tri(const cplx* __restrict__ Ag, 
 #pragma unroll
   for (int c = 0; c < LT_COLS; c++)
     if (tid < jb && c < nc && (MODE != TRI_ROWS || c0 + c >= j0)) column(c)[j0 + tid] = sX[c * LT_LDX + tid];
+}
+
+// X = A^{-1} Y for instances of up to lud::kSmall rows, a CTA each, factors and all
+__global__ void __launch_bounds__(lud::kSmallThreads) k_ls_small(const cplx* __restrict__ Ag, const cplx* __restrict__ Yg,
+                                                                 cplx* __restrict__ Xg, int* __restrict__ ipiv_all,
+                                                                 int* __restrict__ status, int n) {
+  __shared__ lud::SmallShared S;
+  const size_t i = blockIdx.x, n2 = (size_t)n * n;
+  lud::small_solve(Ag + n2 * i, Yg + n2 * i, Xg + n2 * i, n, ipiv_all + n * i, &status[i], S);
 }
 
 // X = P Y: row r from row perm[r]
@@ -591,8 +600,15 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
     const dim3 eg((unsigned)std::min<size_t>((n2 + LS_THREADS - 1) / LS_THREADS, 512), b);
     if (cudaMemsetAsync(norms, 0, 2 * b * sizeof(unsigned long long), st) != cudaSuccess) return TUPS_ERR_CUDA;
     k_ls_form<<<eg, LS_THREADS, 0, st>>>(desc, G, CH, Gg, Ag, norms + b, nn);
+    // X = A^{-1} Y; small instances factor A in the same kernel each time
+    const bool small = nn <= lud::kSmall;
+    const auto solve = [&](const cplx* Y, cplx* X) {
+      if (!small) return ls_solve(st, Ag, Y, X, perm, ozw, b, nn, slices, ozstat, &launches);
+      k_ls_small<<<b, lud::kSmallThreads, 0, st>>>(Ag, Y, X, ipiv, stat, nn);
+      return cudaGetLastError() == cudaSuccess ? TUPS_OK : TUPS_ERR_CUDA;
+    };
     // P A = L U
-    for (int j0 = 0; j0 < nn; j0 += LS_NB) {
+    for (int j0 = 0; !small && j0 < nn; j0 += LS_NB) {
       const int jb = std::min(LS_NB, nn - j0), je = j0 + jb;
       for (int h0 = j0; h0 < je; h0 += kBlock) {
         const int rows = nn - h0;
@@ -611,7 +627,7 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
       }
     }
     if (cudaGetLastError() != cudaSuccess) return TUPS_ERR_CUDA;
-    int rc = ls_solve(st, Ag, Gg, Xg, perm, ozw, b, nn, slices, ozstat, &launches);
+    int rc = solve(Gg, Xg);
     if (rc) return rc;
     // refinement: residual in FP64; stop once max|R_i| <= tol max|Gamma_i| for
     // every instance of the group, else correct with the split-precision factors
@@ -639,7 +655,7 @@ extern "C" int tups_bse_lu_split_batched(int n_inst, const int* n, const int* nl
         worst = std::max(worst, rel[k]);
       }
       if (worst <= tol || steps >= max_refine) break;
-      rc = ls_solve(st, Ag, Rg, Yg, perm, ozw, b, nn, slices, ozstat, &launches);
+      rc = solve(Rg, Yg);
       if (rc) return rc;
       k_ls_update<<<eg, LS_THREADS, 0, st>>>(Xg, Yg, nn);
       steps++;

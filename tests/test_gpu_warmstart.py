@@ -196,3 +196,38 @@ def test_mlp_layers_at_tile_edges(gpu_lib, shape):
     big = np.abs(g_ref) > 1e-3 * np.abs(g_ref).max()
     assert np.abs(net.get_params() - want)[big].max() <= 1e-2 * 2 * MLP_TOL / 1e-3
     net.close()
+
+
+@pytest.mark.parametrize("shape", [(37, 65, 2, 66, 1023), (37, 65, 2, 66, 1024), (130, 64, 1, 3, 1089), (8, 129, 3, 64, 2047)],
+                         ids=["below", "at", "narrow", "wide"])
+def test_mlp_layers_of_large_batches(gpu_lib, shape):
+    """Both sides of the row count from which a layer runs on whole 64 x 64 tiles, with remainders in rows, columns
+    and depth: outputs, loss and gradients against the float64 oracle."""
+    from tups_b200.warmstart import MLP
+    n_in, hidden, layers, n_out, batch = shape
+    net = MLP(n_in, n_out, hidden, layers, max_batch=batch, seed=4)
+    rng = np.random.default_rng(23)
+    p = net.get_params()
+    x = rng.normal(size=(batch, n_in)).astype(np.float32)
+    t = rng.normal(size=(batch, n_out)).astype(np.float32)
+    y_ref, _ = OW.mlp_forward(p, net.widths, x)
+    assert parity.rel(net.forward(x), y_ref) <= 4 * max(n_in, hidden) * 6e-8
+    loss, g = net.gradients(x, t)
+    loss_ref, g_ref = OW.mlp_loss_grad(p, net.widths, x, t)
+    assert abs(loss - loss_ref) <= MLP_TOL * loss_ref
+    assert parity.rel(g, g_ref) <= MLP_TOL
+    # a training pass gathers its rows: one batch of all samples in some order
+    hist = net.train(x, t, batch=batch, epochs=1, lr=1e-3, seed=5)
+    assert abs(hist[0] - loss_ref) <= MLP_TOL * loss_ref
+    net.close()
+
+
+def test_mlp_batches_beyond_two_million_rows(gpu_lib):
+    """More row tiles of 32 than the second grid dimension takes."""
+    from tups_b200.warmstart import MLP
+    batch = 32 * 65535 + 1
+    net = MLP(1, 1, 1, 1, max_batch=batch, seed=4)
+    x = np.linspace(-2.0, 2.0, batch, dtype=np.float32)[:, None]
+    y_ref, _ = OW.mlp_forward(net.get_params(), net.widths, x)
+    assert parity.rel(net.forward(x), y_ref) <= 1e-6
+    net.close()

@@ -132,6 +132,27 @@ __device__ __forceinline__ void wait_predecessor() {
   asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// the output at offset o from its sum v; bias and aux as the epilogue reads them.
+// Returns the squared error (EPI_MSE).
+template <int EPI>
+__device__ __forceinline__ double store(const LinArgs& a, size_t o, float v, float bias, float aux) {
+  if (EPI == EPI_BIAS_SILU) {
+    v += bias;
+    a.C[o] = v;
+    a.C2[o] = v * sigmoid(v);
+  } else if (EPI == EPI_BIAS) {
+    a.C[o] = v + bias;
+  } else if (EPI == EPI_DSILU) {
+    const float s = sigmoid(aux);
+    a.C[o] = v * (s * (1.0f + aux * (1.0f - s)));
+  } else {
+    const float d = v + bias - aux;
+    a.C[o] = (float)(2.0 * a.inv) * d;
+    return (double)d * d;
+  }
+  return 0.0;
+}
+
 constexpr int kTM = 32, kTN = 16, kKC = 256, kSplit = 4, kLinThreads = 256;
 constexpr int kXP = kKC + 4, kWP = kTN + 4;  // pitches: float4 rows on distinct banks
 constexpr size_t kLinSmem = ((size_t)(kTM + kTN) * kXP > (size_t)kTM * kXP + (size_t)kKC * kWP
@@ -251,26 +272,85 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kLinThreads) k_
     float v = 0.0f;
 #pragma unroll
     for (int r = 0; r < kSplit; r++) v += cluster.map_shared_rank(part, r)[eo];
-    if (EPI == EPI_BIAS_SILU) {
-      v += bias;
-      a.C[oo] = v;
-      a.C2[oo] = v * sigmoid(v);
-    } else if (EPI == EPI_BIAS) {
-      a.C[oo] = v + bias;
-    } else if (EPI == EPI_DSILU) {
-      const float s = sigmoid(aux);
-      a.C[oo] = v * (s * (1.0f + aux * (1.0f - s)));
-    } else {
-      const float d = v + bias - aux;
-      a.C[oo] = (float)(2.0 * a.inv) * d;
-      sq = (double)d * d;
-    }
+    sq = store<EPI>(a, oo, v, bias, aux);
   }
   if (EPI == EPI_MSE && tid < kOwn) {
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     if (lane == 0) atomicAdd(a.loss, sq * a.inv);
   }
   cluster.sync();  // the partial tile stays until every rank has read it
+}
+
+// The same product for batches of a thousand rows and more: a CTA per 64 x 64
+// tile, the whole sum over k in steps of 16, 4 x 4 outputs per thread.  Bound by
+// the FP32 pipe and shared memory, where the form above repeats W for every 32
+// rows and adds up 32 partial tiles per output.  A forward pass and copies of
+// 64 -> 3 x 512 -> 68 at 768, 1024, 4096, 16384 rows: 280, 292, 628, 1786 us
+// against 255, 324, 1148, 4278 with the split sums; 200 -> 6 x 128 -> 204: 323,
+// 374, 829, 2709 against 293, 409, 1208, 4454; so the line lies at 1024 rows.
+constexpr int kBigTile = 64, kBigStep = 16, kBigRows = 1024;
+
+template <int EPI, bool WT>
+__global__ void __launch_bounds__(kLinThreads) k_mlp_tile(LinArgs a) {
+  __shared__ float Xs[kBigStep][kBigTile + 4];
+  __shared__ float Ws[kBigStep][kBigTile + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, tiles_n = (a.N + kBigTile - 1) / kBigTile;
+  const int n0 = (int)blockIdx.x % tiles_n * kBigTile, m0 = (int)blockIdx.x / tiles_n * kBigTile;
+  wait_predecessor();
+  // this thread's rows of X and the places it fills
+  constexpr int kPer = kBigTile * kBigStep / kLinThreads;
+  const float* x[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int m = m0 + ty + 16 * i;
+    x[i] = m < a.M ? a.X + (size_t)(a.rows ? a.rows[m] : m) * a.K : nullptr;
+  }
+  float acc[4][4] = {};
+  for (int k0 = 0; k0 < a.K; k0 += kBigStep) {
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      Xs[tx][ty + 16 * i] = x[i] && k0 + tx < a.K ? x[i][k0 + tx] : 0.0f;
+      if (WT) {  // W(k, n), n fastest
+        const int e = tid + i * kLinThreads, k = k0 + e / kBigTile, n = n0 + e % kBigTile;
+        Ws[e / kBigTile][e % kBigTile] = k < a.K && n < a.N ? a.W[(size_t)k * a.N + n] : 0.0f;
+      } else {   // k fastest
+        const int n = n0 + ty + 16 * i;
+        Ws[tx][ty + 16 * i] = n < a.N && k0 + tx < a.K ? a.W[(size_t)n * a.K + k0 + tx] : 0.0f;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kBigStep; k++) {
+      float u[4], v[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) u[i] = Xs[k][ty + 16 * i];
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[j] = Ws[k][tx + 16 * j];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(u[i], v[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+  double sq = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int mo = m0 + ty + 16 * i, no = n0 + tx + 16 * j;
+      if (mo >= a.M || no >= a.N) continue;
+      const size_t o = (size_t)mo * a.N + no;
+      const float bias = EPI != EPI_DSILU ? a.bias[no] : 0.0f;
+      float aux = 0.0f;
+      if (EPI == EPI_DSILU) aux = a.aux[o];
+      if (EPI == EPI_MSE) aux = a.aux[a.trows ? (size_t)a.trows[mo] * a.N + no : o];
+      sq += store<EPI>(a, o, acc[i][j], bias, aux);
+    }
+  if (EPI == EPI_MSE) {
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if ((tid & 31) == 0) atomicAdd(a.loss, sq * a.inv);
+  }
 }
 
 // ---- gradients of all layers, and the Adam step on them ------------------------------
@@ -414,6 +494,10 @@ int launch_dependent(tups_mlp* m, const char* name, void (*kernel)(Args), dim3 g
 
 template <int EPI, bool WT>
 int linear(tups_mlp* m, const LinArgs& a) {
+  if (a.M >= kBigRows) {
+    const long long tiles = ((a.M + kBigTile - 1LL) / kBigTile) * ((a.N + kBigTile - 1) / kBigTile);
+    return launch_dependent(m, "k_mlp_tile", k_mlp_tile<EPI, WT>, dim3((unsigned)tiles), 0, a);
+  }
   const dim3 grid((unsigned)((a.N + kTN - 1) / kTN * kSplit), (unsigned)((a.M + kTM - 1) / kTM));
   return launch_dependent(m, "k_mlp_linear", k_mlp_linear<EPI, WT>, grid, kLinSmem, a);
 }

@@ -231,3 +231,14 @@ def test_mlp_batches_beyond_two_million_rows(gpu_lib):
     y_ref, _ = OW.mlp_forward(net.get_params(), net.widths, x)
     assert parity.rel(net.forward(x), y_ref) <= 1e-6
     net.close()
+
+
+def test_mlp_training_with_a_nan_rate_shows(gpu_lib):
+    """A NaN learning rate is not refused: the parameters turn NaN, they do not stay as if trained."""
+    from tups_b200.warmstart import MLP
+    net = MLP(3, 2, 4, 1, max_batch=8, seed=4)
+    rng = np.random.default_rng(3)
+    net.train(rng.normal(size=(8, 3)).astype(np.float32), rng.normal(size=(8, 2)).astype(np.float32), batch=8, epochs=1,
+              lr=float("nan"))
+    assert np.all(np.isnan(net.get_params()))
+    net.close()

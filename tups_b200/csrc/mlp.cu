@@ -549,8 +549,8 @@ int forward(tups_mlp* m, int batch, const float* x, const int* rows, const float
 }
 
 // gradients of the batch whose forward (with targets) just ran: into m->grads,
-// or with lr > 0 as one Adam step
-int backward(tups_mlp* m, int batch, const float* x, const int* rows, float lr, float weight_decay) {
+// or with `adam` as one step of it
+int backward(tups_mlp* m, int batch, const float* x, const int* rows, bool adam, float lr, float weight_decay) {
   for (int l = n_linear(m) - 1; l > 0; l--) {
     // dZ_{l-1}(b, i) = sum_o dZ_l[b, o] W_l[o, i] silu'(Z_{l-1}(b, i))
     LinArgs a{};
@@ -581,7 +581,7 @@ int backward(tups_mlp* m, int batch, const float* x, const int* rows, float lr, 
     tiles += (L.fout + kGradTO - 1) / kGradTO * L.tiles_i;
   }
   g.grads = m->grads;
-  if (lr > 0.0f) {
+  if (adam) {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     m->adam_t++;
     const double bc1 = 1.0 - std::pow((double)b1, (double)m->adam_t);
@@ -749,7 +749,7 @@ extern "C" int tups_mlp_gradients(tups_mlp* m, const float* x, const float* t, i
   MTRY(h2d(m, m->t, t, (size_t)batch * m->n_out * sizeof(float)));
   MTRY(mlp_cuda(m, cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream), "memset"));
   MTRY(forward(m, batch, m->x, nullptr, m->t, m->loss));
-  MTRY(backward(m, batch, m->x, nullptr, 0.0f, 0.0f));
+  MTRY(backward(m, batch, m->x, nullptr, false, 0.0f, 0.0f));
   if (loss) MTRY(d2h(m, loss, m->loss, sizeof(double)));
   if (grad) MTRY(d2h(m, grad, m->grads, m->n_params * sizeof(float)));
   return mlp_cuda(m, cudaStreamSynchronize(m->stream), "synchronize");
@@ -791,7 +791,7 @@ extern "C" int tups_mlp_train(tups_mlp* m, const float* x, const float* t, int n
     for (int b = 0; b < per_epoch; b++) {
       const int r0 = b * batch, rows = std::min(batch, n_samples - r0);
       MTRY(forward(m, rows, m->data_x, m->idx + r0, m->data_t, m->loss + e));
-      MTRY(backward(m, rows, m->data_x, m->idx + r0, lr, weight_decay));
+      MTRY(backward(m, rows, m->data_x, m->idx + r0, true, lr, weight_decay));
     }
   }
   if (loss_per_epoch && epochs > 0) {

@@ -242,3 +242,40 @@ def test_mlp_training_with_a_nan_rate_shows(gpu_lib):
               lr=float("nan"))
     assert np.all(np.isnan(net.get_params()))
     net.close()
+
+
+def test_mlp_adam_against_the_float64_steps(gpu_lib):
+    """Three steps on one full batch against Adam in float64 with the oracle's gradients, weights and biases apart, a
+    decay of 4 % per step on the weights alone.  Where |g| is within a factor 10 of its largest, a gradient is known
+    to about 1e-5, so its step lr m / sqrt(v) to some 1e-4 of lr; a decay left out or laid on the biases would show
+    as 400 times that."""
+    from tups_b200.warmstart import MLP
+    n_in, hidden, layers, n_out, batch, lr, wd = 20, 33, 2, 17, 32, 1e-2, 4.0
+    net = MLP(n_in, n_out, hidden, layers, max_batch=batch, seed=6)
+    rng = np.random.default_rng(29)
+    layout, _ = OW.mlp_layout(net.widths)
+    p = net.get_params()
+    for _, bo, _, fout in layout:
+        p[bo:bo + fout] = rng.normal(size=fout)
+    net.set_params(p)
+    p = p.astype(np.float64)
+    x = rng.normal(size=(batch, n_in)).astype(np.float32)
+    t = rng.normal(size=(batch, n_out)).astype(np.float32)
+    weight = np.zeros(p.size, dtype=bool)
+    for wo, bo, _, _ in layout:
+        weight[wo:bo] = True
+    b1, b2, eps, m, v = 0.9, 0.999, 1e-8, np.zeros_like(p), np.zeros_like(p)
+    clear = np.ones(p.size, dtype=bool)
+    for step in range(1, 4):
+        _, g = OW.mlp_loss_grad(p, net.widths, x.astype(np.float64), t.astype(np.float64))
+        for part in (weight, ~weight):
+            clear &= ~part | (np.abs(g) > 0.1 * np.abs(g[part]).max())
+        p[weight] *= 1.0 - lr * wd
+        m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+        p -= lr * (m / (1 - b1 ** step)) / (np.sqrt(v / (1 - b2 ** step)) + eps)
+    net.train(x, t, batch=batch, epochs=3, lr=lr, weight_decay=wd, seed=5)
+    got = net.get_params()
+    for part in (weight, ~weight):
+        assert np.count_nonzero(clear & part) >= 10
+        assert np.abs(got - p)[clear & part].max() <= 3 * 1e-4 * lr + 6e-8 * np.abs(p).max()
+    net.close()

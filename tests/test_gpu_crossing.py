@@ -50,3 +50,53 @@ def test_crossing_at_tile_edges(gpu_lib, case, products):
     for r in "dmst":
         assert parity.rel(sol.F(r), st.F[r]) <= TOL, r
     sol.close()
+
+
+def test_crossing_takes_no_memory_of_its_own(gpu_lib):
+    """The gathered operand (0.15 GB here) goes into the BSE's scratch: the first crossing of a context allocates its
+    element lists and no more, so that what fits a card beside a context does not depend on it."""
+    import torch
+    from tups_b200 import Params, Solver
+    sol = Solver(Params(beta=3.0, U=2.0, nParticle=0.95, Nx=8, Nf=32, neighbours=2, f_damping=0.5, ite_max=10))
+    sol.set_autotune(False)
+    sol.calculate_expSqR()
+    sol.calculate_expqSR()
+    for w in ("phbar_to_ph", "pp_to_ph", "ph_to_pp", "phbar_to_pp"):
+        getattr(sol, "calc_M_" + w)()
+    sol.calc_PhiR(0)
+    free0 = torch.cuda.mem_get_info()[0]
+    sol.calculate_PAE()
+    assert free0 - torch.cuda.mem_get_info()[0] <= 16 << 20
+    sol.close()
+
+
+def test_crossing_leaves_the_bse_alone(gpu_lib):
+    """The scratch is the BSE's again in the next iteration: three iterations, two in FP64 and one split, queued as
+    one against the single calls, each of which waits."""
+    from tups_b200 import Params, Solver
+    p = Params(beta=3.0, U=2.0, nParticle=0.95, Nx=4, Nf=10, neighbours=3, f_damping=0.5, ite_max=10)
+    a, b = Solver(p), Solver(p)
+    for ite in range(3):
+        if ite == 2:
+            for s in (a, b):
+                s.set_bse_precision(5)
+        a.iteration(ite)
+        b.calc_Gkw_Grt(ite)
+        b.BSE(ite)
+        if ite == 0:
+            b.calculate_expSqR()
+            b.calculate_expqSR()
+            for w in ("phbar_to_ph", "pp_to_ph", "ph_to_pp", "phbar_to_pp"):
+                getattr(b, "calc_M_" + w)()
+        b.calc_PhiR(ite)
+        b.calculate_PAE()
+        b.calc_SDE(ite)
+        b.conv()
+        if ite % 5 == 0:
+            b.output_block()
+        b.vertex_update()
+        assert np.array_equal(a.Sigma, b.Sigma)
+        for r in "dmst":
+            assert np.array_equal(a.F(r), b.F(r)) and np.array_equal(a.G(r), b.G(r))
+    a.close()
+    b.close()

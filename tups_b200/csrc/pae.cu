@@ -27,7 +27,7 @@
 //     C^T[(target, element), (l1,l2)] = X^T[(target, element), (l3,l4,R)] M^T
 // and F = Phi + Lambda*Nc + C/Nx.  X does not depend on the momentum Q, so a
 // gather pass (k_pae_gather) forms it once per bosonic frequency as a plain
-// matrix, for as many frequencies as a bounded workspace holds, and the GEMM
+// matrix, for as many frequencies as the BSE's scratch holds, and the GEMM
 // (k_pae_gemm, FP64 tensor cores) runs over the columns (Q, l1, l2) of all
 // momenta.  A base pass writes Phi + Lambda*Nc, and each family adds C/Nx to the
 // elements it reaches by reductions in L2, each element at most once per pass,
@@ -408,40 +408,41 @@ static int build_pae_lists(tups_ctx* ctx) {
           }
         cnt[L] = c;
       }
-  // the gathered operand: as many frequencies at a time as 1 GiB holds (less
-  // when the device does not have it), at least one
+  // The gathered operand goes into the BSE's scratch, which holds nothing outside
+  // a BSE call: as many frequencies at a time as it takes, at least one.  Only
+  // a context of very few slots has less there than one frequency needs.
   const long long K = (long long)d.Nl * d.Nl * d.NR;
+  const size_t room = (size_t)d.Nz * d.Nz * ctx->s.bse_chunk;
   std::vector<long long> xoff((size_t)4 * nh, 0);
-  void* px = nullptr;
-  for (size_t cap = (size_t)1 << 30;; cap /= 4) {
-    size_t need = 0;
-    for (int fam = 0; fam < 2; fam++) {
-      std::vector<int>& begin = ctx->pae_chunks[fam];
-      begin.assign(1, 0);
-      size_t used = 0;  // complex entries of the chunk so far
-      for (int W = 1; W <= nh; W++) {
-        size_t own = 0;
-        for (int pair = 0; pair < 2; pair++) own += 2 * (size_t)cnt[pae_list(pair, fam, W, nh)] * K;
-        if (used > 0 && (used + own) * sizeof(cplx) > cap) {
-          begin.push_back(W - 1);
-          used = 0;
-        }
-        for (int pair = 0; pair < 2; pair++) {
-          const int L = pae_list(pair, fam, W, nh);
-          xoff[L] = (long long)used;
-          used += 2 * (size_t)cnt[L] * K;
-        }
-        need = std::max(need, used);
+  size_t need = 0;
+  for (int fam = 0; fam < 2; fam++) {
+    std::vector<int>& begin = ctx->pae_chunks[fam];
+    begin.assign(1, 0);
+    size_t used = 0;  // complex entries of the chunk so far
+    for (int W = 1; W <= nh; W++) {
+      size_t own = 0;
+      for (int pair = 0; pair < 2; pair++) own += 2 * (size_t)cnt[pae_list(pair, fam, W, nh)] * K;
+      if (used > 0 && used + own > room) {
+        begin.push_back(W - 1);
+        used = 0;
       }
-      begin.push_back(nh);
+      for (int pair = 0; pair < 2; pair++) {
+        const int L = pae_list(pair, fam, W, nh);
+        xoff[L] = (long long)used;
+        used += 2 * (size_t)cnt[L] * K;
+      }
+      need = std::max(need, used);
     }
-    const cudaError_t e = cudaMalloc(&px, std::max<size_t>(need, 1) * sizeof(cplx));
-    if (e == cudaSuccess) break;
-    cudaGetLastError();
-    if (cap < 1024) return set_error(ctx, TUPS_ERR_OOM, "crossing workspace");
+    begin.push_back(nh);
   }
-  ctx->allocations.push_back(px);
-  ctx->t.pae_x = (cplx*)px;
+  ctx->t.pae_x = ctx->s.bse_A;
+  if (need > room) {
+    void* px = nullptr;
+    const int rc = cuda_check(ctx, cudaMalloc(&px, need * sizeof(cplx)), "crossing workspace");
+    if (rc) return rc;
+    ctx->allocations.push_back(px);
+    ctx->t.pae_x = (cplx*)px;
+  }
   ctx->pae_cnt = cnt;
   void* pe = nullptr;
   void* pc = nullptr;

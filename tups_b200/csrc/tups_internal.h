@@ -42,7 +42,7 @@ struct DeviceTables {
   int4* pae_elems = nullptr;  // crossing: elements per (pair, family, W), see pae.cu
   int* pae_counts = nullptr;
   long long* pae_xoff = nullptr;  // crossing: a list's place in the gathered operand
-  cplx* pae_x = nullptr;          // crossing: the gathered operand of one chunk of frequencies
+  cplx* pae_x = nullptr;          // crossing: the gathered operand of one chunk of frequencies (BSE scratch)
 };
 
 struct DeviceState {
@@ -56,7 +56,7 @@ struct DeviceState {
   cplx* G[4] = {};            // (Nz, Nz, Nb)
   cplx* chi_ph = nullptr;     // (Nl, Nl, Nf, Nb) nu-diagonal blocks of chi_ph_LL
   cplx* chi_pp = nullptr;
-  cplx* bse_A = nullptr;      // BSE scratch: Gamma*chi per instance of a chunk
+  cplx* bse_A = nullptr;      // BSE scratch: Gamma*chi per instance of a chunk; the crossing's gathered operand
   cplx* bse_B = nullptr;      // chi*Gamma
   size_t bse_chunk = 0;       // instances per chunk
   cplx* PhiR[4] = {};         // (Nz*Nz, Nf/2, NR)

@@ -100,3 +100,51 @@ def test_crossing_leaves_the_bse_alone(gpu_lib):
             assert np.array_equal(a.F(r), b.F(r)) and np.array_equal(a.G(r), b.G(r))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("neighbours,ntasks", [(2, 30), (2, 15), (2, 10), (2, 6), (2, 5), (2, 3), (2, 2), (3, 30), (3, 10)])
+def test_crossing_of_a_ranks_slots(gpu_lib, neighbours, ntasks):
+    """One slot, some frequencies of a momentum, of two, whole momenta: the crossing of a rank's slots, by the form
+    that gathers in the GEMM (up to 64 columns) or ahead of it, against the crossing of all slots."""
+    import torch
+    from tups_b200 import Params, Solver
+    from tups_b200.sharded import _DeviceBuffer
+    p = Params(beta=3.0, U=2.0, nParticle=0.95, Nx=4, Nf=10, neighbours=neighbours, f_damping=0.5, ite_max=10)
+    full = Solver(p)
+    rng = np.random.default_rng(ntasks)
+    shape = (full.Nz, full.Nz, full.Nb)
+    G = {r: rng.standard_normal(shape) + 1j * rng.standard_normal(shape) for r in "dmst"}
+    phir = {}
+
+    def whole_phir(what, ptr, count, op):
+        t = torch.as_tensor(_DeviceBuffer(ptr, count), device="cuda:0")
+        t.copy_(torch.from_numpy(phir["dmst"[what]]))
+        torch.cuda.synchronize()
+
+    def crossing(sol, slots):
+        sol.calculate_expSqR()
+        sol.calculate_expqSR()
+        for w in ("phbar_to_ph", "pp_to_ph", "ph_to_pp", "phbar_to_pp"):
+            getattr(sol, "calc_M_" + w)()
+        for r in "dmst":
+            sol.set_vertex(r, 1, np.asfortranarray(G[r][..., slots]))
+        sol.calc_PhiR(0)
+
+    crossing(full, slice(None))
+    phir.update({r: np.ravel(full.PhiR(r), order="F").view(np.float64).copy() for r in "dmst"})
+    want = {}
+    for products in (3, 4):
+        full.set_crossing_products(products)
+        full.calculate_PAE()
+        want[products] = {r: full.F(r).copy() for r in "dmst"}
+    full.close()
+    for rank in sorted({0, ntasks // 2, ntasks - 1}):
+        sol = Solver(p, 0, rank, ntasks, whole_phir)
+        slots = slice(sol.slot0, sol.slot0 + sol.Nb)
+        crossing(sol, slots)
+        for products in (3, 4):
+            sol.set_crossing_products(products)
+            sol.calculate_PAE()
+            for r in "dmst":
+                assert parity.rel(sol.F(r), want[products][r][..., slots]) <= TOL, (rank, products, r)
+        sol.close()

@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_ls_panel(cplx* __restrict_
 using LsTile = ZgemmTile<1, 2, 2, 2, 16, 2, false, false>;
 
 struct LsSource {
+  static constexpr bool kGather = false;
   const cplx *l, *r;
   int n, K, n0;
   __device__ int ktiles() const { return (K + 15) / 16; }

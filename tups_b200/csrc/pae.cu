@@ -32,8 +32,8 @@
 // momenta.  A base pass writes Phi + Lambda*Nc, and each family adds C/Nx to the
 // elements it reaches by reductions in L2, each element at most once per pass,
 // so the result does not depend on the order of the CTAs (deterministic).
-// Gathering X inside the GEMM, as it was done before, repeated the scattered
-// loads and the dispatch arithmetic for every column tile.
+// Gathering X inside the GEMM repeats the scattered loads and the dispatch
+// arithmetic for every column tile: that form serves contexts of few columns.
 // With one form factor the sum over k has NR terms only: k_pae_direct forms
 // every element at once without the lists.
 #include <string>
@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(32 * PG_WARPS) k_pae_gather(PaePtrs P, const i
 // X^T tile rows from the workspace, M^T columns (Q, l1, l2) with k fastest
 template <int BK>
 struct PaeSource {
+  static constexpr bool kGather = false;
   const cplx *x, *m;  // first row of the tile, first column of the tile
   size_t ld;          // rows of X
   int K;
@@ -233,15 +234,64 @@ struct PaeSource {
   __device__ size_t roff(int n) const { return (size_t)K * n; }
 };
 
+// The same operands with the tile's X formed from Phi(R) in the GEMM's own stages,
+// as k_pae_gather does: the tile's rows are both targets of BM / 2 elements,
+// target 0 first, so a source entry is read once for the two.  koff: of every k,
+// in shared memory, twice its offset in Phi(R) plus one where s(l3) s(l4) = -1.
+template <class Tile, int BK>
+struct PaeGatherSource {
+  static constexpr bool kGather = true;
+  static constexpr int kElems = Tile::BM / 2, kStep = Tile::NT / kElems, kPer = BK / kStep;
+  static_assert(Tile::NT % kElems == 0 && BK % kStep == 0, "a thread keeps its element");
+  const cplx *x0, *x1;  // the element's source entries at l3 = l4 = R = 0
+  const double (*fac)[2];  // dispatch factors [source][target]
+  bool in, tr;
+  const cplx* m;
+  const long long* koff;
+  int K;
+  cplx v0[kPer], v1[kPer];
+  double sg[kPer];
+  __device__ int ktiles() const { return (K + BK - 1) / BK; }
+  __device__ int depth(int kt) const { return min(BK, K - kt * BK); }
+  __device__ size_t ldl() const { return 0; }
+  __device__ const cplx* left(int) const { return m; }
+  __device__ const cplx* right(int kt) const { return m + kt * BK; }
+  __device__ size_t roff(int n) const { return (size_t)K * n; }
+  __device__ void fetch(int kt) {
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int k = kt * BK + (int)threadIdx.x / kElems + i * kStep;
+      v0[i] = v1[i] = cmk(0.0, 0.0);
+      sg[i] = 1.0;
+      if (in && k < K) {
+        const long long o = koff[k];
+        v0[i] = x0[o >> 1];
+        v1[i] = x1[o >> 1];
+        sg[i] = o & 1 ? -1.0 : 1.0;
+      }
+    }
+  }
+  __device__ void put(cplx* stage) const {
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      cplx* d = stage + ((int)threadIdx.x / kElems + i * kStep) * Tile::LDL + threadIdx.x % kElems;
+      d[0] = pae_combine(v0[i], v1[i], fac[0][0], fac[1][0], tr, sg[i]);
+      d[kElems] = pae_combine(v0[i], v1[i], fac[0][1], fac[1][1], tr, sg[i]);
+    }
+  }
+};
+
 // F_target += C / Nx for one family: tiles of (target, element) rows and
 // (momentum, l1, l2) columns, the columns of all the context's momenta numbered
 // flat so that only the last tile pads.  The columns are the fastest grid
-// dimension: the CTAs in flight share X rows, and M^T stays in L2.
-template <class Tile, int BK, int MINB>
+// dimension: the CTAs in flight share X rows, and M^T stays in L2.  GATHER: X is
+// formed here (PaeGatherSource), once per column tile.
+template <class Tile, int BK, int MINB, bool GATHER>
 __global__ void __launch_bounds__(Tile::NT, MINB) k_pae_gemm(PaePtrs P, const cplx* __restrict__ X,
                                                              const int4* __restrict__ elems,
                                                              const int* __restrict__ counts,
-                                                             const long long* __restrict__ xoff, int Nz, int Nf, int Nl,
+                                                             const long long* __restrict__ xoff,
+                                                             const int* __restrict__ signs, int Nz, int Nf, int Nl,
                                                              int NR, int fam, int w_begin, int nw, int slot0, int Nb,
                                                              double inv_nx) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -249,8 +299,11 @@ __global__ void __launch_bounds__(Tile::NT, MINB) k_pae_gemm(PaePtrs P, const cp
   __shared__ long long fcol[Tile::BN];  // offset of the column's (l1, l2, slot), -1 if not of this context
   const int pair = blockIdx.z / nw, w = w_begin + blockIdx.z % nw, nh = Nf / 2;
   const int list = pae_list(pair, fam, w + 1, nh);
-  const int cnt = counts[list], rows = 2 * cnt, m0 = blockIdx.y * Tile::BM, n0 = blockIdx.x * Tile::BN;
-  if (m0 >= rows) return;
+  const int cnt = counts[list], n0 = blockIdx.x * Tile::BN;
+  // GATHER: rows of a tile stand for both targets of half as many elements
+  const int e0 = blockIdx.y * (Tile::BM / 2), m0 = GATHER ? 0 : blockIdx.y * Tile::BM;
+  const int rows = GATHER ? Tile::BM : 2 * cnt;
+  if (GATHER ? e0 >= cnt : m0 >= rows) return;
   const int nl2 = Nl * Nl, Q0 = slot0 / nh, Q1 = (slot0 + Nb - 1) / nh, cols = (Q1 - Q0 + 1) * nl2;
   const size_t n2 = (size_t)Nz * Nz;
   auto local_slot = [&](int iq) {  // local index of slot (Q0 + iq, w), or -1
@@ -262,8 +315,10 @@ __global__ void __launch_bounds__(Tile::NT, MINB) k_pae_gemm(PaePtrs P, const cp
   if (!any) return;
   for (int r = threadIdx.x; r < Tile::BM; r += Tile::NT) {
     cplx* f = nullptr;
-    if (m0 + r < rows) {
-      const int t = m0 + r >= cnt, x = elems[(size_t)list * Nf * Nf + (m0 + r - t * cnt)].x;
+    const int t = GATHER ? r >= Tile::BM / 2 : m0 + r >= cnt;
+    const int e = GATHER ? e0 + r - t * (Tile::BM / 2) : m0 + r - t * cnt;
+    if (GATHER ? e < cnt : m0 + r < rows) {
+      const int x = elems[(size_t)list * Nf * Nf + e].x;
       // constant indices keep the parameter struct out of local memory
       cplx* F = pair == 0 ? (t ? P.F[1] : P.F[0]) : (t ? P.F[3] : P.F[2]);
       f = F + ((x & 255) - 1) + (size_t)Nz * ((x >> 8) - 1);
@@ -276,15 +331,38 @@ __global__ void __launch_bounds__(Tile::NT, MINB) k_pae_gemm(PaePtrs P, const cp
   }
   Tile t;
   const int K = nl2 * NR;
-  t.run(PaeSource<BK>{X + xoff[list] + m0, pae_tensor(P, pair, fam) + (size_t)K * ((size_t)Q0 * nl2 + n0), (size_t)rows,
-                      K},
-        reinterpret_cast<cplx*>(smraw), rows - m0, cols - n0);
+  const cplx* right = pae_tensor(P, pair, fam) + (size_t)K * ((size_t)Q0 * nl2 + n0);
+  if constexpr (GATHER) {
+    long long* koff = reinterpret_cast<long long*>(smraw + Tile::kSmem);
+    for (int k = threadIdx.x; k < K; k += Tile::NT) {
+      const int l34 = k % nl2, l3 = l34 % Nl, l4 = l34 / Nl;
+      koff[k] = 2 * ((long long)l3 * Nf + (long long)Nz * l4 * Nf + (long long)(n2 * nh) * (k / nl2)) +
+                (signs[l3] * signs[l4] < 0);
+    }
+    __syncthreads();
+    PaeGatherSource<Tile, BK> src;
+    const int e = e0 + threadIdx.x % PaeGatherSource<Tile, BK>::kElems;
+    src.in = e < cnt;
+    const int4 rec = elems[(size_t)list * Nf * Nf + min(e, cnt - 1)];
+    const size_t eo = (size_t)(rec.z - 1) + (size_t)Nz * ((rec.w & 65535) - 1) + n2 * (rec.y - 1);
+    src.x0 = pae_source(P, pair, fam, 0) + eo;
+    src.x1 = pae_source(P, pair, fam, 1) + eo;
+    src.fac = c_pae_fac[pair][fam];
+    src.tr = (rec.w >> 16) != 0;
+    src.m = right;
+    src.koff = koff;
+    src.K = K;
+    t.run(src, reinterpret_cast<cplx*>(smraw), rows - m0, cols - n0);
+  } else {
+    t.run(PaeSource<BK>{X + xoff[list] + m0, right, (size_t)rows, K}, reinterpret_cast<cplx*>(smraw), rows - m0,
+          cols - n0);
+  }
   // a reduction in L2 (no value returned, so no wait for the old F); each
   // element is in a family's list once, so no two CTAs of a launch add to the
   // same entry
   t.each(rows - m0, cols - n0, [&](int row, int col, cplx c) {
     const long long o = fcol[col];
-    if (o < 0) return;
+    if (o < 0 || (GATHER && !frow[row])) return;
     cplx* f = frow[row] + o;
     atomicAdd(&f->x, __dmul_rn(inv_nx, c.x));
     atomicAdd(&f->y, __dmul_rn(inv_nx, c.y));
@@ -332,6 +410,12 @@ __global__ void k_pae_direct(PaePtrs P, const int* __restrict__ ibz, const int* 
   (pair ? P.F[3] : P.F[1])[e] = f1;
 }
 
+// Columns up to which the GEMM gathers X itself (ranks that hold one or two
+// momenta).  Five form factors, 32 frequencies, in the GEMM against ahead of it:
+// 25 columns 0.140 against 0.206 ms, 50 0.223 against 0.250, 75 0.329 against
+// 0.325, 100 0.406 against 0.384; nine form factors, 81 columns 0.184, 0.178.
+constexpr int kPaeFewColumns = 64;
+
 static int run_base(tups_ctx* ctx, const PaePtrs& P) {
   const auto& d = ctx->d;
   const size_t n = (size_t)d.Nz * d.Nz * d.Nb;
@@ -342,36 +426,41 @@ static int run_base(tups_ctx* ctx, const PaePtrs& P) {
 }
 
 // F = Phi + Lambda Nc, then the diagonal family, then the anti-diagonal one
-template <class Tile, int BK, int MINB>
+template <class Tile, int BK, int MINB, bool GATHER = false>
 static int run_pae(tups_ctx* ctx, const PaePtrs& P) {
   const auto& d = ctx->d;
-  auto kern = k_pae_gemm<Tile, BK, MINB>;
-  if (Tile::kSmem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem);
+  auto kern = k_pae_gemm<Tile, BK, MINB, GATHER>;
+  const int nh = d.Nf / 2, K = d.Nl * d.Nl * d.NR;
+  const size_t smem = Tile::kSmem + (GATHER ? K * sizeof(long long) : 0);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_check(ctx, e, "k_pae_gemm smem attribute");
   }
   int rc = run_base(ctx, P);
-  const int nh = d.Nf / 2, K = d.Nl * d.Nl * d.NR;
   const int nQ = (ctx->slot0 + d.Nb - 1) / nh - ctx->slot0 / nh + 1;  // momenta holding this context's slots
   const unsigned gx = (unsigned)cdiv((long long)nQ * d.Nl * d.Nl, Tile::BN);
+  const std::vector<int> whole = {0, nh};
   for (int fam = 0; fam < 2 && !rc; fam++) {
-    const std::vector<int>& begin = ctx->pae_chunks[fam];  // first frequency of each chunk, then nh
+    // first frequency of each chunk, then nh
+    const std::vector<int>& begin = GATHER ? whole : ctx->pae_chunks[fam];
     for (size_t c = 0; c + 1 < begin.size() && !rc; c++) {
       const int w0 = begin[c], nw = begin[c + 1] - w0;
       int longest = 0;
       for (int pair = 0; pair < 2; pair++)
         for (int w = w0; w < w0 + nw; w++) longest = std::max(longest, ctx->pae_cnt[pae_list(pair, fam, w + 1, nh)]);
       if (longest == 0) continue;
-      // few elements: split k over CTAs until the grid fills the SMs
-      const long long ctas = (long long)cdiv(longest, 32) * 2 * nw;
-      const int ksplit = (int)std::max<long long>(1, std::min<long long>(cdiv(K, 4 * PG_WARPS), cdiv(148 * 6, ctas)));
-      k_pae_gather<<<dim3((unsigned)cdiv(longest, 32), ksplit, 2 * nw), 32 * PG_WARPS, 0, ctx->stream>>>(
-          P, ctx->t.pae_elems, ctx->t.pae_counts, ctx->t.pae_xoff, ctx->t.signs, ctx->t.pae_x, d.Nz, d.Nf, d.Nl, d.NR,
-          fam, w0, nw);
-      if ((rc = after_launch(ctx, "k_pae_gather"))) break;
-      kern<<<dim3(gx, (unsigned)cdiv(2LL * longest, Tile::BM), 2 * nw), Tile::NT, Tile::kSmem, ctx->stream>>>(
-          P, ctx->t.pae_x, ctx->t.pae_elems, ctx->t.pae_counts, ctx->t.pae_xoff, d.Nz, d.Nf, d.Nl, d.NR, fam, w0, nw,
-          ctx->slot0, d.Nb, 1.0 / d.Nx);
+      if (!GATHER) {
+        // few elements: split k over CTAs until the grid fills the SMs
+        const long long ctas = (long long)cdiv(longest, 32) * 2 * nw;
+        const int ksplit = (int)std::max<long long>(1, std::min<long long>(cdiv(K, 4 * PG_WARPS), cdiv(148 * 6, ctas)));
+        k_pae_gather<<<dim3((unsigned)cdiv(longest, 32), ksplit, 2 * nw), 32 * PG_WARPS, 0, ctx->stream>>>(
+            P, ctx->t.pae_elems, ctx->t.pae_counts, ctx->t.pae_xoff, ctx->t.signs, ctx->t.pae_x, d.Nz, d.Nf, d.Nl,
+            d.NR, fam, w0, nw);
+        if ((rc = after_launch(ctx, "k_pae_gather"))) break;
+      }
+      kern<<<dim3(gx, (unsigned)cdiv(2LL * longest, Tile::BM), 2 * nw), Tile::NT, smem, ctx->stream>>>(
+          P, ctx->t.pae_x, ctx->t.pae_elems, ctx->t.pae_counts, ctx->t.pae_xoff, ctx->t.signs, d.Nz, d.Nf, d.Nl, d.NR,
+          fam, w0, nw, ctx->slot0, d.Nb, 1.0 / d.Nx);
       rc = after_launch(ctx, "k_pae_gemm");
     }
   }
@@ -388,8 +477,16 @@ static int run_direct(tups_ctx* ctx, const PaePtrs& P) {
   return after_launch(ctx, "k_pae_direct");
 }
 
+// few columns per frequency: no pass that gathers X once for all of them
+static bool pae_few_columns(const tups_ctx* ctx) {
+  const auto& d = ctx->d;
+  const int nh = d.Nf / 2, nQ = (ctx->slot0 + d.Nb - 1) / nh - ctx->slot0 / nh + 1;
+  return nQ * d.Nl * d.Nl <= kPaeFewColumns;
+}
+
 // Element lists of the two families per target pair and bosonic index W,
 // built on the host from the frequency maps (pae_family) at the first call.
+// Frequencies of which the context has no slot get empty lists.
 static int build_pae_lists(tups_ctx* ctx) {
   const auto& d = ctx->d;
   const int Nf = d.Nf, nh = Nf / 2;
@@ -398,6 +495,7 @@ static int build_pae_lists(tups_ctx* ctx) {
   for (int pair = 0; pair < 2; pair++)
     for (int fam = 0; fam < 2; fam++)
       for (int W = 1; W <= nh; W++) {
+        if (d.Nb < nh && (W - 1 - ctx->slot0 % nh + nh) % nh >= d.Nb) continue;
         const int L = pae_list(pair, fam, W, nh);
         int c = 0;
         for (int nu2 = 1; nu2 <= Nf; nu2++)
@@ -410,39 +508,48 @@ static int build_pae_lists(tups_ctx* ctx) {
       }
   // The gathered operand goes into the BSE's scratch, which holds nothing outside
   // a BSE call: as many frequencies at a time as it takes, at least one.  Only
-  // a context of very few slots has less there than one frequency needs.
+  // contexts of few slots (ranks) have less there than all frequencies need;
+  // they take a workspace of their own where that is small (8x8, 9 form factors,
+  // 16 frequencies, two momenta: 44 MB, 316 us for a crossing, 344 in two chunks)
+  // or where not even one frequency fits.
   const long long K = (long long)d.Nl * d.Nl * d.NR;
-  const size_t room = (size_t)d.Nz * d.Nz * ctx->s.bse_chunk;
+  constexpr size_t kOwn = ((size_t)64 << 20) / sizeof(cplx);
   std::vector<long long> xoff((size_t)4 * nh, 0);
-  size_t need = 0;
-  for (int fam = 0; fam < 2; fam++) {
-    std::vector<int>& begin = ctx->pae_chunks[fam];
-    begin.assign(1, 0);
-    size_t used = 0;  // complex entries of the chunk so far
-    for (int W = 1; W <= nh; W++) {
-      size_t own = 0;
-      for (int pair = 0; pair < 2; pair++) own += 2 * (size_t)cnt[pae_list(pair, fam, W, nh)] * K;
-      if (used > 0 && used + own > room) {
-        begin.push_back(W - 1);
-        used = 0;
+  const auto plan = [&](size_t room) {  // chunks of up to `room` entries; returns the largest
+    size_t need = 0;
+    for (int fam = 0; fam < 2; fam++) {
+      std::vector<int>& begin = ctx->pae_chunks[fam];
+      begin.assign(1, 0);
+      size_t used = 0;  // complex entries of the chunk so far
+      for (int W = 1; W <= nh; W++) {
+        size_t own = 0;
+        for (int pair = 0; pair < 2; pair++) own += 2 * (size_t)cnt[pae_list(pair, fam, W, nh)] * K;
+        if (used > 0 && used + own > room) {
+          begin.push_back(W - 1);
+          used = 0;
+        }
+        for (int pair = 0; pair < 2; pair++) {
+          const int L = pae_list(pair, fam, W, nh);
+          xoff[L] = (long long)used;
+          used += 2 * (size_t)cnt[L] * K;
+        }
+        need = std::max(need, used);
       }
-      for (int pair = 0; pair < 2; pair++) {
-        const int L = pae_list(pair, fam, W, nh);
-        xoff[L] = (long long)used;
-        used += 2 * (size_t)cnt[L] * K;
-      }
-      need = std::max(need, used);
+      begin.push_back(nh);
     }
-    begin.push_back(nh);
+    return need;
+  };
+  const size_t room = 2 * ctx->s.bse_half;
+  size_t need = plan(SIZE_MAX);
+  if (need > kOwn) need = plan(room);
+  void* px = nullptr;
+  if (need > room && cudaMalloc(&px, need * sizeof(cplx)) != cudaSuccess) {
+    cudaGetLastError();
+    px = nullptr;
+    if (plan(room) > room) return set_error(ctx, TUPS_ERR_OOM, "crossing workspace");
   }
-  ctx->t.pae_x = ctx->s.bse_A;
-  if (need > room) {
-    void* px = nullptr;
-    const int rc = cuda_check(ctx, cudaMalloc(&px, need * sizeof(cplx)), "crossing workspace");
-    if (rc) return rc;
-    ctx->allocations.push_back(px);
-    ctx->t.pae_x = (cplx*)px;
-  }
+  if (px) ctx->allocations.push_back(px);
+  ctx->t.pae_x = px ? (cplx*)px : ctx->s.bse_A;
   ctx->pae_cnt = cnt;
   void* pe = nullptr;
   void* pc = nullptr;
@@ -500,6 +607,17 @@ static const PaeCand kPaeG4[] = {
     {"32x32_s3", run_pae<ZgemmTile<1, 2, 2, 2, 16, 3, false>, 16, 3>},
     {"32x32_s3_x4", run_pae<ZgemmTile<1, 2, 2, 2, 16, 3, false, false>, 16, 4>},
 };
+// up to kPaeFewColumns columns
+static const PaeCand kPaeG3Few[] = {
+    {"g3_32x32_s2_x4_gather", run_pae<ZgemmTile<1, 2, 2, 2, 16, 2, true, false>, 16, 4, true>},
+    {"g3_32x32_s2_x5", run_pae<ZgemmTile<1, 2, 2, 2, 16, 2, true, false>, 16, 5>},
+    {"g3_32x32_s3_x4", run_pae<ZgemmTile<1, 2, 2, 2, 16, 3, true, false>, 16, 4>},
+    {"g3_32x32_s3", run_pae<ZgemmTile<1, 2, 2, 2, 16, 3, true>, 16, 3>},
+};
+static const PaeCand kPaeG4Few[] = {
+    {"32x32_s2_x4_gather", run_pae<ZgemmTile<1, 2, 2, 2, 16, 2, false, false>, 16, 4, true>},
+    {"32x32_s3_x4", run_pae<ZgemmTile<1, 2, 2, 2, 16, 3, false, false>, 16, 4>},
+};
 static const PaeCand kPaeDirect[] = {
     {"direct_b128", run_direct<128>},
     {"direct_b256", run_direct<256>},
@@ -526,10 +644,16 @@ int launch_pae(tups_ctx* ctx) {
   }
   const bool g3 = ctx->pae_products == 3 && nl2 > 8;
   const bool brief = nl2 * d.NR < 256;
-  const PaeCand* cands = nl2 <= 8 ? kPaeDirect : g3 ? (brief ? kPaeG3Short : kPaeG3) : kPaeG4;
-  const int n_cand = (int)(nl2 <= 8 ? sizeof(kPaeDirect)
-                           : g3     ? (brief ? sizeof(kPaeG3Short) : sizeof(kPaeG3))
-                                    : sizeof(kPaeG4)) / (int)sizeof(PaeCand);
+  const PaeCand* cands = nullptr;
+  int n_cand = 0;
+  const auto take = [&](const PaeCand* c, size_t bytes) {
+    cands = c;
+    n_cand = (int)(bytes / sizeof(PaeCand));
+  };
+  if (nl2 <= 8) take(kPaeDirect, sizeof(kPaeDirect));
+  else if (pae_few_columns(ctx)) g3 ? take(kPaeG3Few, sizeof(kPaeG3Few)) : take(kPaeG4Few, sizeof(kPaeG4Few));
+  else if (!g3) take(kPaeG4, sizeof(kPaeG4));
+  else brief ? take(kPaeG3Short, sizeof(kPaeG3Short)) : take(kPaeG3, sizeof(kPaeG3));
   const std::string key = std::string(g3 ? "k_pae_mma(3M)" : "k_pae_mma") + " Nl=" + std::to_string(d.Nl) +
                           " Nf=" + std::to_string(d.Nf) +
                           " NIBZ=" + std::to_string(d.NIBZ) + " NR=" + std::to_string(d.NR) +

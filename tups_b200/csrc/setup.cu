@@ -719,8 +719,10 @@ static int alloc_state(tups_ctx* ctx) {
   size_t cap = ((size_t)4 << 30) / per;
   size_t want = 4 * Nb;
   s.bse_chunk = std::max<size_t>(4, std::min(want, cap)) / 4 * 4;
-  TRY(dalloc(ctx, &s.bse_A, Nz * Nz * s.bse_chunk));
-  TRY(dalloc(ctx, &s.bse_B, Nz * Nz * s.bse_chunk));
+  // one buffer, which the crossing uses as a whole between BSE calls
+  s.bse_half = (Nz * Nz * s.bse_chunk + 15) / 16 * 16;
+  TRY(dalloc(ctx, &s.bse_A, 2 * s.bse_half));
+  s.bse_B = s.bse_A + s.bse_half;
   TRY(dalloc(ctx, &ctx->t.expSqR, (size_t)d.NIBZ * d.NR * NS));
   TRY(dalloc(ctx, &ctx->t.expqSR, (size_t)d.Nc * d.NR * NS));
   TRY(dalloc(ctx, &s.chi_aux_ph, (size_t)d.Nl * d.nbox * Nb));

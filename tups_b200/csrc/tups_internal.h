@@ -57,7 +57,8 @@ struct DeviceState {
   cplx* chi_ph = nullptr;     // (Nl, Nl, Nf, Nb) nu-diagonal blocks of chi_ph_LL
   cplx* chi_pp = nullptr;
   cplx* bse_A = nullptr;      // BSE scratch: Gamma*chi per instance of a chunk; the crossing's gathered operand
-  cplx* bse_B = nullptr;      // chi*Gamma
+  cplx* bse_B = nullptr;      // chi*Gamma, the second half of the same buffer
+  size_t bse_half = 0;        // entries of a half
   size_t bse_chunk = 0;       // instances per chunk
   cplx* PhiR[4] = {};         // (Nz*Nz, Nf/2, NR)
   cplx* M[4] = {};            // (Nl^2 NR, Nl^2, NIBZ): 0 phbar_to_ph 1 pp_to_ph 2 ph_to_pp 3 phbar_to_pp

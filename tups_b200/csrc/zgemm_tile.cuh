@@ -65,9 +65,13 @@ struct ZgemmTile {
   // columns of the left operand, element (m, k) at src.left(kt)[m + ld k],
   // ld = src.ldl(), and as many rows of the right one, element (k, n) at
   // src.right(kt)[src.roff(n) + k].  rows, cols: extent of the matrix from the
-  // tile on.  sm: kSmem bytes, 16-byte aligned.
+  // tile on.  sm: kSmem bytes, 16-byte aligned.  With Src::kGather the source
+  // forms the left operand itself: src.fetch(kt) reads what stage kt needs into
+  // registers and src.put(stage) writes it, entry (m, k) at stage[k LDL + m],
+  // after the products of the step between (only without AHEAD).
   template <class Src>
-  __device__ __forceinline__ void run(const Src& src, cplx* sm, int rows, int cols) {
+  __device__ __forceinline__ void run(Src src, cplx* sm, int rows, int cols) {
+    static_assert(!(Src::kGather && AHEAD), "a gathering source has no read-ahead form");
     cplx* sL = sm;                         // [ST][BK][LDL]
     cplx* sR = sL + (size_t)ST * BK * LDL; // [ST][BN][LDR]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -91,12 +95,14 @@ struct ZgemmTile {
       const cplx *pl = src.left(kt), *pr = src.right(kt);
       cplx* dL = sL + (size_t)st * BK * LDL;
       cplx* dR = sR + (size_t)st * BN * LDR;
+      if constexpr (!Src::kGather) {
 #pragma unroll
-      for (int i = 0; i < (BK * BM + NT - 1) / NT; i++) {
-        const int e = tid + i * NT, m = e % BM, k = e / BM;
-        if (BK * BM % NT == 0 || e < BK * BM) {
-          const bool ok = m < rows && k < kv;
-          zg_cp_async16(dL + k * LDL + m, ok ? pl + m + ld * k : pl, ok);
+        for (int i = 0; i < (BK * BM + NT - 1) / NT; i++) {
+          const int e = tid + i * NT, m = e % BM, k = e / BM;
+          if (BK * BM % NT == 0 || e < BK * BM) {
+            const bool ok = m < rows && k < kv;
+            zg_cp_async16(dL + k * LDL + m, ok ? pl + m + ld * k : pl, ok);
+          }
         }
       }
 #pragma unroll
@@ -124,7 +130,13 @@ struct ZgemmTile {
     };
 #pragma unroll
     for (int s = 0; s < ST - 1; s++) {
-      if (s < ktiles) load(s, s);
+      if (s < ktiles) {
+        load(s, s);
+        if constexpr (Src::kGather) {
+          src.fetch(s);
+          src.put(sL + (size_t)s * BK * LDL);
+        }
+      }
       asm volatile("cp.async.commit_group;\n" ::);
     }
     // this thread's copies of the next stage, and every warp past its reads of
@@ -134,16 +146,30 @@ struct ZgemmTile {
       asm volatile("bar.sync 0;\n" ::: "memory");  // working and idle warps meet here from different loops
     };
     int st = 0, ldst = ST - 1;
+    cplx* filling = nullptr;  // kGather: the stage whose left operand is in registers
     auto refill = [&](int kt) {
-      if (kt + ST - 1 < ktiles) load(ldst, kt + ST - 1);
+      if (kt + ST - 1 < ktiles) {
+        load(ldst, kt + ST - 1);
+        if constexpr (Src::kGather) {
+          src.fetch(kt + ST - 1);
+          filling = sL + (size_t)ldst * BK * LDL;
+        }
+      }
       asm volatile("cp.async.commit_group;\n" ::);
       ldst = ldst + 1 == ST ? 0 : ldst + 1;
+    };
+    auto fill = [&] {
+      if constexpr (Src::kGather) {
+        if (filling) src.put(filling);
+        filling = nullptr;
+      }
     };
     if (AHEAD) land();
     if (wm0 >= rows || wn0 >= cols) {
       for (int kt = 0; kt < ktiles; kt++) {
         if (!AHEAD) land();
         refill(kt);
+        fill();
         if (AHEAD) land();
       }
       return;
@@ -206,6 +232,7 @@ struct ZgemmTile {
           }
         }
       }
+      fill();
     }
   }
 
@@ -258,6 +285,7 @@ struct ZgemmTile {
 // stages of its own.  a, f, b: (Nz, Nz) matrices of one instance
 template <int BK>
 struct BseSource {
+  static constexpr bool kGather = false;
   const cplx *a, *f, *b;
   int Nz, m0, n0;
   __device__ int half() const { return (Nz + BK - 1) / BK; }

@@ -143,3 +143,29 @@ def test_bse_noalloc_multiple_chunks(gpu_lib, shape):
         out = np.transpose(g.cpu().numpy(), (0, 2, 1))
         err = np.abs(out - ref).max() / np.abs(ref).max()
         assert err < TOL, (call, err)
+
+
+@pytest.mark.parametrize("Nf,Nl", [(1, 1), (16, 1), (17, 1), (31, 1), (33, 1), (41, 1), (9, 2), (10, 2), (10, 3), (5, 5),
+                                   (9, 13), (10, 14), (10, 16), (10, 17), (50, 5), (13, 20), (40, 1)])
+def test_bse_noalloc_at_the_edges_of_its_forms(gpu_lib, Nf, Nl):
+    """One form factor, few frequencies, more form factors than a line keeps; sizes around 16 and 32 rows, a last K
+    step of less and of more than half, 250 and 260 rows."""
+    import torch
+
+    Nz, n_inst = Nf * Nl, 3
+    rng = np.random.default_rng(Nz)
+
+    def crandn(*s):
+        return rng.standard_normal(s) + 1j * rng.standard_normal(s)
+
+    gam, fv, chi_cm = crandn(n_inst, Nz, Nz), crandn(n_inst, Nz, Nz), 0.1 * crandn(n_inst, Nl, Nl, Nf)
+    scale, f_damping = 0.37, 0.25
+    ref = _reference_update(np.transpose(gam, (0, 2, 1)), np.transpose(fv, (0, 2, 1)), chi_cm, scale, f_damping)
+    g, f, chi = (torch.from_numpy(np.ascontiguousarray(x)).cuda()
+                 for x in (gam, fv, np.transpose(chi_cm, (0, 3, 2, 1))))
+    rc = gpu_lib.tups_bse_noalloc(n_inst, Nz, Nf, Nl, *(C.c_void_p(x.data_ptr()) for x in (g, f, chi)), scale, f_damping,
+                                  C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    out = np.transpose(g.cpu().numpy(), (0, 2, 1))
+    # sums of 2 Nz products of the prep's sums
+    assert np.abs(out - ref).max() <= max(TOL, 4 * Nz * 2.3e-16) * np.abs(ref).max()

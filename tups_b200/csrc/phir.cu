@@ -235,18 +235,18 @@ __global__ void __launch_bounds__(phir_max_threads(OPT, NR)) k_phir(PhirPtrs P, 
   }
 }
 
-// Crossing tensors per IBZ momentum Q; layout (Nl^4, NIBZ, NR) with l1 fastest.
+// Crossing tensors per IBZ momentum Q, stored as the crossing GEMM's right operand:
+// (l3, l4, R) fastest, then (l1, l2), then Q.  One lattice vector R per grid row,
+// as the symmetries that contribute are R's: with R within a warp, 6 % slower.
 // which: 0 phbar_to_ph, 1 pp_to_ph, 2 ph_to_pp, 3 phbar_to_pp.
 __global__ void k_M(cplx* __restrict__ M, int which, const double* __restrict__ FF, const double* __restrict__ FFinv,
                     const cplx* __restrict__ E, const int* __restrict__ qibz_xy, const int* __restrict__ symlistR,
                     int Nx, int Ny, int Nl, int NIBZ, int NR) {
-  const int nl4 = Nl * Nl * Nl * Nl;
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)nl4 * NIBZ * NR) return;
-  // stored as the crossing GEMM's right operand: (l3, l4, R) fastest, then (l1, l2), then Q
-  const int nl2 = Nl * Nl, K = nl2 * NR, k = (int)(e % K), R = k / nl2;
-  const int l12 = (int)((e / K) % nl2), Q = (int)(e / ((size_t)K * nl2));
-  const int l1 = l12 % Nl, l2 = l12 / Nl, l3 = k % nl2 % Nl, l4 = k % nl2 / Nl;
+  const int nl2 = Nl * Nl, R = blockIdx.y;
+  if (e >= (size_t)nl2 * nl2 * NIBZ) return;
+  const int l34 = (int)(e % nl2), l12 = (int)((e / nl2) % nl2), Q = (int)(e / ((size_t)nl2 * nl2));
+  const int l1 = l12 % Nl, l2 = l12 / Nl, l3 = l34 % Nl, l4 = l34 / Nl;
   const int qx = qibz_xy[2 * Q] - 1, qy = qibz_xy[2 * Q + 1] - 1;  // 0-based
   const int Nc = Nx * Ny;
   auto ff = [&](int kx, int ky, int l) { return FF[kx + Nx * (ky + Ny * l)]; };
@@ -289,7 +289,7 @@ __global__ void k_M(cplx* __restrict__ M, int which, const double* __restrict__ 
       out = cfma(m1, m2, out);
     }
   }
-  M[e] = out;
+  M[(e / nl2 * NR + R) * nl2 + l34] = out;
 }
 
 // k_phir instantiations by outputs per thread (OPT) and NR; every candidate
@@ -402,8 +402,8 @@ int launch_M(tups_ctx* ctx, int which) {
     if (rc) return rc;
     ctx->t.ibz_xy = (int*)p;
   }
-  const size_t n = (size_t)d.Nl * d.Nl * d.Nl * d.Nl * d.NIBZ * d.NR;
-  k_M<<<cdiv(n, 128), 128, 0, ctx->stream>>>(ctx->s.M[which], which, ctx->t.FF, ctx->t.FF_inv, ctx->t.expqSR,
+  const size_t n = (size_t)d.Nl * d.Nl * d.Nl * d.Nl * d.NIBZ;
+  k_M<<<dim3((unsigned)cdiv(n, 128), d.NR), 128, 0, ctx->stream>>>(ctx->s.M[which], which, ctx->t.FF, ctx->t.FF_inv, ctx->t.expqSR,
                                              ctx->t.ibz_xy, ctx->t.ibz_xy + 2 * (size_t)d.NIBZ, d.Nx, d.Ny, d.Nl,
                                              d.NIBZ, d.NR);
   return after_launch(ctx, "k_M");

@@ -13,9 +13,9 @@ further iterations launched kernel by kernel with phase events.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl {tups,reference}]
 
-Prints one JSON line (rank 0).  ``--impl reference`` times the CPU
-restatement of the reference (the reference's Fortran cannot be built in
-this image) on the host cores.
+Prints one JSON line (rank 0).  ``--impl reference`` says that the reference
+is unavailable: its Fortran cannot be built in this image.  The CPU
+restatement of it is timed on the host cores as ``cpu_baseline``.
 """
 from __future__ import annotations
 
@@ -235,28 +235,14 @@ def fortran_toolchain() -> dict:
     return {t: shutil.which(t) for t in ("gfortran", "mpif90", "mpifort", "ifort", "ifx", "h5fc")}
 
 
-def run_reference(args, wl_name: str, wl: dict):
-    ws, rank, _ = dist_env()
-    if rank != 0:
+def run_reference():
+    """The reference arm: the unmodified reference or nothing.  Its own CPU restatement is timed beside this
+    framework's arm (``cpu_baseline``)."""
+    if dist_env()[1] != 0:
         return
-    steps, warm = args.steps, args.warmup
-    spi = cpu_oracle_seconds_per_iteration(wl, timed_iterations=steps, warm_iterations=warm)
-    cores = max(blas_threads(), os.cpu_count() or 1)
-    tools = fortran_toolchain()
-    line = {
-        "impl": "reference", "metric": METRIC, "metric_full": METRIC_FULL, "value": spi, "unit": "s/iter",
-        "n_gpus": ws, "steps": steps, "warmup": warm, "ms_per_step": spi * 1e3, "higher_is_better": False,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-        "config": workload_config(wl_name, wl, ws),
-        "cpu_baseline": {"value": spi, "unit": "s/iter", "cores": cores, "kind": "port",
-                         "sample": f"{steps} iteration(s) after {warm} untimed; " + CPU_PORT_SAMPLE},
-        "reference_toolchain": tools,
-        "reference_note": ("the Fortran reference needs mpif90 + MKL + HDF5-Fortran; none of the compilers "
-                           "probed here is present" if not any(tools.values()) else
-                           "a Fortran compiler is present; the port is still the timed arm"),
-        "e2e": {"value": spi, "unit": "s/iter", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-    }
-    print(json.dumps(line), flush=True)
+    found = [t for t, path in fortran_toolchain().items() if path]
+    why = "the reference is Fortran and needs mpif90, MKL and HDF5-Fortran; compilers found here: "
+    print(json.dumps({"impl": "reference", "unavailable": why + (", ".join(found) or "none")}), flush=True)
 
 
 def run_tups(args, wl_name: str, wl: dict):
@@ -612,8 +598,6 @@ def run_bse_batched(args):
     Hermitian Gaussian Gamma scaled to rho(Gamma chi) = 0.9, chi the beta = 10
     bare bubble.  One step = the whole batch, F = (1 - Gamma chi)^{-1} Gamma."""
     ws, rank, local = dist_env()
-    if args.impl == "reference" and rank != 0:
-        return
     from tups_b200.bse_batched import algorithmic_flops, make_instances
     from oracle import lu as LU
     workers = min(16, os.cpu_count() or 1)
@@ -632,13 +616,6 @@ def run_bse_batched(args):
                      "zgetrf+zgetrs, FP64"}
     cfg = {"workload": LU_WORKLOAD, "instances": int(len(inst.n)), "n_sizes": sorted(set(inst.n.tolist())),
            "Nnu": 64, "lattice": "8x8", "beta": 10.0, "rho": 0.9, "l2": "inputs 4.7 GB > L2; no flush"}
-    if args.impl == "reference":
-        line = {"impl": "reference", "metric": "BSE TFLOP/s", "value": cpu_tf, "unit": "TFLOP/s", "n_gpus": ws,
-                "steps": 1, "warmup": 0, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": "f64", "data": "synthetic", "config": cfg, "cpu_baseline": cpu,
-                "e2e": {"value": cpu_tf, "unit": "TFLOP/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-        print(json.dumps(line), flush=True)
-        return
     import torch
     from tups_b200.bse_batched import LuBatch
     device = local
@@ -829,22 +806,17 @@ def main():
     ap.add_argument("--no-target", action="store_true",
                     help="skip the 16x16 / 9 form factor FP64-vs-ladder record (about 6 minutes)")
     args = ap.parse_args()
-    if args.warmup < 3 and args.impl == "tups":
-        args.warmup = 3
+    if args.impl == "reference":
+        run_reference()
+        return
+    args.warmup = max(args.warmup, 3)
     if args.workload == LU_WORKLOAD:
         run_bse_batched(args)
         return
     if args.workload == ZGEMM_WORKLOAD:
-        if args.impl == "reference":
-            print(json.dumps({"impl": "reference", "unavailable": "the split ZGEMM has no CPU counterpart"}))
-            return
         run_zgemm_split(args)
         return
-    wl = WORKLOADS[args.workload]
-    if args.impl == "reference":
-        run_reference(args, args.workload, wl)
-    else:
-        run_tups(args, args.workload, wl)
+    run_tups(args, args.workload, WORKLOADS[args.workload])
 
 
 if __name__ == "__main__":

@@ -383,13 +383,14 @@ long long tups_kernel_launches(const tups_ctx* ctx);
  *   F_i = (1 - scale_i Gamma_i chi_i)^{-1} Gamma_i   (want_phi: F_i - Gamma_i)
  * for n_inst instances of size n[i] = nl[i] * Nnu_i, block by block
  * (partial-pivoting LU, blocks of 64 columns, every launch over the instances
- * that still have a block, FP64 tensor-core updates; n[i] right-hand sides).
- * n, nl, scale: host arrays.  gamma, out, work: device, instances packed consecutively as
- * (n, n) column-major complex128; chi: device, packed (nl, nl, Nnu) blocks;
- * ipiv: device int, packed n[i].  work: scratch of n[i]^2, its content on
- * return is not the LU factors.  status (host, optional): per instance 0, or
- * k+1 when column k had a zero pivot; when given, the call synchronises.
- * Allocates nothing; limit n_inst <= 16384. */
+ * that still have a block, FP64 tensor-core updates; instances of up to 32 rows
+ * whole; n[i] right-hand sides).  n, nl, scale: host arrays.  gamma, out, work:
+ * device, instances packed consecutively as (n, n) column-major complex128;
+ * chi: device, packed (nl, nl, Nnu) blocks; ipiv: device int, packed n[i].
+ * work: scratch of n[i]^2.  status (host, optional): per instance 0, or k+1 when
+ * column k had a zero pivot; when given, the call synchronises.  Allocates
+ * nothing; limit n_inst <= 16384.  The instance and interchange tables are
+ * static device arrays (9 MB): calls that overlap on the GPU race on them. */
 int tups_bse_lu_batched(int n_inst, const int* n, const int* nl, const double* scale, const double* gamma,
                         const double* chi, double* out, double* work, int* ipiv, int want_phi, int* status,
                         void* stream);

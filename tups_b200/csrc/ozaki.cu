@@ -16,10 +16,10 @@
 // Layout: slices of A' as rows of Kpad bytes (K-major), slices of B' as rows
 // of Kpad bytes (one row per column of B'); Kpad = 2K rounded up to 128.
 // The GEMM kernel reads 128-byte K chunks of both with TMA (128-byte
-// swizzle), accumulates one diagonal d at a time in TMEM (two buffers, so
-// the FP64 drain of diagonal d overlaps the MMAs of diagonal d+1), and
-// folds each diagonal into an FP64 partial sum in global memory; the last
-// diagonal applies the scales and the caller's epilogue.
+// swizzle), accumulates two diagonals at a time in TMEM (four buffers, so the
+// FP64 drain of two diagonals overlaps the MMAs of the next two), and folds
+// each diagonal into FP64 sums in registers; after the last one the scales and
+// the caller's epilogue are applied.
 #include <cuda.h>
 
 #include <algorithm>
@@ -549,9 +549,12 @@ __device__ __forceinline__ uint32_t oz_uniform(uint32_t v) { return __shfl_sync(
 // diagonals per stage; 490 with one wait and one commit per two products; 430
 // with a warp-uniform schedule and one elected lane; 397 with the drain in loads of
 // 16 columns, FP64 conversions by addition and four columns' reads ahead (2.6
-// POPS).  Then it is near what shared memory gives: 16 KB of copies and 32 KB
-// of operand reads per product, 384 cycles at 128 bytes per cycle, 367 measured;
-// the drain runs four times slower under the MMAs than alone for the same reason.
+// POPS).  The tensor pipe is 75 % busy then, and the clock falls to 1.64 GHz under
+// the power limit: 367 cycles per product (cycles elapsed, mean over the SMs, over
+// the mean number of products of an SM).  The rest is the drain, four times slower
+// under the MMAs than alone, and shared memory: 16 KB of copies per product beside
+// operand reads of up to 32 KB, which at 128 bytes per cycle would be 384 cycles
+// if each MMA fetched both of its operands anew.
 enum { OZ_EPI_ZGEMM = 0, OZ_EPI_BSE = 1, OZ_EPI_SUB = 2 };
 
 constexpr int OZ_NBUF = 4;            // TMEM accumulator buffers
@@ -1243,9 +1246,8 @@ OzWork oz_work_layout(int batch, int M, int N, int K, int s) {
   w.b_bytes = (size_t)batch * s * 2 * N * w.Kpad;
   w.rs_bytes = (size_t)batch * M * sizeof(double);
   w.cs_bytes = (size_t)batch * N * sizeof(double);
-  w.acc_bytes = 0;  // the FP64 sums live in registers
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-  w.total = up(w.a_bytes) + up(w.b_bytes) + up(w.rs_bytes) + up(w.cs_bytes) + up(w.acc_bytes) + 256;
+  w.total = up(w.a_bytes) + up(w.b_bytes) + up(w.rs_bytes) + up(w.cs_bytes) + 256;
   return w;
 }
 
@@ -1259,7 +1261,6 @@ void oz_bind_work(OzRun& R, const OzWork& w, void* base) {
   R.rscale = (double*)p;
   p += up(w.rs_bytes);
   R.cscale = (double*)p;
-  R.acc = nullptr;
 }
 
 // a failed CUDA step of oz_run on stderr (the batched ZGEMM entry point has no

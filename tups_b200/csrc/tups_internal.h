@@ -206,7 +206,7 @@ struct OzOperand {
 
 struct OzWork {
   int Kpad = 0;
-  size_t a_bytes = 0, b_bytes = 0, rs_bytes = 0, cs_bytes = 0, acc_bytes = 0, total = 0;
+  size_t a_bytes = 0, b_bytes = 0, rs_bytes = 0, cs_bytes = 0, total = 0;
 };
 
 struct OzRun {
@@ -216,7 +216,6 @@ struct OzRun {
   int8_t* b_slices = nullptr;
   double* rscale = nullptr;
   double* cscale = nullptr;
-  double* acc = nullptr;
   double* status = nullptr;   // receives status_code when a wait times out
   double status_code = 0.0;
   int epi = 0;         // 0: C = A B; 1: BSE update written over G; 2: C -= A B

@@ -1,6 +1,6 @@
 // One CTA tile of a complex GEMM on the FP64 tensor cores (mma.sync m16n8k8
-// f64), shared by the BSE GEMM, its no-allocation form, the LU updates and
-// the split LU's residual.
+// f64), shared by the BSE GEMM, its no-allocation form, the crossing and, in the
+// split LU, the second panel's update and the residual.
 //
 // Operands arrive by cp.async into ST shared-memory stages of BK columns; the
 // fragments of the next k8 step are read into a second register set before the
@@ -41,15 +41,15 @@ __device__ __forceinline__ void zg_dmma(double* c, const double* a, const double
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// Without AHEAD the fragments of a step are read when it starts: fewer
-// registers, so more CTAs per SM, which is the better side for short sums (a
-// 64-column LU update: 5 CTAs per SM 6.4 ms, 3 with AHEAD 9.6).
-//
-// WM x WN warps of 16 TM x 8 TN
+// what an epilogue reads per entry: two matrices
 struct ZgPair {
   cplx a, b;
 };
 
+// WM x WN warps of 16 TM x 8 TN.  Without AHEAD the fragments of a step are read
+// when it starts: fewer registers, so more CTAs per SM, and the padding of a last
+// stage is skipped, which is the better side for short sums (the crossing at K =
+// 100: 5 CTAs per SM 1.03 ms, 3 with AHEAD 1.30).
 template <int TM, int TN, int WM, int WN, int BK, int ST, bool M3, bool AHEAD = true>
 struct ZgemmTile {
   static constexpr int BM = 16 * TM * WM, BN = 8 * TN * WN, NW = WM * WN, NT = 32 * NW;
